@@ -237,7 +237,11 @@ int derivatives(gsph_ctx* c, cudaStream_t s) {
     cudaError_t e;
     if (c->fp64) {
         int launches = 0;
-        e = launch64_derivatives(c->a64, c->dp64, s, launches);
+        Fork64 f;
+        f.side = c->side;
+        f.fork = c->ev_fork;
+        f.join = c->ev_join;
+        e = launch64_derivatives(c->a64, c->dp64, s, launches, f);
         c->launches += launches;
         if (e != cudaSuccess) return cuda_fail(c, e, "FP64 derivatives");
         return GSPH_OK;
@@ -296,9 +300,16 @@ int derivatives(gsph_ctx* c, cudaStream_t s) {
 }
 
 int reorder(gsph_ctx* c, cudaStream_t s) {
-    if (!c->L.cull) return GSPH_OK;
+    if (!c->L.cull && !c->a64.order) return GSPH_OK;
     int launches = 0;
-    const cudaError_t e = reorder_particles(c->a, c->sp, s, launches);
+    cudaError_t e;
+    if (c->fp64) {  // the particles stay in place; the culled passes go through the order
+        e = launch64_to32(c->a64, c->a.posm, s);
+        if (e == cudaSuccess) e = curve_order(c->a, c->sp, s, launches);
+        launches += 1;
+    } else {
+        e = reorder_particles(c->a, c->sp, s, launches);
+    }
     c->launches += launches;
     c->steps_since_sort = 0;
     if (e != cudaSuccess) return cuda_fail(c, e, "particle reorder");
@@ -555,6 +566,33 @@ int gsph_create(const gsph_params* p, const gsph_options* opt, int64_t n, gsph_c
         b.balsara = static_cast<double*>(dalloc(c, n_pad * sizeof(double), ae));
         b.dt_state = static_cast<double*>(dalloc(c, 4 * sizeof(double), ae));
         c->diag64 = static_cast<double*>(dalloc(c, diag64_scratch_doubles(n_pad) * sizeof(double), ae));
+        const bool slots = n_pad <= kMaxSlots64;
+        if (slots && (p->flags & GSPH_SELF_GRAVITY) && o.gravity_form != GSPH_GRAVITY_ONE_SIDED &&
+            !((p->flags & GSPH_SPH) && o.no_cull)) {
+            gravity64_shape(b);
+            b.gpart = static_cast<double*>(dalloc(c, gravity64_doubles(b) * sizeof(double), ae));
+            b.gfold = static_cast<double*>(dalloc(c, 3 * n_pad * sizeof(double), ae));
+        }
+        // the culled passes take their gravity from the slots, so a context that asks for the one-sided sum
+        // keeps the sweep over all pairs
+        if (slots && (p->flags & GSPH_SPH) && !o.no_cull && (b.gpart || !(p->flags & GSPH_SELF_GRAVITY))) {
+            SpatialArrays& sp = c->sp;
+            b.order = static_cast<int*>(dalloc(c, n_pad * sizeof(int), ae));
+            b.P = D4();
+            b.J = static_cast<double4*>(dalloc(c, 4 * n_pad * sizeof(double4), ae));
+            b.box_lo = static_cast<float4*>(dalloc(c, boxes64(n_pad) * sizeof(float4), ae));
+            b.box_hi = static_cast<float4*>(dalloc(c, boxes64(n_pad) * sizeof(float4), ae));
+            b.nb = static_cast<int*>(dalloc(c, lists64_ints(n_pad) * sizeof(int), ae));
+            b.nbcnt = static_cast<int*>(dalloc(c, counts64_ints(n_pad) * sizeof(int), ae));
+            sp.order = static_cast<int*>(dalloc(c, n_pad * sizeof(int), ae));
+            sp.order_out = b.order;
+            sp.keys = static_cast<unsigned*>(dalloc(c, 2 * n_pad * sizeof(unsigned), ae));
+            sp.sort_tmp_bytes = spatial_sort_tmp_bytes(n_pad);
+            sp.sort_tmp = dalloc(c, sp.sort_tmp_bytes, ae);
+            sp.bbox = static_cast<int*>(dalloc(c, 8 * sizeof(int), ae));
+            sp.ext_of_int = b.order;  // identity until positions are uploaded
+            if (ae == cudaSuccess) ae = cudaMemset(b.J, 0, 4 * n_pad * sizeof(double4));
+        }
         const double q = p->normalsep / p->H;
         double wn = 0.0;
         if (q <= 1.0) wn = (q < 0.5) ? (6 * q * q * q - 6 * q * q + 1) : 2 * (1 - q) * (1 - q) * (1 - q);
@@ -573,12 +611,12 @@ int gsph_create(const gsph_params* p, const gsph_options* opt, int64_t n, gsph_c
     e = cudaMemset(a.dt_state, 0, 4 * sizeof(float));
     if (e == cudaSuccess) e = cudaMemset(a.status, 0, 4 * sizeof(int));
     if (e == cudaSuccess) e = launch_init_padding(a, 0);
-    if (e == cudaSuccess && L.cull) e = launch_identity_order(c->sp, n_pad, 0);
+    if (e == cudaSuccess && (L.cull || c->a64.order)) e = launch_identity_order(c->sp, n_pad, 0);
     if (e == cudaSuccess && c->fp64) {
         e = launch64_init(c->a64, 0);
         if (e == cudaSuccess) e = cudaMemset(c->a64.dt_state, 0, 4 * sizeof(double));
     }
-    if (e == cudaSuccess && L.cull) {
+    if (e == cudaSuccess && (L.cull || c->a64.order)) {
         e = cudaStreamCreateWithFlags(&c->side, cudaStreamNonBlocking);
         if (e == cudaSuccess) e = cudaEventCreateWithFlags(&c->ev_fork, cudaEventDisableTiming);
         if (e == cudaSuccess) e = cudaEventCreateWithFlags(&c->ev_join, cudaEventDisableTiming);
@@ -837,7 +875,7 @@ int gsph_step(gsph_ctx* c, int32_t nsteps, void* stream) {
         c->graph_slots = slots;
     }
     for (int32_t k = 0; k < nsteps; ++k) {
-        if (c->L.cull && c->opt.resort_interval > 0 && c->steps_since_sort >= c->opt.resort_interval) {
+        if ((c->L.cull || c->a64.order) && c->opt.resort_interval > 0 && c->steps_since_sort >= c->opt.resort_interval) {
             const int rc = reorder(c, s);  // permutes in place: the graph's pointers stay valid
             if (rc != GSPH_OK) return rc;
         }

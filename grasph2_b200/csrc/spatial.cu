@@ -200,7 +200,7 @@ cudaError_t launch_identity_order(const SpatialArrays& s, int64_t n_pad, cudaStr
     return cudaGetLastError();
 }
 
-cudaError_t reorder_particles(const DevArrays& a, const SpatialArrays& s, cudaStream_t st, int& launches) {
+cudaError_t curve_order(const DevArrays& a, const SpatialArrays& s, cudaStream_t st, int& launches) {
     const int64_t np = a.n_pad;
     k_bbox_init<<<1, 32, 0, st>>>(s.bbox);
     k_bbox<<<256, 256, 0, st>>>(a, s.bbox);
@@ -213,6 +213,12 @@ cudaError_t reorder_particles(const DevArrays& a, const SpatialArrays& s, cudaSt
                                         static_cast<int>(np), 0, 32, st);
     if (e != cudaSuccess) return e;
     launches += 4;  // onesweep radix sort passes (approximate count for the launch counter)
+    return e;
+}
+
+cudaError_t reorder_particles(const DevArrays& a, const SpatialArrays& s, cudaStream_t st, int& launches) {
+    const cudaError_t e = curve_order(a, s, st, launches);
+    if (e != cudaSuccess) return e;
     return permute_particles(a, s.order_out, s.tmp4, s.tmp8, s.ext_of_int, st, launches);
 }
 

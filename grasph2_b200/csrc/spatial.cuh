@@ -82,6 +82,8 @@ cudaError_t launch_chunk_bounds(const DevArrays& a, const SpatialArrays& s, cuda
 cudaError_t launch_chunk_lists(const DevArrays& a, const SpatialArrays& s, float h, cudaStream_t st);
 // Sort the n real particles of `a` along the Hilbert curve and permute every per-particle array in place.
 cudaError_t reorder_particles(const DevArrays& a, const SpatialArrays& s, cudaStream_t st, int& launches);
+// The first half of it: order_out[k] = slot of the k-th particle along the curve (padding last, in place).
+cudaError_t curve_order(const DevArrays& a, const SpatialArrays& s, cudaStream_t st, int& launches);
 cudaError_t launch_identity_order(const SpatialArrays& s, int64_t n_pad, cudaStream_t st);
 // Gather every per-particle array of `a` (all n_pad slots) and `ext_of_int` by `order` (new slot i takes
 // old slot order[i]); t4 / t8 are n_pad-element scratch.
