@@ -8,6 +8,7 @@
 // the FP32 rate, so this mode is the accuracy reference for trajectories the FP32 forms are measured
 // against (energy drift), and the drop-in for callers of the reference's FP64 build.
 #include "fp64.cuh"
+#include "potential.cuh"
 #include "rsqrt64.cuh"
 
 namespace gsph {
@@ -895,7 +896,6 @@ __global__ void k64_init(DevArrays64 a) {
 // ---- FP64 diagnostics (same quantities as the FP32 path) ---------------------------------------------
 constexpr int kDiag64 = 12;
 __global__ void __launch_bounds__(kT64) k64_diag(DevArrays64 a, DevParams64 p, double half_kick, double* blocks) {
-    __shared__ double4 tile[kT64];
     __shared__ double red[kT64 / 32][kDiag64];
     const int64_t i = static_cast<int64_t>(blockIdx.x) * kT64 + threadIdx.x;
     double f[kDiag64] = {};
@@ -924,21 +924,6 @@ __global__ void __launch_bounds__(kT64) k64_diag(DevArrays64 a, DevParams64 p, d
             }
         }
     }
-    if (has64(p, GSPH_SELF_GRAVITY)) {  // -G m_i sum_{j > i} m_j / sqrt(r^2 + eps^2)
-        double phi = 0.0;
-        for (int64_t t0 = static_cast<int64_t>(blockIdx.x) * kT64; t0 < a.n_pad; t0 += kT64) {
-            __syncthreads();
-            tile[threadIdx.x] = a.posm[t0 + threadIdx.x];
-            __syncthreads();
-            for (int jj = 0; jj < kT64; ++jj) {
-                if (t0 + jj <= i) continue;
-                const double4 q = tile[jj];
-                const double dx = q.x - x.x, dy = q.y - x.y, dz = q.z - x.z;
-                phi += q.w / sqrt(dx * dx + dy * dy + dz * dz + p.eps2);
-            }
-        }
-        if (i < a.n) f[1] = -p.G * x.w * phi;
-    }
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     for (int k = 0; k < kDiag64; ++k) {
         double v = f[k];
@@ -952,14 +937,6 @@ __global__ void __launch_bounds__(kT64) k64_diag(DevArrays64 a, DevParams64 p, d
         blocks[static_cast<int64_t>(blockIdx.x) * kDiag64 + threadIdx.x] = s;
     }
 }
-__global__ void k64_diag_reduce(const double* blocks, int nblocks, double* out) {
-    const int k = threadIdx.x;
-    if (k >= kDiag64) return;
-    double s = 0.0;
-    for (int b = 0; b < nblocks; ++b) s += blocks[static_cast<int64_t>(b) * kDiag64 + k];
-    out[k] = s;
-}
-
 }  // namespace
 
 DevParams64 make_dev_params64(const gsph_params& p, double w_pref, double dw_pref, double inv_w_normalsep) {
@@ -1165,14 +1142,22 @@ cudaError_t launch64_pack_pos(const DevArrays64& a, const double* src, cudaStrea
     k64_pack_pos<<<blocks_for(a.n, 256), 256, 0, s>>>(a, src);
     return cudaGetLastError();
 }
-size_t diag64_scratch_doubles(int64_t n_pad) { return static_cast<size_t>(n_pad / kT64) * kDiag64 + kDiag64; }
+size_t diag64_scratch_doubles(int64_t n_pad) {
+    return static_cast<size_t>(n_pad / kT64) * kDiag64 + kDiag64 + potential_partials();
+}
 cudaError_t launch64_diagnostics(const DevArrays64& a, const DevParams64& p, double half_kick, double* scratch,
                                  double* out, cudaStream_t s) {
     const int nb = static_cast<int>(a.n_pad / kT64);
     k64_diag<<<nb, kT64, 0, s>>>(a, p, half_kick, scratch);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    k64_diag_reduce<<<1, 32, 0, s>>>(scratch, nb, out);
+    double* pot = scratch + static_cast<int64_t>(nb) * kDiag64;
+    int npot = 0;
+    if (has64(p, GSPH_SELF_GRAVITY)) {
+        e = launch_pair_potential(PotSource64{a.posm}, a.n, p.eps2, pot, npot, s);
+        if (e != cudaSuccess) return e;
+    }
+    k_sum_partials<kDiag64><<<1, 32 * kDiag64, 0, s>>>(scratch, nb, pot, npot, -p.G, out);
     return cudaGetLastError();
 }
 

@@ -3,6 +3,7 @@
 //
 // HBM-bound: each kernel touches each particle once with coalesced float4 / double streams.
 #include "integrate.cuh"
+#include "potential.cuh"
 #include "sph.cuh"
 
 namespace gsph {
@@ -87,52 +88,15 @@ __device__ __forceinline__ double block_sum(double v, double* sh) {
     return r;
 }
 
-// per-particle terms and, per i, its share of the pair potential against j > i; one row of
-// kDiagFields block partials per CTA (deterministic second stage)
+// per-particle terms, one row of kDiagFields block partials per CTA (the pair potential, field 1, has a kernel of
+// its own: potential.cuh)
 __global__ void __launch_bounds__(kDiagThreads) k_diag(DevArrays a, DevParams p, double half_kick) {
-    __shared__ double tile[4][kDiagThreads];
     __shared__ double red[32];
     const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    const int64_t np = a.n_pad;
     double f[kDiagFields];
 #pragma unroll
     for (int k = 0; k < kDiagFields; ++k) f[k] = 0.0;
-    double xi = 0, yi = 0, zi = 0, mi = 0;
-    if (i < a.n) {
-        diag_terms(a, p, i, half_kick, f);
-        mi = a.posm[i].w;
-        xi = a.pos64[i]; yi = a.pos64[np + i]; zi = a.pos64[2 * np + i];
-    }
-    // pair potential: -G m_i sum_{j>i} m_j / sqrt(r^2 + eps^2), j-tiles of blockDim through shared memory
-    if (has(p, GSPH_SELF_GRAVITY)) {
-        const double eps2 = p.eps2_d;
-        double phi = 0.0;
-        const int64_t j_first = static_cast<int64_t>(blockIdx.x) * blockDim.x;  // j > i needs j >= block start
-        for (int64_t t0 = j_first; t0 < a.n; t0 += blockDim.x) {
-            const int64_t j = t0 + threadIdx.x;
-            __syncthreads();
-            if (j < a.n) {
-                tile[0][threadIdx.x] = a.pos64[j];
-                tile[1][threadIdx.x] = a.pos64[np + j];
-                tile[2][threadIdx.x] = a.pos64[2 * np + j];
-                tile[3][threadIdx.x] = a.posm[j].w;
-            } else {
-                tile[3][threadIdx.x] = 0.0;
-                tile[0][threadIdx.x] = tile[1][threadIdx.x] = tile[2][threadIdx.x] = 0.0;
-            }
-            __syncthreads();
-            if (i < a.n) {
-                const int64_t rem = a.n - t0;
-                const int cnt = rem < static_cast<int64_t>(blockDim.x) ? static_cast<int>(rem) : static_cast<int>(blockDim.x);
-                for (int jj = 0; jj < cnt; ++jj) {
-                    if (t0 + jj <= i) continue;
-                    const double dx = tile[0][jj] - xi, dy = tile[1][jj] - yi, dz = tile[2][jj] - zi;
-                    phi += tile[3][jj] / sqrt(dx * dx + dy * dy + dz * dz + eps2);
-                }
-            }
-        }
-        f[1] = -p.G_d * mi * phi;
-    }
+    if (i < a.n) diag_terms(a, p, i, half_kick, f);
     for (int k = 0; k < kDiagFields; ++k) {
         const double s = block_sum(f[k], red);
         if (threadIdx.x == 0) a.diag[static_cast<int64_t>(blockIdx.x) * kDiagFields + k] = s;
@@ -275,14 +239,6 @@ __global__ void k_energy_adjust(DevArrays a, DevParams p, const double* __restri
     }
 }
 
-__global__ void k_diag_reduce(DevArrays a, int nblocks, double* out) {
-    const int k = threadIdx.x;
-    if (k >= kDiagFields) return;
-    double s = 0.0;
-    for (int b = 0; b < nblocks; ++b) s += a.diag[static_cast<int64_t>(b) * kDiagFields + k];
-    out[k] = s;
-}
-
 // ---- host layout <-> device layout ------------------------------------------------------------
 // attribute ids follow the bit order of GSPH_POS ... GSPH_MAXVSIG
 // `ext` maps the device slot i to the caller's particle index e (identity when null); the staging
@@ -421,14 +377,30 @@ cudaError_t launch_leapfrog(const DevArrays& a, const DevParams& p, int not_firs
 
 int leapfrog_kernel_count(const DevParams& p) { return has(p, GSPH_VARIABLE_TIMESTEP) ? 3 : 1; }
 
-size_t diag_scratch_doubles(int64_t n) { return static_cast<size_t>(blocks_for(n, kDiagThreads)) * kDiagFields + kDiagFields; }
+size_t diag_scratch_doubles(int64_t n) {
+    return static_cast<size_t>(blocks_for(n, kDiagThreads)) * kDiagFields + kDiagFields + potential_partials();
+}
+
+namespace {
+// the sums of `rows` rows of block partials
+cudaError_t reduce_diag(const double* part, unsigned rows, double* out, cudaStream_t s) {
+    k_sum_partials<kDiagFields><<<1, 32 * kDiagFields, 0, s>>>(part, static_cast<int>(rows), nullptr, 0, 0.0, out);
+    return cudaGetLastError();
+}
+}  // namespace
 
 cudaError_t launch_diagnostics(const DevArrays& a, const DevParams& p, double half_kick, double* out_dev, cudaStream_t s) {
     const unsigned nb = blocks_for(a.n, kDiagThreads);
     k_diag<<<nb, kDiagThreads, 0, s>>>(a, p, half_kick);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    k_diag_reduce<<<1, 32, 0, s>>>(a, static_cast<int>(nb), out_dev);
+    double* pot = a.diag + static_cast<int64_t>(nb) * kDiagFields;
+    int npot = 0;
+    if (has(p, GSPH_SELF_GRAVITY)) {
+        e = launch_pair_potential(PotSource32{a.pos64, a.posm, a.n_pad}, a.n, p.eps2_d, pot, npot, s);
+        if (e != cudaSuccess) return e;
+    }
+    k_sum_partials<kDiagFields><<<1, 32 * kDiagFields, 0, s>>>(a.diag, static_cast<int>(nb), pot, npot, -p.G_d, out_dev);
     return cudaGetLastError();
 }
 
@@ -438,8 +410,7 @@ cudaError_t launch_diagnostics_fast(const DevArrays& a, const DevParams& p, doub
     k_diag_fast<<<nb, kDiagThreads, 0, s>>>(a, p, half_kick);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    k_diag_reduce<<<1, 32, 0, s>>>(a, static_cast<int>(nb), out_dev);
-    return cudaGetLastError();
+    return reduce_diag(a.diag, nb, out_dev, s);
 }
 
 cudaError_t launch_state_compare(const DevArrays& q, const DevArrays& p_state, const DevArrays& x0, const DevParams& p,
@@ -450,8 +421,7 @@ cudaError_t launch_state_compare(const DevArrays& q, const DevArrays& p_state, c
     k_state_compare<<<nb, kDiagThreads, 0, s>>>(qq, p_state, x0, p);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    k_diag_reduce<<<1, 32, 0, s>>>(qq, static_cast<int>(nb), out_dev);
-    return cudaGetLastError();
+    return reduce_diag(qq.diag, nb, out_dev, s);
 }
 
 cudaError_t launch_energy_adjust(const DevArrays& a, const DevParams& p, double d_kin, double d_shear, double* tot_dev,
@@ -460,8 +430,7 @@ cudaError_t launch_energy_adjust(const DevArrays& a, const DevParams& p, double 
     k_energy_parts<<<nb, kDiagThreads, 0, s>>>(a, p);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    k_diag_reduce<<<1, 32, 0, s>>>(a, static_cast<int>(nb), tot_dev);
-    e = cudaGetLastError();
+    e = reduce_diag(a.diag, nb, tot_dev, s);
     if (e != cudaSuccess) return e;
     k_energy_adjust<<<nb, kDiagThreads, 0, s>>>(a, p, tot_dev, d_kin, d_shear);
     return cudaGetLastError();
