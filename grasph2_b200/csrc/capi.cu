@@ -42,8 +42,10 @@ struct gsph_ctx {
     float* staging = nullptr;     // kStagingFloats * n floats: every attribute its own region
     double* staging64 = nullptr;  // 9 * n doubles
     double* diag_out = nullptr;   // device, 12 doubles
-    size_t part_cap = 0, gpart_cap = 0, item_cap = 0;  // floats allocated for a.part, a.gpart, sp.item_part
-    size_t item_nb_items = 0;                          // work items the neighbour-list buffers hold
+    size_t part_cap = 0, gpart_cap = 0;  // floats allocated for a.part, a.gpart
+    // derivatives of network proposals (pairs_fixed.cu): launch shapes as created, buffers of the first proposal
+    Launch fixed_L;
+    FixedArrays fixed;
     std::vector<void*> snap[4];    // gsph_snapshot slots: saved copies of the state arrays (allocated on first save)
     cudaStream_t capture_stream = nullptr;
     cudaGraph_t graph = nullptr;
@@ -259,10 +261,10 @@ int derivatives(gsph_ctx* c, cudaStream_t s) {
             join = c->ev_join;
             c->launches += 1;
         }
-        if (sp) {  // bounds of every chunk at the current positions, each group's near chunks, work items
+        if (sp) {  // bounds of every chunk at the current positions, each group's near chunks, the groups' order
             e = launch_chunk_bounds(c->a, c->sp, s);
             if (e == cudaSuccess) e = launch_chunk_lists(c->a, c->sp, p.H, s);
-            if (e == cudaSuccess) e = launch_work_items(c->a, c->sp, c->sp.item_target, s);
+            if (e == cudaSuccess) e = launch_group_order(c->a, c->sp, s);
             if (e != cudaSuccess) return cuda_fail(c, e, "chunk lists");
             c->launches += 3;
         }
@@ -296,6 +298,64 @@ int derivatives(gsph_ctx* c, cudaStream_t s) {
         if (e != cudaSuccess) return cuda_fail(c, e, "gravity pass");
         c->launches += has(p, GSPH_SELF_GRAVITY) ? 2 : 1;
     }
+    return GSPH_OK;
+}
+
+// replace the tracked allocation *p by one of `floats` floats when it holds fewer (contents are scratch)
+int grow(gsph_ctx* c, float** p, size_t& cap, size_t floats) {
+    if (floats <= cap) return GSPH_OK;
+    float* q = nullptr;
+    GSPH_CK(c, cudaMalloc(&q, floats * sizeof(float)), "autotune allocation");
+    for (auto& a : c->allocations)
+        if (a == *p) a = q;
+    cudaFree(*p);
+    *p = q;
+    cap = floats;
+    return GSPH_OK;
+}
+
+// derivatives in the fixed order of summation (a culled context in single precision)
+int fixed_derivatives(gsph_ctx* c, cudaStream_t s) {
+    const DevParams& p = c->dp;
+    const int64_t np = c->a.n_pad;
+    cudaError_t e = cudaSuccess;
+    FixedArrays& fx = c->fixed;
+    if (!fx.item_start) {
+        // one allocation, the largest alignment first
+        const size_t items = fixed_items(np, c->sm_count);
+        const size_t parts = items * fixed_part_floats(), lists = items * fixed_list_ints();
+        int* base = static_cast<int*>(dalloc(c, (parts + lists + items * (kGroup + 1) + np / kGroup + 2) * sizeof(int), e));
+        if (e != cudaSuccess) return fail(c, GSPH_E_NOMEM, std::string("proposal buffers: ") + cudaGetErrorString(e));
+        fx.part = reinterpret_cast<float*>(base);
+        fx.nb = base + parts;
+        fx.nbcnt = fx.nb + lists;
+        fx.nbover = fx.nbcnt + items * kGroup;
+        fx.item_start = fx.nbover + items;
+    }
+    const bool grav = has(p, GSPH_SELF_GRAVITY);
+    cudaEvent_t join = nullptr;
+    if (grav) {
+        const size_t need = gravity_partial_floats(c->fixed_L, np);
+        if (need > c->gpart_cap) {
+            drop_graph(c);  // it holds the old pointer
+            const int rc = grow(c, &c->a.gpart, c->gpart_cap, need);
+            if (rc != GSPH_OK) return rc;
+        }
+        e = cudaEventRecord(c->ev_fork, s);
+        if (e == cudaSuccess) e = cudaStreamWaitEvent(c->side, c->ev_fork, 0);
+        if (e == cudaSuccess) e = launch_fixed_gravity(c->a, p, c->fixed_L, c->side);
+        if (e == cudaSuccess) e = cudaEventRecord(c->ev_join, c->side);
+        if (e != cudaSuccess) return cuda_fail(c, e, "gravity pass");
+        join = c->ev_join;
+        c->launches += 2;
+    }
+    e = launch_chunk_bounds(c->a, c->sp, s);
+    if (e == cudaSuccess) e = launch_chunk_lists(c->a, c->sp, p.H, s);
+    if (e != cudaSuccess) return cuda_fail(c, e, "chunk lists");
+    int launches = 2;
+    e = launch_fixed_sph(c->a, p, c->fixed_L, c->sp, fx, c->sm_count, grav, join, s, launches);
+    c->launches += launches;
+    if (e != cudaSuccess) return cuda_fail(c, e, "SPH passes");
     return GSPH_OK;
 }
 
@@ -346,6 +406,12 @@ bool gsph_ctx_state(gsph_ctx* c, DevArrays* a, const int** ext) {
     *a = c->a;
     *ext = ext_map(c);
     return true;
+}
+
+// the derivatives of a network proposal (surrogate_run.cu)
+int gsph_ctx_proposal_derivatives(gsph_ctx* c, void* stream) {
+    if (c->fp64 || !c->L.cull) return gsph_compute_derivatives(c, stream);  // the features will refuse the context
+    return fixed_derivatives(c, as_stream(stream));
 }
 
 extern "C" {
@@ -505,6 +571,8 @@ int gsph_create(const gsph_params* p, const gsph_options* opt, int64_t n, gsph_c
         if (sym && own_kernel && !c->fp64) sym_groups(nblocks, o.gravity_groups ? o.gravity_groups : 64, L.grav_sym_G, L.grav_sym_gs);
     }
 
+    c->fixed_L = L;
+
     cudaError_t ae = cudaSuccess;
     auto F4 = [&](void) { return static_cast<float4*>(dalloc(c, n_pad * sizeof(float4), ae)); };
     DevArrays& a = c->a;
@@ -521,20 +589,14 @@ int gsph_create(const gsph_params* p, const gsph_options* opt, int64_t n, gsph_c
     if (L.cull) {
         SpatialArrays& sp = c->sp;
         const int64_t nchunks = n_pad / kChunk, ngroups = n_pad / kGroup;
-        L.item_grid = c->sm_count * 5;      // 41 KB of shared memory and at most 102 registers: 5 per SM
-        L.density_grid = c->sm_count * 12;  // 40 registers (launch bound) and 8 KB of shared memory: 12 per SM
-        sp.item_target = 6 * L.item_grid;
-        sp.item_start = static_cast<int*>(dalloc(c, (ngroups + 2) * sizeof(int), ae));
-        // worst case fields per item: fused solids pass without gravity, compensated (x2); items are at
-        // most target + one per group (rounding up per group)
-        const size_t kk = 2 * static_cast<size_t>(popc_c(field_mask<PASS_FUSED, false, true>()));
-        const size_t cap = static_cast<size_t>(sp.item_target) + static_cast<size_t>(ngroups);
-        c->item_cap = cap * kk * kGroup;
-        sp.item_part = static_cast<float*>(dalloc(c, c->item_cap * sizeof(float), ae));
-        c->item_nb_items = cap;
-        sp.item_nb = static_cast<int*>(dalloc(c, cap * kItemNb * kGroup * sizeof(int), ae));
-        sp.item_nbcnt = static_cast<int*>(dalloc(c, cap * kGroup * sizeof(int), ae));
-        sp.item_nbover = static_cast<int*>(dalloc(c, cap * sizeof(int), ae));
+        sp.group_order = static_cast<int*>(dalloc(c, ngroups * sizeof(int), ae));
+        sp.sub_lo = static_cast<float4*>(dalloc(c, n_pad / kSub * sizeof(float4), ae));
+        sp.sub_hi = static_cast<float4*>(dalloc(c, n_pad / kSub * sizeof(float4), ae));
+        // 256 neighbours per particle in equal shares; 96 in very large contexts, whose chunk lists already take
+        // n^2 / 2048 bytes (a longer list costs its warp a second search, not correctness)
+        sp.nb_cap = n_pad <= (int64_t(1) << 22) ? 64 : 24;
+        sp.nb = static_cast<int*>(dalloc(c, static_cast<size_t>(kShares) * sp.nb_cap * n_pad * sizeof(int), ae));
+        sp.nbcnt = static_cast<int*>(dalloc(c, static_cast<size_t>(kShares) * n_pad * sizeof(int), ae));
         a.jrec = static_cast<float4*>(dalloc(c, 4 * n_pad * sizeof(float4), ae));
         if (ae == cudaSuccess) ae = cudaMemset(a.jrec, 0, 4 * n_pad * sizeof(float4));
         sp.box_lo = static_cast<float4*>(dalloc(c, nchunks * sizeof(float4), ae));
@@ -1016,19 +1078,6 @@ int gsph_snapshot(gsph_ctx* c, int32_t slot, int32_t restore, void* stream) {
 
 namespace {
 
-// replace the tracked allocation *p by one of `floats` floats when it holds fewer (contents are scratch)
-int grow(gsph_ctx* c, float** p, size_t& cap, size_t floats) {
-    if (floats <= cap) return GSPH_OK;
-    float* q = nullptr;
-    GSPH_CK(c, cudaMalloc(&q, floats * sizeof(float)), "autotune allocation");
-    for (auto& a : c->allocations)
-        if (a == *p) a = q;
-    cudaFree(*p);
-    *p = q;
-    cap = floats;
-    return GSPH_OK;
-}
-
 // median over `reps` launches of f(stream), in ms (events on the stream, after one warm-up)
 template <typename F>
 int time_ms(gsph_ctx* c, cudaStream_t s, int reps, F&& f, float& ms) {
@@ -1141,19 +1190,12 @@ int gsph_autotune(gsph_ctx* c, int32_t reps, void* stream) {
             L.grav_sym_gs = best.grav_sym_gs;
         }
     }
-    // 2. the SPH passes: work items of the culled kernels, or the all-pairs tile shape
-    if (rc == GSPH_OK && sph) {
+    // 2. the all-pairs SPH passes' tile shape (the culled kernels have one shape)
+    if (rc == GSPH_OK && sph && !L.cull) {
         Launch best = L;
         float best_ms = 1e30f;
         std::vector<Launch> cands;
-        if (L.cull) {
-            for (int f : {3, 6, 12, 24}) {
-                Launch t = L;
-                t.item_grid = L.item_grid;
-                cands.push_back(t);
-                cands.back().nseg = -f;  // marks the item multiple (restored below)
-            }
-        } else {
+        {
             for (int th : {64, 128, 256})
                 for (int jt : {128, 256, 512}) {
                     if (np % jt || np % th) continue;
@@ -1168,30 +1210,9 @@ int gsph_autotune(gsph_ctx* c, int32_t reps, void* stream) {
                     }
                 }
         }
-        const int ngroups = static_cast<int>(np / kGroup);
-        const size_t kk = 2 * static_cast<size_t>(popc_c(field_mask<PASS_FUSED, false, true>()));
-        for (Launch t : cands) {
-            const int target_mult = t.nseg < 0 ? -t.nseg : 0;
-            if (target_mult) {
-                t.nseg = L.nseg;
-                const size_t items = static_cast<size_t>(target_mult) * L.item_grid + ngroups;
-                rc = grow(c, &c->sp.item_part, c->item_cap, items * kk * kGroup);
-                if (rc == GSPH_OK && items > c->item_nb_items) {
-                    size_t cap_nb = c->item_nb_items * kItemNb * kGroup, cap_cnt = c->item_nb_items * kGroup,
-                           cap_over = c->item_nb_items;
-                    rc = grow(c, reinterpret_cast<float**>(&c->sp.item_nb), cap_nb, items * kItemNb * kGroup);
-                    if (rc == GSPH_OK)
-                        rc = grow(c, reinterpret_cast<float**>(&c->sp.item_nbcnt), cap_cnt, items * kGroup);
-                    if (rc == GSPH_OK)
-                        rc = grow(c, reinterpret_cast<float**>(&c->sp.item_nbover), cap_over, items);
-                    if (rc == GSPH_OK) c->item_nb_items = items;
-                }
-                if (rc != GSPH_OK) break;
-                c->sp.item_target = target_mult * L.item_grid;
-            } else {
-                rc = grow(c, &c->a.part, c->part_cap, partial_floats(c->dp, t, np));
-                if (rc != GSPH_OK) break;
-            }
+        for (const Launch& t : cands) {
+            rc = grow(c, &c->a.part, c->part_cap, partial_floats(c->dp, t, np));
+            if (rc != GSPH_OK) break;
             const Launch saved = L;
             L = t;
             float ms = 0.0f;
@@ -1201,17 +1222,12 @@ int gsph_autotune(gsph_ctx* c, int32_t reps, void* stream) {
             if (ms < best_ms) {
                 best_ms = ms;
                 best = t;
-                if (target_mult) best.item_grid = -target_mult;  // remembered as a multiple
             }
         }
         if (rc == GSPH_OK) {
-            if (L.cull) {
-                c->sp.item_target = -best.item_grid * L.item_grid;
-            } else {
-                L.threads = best.threads;
-                L.jt = best.jt;
-                L.nseg = best.nseg;
-            }
+            L.threads = best.threads;
+            L.jt = best.jt;
+            L.nseg = best.nseg;
         }
     }
     c->profiling = profiling;
@@ -1231,7 +1247,7 @@ int gsph_launch_shape_get(gsph_ctx* c, gsph_launch_shape* out) {
     out->sph_threads = c->L.threads;
     out->sph_jt = c->L.jt;
     out->sph_nseg = c->L.nseg;
-    out->items = c->L.cull ? c->sp.item_target : 0;
+    out->items = c->L.cull ? kShares : 0;
     return GSPH_OK;
 }
 

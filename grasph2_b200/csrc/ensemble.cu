@@ -31,6 +31,7 @@
 
 #include <cub/device/device_radix_sort.cuh>
 
+#include "f32x2.cuh"
 #include "integrate.cuh"
 #include "spatial.cuh"
 #include "sph.cuh"
@@ -75,30 +76,6 @@ struct EnsView {
     float* gslot;        // all simulations' slots; simulation k's start at slot_base[k]
     const long long* slot_base;
 };
-
-// ---- paired FP32 (PTX ISA 8.6, sm_100+): two lanes per instruction, IEEE single precision ---------
-__device__ __forceinline__ uint64_t u64_of(float2 v) { return *reinterpret_cast<uint64_t*>(&v); }
-__device__ __forceinline__ float2 f2_of(uint64_t v) { return *reinterpret_cast<float2*>(&v); }
-__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
-    uint64_t d;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(u64_of(a)), "l"(u64_of(b)), "l"(u64_of(c)));
-    return f2_of(d);
-}
-__device__ __forceinline__ float2 sub2(float2 a, float2 b) {
-    uint64_t d;
-    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(u64_of(a)), "l"(u64_of(b)));
-    return f2_of(d);
-}
-__device__ __forceinline__ float2 add2(float2 a, float2 b) {
-    uint64_t d;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(u64_of(a)), "l"(u64_of(b)));
-    return f2_of(d);
-}
-__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
-    uint64_t d;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(u64_of(a)), "l"(u64_of(b)));
-    return f2_of(d);
-}
 
 // ---- cross-CTA counters --------------------------------------------------------------------------
 __device__ __forceinline__ int64_t lmin(int64_t x, int64_t y) { return x < y ? x : y; }

@@ -15,6 +15,7 @@
 #include <algorithm>
 #include <cfloat>
 
+#include "f32x2.cuh"
 #include "pairs.cuh"
 #include "sph.cuh"
 
@@ -25,27 +26,15 @@ namespace {
 // ================================================================================================
 // density
 // ================================================================================================
-// Where the partial sums of particle i live: j-segments [seg][field][n_pad] (all-pairs kernels) or
-// work items [w][field][kGroup] (culled kernels); KK = fields per slot (2K when compensated).
+// The partial sums of particle i: j-segments [seg][field][n_pad] (the culled pass: one); KK = fields per slot (2K
+// with compensation terms).
 struct PartView {
     const float* part;
     int64_t n_pad;
     int nseg;
-    const int* item_start;  // non-null: item layout
     int KK;
-    bool err;               // compensation terms stored after the K sums (all-pairs segments, compensated)
-    __device__ __forceinline__ void range(int64_t i, int& b, int& e) const {
-        if (item_start) {
-            const int64_t g = i / kGroup;
-            b = item_start[g];
-            e = item_start[g + 1];
-        } else {
-            b = 0;
-            e = nseg;
-        }
-    }
+    bool err;  // compensation terms stored after the K sums (all-pairs segments, compensated)
     __device__ __forceinline__ float at(int slot, int o, int64_t i) const {
-        if (item_start) return part[(static_cast<int64_t>(slot) * KK + o) * kGroup + (i % kGroup)];
         return part[(static_cast<int64_t>(slot) * KK + o) * n_pad + i];
     }
 };
@@ -95,111 +84,54 @@ __global__ void __launch_bounds__(256) k_density(const float4* __restrict__ posm
     if (COMP) part[(seg * 2 + 1) * n_pad + i] = rho_c;
 }
 
-// culled density sum over the near-chunk work items (persistent grid); with LISTS every lane also
-// records the indices of its neighbours in this item (for the SPH passes of the same step)
-template <bool COMP, bool LISTS>
-__global__ void __launch_bounds__(kGroup, 12) k_density_items(const float4* __restrict__ posm, DevParams p, CullView cv,
-                                                          int* status) {
-    constexpr int SJ = kStageChunks * kChunk;
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    ItemPipe<1> pipe;
-    pipe.buf = reinterpret_cast<float4*>(smem_raw);
-    pipe.bar = reinterpret_cast<uint64_t*>(smem_raw + 2 * SJ * sizeof(float4));
-    pipe.src[0] = posm;
-    pipe.status = status;
-    pipe.init();
-    const uint32_t span = __float_as_uint(p.H2);
-    const int total = cv.items();
-    __shared__ float4 wbox[kGroup / 32][2];  // each warp's bounding box for the current item
-    for (int w = blockIdx.x; w < total; w += gridDim.x) {
-        int g, c0, c1;
-        cv.item(w, g, c0, c1);
-        const float4 pi = posm[static_cast<int64_t>(g) * kGroup + threadIdx.x];
-        float rho_s = 0.0f, rho_c = 0.0f;
-        int cnt = 0;
-        // the warp's bounding box: a chunk of the group's list that lies farther than h (1 + kMargin)
-        // from it (the list's own conservative bound) holds no neighbour of the warp's 32 particles, and
-        // the warp skips its tests (same sums, same lists; padding lanes only widen the box)
-        if (LISTS) {
-            float wlo[3] = {pi.x, pi.y, pi.z}, whi[3] = {pi.x, pi.y, pi.z};
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1)
-#pragma unroll
-                for (int c = 0; c < 3; ++c) {
-                    wlo[c] = fminf(wlo[c], __shfl_xor_sync(0xffffffffu, wlo[c], o));
-                    whi[c] = fmaxf(whi[c], __shfl_xor_sync(0xffffffffu, whi[c], o));
-                }
-            __syncwarp();  // the previous item's reads of this warp's box are done
-            if ((threadIdx.x & 31) == 0) {
-                wbox[threadIdx.x >> 5][0] = make_float4(wlo[0], wlo[1], wlo[2], 0.0f);
-                wbox[threadIdx.x >> 5][1] = make_float4(whi[0], whi[1], whi[2], 0.0f);
-            }
-            __syncwarp();
+// Culled density sum of 32 particles per CTA, with the epilogue; every share's neighbours go to its list.
+template <bool COMP>
+__global__ void __launch_bounds__(kSub * kShares) k_density_near(const float4* __restrict__ posm, float4* __restrict__ velrho,
+                                                                 DevParams p, NearView v) {
+    __shared__ float4 sh[kShares][kSub];
+    __shared__ float red[COMP ? 2 : 1][kShares][kSub];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int g = v.group();
+    const int64_t s0 = v.first(g), i = s0 + lane;
+    if (s0 >= v.n) return;
+    const float4 pi = posm[i];
+    float rho_s = 0.0f, rho_c = 0.0f;
+    int cnt = 0;
+    int* lst = v.nb + static_cast<int64_t>(warp) * v.cap * v.n_pad + i;
+    near_scan(v, posm, g, s0, __float_as_uint(p.H2), pi, sh[warp], [&](unsigned m, int jb) {
+        float t = 0.0f;
+        while (m) {
+            const int k = __ffs(m) - 1;
+            m &= m - 1;
+            const float4 q = sh[warp][k];
+            const float dx = q.x - pi.x, dy = q.y - pi.y, dz = q.z - pi.z;
+            const float r2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
+            t = fmaf(q.w, w_poly(r2 * rsqrtf(r2) * p.inv_h), t);
+            if (cnt < v.cap) lst[static_cast<int64_t>(cnt) * v.n_pad] = jb + k;
+            ++cnt;
         }
-        int* lst = LISTS ? cv.nb + static_cast<int64_t>(w) * kItemNb * kGroup + threadIdx.x : nullptr;
-        const int* chunks = cv.list + static_cast<int64_t>(g) * cv.nchunks + c0;
-        int chunk_base = 0;
-        if (!pipe.run(chunks, c1 - c0, [&](const float4* J, int nj) {
-                float t;
-                if (LISTS) {  // the density_tile sum, recording the neighbours as well (same order)
-                    t = 0.0f;
-                    for (int s0 = 0; s0 < nj; s0 += kChunk) {
-                        const int jc = chunks[chunk_base + s0 / kChunk], jb = jc * kChunk;
-                        {
-                            const float4 l = cv.box_lo[jc], u = cv.box_hi[jc];
-                            const float4 wl = wbox[threadIdx.x >> 5][0], wh = wbox[threadIdx.x >> 5][1];
-                            const float gx = fmaxf(0.0f, fmaxf(l.x - wh.x, wl.x - u.x)),
-                                        gy = fmaxf(0.0f, fmaxf(l.y - wh.y, wl.y - u.y)),
-                                        gz = fmaxf(0.0f, fmaxf(l.z - wh.z, wl.z - u.z));
-                            const float hm = p.H * (1.0f + kMargin);
-                            if (gx * gx + gy * gy + gz * gz > hm * hm) continue;  // warp-uniform
-                        }
-                        // the chunk's 64 tests into a bit mask without branches, then its set bits in
-                        // ascending order (the neighbours, about 2 % of the tests)
-                        unsigned m8[8];
+        if (COMP) fold(rho_s, rho_c, t);
+        else rho_s += t;
+    });
+    v.nbcnt[static_cast<int64_t>(warp) * v.n_pad + i] = cnt;
+    red[0][warp][lane] = rho_s;
+    if (COMP) red[COMP ? 1 : 0][warp][lane] = rho_c;
+    __syncthreads();
+    if (warp != 0 || i >= v.n) return;
+    float rho;
+    if (COMP) {
+        double s = 0.0;
 #pragma unroll
-                        for (int b = 0; b < 8; ++b) {
-                            unsigned m = 0;
+        for (int w = 0; w < kShares; ++w) s += static_cast<double>(red[0][w][lane]) + static_cast<double>(red[COMP ? 1 : 0][w][lane]);
+        rho = static_cast<float>(s * static_cast<double>(p.w_pref));
+    } else {
+        float s = 0.0f;
 #pragma unroll
-                            for (int u = 0; u < 8; ++u) {
-                                const float4 q = J[s0 + b * 8 + u];
-                                const float dx = q.x - pi.x, dy = q.y - pi.y, dz = q.z - pi.z;
-                                const float r2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
-                                m |= static_cast<unsigned>(in_open_closed(r2, 0u, span)) << u;
-                            }
-                            m8[b] = m;
-                        }
-                        uint64_t bits = static_cast<uint64_t>(m8[0] | (m8[1] << 8) | (m8[2] << 16) | (m8[3] << 24)) |
-                                        (static_cast<uint64_t>(m8[4] | (m8[5] << 8) | (m8[6] << 16) | (m8[7] << 24)) << 32);
-                        while (bits) {
-                            const int j = __ffsll(static_cast<long long>(bits)) - 1;
-                            bits &= bits - 1;
-                            const float4 q = J[s0 + j];
-                            const float dx = q.x - pi.x, dy = q.y - pi.y, dz = q.z - pi.z;
-                            const float r2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
-                            const float r = r2 * rsqrtf(r2);
-                            t = fmaf(q.w, w_poly(r * p.inv_h), t);
-                            if (cnt < kItemNb) lst[cnt * kGroup] = jb + j;
-                            ++cnt;
-                        }
-                    }
-                    chunk_base += nj / kChunk;
-                } else {
-                    t = density_tile(J, nj, pi, span, p.inv_h);
-                }
-                if (COMP) fold(rho_s, rho_c, t);
-                else rho_s += t;
-            }))
-            return;
-        float* out = cv.part + static_cast<int64_t>(w) * (COMP ? 2 : 1) * kGroup + threadIdx.x;
-        out[0] = rho_s;
-        if (COMP) out[kGroup] = rho_c;
-        if (LISTS) {
-            cv.nbcnt[static_cast<int64_t>(w) * kGroup + threadIdx.x] = min(cnt, kItemNb + 1);
-            const int over = __syncthreads_or(cnt > kItemNb);  // the SPH passes read one flag per item
-            if (threadIdx.x == 0) cv.nbover[w] = over;
-        }
+        for (int w = 0; w < kShares; ++w) s += red[0][w][lane];
+        rho = s * p.w_pref;
     }
+    if (has(p, GSPH_DEAL_WITH_NO_PARTNERS) && rho < 0.001f) rho = p.rho0 * 0.01f;  // computeDerivatives.h:85-88
+    reinterpret_cast<float*>(velrho + i)[3] = rho;
 }
 
 // sum the slots, apply the prefactor and the optional floor (computeDerivatives.h:85-88), then
@@ -208,16 +140,14 @@ template <bool COMP>
 __global__ void k_density_finish(DevArrays a, DevParams p, PartView pv) {
     const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (i >= a.n) return;
-    int b, e;
-    pv.range(i, b, e);
     float rho;
     if (COMP) {
         double s = 0.0;
-        for (int k = b; k < e; ++k) s += static_cast<double>(pv.at(k, 0, i)) + static_cast<double>(pv.at(k, 1, i));
+        for (int k = 0; k < pv.nseg; ++k) s += static_cast<double>(pv.at(k, 0, i)) + static_cast<double>(pv.at(k, 1, i));
         rho = static_cast<float>(s * static_cast<double>(p.w_pref));
     } else {
         float s = 0.0f;
-        for (int k = b; k < e; ++k) s += pv.at(k, 0, i);
+        for (int k = 0; k < pv.nseg; ++k) s += pv.at(k, 0, i);
         rho = s * p.w_pref;
     }
     if (has(p, GSPH_DEAL_WITH_NO_PARTNERS) && rho < 0.001f) rho = p.rho0 * 0.01f;
@@ -234,7 +164,7 @@ __global__ void k_density_finish(DevArrays a, DevParams p, PartView pv) {
     }
 }
 
-// j-records from the current density (INTEGRATE_DENSITY: no density pass precedes the pairs)
+// j-records from the current density
 __global__ void k_prepare(DevArrays a, DevParams p) {
     const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (i >= a.n) return;
@@ -346,147 +276,102 @@ __global__ void __launch_bounds__(256) k_pairs(DevArrays a, DevParams p, int jt,
                                S, C, maxv);
 }
 
-// Culled SPH pass (no gravity): a persistent grid walks the work items; item w covers some near
-// chunks of one i-group and writes its partials to part[w][field][kGroup]. Phase 1 streams only the
-// positions of those chunks through shared memory and lets every lane record the indices of its own
-// neighbours (kNbCap per lane, flushed early when a lane's list is nearly full); phase 2 walks the
-// per-lane lists and gathers each neighbour's records from L2, so the SPH terms run lane-dense.
-constexpr int kNbCap = 64;
-template <int PASS, bool SOLIDS, bool COMP>
-__global__ void __launch_bounds__(kGroup, 5) k_pairs_items(DevArrays a, DevParams p, CullView cv) {
+// Culled SPH pass (no gravity) of 32 particles per CTA. LISTS: an earlier pass of the step stored the neighbour lists;
+// otherwise every share first searches its boxes and stores them (for itself and a later pass). The terms then run
+// over the lists, one packed 64-byte record per neighbour, the next record and the index after it in flight; a warp
+// with an incomplete list (more than v.cap in one share) goes back to the boxes. The shares of a field are added in
+// order (compensated: in FP64; a share holds a few to tens of terms, so it carries no compensation term itself).
+//
+// Bound: instruction issue and the L2 latency of the gathers. All neighbours of a particle in four lists instead of one
+// list per work item of a few chunks: a warp runs as long as its longest list, and the longer lists differ less
+// (18.8 of 32 lanes were active). No partial sums per item: the finish kernel reads one value per field.
+template <int PASS, bool SOLIDS, bool LISTS, bool COMP>
+__global__ void __launch_bounds__(kSub * kShares, 5) k_pairs_near(DevArrays a, DevParams p, NearView v) {
     constexpr uint32_t MASK = field_mask<PASS, false, SOLIDS>();
     constexpr int K = popc_c(MASK);
     constexpr bool DO_A = PASS != PASS_VGRAD;
-    constexpr int SJ = kStageChunks * kChunk;
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    ItemPipe<1> pipe;
-    pipe.buf = reinterpret_cast<float4*>(smem_raw);
-    pipe.bar = reinterpret_cast<uint64_t*>(smem_raw + 2 * SJ * sizeof(float4));
-    pipe.src[0] = a.posm;
-    pipe.status = a.status;
-    const int lane = threadIdx.x & 31;
-    int* nb = reinterpret_cast<int*>(smem_raw + pipe_smem_bytes(1, SJ)) + (threadIdx.x >> 5) * (kNbCap * 32);
-    pipe.init();
-    const int total = cv.items();
-    for (int w = blockIdx.x; w < total; w += gridDim.x) {
-        int g, c0, c1;
-        cv.item(w, g, c0, c1);
-        const int64_t i = static_cast<int64_t>(g) * kGroup + threadIdx.x;
-        const ISph I = load_isph<PASS, SOLIDS>(a, p, i, 0.0f);
-        PairAcc S, C, T;
-#pragma unroll
-        for (int f = 0; f < F_COUNT; ++f) S.f[f] = C.f[f] = T.f[f] = 0.0f;
-        float maxv = 0.0f;
-        // the density pass's neighbour lists of this item, when every lane's list is complete (one flag
-        // per item, so no block-wide vote: the warps of a block run through list items independently)
-        if (cv.nb && cv.nbover[w] == 0) {
-            const int lcnt = cv.nbcnt[static_cast<int64_t>(w) * kGroup + threadIdx.x];
-            const int* lst = cv.nb + static_cast<int64_t>(w) * kItemNb * kGroup + threadIdx.x;
-            const float4 zero = make_float4(0, 0, 0, 0);
-            const int j0 = lcnt > 0 ? lst[0] : 0;
-            int jn = lcnt > 1 ? lst[kGroup] : 0;  // the index of neighbour k+1
-            const float4* r0 = a.jrec + 4 * static_cast<int64_t>(j0);  // one 64-byte record per neighbour
-            float4 qn = __ldg(r0), vn = __ldg(r0 + 1);
-            float4 an = DO_A ? __ldg(r0 + 2) : zero, bn = DO_A ? __ldg(r0 + 3) : zero;
-            // software pipeline: neighbour k+1's records and neighbour k+2's index in flight during k
-            for (int k = 0; k < lcnt; ++k) {
-                const float4 q = qn, vj = vn, ja = an, jb = bn;
-                if (k + 1 < lcnt) {
-                    const float4* r = a.jrec + 4 * static_cast<int64_t>(jn);
-                    qn = __ldg(r);
-                    vn = __ldg(r + 1);
-                    if (DO_A) {
-                        an = __ldg(r + 2);
-                        bn = __ldg(r + 3);
-                    }
-                }
-                if (k + 2 < lcnt) jn = lst[(k + 2) * kGroup];
-                const float dx = q.x - I.pi.x, dy = q.y - I.pi.y, dz = q.z - I.pi.z;
-                const float r2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
-                sph_neighbour<PASS, SOLIDS>(T, maxv, I, q.w, dx, dy, dz, r2, vj, ja, jb, p);
+    __shared__ float4 sh[kShares][kSub];
+    __shared__ float red[kShares][K][kSub];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int g = v.group();
+    const int64_t s0 = v.first(g), i = s0 + lane;
+    if (s0 >= v.n) return;
+    const ISph I = load_isph<PASS, SOLIDS>(a, p, i, 0.0f);
+    int* lst = v.nb + static_cast<int64_t>(warp) * v.cap * v.n_pad + i;
+    int cnt = 0;
+    if (LISTS) {
+        cnt = v.nbcnt[static_cast<int64_t>(warp) * v.n_pad + i];
+    } else {
+        near_scan(v, a.posm, g, s0, I.span, I.pi, sh[warp], [&](unsigned m, int jb) {
+            while (m) {
+                const int k = __ffs(m) - 1;
+                m &= m - 1;
+                if (cnt < v.cap) lst[static_cast<int64_t>(cnt) * v.n_pad] = jb + k;
+                ++cnt;
             }
-            fold_tile<MASK, COMP>(S, C, T);
-            store_partials<MASK, COMP>(cv.part + static_cast<int64_t>(w) * (COMP ? 2 * K : K) * kGroup + threadIdx.x,
-                                       kGroup, S, C, maxv);
-            continue;
+        });
+        v.nbcnt[static_cast<int64_t>(warp) * v.n_pad + i] = cnt;
+    }
+    PairAcc T;
+#pragma unroll
+    for (int f = 0; f < F_COUNT; ++f) T.f[f] = 0.0f;
+    float maxv = 0.0f;
+    const float4 zero = make_float4(0, 0, 0, 0);
+    auto term = [&](float4 q, float4 vj, float4 ja, float4 jb) {
+        const float dx = q.x - I.pi.x, dy = q.y - I.pi.y, dz = q.z - I.pi.z;
+        sph_neighbour<PASS, SOLIDS>(T, maxv, I, q.w, dx, dy, dz, fmaf(dz, dz, fmaf(dy, dy, dx * dx)), vj, ja, jb, p);
+    };
+    if (!__any_sync(0xffffffffu, cnt > v.cap)) {
+        int jn = cnt > 0 ? lst[0] : 0;
+        const float4* r0 = a.jrec + 4 * static_cast<int64_t>(jn);
+        float4 qn = __ldg(r0), vn = __ldg(r0 + 1);
+        float4 an = DO_A ? __ldg(r0 + 2) : zero, bn = DO_A ? __ldg(r0 + 3) : zero;
+        jn = cnt > 1 ? lst[v.n_pad] : 0;  // the index of neighbour k + 1
+        for (int k = 0; k < cnt; ++k) {
+            const float4 q = qn, vj = vn, ja = an, jb = bn;
+            if (k + 1 < cnt) {
+                const float4* r = a.jrec + 4 * static_cast<int64_t>(jn);
+                qn = __ldg(r);
+                vn = __ldg(r + 1);
+                if (DO_A) {
+                    an = __ldg(r + 2);
+                    bn = __ldg(r + 3);
+                }
+            }
+            if (k + 2 < cnt) jn = lst[static_cast<int64_t>(k + 2) * v.n_pad];
+            term(q, vj, ja, jb);
         }
-        int cnt = 0;
-        // phase 2 over the lane lists collected so far
-        auto drain = [&]() {
-            int m = cnt;
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
-            // software pipeline: the records of neighbour k+1 are in flight while k is computed
-            const float4 zero = make_float4(0, 0, 0, 0);
-            int jn = cnt > 0 ? nb[lane] : 0;
-            const float4* r0 = a.jrec + 4 * static_cast<int64_t>(jn);
-            float4 qn = __ldg(r0), vn = __ldg(r0 + 1);
-            float4 an = DO_A ? __ldg(r0 + 2) : zero, bn = DO_A ? __ldg(r0 + 3) : zero;
-            for (int k = 0; k < m; ++k) {
-                const float4 q = qn, vj = vn, ja = an, jb = bn;
-                if (k + 1 < cnt) {
-                    jn = nb[(k + 1) * 32 + lane];
-                    const float4* r = a.jrec + 4 * static_cast<int64_t>(jn);
-                    qn = __ldg(r);
-                    vn = __ldg(r + 1);
-                    if (DO_A) {
-                        an = __ldg(r + 2);
-                        bn = __ldg(r + 3);
-                    }
-                }
-                if (k < cnt) {
-                    const float dx = q.x - I.pi.x, dy = q.y - I.pi.y, dz = q.z - I.pi.z;
-                    const float r2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
-                    sph_neighbour<PASS, SOLIDS>(T, maxv, I, q.w, dx, dy, dz, r2, vj, ja, jb, p);
-                }
+    } else {
+        near_scan(v, a.posm, g, s0, I.span, I.pi, sh[warp], [&](unsigned m, int jb) {
+            while (m) {
+                const float4* r = a.jrec + 4 * static_cast<int64_t>(jb + __ffs(m) - 1);
+                m &= m - 1;
+                term(r[0], r[1], DO_A ? r[2] : zero, DO_A ? r[3] : zero);
             }
-            cnt = 0;
-            __syncwarp();
-        };
-        const int* chunks = cv.list + static_cast<int64_t>(g) * cv.nchunks + c0;
-        int chunk_base = 0;  // position in `chunks` of the current stage
-        if (!pipe.run(chunks, c1 - c0, [&](const float4* J, int nj) {
-                for (int s0 = 0; s0 < nj; s0 += kChunk) {
-                    const int jbase = chunks[chunk_base + s0 / kChunk] * kChunk;
-                    // 64 independent tests into eight 8-bit masks (no serial chain), then the set bits
-                    unsigned m8[8];
+        });
+    }
 #pragma unroll
-                    for (int b = 0; b < 8; ++b) {
-                        unsigned m = 0;
+    for (int f = 0; f < F_COUNT; ++f)
+        if ((MASK >> f) & 1u) red[warp][field_offset<MASK>(f)][lane] = f == F_MAXV ? maxv : T.f[f];
+    __syncthreads();
+    for (int o = warp; o < K; o += kShares) {  // each warp adds the shares of its fields
+        const bool mx = ((MASK >> F_MAXV) & 1u) && o == field_offset<MASK>(F_MAXV);
+        float s = red[0][o][lane];
+        if (mx) {
 #pragma unroll
-                        for (int t = 0; t < 8; ++t) {
-                            const float4 q = J[s0 + b * 8 + t];
-                            const float dx = q.x - I.pi.x, dy = q.y - I.pi.y, dz = q.z - I.pi.z;
-                            const float r2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
-                            m |= static_cast<unsigned>(in_open_closed(r2, 0u, I.span)) << t;
-                        }
-                        m8[b] = m;
-                    }
-                    unsigned lo = m8[0] | (m8[1] << 8) | (m8[2] << 16) | (m8[3] << 24);
-                    unsigned hi = m8[4] | (m8[5] << 8) | (m8[6] << 16) | (m8[7] << 24);
-                    while (lo) {
-                        nb[cnt * 32 + lane] = jbase + __ffs(lo) - 1;
-                        ++cnt;
-                        lo &= lo - 1u;
-                    }
-                    while (hi) {
-                        nb[cnt * 32 + lane] = jbase + 32 + __ffs(hi) - 1;
-                        ++cnt;
-                        hi &= hi - 1u;
-                    }
-                    // a lane could overflow on the next chunk: process the lists now
-                    if (__any_sync(0xffffffffu, cnt > kNbCap - kChunk)) drain();
-                }
-                chunk_base += nj / kChunk;
-            }))
-            return;
-        drain();
-        fold_tile<MASK, COMP>(S, C, T);
-        store_partials<MASK, COMP>(cv.part + static_cast<int64_t>(w) * (COMP ? 2 * K : K) * kGroup + threadIdx.x,
-                                   kGroup, S, C, maxv);
+            for (int w = 1; w < kShares; ++w) s = fmaxf(s, red[w][o][lane]);
+        } else if (COMP) {
+            double d = s;
+#pragma unroll
+            for (int w = 1; w < kShares; ++w) d += static_cast<double>(red[w][o][lane]);
+            s = static_cast<float>(d);
+        } else {
+#pragma unroll
+            for (int w = 1; w < kShares; ++w) s += red[w][o][lane];
+        }
+        a.part[static_cast<int64_t>(o) * a.n_pad + i] = s;
     }
 }
-
 
 // Sum the slots of one field in a fixed order: FP32 in plain mode, FP64 of (sum + error) in
 // compensated mode. The max signal velocity is a max over slots.
@@ -494,23 +379,21 @@ template <uint32_t MASK, bool COMP>
 __device__ __forceinline__ float seg_sum(const PartView& v, int64_t i, int f) {
     constexpr int K = popc_c(MASK);
     const int o = field_offset<MASK>(f);
-    int b, e;
-    v.range(i, b, e);
     if (f == F_MAXV) {
         float m = 0.0f;
-        for (int k = b; k < e; ++k) m = fmaxf(m, v.at(k, o, i));
+        for (int k = 0; k < v.nseg; ++k) m = fmaxf(m, v.at(k, o, i));
         return m;
     }
     if (COMP) {
         double s = 0.0;
-        for (int k = b; k < e; ++k) {
+        for (int k = 0; k < v.nseg; ++k) {
             s += static_cast<double>(v.at(k, o, i));
             if (v.err) s += static_cast<double>(v.at(k, K + o, i));
         }
         return static_cast<float>(s);
     }
     float s = 0.0f;
-    for (int k = b; k < e; ++k) s += v.at(k, o, i);
+    for (int k = 0; k < v.nseg; ++k) s += v.at(k, o, i);
     return s;
 }
 
@@ -591,32 +474,6 @@ __global__ void k_pairs_finish(DevArrays a, DevParams p, PartView pv, GravSum gs
 // ================================================================================================
 // pure gravity (ENABLE_SPH off): I i-particles per thread share every j read from shared memory
 // ================================================================================================
-// Paired FP32 (PTX ISA 8.6, sm_100+): one add/sub/mul/fma.rn.f32x2 instruction performs the same
-// IEEE single-precision operation on two lanes of a 64-bit register pair, so two i-particles advance
-// per issued instruction with bit-identical results to the scalar form.
-__device__ __forceinline__ uint64_t u64_of(float2 v) { return *reinterpret_cast<uint64_t*>(&v); }
-__device__ __forceinline__ float2 f2_of(uint64_t v) { return *reinterpret_cast<float2*>(&v); }
-__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
-    uint64_t d;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(u64_of(a)), "l"(u64_of(b)), "l"(u64_of(c)));
-    return f2_of(d);
-}
-__device__ __forceinline__ float2 sub2(float2 a, float2 b) {
-    uint64_t d;
-    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(u64_of(a)), "l"(u64_of(b)));
-    return f2_of(d);
-}
-__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
-    uint64_t d;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(u64_of(a)), "l"(u64_of(b)));
-    return f2_of(d);
-}
-__device__ __forceinline__ float2 add2(float2 a, float2 b) {
-    uint64_t d;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(u64_of(a)), "l"(u64_of(b)));
-    return f2_of(d);
-}
-
 // I (even) i-particles per thread in I/2 register pairs; same arithmetic order as k_gravity
 template <int I, int GRAV, bool COMP>
 __global__ void __launch_bounds__(128) k_gravity_x2(const float4* __restrict__ posm, float* __restrict__ part,
@@ -1032,105 +889,37 @@ cudaError_t timer_record(cudaEvent_t ev, cudaStream_t s) {
     } while (0)
 
 namespace {
-CullView cull_view(const DevArrays& a, const SpatialArrays& sp) {
-    CullView cv;
-    cv.list = sp.list;
-    cv.count = sp.count;
-    cv.item_start = sp.item_start;
-    cv.ngroups = static_cast<int>(a.n_pad / kGroup);
-    cv.nchunks = a.n_pad / kChunk;
-    cv.part = sp.item_part;
-    cv.nb = nullptr;
-    cv.nbcnt = nullptr;
-    cv.nbover = nullptr;
-    cv.box_lo = sp.box_lo;
-    cv.box_hi = sp.box_hi;
-    return cv;
+NearView near_view(const DevArrays& a, const DevParams& p, const SpatialArrays& sp) {
+    NearView v;
+    v.list = sp.list;
+    v.count = sp.count;
+    v.order = sp.group_order;
+    v.lo = sp.sub_lo;
+    v.hi = sp.sub_hi;
+    v.nchunks = a.n_pad / kChunk;
+    v.n = a.n;
+    v.n_pad = a.n_pad;
+    const float hm = p.H * (1.0f + kMargin);
+    v.hm2 = hm * hm;
+    v.nb = sp.nb;
+    v.nbcnt = sp.nbcnt;
+    v.cap = sp.nb_cap;
+    return v;
 }
+unsigned near_blocks(const DevArrays& a) { return static_cast<unsigned>(a.n_pad / kSub); }
 PartView seg_view(const DevArrays& a, int nseg, int KK, bool err) {
-    return PartView{a.part, a.n_pad, nseg, nullptr, KK, err};
-}
-PartView item_view(const DevArrays& a, const SpatialArrays& sp, int KK, bool err) {
-    return PartView{sp.item_part, a.n_pad, 0, sp.item_start, KK, err};
-}
-
-// One block: chunks per item ic = ceil(total near chunks / target) so that items carry equal work,
-// then the exclusive scan of the per-group item counts ceil(count / ic) in a fixed order.
-constexpr int kScanThreads = 1024;
-__global__ void __launch_bounds__(kScanThreads) k_work_items(const int* __restrict__ count, int* __restrict__ start,
-                                                             int ngroups, int target) {
-    __shared__ int warp_sums[kScanThreads / 32];
-    __shared__ int carry;
-    __shared__ int ic_sh;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    int part = 0;  // total near chunks
-    for (int g = threadIdx.x; g < ngroups; g += kScanThreads) part += count[g];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
-    if (lane == 0) warp_sums[warp] = part;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        long long total = 0;
-        for (int w = 0; w < kScanThreads / 32; ++w) total += warp_sums[w];
-        const long long ic = (total + target - 1) / target;
-        ic_sh = static_cast<int>(ic < 1 ? 1 : ic);
-        carry = 0;
-    }
-    __syncthreads();
-    const int ic = ic_sh;
-    for (int base = 0; base < ngroups; base += kScanThreads) {
-        const int g = base + threadIdx.x;
-        const int v = (g < ngroups) ? (count[g] + ic - 1) / ic : 0;
-        int x = v;  // inclusive warp scan
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int y = __shfl_up_sync(0xffffffffu, x, o);
-            if (lane >= o) x += y;
-        }
-        __syncthreads();
-        if (lane == 31) warp_sums[warp] = x;
-        __syncthreads();
-        if (warp == 0) {
-            int w = warp_sums[lane];
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const int y = __shfl_up_sync(0xffffffffu, w, o);
-                if (lane >= o) w += y;
-            }
-            warp_sums[lane] = w;  // inclusive over warps
-        }
-        __syncthreads();
-        const int before = carry + (warp ? warp_sums[warp - 1] : 0) + x - v;
-        if (g < ngroups) start[g] = before;
-        __syncthreads();
-        if (threadIdx.x == kScanThreads - 1) carry = before + v;
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) {
-        start[ngroups] = carry;
-        start[ngroups + 1] = ic;
-    }
+    return PartView{a.part, a.n_pad, nseg, KK, err};
 }
 }  // namespace
-
-cudaError_t launch_work_items(const DevArrays& a, const SpatialArrays& sp, int target, cudaStream_t s) {
-    k_work_items<<<1, kScanThreads, 0, s>>>(sp.count, sp.item_start, static_cast<int>(a.n_pad / kGroup), target);
-    return cudaGetLastError();
-}
 
 cudaError_t launch_density(const DevArrays& a, const DevParams& p, const Launch& L, cudaStream_t s, const KTimer* t,
                            const SpatialArrays* sp) {
     const bool comp = L.accum == GSPH_ACCUM_COMPENSATED;
     GSPH_TIMER_MARK(t, start);
     if (sp) {
-        const size_t smem = pipe_smem_bytes(1, kStageChunks * kChunk);
-        const CullView cv = cull_view(a, *sp);
-        CullView cvl = cv;
-        cvl.nb = sp->item_nb;
-        cvl.nbcnt = sp->item_nbcnt;
-        cvl.nbover = sp->item_nbover;
-        if (comp) k_density_items<true, true><<<L.density_grid, kGroup, smem, s>>>(a.posm, p, cvl, a.status);
-        else k_density_items<false, true><<<L.density_grid, kGroup, smem, s>>>(a.posm, p, cvl, a.status);
+        const NearView v = near_view(a, p, *sp);
+        if (comp) k_density_near<true><<<near_blocks(a), kSub * kShares, 0, s>>>(a.posm, a.velrho, p, v);
+        else k_density_near<false><<<near_blocks(a), kSub * kShares, 0, s>>>(a.posm, a.velrho, p, v);
     } else {
         const int T = 256;
         const dim3 grid(static_cast<unsigned>(a.n_pad / T), static_cast<unsigned>(L.nseg));
@@ -1141,8 +930,8 @@ cudaError_t launch_density(const DevArrays& a, const DevParams& p, const Launch&
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     GSPH_TIMER_MARK(t, stop);
-    const int KK = comp ? 2 : 1;
-    const PartView pv = sp ? item_view(a, *sp, KK, comp) : seg_view(a, L.nseg, KK, comp);
+    if (sp) return launch_prepare(a, p, s);  // the density is final: the j-records
+    const PartView pv = seg_view(a, L.nseg, comp ? 2 : 1, comp);
     if (comp) k_density_finish<true><<<blocks_for(a.n, 256), 256, 0, s>>>(a, p, pv);
     else k_density_finish<false><<<blocks_for(a.n, 256), 256, 0, s>>>(a, p, pv);
     return cudaGetLastError();
@@ -1158,27 +947,13 @@ template <int PASS, int GRAV, bool SOLIDS, bool COMP>
 cudaError_t pairs_t(const DevArrays& a, const DevParams& p, const Launch& L, cudaStream_t s, const KTimer* t,
                     const SpatialArrays* sp, int gnseg, cudaEvent_t join, bool lists) {
     constexpr int NS = (PASS == PASS_VGRAD) ? 2 : 4;
-    if (sp) {  // SPH terms over the near-chunk work items; gravity partials come from elsewhere
+    if (sp) {  // SPH terms over the near chunks; gravity partials come from elsewhere
         constexpr uint32_t MASK = field_mask<PASS, false, SOLIDS>();
         constexpr int K = popc_c(MASK);
-        // position stages, then per warp the [kNbCap][32] neighbour-index lists
-        const size_t smem = pipe_smem_bytes(1, kStageChunks * kChunk) + (kGroup / 32) * kNbCap * 32 * sizeof(int);
-        if (smem > 48 * 1024) {
-            cudaError_t e = cudaFuncSetAttribute(k_pairs_items<PASS, SOLIDS, false>,
-                                                 cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-            if (e != cudaSuccess) return e;
-        }
         GSPH_TIMER_MARK(t, start);
-        CullView cv = cull_view(a, *sp);
-        if (lists) {
-            cv.nb = sp->item_nb;
-            cv.nbcnt = sp->item_nbcnt;
-            cv.nbover = sp->item_nbover;
-        }
-        // one work item is one tile of its particles' neighbour sums (a few to tens of terms): its
-        // partials carry no compensation term, and the compensated form folds the items in FP64 in the
-        // finish, so both forms run the plain kernel
-        k_pairs_items<PASS, SOLIDS, false><<<L.item_grid, kGroup, smem, s>>>(a, p, cv);
+        const NearView v = near_view(a, p, *sp);
+        if (lists) k_pairs_near<PASS, SOLIDS, true, COMP><<<near_blocks(a), kSub * kShares, 0, s>>>(a, p, v);
+        else k_pairs_near<PASS, SOLIDS, false, COMP><<<near_blocks(a), kSub * kShares, 0, s>>>(a, p, v);
         cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) return e;
         GSPH_TIMER_MARK(t, stop);
@@ -1187,7 +962,7 @@ cudaError_t pairs_t(const DevArrays& a, const DevParams& p, const Launch& L, cud
             if (e != cudaSuccess) return e;
         }
         k_pairs_finish<PASS, false, SOLIDS, COMP><<<blocks_for(a.n, 256), 256, 0, s>>>(
-            a, p, item_view(a, *sp, K, false), grav_sum(L, PASS == PASS_VGRAD ? 0 : gnseg));
+            a, p, seg_view(a, 1, K, false), grav_sum(L, PASS == PASS_VGRAD ? 0 : gnseg));
         return cudaGetLastError();
     }
     constexpr uint32_t MASK = field_mask<PASS, (GRAV != 0), SOLIDS>();
@@ -1311,6 +1086,13 @@ cudaError_t launch_gravity(const DevArrays& a, const DevParams& p, const Launch&
 cudaError_t launch_gravity_partials(const DevArrays& a, const DevParams& p, const Launch& L, cudaStream_t s,
                                     const KTimer* t) {
     return gravity_any(a, p, L, s, t, false);
+}
+
+cudaError_t launch_gravity_fold(const DevArrays& a, const Launch& L, int S, cudaStream_t s) {
+    const unsigned nb = blocks_for(a.n * kFoldT, 256);
+    if (L.accum == GSPH_ACCUM_COMPENSATED) k_gravity_fold<true><<<nb, 256, 0, s>>>(a.gpart, a.n, a.n_pad, S, a.gfold);
+    else k_gravity_fold<false><<<nb, 256, 0, s>>>(a.gpart, a.n, a.n_pad, S, a.gfold);
+    return cudaGetLastError();
 }
 
 // Gravity partials of caller-provided, already padded j-records into caller-provided partials

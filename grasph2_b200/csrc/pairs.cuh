@@ -84,95 +84,88 @@ struct JTilePipe {
     }
 };
 
-// ---- culled passes: work items over the near-chunk lists ------------------------------------------
-constexpr int kStageChunks = 4;  // chunks staged per pipeline stage (256 j-particles)
-constexpr int kItemNb = 96;      // neighbour-list slots per lane and work item (density pass -> SPH passes)
+// ---- culled passes -------------------------------------------------------------------------------
+// Every 32 consecutive particles (a quarter of an i-group) belong to one CTA of kShares warps; lane l of each warp
+// holds particle l. The warps share the group's near chunks, half a chunk (32 particles, one box) at a time: half h
+// goes to warp h % kShares, since near chunks come in runs along the curve. A particle's neighbours found by a warp
+// are its share; the CTA adds the shares in order, so no partial sums leave it.
+constexpr int kShares = 4;
+constexpr int kSub = 32;                 // particles per CTA and per box
+constexpr int kSubs = kGroup / kSub;     // CTAs per i-group
 
-// Work item w of the culled passes: i-group g, positions [c0, c1) of g's near-chunk list. Items are
-// numbered group by group (item_start[g] .. item_start[g+1]-1), at most item_chunks chunks each.
-struct CullView {
-    const int* list;
+struct NearView {
+    const int* list;     // near chunks of each i-group, row stride nchunks
     const int* count;
-    const int* item_start;  // [ngroups + 2]: first item of each group, the number of items, the
-                            // chunks per item (chosen on the device from the total near-chunk count)
-    int ngroups;
-    int64_t nchunks;        // row stride of `list`
-    float* part;            // [item][field][kGroup]
-    int* nb;                // nullable: per item, each lane's neighbour indices [item][kItemNb][kGroup] ...
-    int* nbcnt;             // ... and their count [item][kGroup] (kItemNb + 1: the list overflowed) ...
-    int* nbover;            // ... and per item whether any lane's list overflowed
-    const float4* box_lo;   // per-chunk bounding boxes (the culled density pass skips, warp by warp, the
-    const float4* box_hi;   // chunks of an item that are farther than h (1 + kMargin) from the warp's box)
-    __device__ __forceinline__ int items() const { return item_start[ngroups]; }
-    __device__ __forceinline__ void item(int w, int& g, int& c0, int& c1) const {
-        int lo = 0, hi = ngroups;  // item_start[lo] <= w < item_start[hi]
-        while (hi - lo > 1) {
-            const int mid = (lo + hi) >> 1;
-            if (item_start[mid] <= w) lo = mid;
-            else hi = mid;
-        }
-        g = lo;
-        const int ic = item_start[ngroups + 1];
-        c0 = (w - item_start[g]) * ic;
-        c1 = min(c0 + ic, count[g]);
+    const int* order;    // i-groups, the longest lists first
+    const float4 *lo, *hi;  // bounds of every 32 particles
+    int64_t nchunks, n, n_pad;
+    float hm2;           // (h (1 + kMargin))^2
+    int* nb;             // neighbour lists [share][cap][n_pad] ...
+    int* nbcnt;          // ... and their lengths [share][n_pad]; more than cap: the list is incomplete
+    int cap;
+    __device__ __forceinline__ int group() const { return order[blockIdx.x / kSubs]; }
+    __device__ __forceinline__ int64_t first(int g) const {
+        return static_cast<int64_t>(g) * kGroup + (blockIdx.x % kSubs) * kSub;
     }
 };
 
-// Two-stage pipeline over a list of chunks, kStageChunks chunks per stage; the stage counter runs on
-// across items so the mbarrier phases stay in step.
-template <int NS>
-struct ItemPipe {
-    static constexpr int SJ = kStageChunks * kChunk;
-    float4* buf;     // shared: [2][NS][SJ]
-    uint64_t* bar;   // shared: [2]
-    const float4* src[NS];
-    int* status;
-    uint32_t kst = 0;
-
-    __device__ __forceinline__ void init() {
-        if (threadIdx.x == 0) {
-            mbar_init(&bar[0], 1);
-            mbar_init(&bar[1], 1);
-            fence_barrier_init();
+// One warp's share of the near chunks of the 32 particles from s0 (group g): the boxes farther than h (1 + kMargin)
+// from the 32 particles' own box are skipped (32 of them per vote), the positions of the others go through the
+// warp's shared buffer `sh`, the next box's load in flight while one is tested, and body(mask, jb) gets each lane's
+// mask of the neighbours (0 < r^2 <= H^2, bit k: particle jb + k, its record in sh[k]). No block barriers.
+template <typename Body>
+__device__ __forceinline__ void near_scan(const NearView& v, const float4* __restrict__ posm, int g, int64_t s0,
+                                          uint32_t span, float4 pi, float4* sh, Body&& body) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const float4 l = v.lo[s0 / kSub], u = v.hi[s0 / kSub];
+    const int nh = v.count[g] * (kChunk / kSub);
+    const int* chunks = v.list + static_cast<int64_t>(g) * v.nchunks;
+    for (int h0 = 0; h0 < nh; h0 += 32 * kShares) {
+        const int h = h0 + kShares * lane + warp;
+        int bx = 0;
+        bool near = false;
+        if (h < nh) {
+            bx = chunks[h / (kChunk / kSub)] * (kChunk / kSub) + h % (kChunk / kSub);
+            const float4 bl = v.lo[bx], bu = v.hi[bx];
+            const float gx = fmaxf(0.0f, fmaxf(bl.x - u.x, l.x - bu.x)), gy = fmaxf(0.0f, fmaxf(bl.y - u.y, l.y - bu.y)),
+                        gz = fmaxf(0.0f, fmaxf(bl.z - u.z, l.z - bu.z));
+            near = !(gx * gx + gy * gy + gz * gz > v.hm2);
         }
-        __syncthreads();
-    }
-    __device__ __forceinline__ void issue(int b, const int* chunks, int first, int nc) {
-        mbar_expect_tx(&bar[b], static_cast<uint32_t>(NS * nc * kChunk * sizeof(float4)));
-        for (int c = 0; c < nc; ++c) {
-            const int64_t ch = chunks[first + c];
-#pragma unroll
-            for (int s = 0; s < NS; ++s)
-                bulk_g2s(buf + (static_cast<int64_t>(b) * NS + s) * SJ + c * kChunk, src[s] + ch * kChunk,
-                         static_cast<uint32_t>(kChunk * sizeof(float4)), &bar[b]);
+        unsigned todo = __ballot_sync(0xffffffffu, near);
+        int jn = 0;
+        float4 qn = make_float4(0, 0, 0, 0);
+        if (todo) {
+            jn = kSub * __shfl_sync(0xffffffffu, bx, __ffs(todo) - 1);
+            qn = posm[jn + lane];
         }
-    }
-    // body(stage, nj) for every stage of the n chunks chunks[0..n); false if a wait gave up
-    template <typename Body>
-    __device__ __forceinline__ bool run(const int* chunks, int n, Body&& body) {
-        const int nst = (n + kStageChunks - 1) / kStageChunks;
-        if (threadIdx.x == 0)
-            for (int st = 0; st < 2 && st < nst; ++st)
-                issue((kst + st) & 1, chunks, st * kStageChunks, min(kStageChunks, n - st * kStageChunks));
-        for (int st = 0; st < nst; ++st) {
-            const int b = kst & 1;
-            const bool ok = mbar_wait_bounded(&bar[b], (kst >> 1) & 1, status);
-            if (__syncthreads_or(!ok)) {
-                if (threadIdx.x == 0 && st + 1 < nst)
-                    mbar_wait_bounded(&bar[(kst + 1) & 1], ((kst + 1) >> 1) & 1, status);
-                __syncthreads();
-                return false;
+        while (todo) {
+            todo &= todo - 1;
+            const int jb = jn;
+            const float4 q0 = qn;
+            if (todo) {
+                jn = kSub * __shfl_sync(0xffffffffu, bx, __ffs(todo) - 1);
+                qn = posm[jn + lane];
             }
-            const int nc = min(kStageChunks, n - st * kStageChunks);
-            body(buf + static_cast<int64_t>(b) * NS * SJ, nc * kChunk);
-            __syncthreads();
-            if (threadIdx.x == 0 && st + 2 < nst)
-                issue(b, chunks, (st + 2) * kStageChunks, min(kStageChunks, n - (st + 2) * kStageChunks));
-            ++kst;
+            __syncwarp();  // the previous box's reads are done
+            sh[lane] = q0;
+            __syncwarp();
+            unsigned m4[4];  // four independent masks: no serial chain over the 32 tests
+#pragma unroll
+            for (int b = 0; b < 4; ++b) {
+                unsigned m = 0;
+#pragma unroll
+                for (int t = 0; t < 8; ++t) {
+                    const float4 q = sh[8 * b + t];
+                    const float dx = q.x - pi.x, dy = q.y - pi.y, dz = q.z - pi.z;
+                    const float r2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
+                    m |= static_cast<unsigned>((__float_as_uint(r2) - 1u) < span) << t;  // 0 < r2 <= H2
+                }
+                m4[b] = m;
+            }
+            body(m4[0] | (m4[1] << 8) | (m4[2] << 16) | (m4[3] << 24), jb);
         }
-        return true;
     }
-};
+}
 
 // shared-memory bytes of a pipeline: 2 stages of NS streams plus the two barriers
 __host__ __device__ inline size_t pipe_smem_bytes(int ns, int jt) {
@@ -254,8 +247,6 @@ struct Launch {
     int grav_sym_G = 0;   // > 0: symmetric gravity kernel over G groups of grav_sym_gs blocks of 1024
     int grav_sym_gs = 0;
     int accum;       // GSPH_ACCUM_*
-    int item_grid;   // persistent grid of the culled SPH kernel (its resident capacity)
-    int density_grid;  // persistent grid of the culled density kernel
 };
 
 // the finish kernels' view of the gravity partials of launch shape L; nseg == 0: no gravity partials
@@ -277,17 +268,14 @@ inline void sym_groups(int64_t nblocks, int target, int& G, int& gs) {
     G = static_cast<int>((nblocks + gs - 1) / gs);
 }
 
-// With `sp`, the culled density pass also stores every lane's neighbour indices per work item
-// (sp->item_nb), which the SPH passes of the same step then use instead of scanning the chunks again.
+// With `sp`, the culled density pass over the near chunks, which also stores every particle's neighbours
+// (sp->nb): the SPH passes of the same step read them instead of searching again.
 cudaError_t launch_density(const DevArrays& a, const DevParams& p, const Launch& L, cudaStream_t s,
                            const KTimer* t = nullptr, const SpatialArrays* sp = nullptr);
-// near-chunk work items of the culled passes (item_start scan); needs launch_chunk_lists first.
-// `target` items in total (plus at most one per group for rounding).
-cudaError_t launch_work_items(const DevArrays& a, const SpatialArrays& sp, int target, cudaStream_t s);
 cudaError_t launch_prepare(const DevArrays& a, const DevParams& p, cudaStream_t s);
-// With `sp`, the SPH terms come from the near-chunk work items; the finish kernel then adds `gnseg`
-// segments of gravity partials (a.gpart, from launch_gravity_partials), after waiting for `join`
-// when it is given (the gravity kernel may run on another stream).
+// With `sp`, the SPH terms come from the near chunks, or (`lists`) from the neighbour lists an earlier pass of the step
+// stored; the finish kernel then adds the gravity sums (a.gfold, from launch_gravity_partials), after waiting for
+// `join` when it is given (the gravity kernel may run on another stream).
 cudaError_t launch_pairs(int pass, const DevArrays& a, const DevParams& p, const Launch& L, cudaStream_t s,
                          const KTimer* t = nullptr, const SpatialArrays* sp = nullptr, int gnseg = 0,
                          cudaEvent_t join = nullptr, bool lists = false);
@@ -298,7 +286,26 @@ cudaError_t launch_gravity(const DevArrays& a, const DevParams& p, const Launch&
 cudaError_t launch_fp32_peak(int sm_count, int iters, float* sink, cudaStream_t s);
 cudaError_t launch_gravity_raw(const float4* posm_padded, float* part, int64_t n_pad, int ipt, int jt, int nseg,
                                float eps2, int* status, cudaStream_t s);
+// the FP64 fold of `S` slots of a.gpart into a.gfold
+cudaError_t launch_gravity_fold(const DevArrays& a, const Launch& L, int S, cudaStream_t s);
 int64_t fp32_peak_flops(int sm_count, int iters);
+
+// ---- derivatives in a fixed order of summation (pairs_fixed.cu) ---------------------------------------
+struct FixedArrays {
+    int* item_start = nullptr;  // [n_pad / kGroup + 2] first work item of each group, number of items, chunks per item
+    float* part = nullptr;      // [items][fields][kGroup] partial sums
+    int* nb = nullptr;          // [items][kItemNb][kGroup] neighbour indices the density pass found
+    int* nbcnt = nullptr;       // [items][kGroup]
+    int* nbover = nullptr;      // [items]
+};
+size_t fixed_items(int64_t n_pad, int sms);
+size_t fixed_part_floats();  // per item
+size_t fixed_list_ints();    // per item
+cudaError_t launch_fixed_gravity(const DevArrays& a, const DevParams& p, const Launch& L, cudaStream_t s);
+// near-chunk lists first; `join` as in launch_pairs
+cudaError_t launch_fixed_sph(const DevArrays& a, const DevParams& p, const Launch& L, const SpatialArrays& sp,
+                             const FixedArrays& fx, int sms, bool grav, cudaEvent_t join, cudaStream_t s, int& launches);
+
 size_t partial_floats(const DevParams& p, const Launch& L, int64_t n_pad);
 size_t gravity_partial_floats(const Launch& L, int64_t n_pad);
 int gravity_blocks_per_sm(int ipt, int threads, int jt, bool comp);

@@ -9,46 +9,51 @@ namespace {
 
 inline unsigned blocks_for(int64_t n, int t) { return static_cast<unsigned>((n + t - 1) / t); }
 
-// one warp per chunk: min/max over its real particles (empty chunk: lo = +inf, hi = -inf)
-__global__ void k_chunk_bounds(DevArrays a, float4* __restrict__ lo, float4* __restrict__ hi, int64_t nchunks) {
-    const int64_t w = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
-    const int lane = threadIdx.x & 31;
-    if (w >= nchunks) return;
-    float mnx = INFINITY, mny = INFINITY, mnz = INFINITY, mxx = -INFINITY, mxy = -INFINITY, mxz = -INFINITY;
-    for (int k = lane; k < kChunk; k += 32) {
-        const int64_t i = w * kChunk + k;
-        if (i < a.n) {
-            const float4 p = a.posm[i];
-            mnx = fminf(mnx, p.x); mny = fminf(mny, p.y); mnz = fminf(mnz, p.z);
-            mxx = fmaxf(mxx, p.x); mxy = fmaxf(mxy, p.y); mxz = fmaxf(mxz, p.z);
-        }
+// one warp per half chunk, two halves per chunk: min/max over the real particles (none: lo = +inf, hi = -inf)
+static_assert(kChunk == 64, "two halves per chunk");
+__global__ void __launch_bounds__(256) k_chunk_bounds(DevArrays a, SpatialArrays s, int64_t nsub) {
+    __shared__ float4 box[8][2];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int64_t w = static_cast<int64_t>(blockIdx.x) * 8 + warp, i = w * 32 + lane;
+    float mn[3] = {INFINITY, INFINITY, INFINITY}, mx[3] = {-INFINITY, -INFINITY, -INFINITY};
+    if (i < a.n) {
+        const float4 p = a.posm[i];
+        mn[0] = mx[0] = p.x; mn[1] = mx[1] = p.y; mn[2] = mx[2] = p.z;
     }
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        mnx = fminf(mnx, __shfl_xor_sync(0xffffffffu, mnx, o));
-        mny = fminf(mny, __shfl_xor_sync(0xffffffffu, mny, o));
-        mnz = fminf(mnz, __shfl_xor_sync(0xffffffffu, mnz, o));
-        mxx = fmaxf(mxx, __shfl_xor_sync(0xffffffffu, mxx, o));
-        mxy = fmaxf(mxy, __shfl_xor_sync(0xffffffffu, mxy, o));
-        mxz = fmaxf(mxz, __shfl_xor_sync(0xffffffffu, mxz, o));
-    }
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            mn[c] = fminf(mn[c], __shfl_xor_sync(0xffffffffu, mn[c], o));
+            mx[c] = fmaxf(mx[c], __shfl_xor_sync(0xffffffffu, mx[c], o));
+        }
     if (lane == 0) {
-        lo[w] = make_float4(mnx, mny, mnz, 0.0f);
-        hi[w] = make_float4(mxx, mxy, mxz, 0.0f);
+        box[warp][0] = make_float4(mn[0], mn[1], mn[2], 0.0f);
+        box[warp][1] = make_float4(mx[0], mx[1], mx[2], 0.0f);
     }
+    __syncthreads();
+    if (lane != 0 || w >= nsub) return;
+    const float4 l = box[warp][0], u = box[warp][1];
+    s.sub_lo[w] = l;
+    s.sub_hi[w] = u;
+    if (warp & 1) return;
+    const float4 m = box[warp + 1][0], v = box[warp + 1][1];
+    s.box_lo[w / 2] = make_float4(fminf(l.x, m.x), fminf(l.y, m.y), fminf(l.z, m.z), 0.0f);
+    s.box_hi[w / 2] = make_float4(fmaxf(u.x, v.x), fmaxf(u.y, v.y), fmaxf(u.z, v.z), 0.0f);
 }
 
 __device__ __forceinline__ float gap(float lo_a, float hi_a, float lo_b, float hi_b) {
     return fmaxf(0.0f, fmaxf(lo_b - hi_a, lo_a - hi_b));
 }
 
-// one block per i-group: the ordered list of chunks within h of the group's box
-constexpr int kListThreads = 256;
-__global__ void __launch_bounds__(kListThreads) k_chunk_lists(const float4* __restrict__ lo,
-                                                              const float4* __restrict__ hi, int* __restrict__ list,
-                                                              int* __restrict__ count, int64_t nchunks, float h2m) {
+// one warp per i-group: the ordered list of chunks within h of the group's box, 128 chunks per round
+__global__ void __launch_bounds__(128) k_chunk_lists(const float4* __restrict__ lo, const float4* __restrict__ hi,
+                                                     int* __restrict__ list, int* __restrict__ count, int64_t ngroups,
+                                                     int64_t nchunks, float h2m) {
     constexpr int per_group = kGroup / kChunk;
-    const int64_t g = blockIdx.x;
+    const int lane = threadIdx.x & 31;
+    const int64_t g = static_cast<int64_t>(blockIdx.x) * 4 + (threadIdx.x >> 5);
+    if (g >= ngroups) return;
     float4 glo = lo[g * per_group], ghi = hi[g * per_group];
 #pragma unroll
     for (int k = 1; k < per_group; ++k) {
@@ -56,37 +61,70 @@ __global__ void __launch_bounds__(kListThreads) k_chunk_lists(const float4* __re
         glo.x = fminf(glo.x, l.x); glo.y = fminf(glo.y, l.y); glo.z = fminf(glo.z, l.z);
         ghi.x = fmaxf(ghi.x, u.x); ghi.y = fmaxf(ghi.y, u.y); ghi.z = fmaxf(ghi.z, u.z);
     }
-    __shared__ int warp_tot[kListThreads / 32];
-    __shared__ int base_sh;
-    if (threadIdx.x == 0) base_sh = 0;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     int* out = list + g * nchunks;
-    for (int64_t r = 0; r < nchunks; r += kListThreads) {
-        const int64_t c = r + threadIdx.x;
-        bool near = false;
-        if (c < nchunks) {
-            const float4 l = lo[c], u = hi[c];
-            const float dx = gap(glo.x, ghi.x, l.x, u.x), dy = gap(glo.y, ghi.y, l.y, u.y),
-                        dz = gap(glo.z, ghi.z, l.z, u.z);
-            near = dx * dx + dy * dy + dz * dz <= h2m;
+    int n = 0;
+    for (int64_t r = 0; r < nchunks; r += 128) {
+        bool near[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const int64_t c = r + 32 * k + lane;
+            near[k] = false;
+            if (c < nchunks) {
+                const float4 l = lo[c], u = hi[c];
+                const float dx = gap(glo.x, ghi.x, l.x, u.x), dy = gap(glo.y, ghi.y, l.y, u.y),
+                            dz = gap(glo.z, ghi.z, l.z, u.z);
+                near[k] = dx * dx + dy * dy + dz * dz <= h2m;
+            }
         }
-        const unsigned ballot = __ballot_sync(0xffffffffu, near);
-        const int rank = __popc(ballot & ((1u << lane) - 1u));
-        __syncthreads();
-        if (lane == 0) warp_tot[warp] = __popc(ballot);
-        __syncthreads();
-        int off = base_sh;
-        for (int w = 0; w < warp; ++w) off += warp_tot[w];
-        if (near) out[off + rank] = static_cast<int>(c);
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            int t = 0;
-            for (int w = 0; w < kListThreads / 32; ++w) t += warp_tot[w];
-            base_sh += t;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const unsigned b = __ballot_sync(0xffffffffu, near[k]);
+            if (near[k]) out[n + __popc(b & ((1u << lane) - 1u))] = static_cast<int>(r + 32 * k + lane);
+            n += __popc(b);
         }
     }
+    if (lane == 0) count[g] = n;
+}
+
+// The groups by falling near-chunk count (to a 256th of the largest), so that the CTAs of long lists start first and
+// the short ones fill the last wave. One block: counting sort. The order within a bucket is not fixed, and need not
+// be: every group's results are its own.
+constexpr int kOrderThreads = 1024, kBuckets = 256;
+__global__ void __launch_bounds__(kOrderThreads) k_group_order(const int* __restrict__ count, int* __restrict__ order,
+                                                               int ngroups) {
+    __shared__ int most, bins[kBuckets], warp_sum[kBuckets / 32];
+    if (threadIdx.x == 0) most = 1;
+    if (threadIdx.x < kBuckets) bins[threadIdx.x] = 0;
     __syncthreads();
-    if (threadIdx.x == 0) count[g] = base_sh;
+    int m = 0;
+    for (int g = threadIdx.x; g < ngroups; g += kOrderThreads) m = max(m, count[g]);
+    atomicMax(&most, m);
+    __syncthreads();
+    const int top = most;
+    auto bucket = [&](int g) {
+        return kBuckets - 1 - static_cast<int>(static_cast<long long>(count[g]) * (kBuckets - 1) / top);
+    };
+    for (int g = threadIdx.x; g < ngroups; g += kOrderThreads) atomicAdd(&bins[bucket(g)], 1);
+    __syncthreads();
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int v = 0, x = 0;
+    if (threadIdx.x < kBuckets) {
+        v = x = bins[threadIdx.x];
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(0xffffffffu, x, o);
+            if (lane >= o) x += y;
+        }
+        if (lane == 31) warp_sum[warp] = x;
+    }
+    __syncthreads();
+    if (threadIdx.x < kBuckets) {
+        int before = x - v;
+        for (int w = 0; w < warp; ++w) before += warp_sum[w];
+        bins[threadIdx.x] = before;
+    }
+    __syncthreads();
+    for (int g = threadIdx.x; g < ngroups; g += kOrderThreads) order[atomicAdd(&bins[bucket(g)], 1)] = g;
 }
 
 // ---- space-filling-curve reorder ----------------------------------------------------------------
@@ -182,16 +220,20 @@ size_t spatial_sort_tmp_bytes(int64_t n_pad) {
 }
 
 cudaError_t launch_chunk_bounds(const DevArrays& a, const SpatialArrays& s, cudaStream_t st) {
-    const int64_t nchunks = a.n_pad / kChunk;
-    k_chunk_bounds<<<blocks_for(nchunks * 32, 256), 256, 0, st>>>(a, s.box_lo, s.box_hi, nchunks);
+    const int64_t nsub = a.n_pad / 32;
+    k_chunk_bounds<<<blocks_for(nsub, 8), 256, 0, st>>>(a, s, nsub);
     return cudaGetLastError();
 }
 
 cudaError_t launch_chunk_lists(const DevArrays& a, const SpatialArrays& s, float h, cudaStream_t st) {
-    const int64_t nchunks = a.n_pad / kChunk;
+    const int64_t nchunks = a.n_pad / kChunk, ngroups = a.n_pad / kGroup;
     const float hm = h * (1.0f + kMargin);
-    k_chunk_lists<<<static_cast<unsigned>(a.n_pad / kGroup), kListThreads, 0, st>>>(s.box_lo, s.box_hi, s.list,
-                                                                                     s.count, nchunks, hm * hm);
+    k_chunk_lists<<<blocks_for(ngroups, 4), 128, 0, st>>>(s.box_lo, s.box_hi, s.list, s.count, ngroups, nchunks, hm * hm);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_group_order(const DevArrays& a, const SpatialArrays& s, cudaStream_t st) {
+    k_group_order<<<1, kOrderThreads, 0, st>>>(s.count, s.group_order, static_cast<int>(a.n_pad / kGroup));
     return cudaGetLastError();
 }
 

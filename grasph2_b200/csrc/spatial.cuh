@@ -22,12 +22,12 @@ struct SpatialArrays {
     float4* box_hi;
     int* list;         // [n_pad / kGroup][n_pad / kChunk] near chunks of each i-group
     int* count;        // [n_pad / kGroup]
-    int* item_start;   // [n_pad / kGroup + 2] first work item of each group, number of items, chunks per item
-    int item_target;   // items aimed at per pass (the item buffer holds item_target + groups items)
-    float* item_part;  // [items][fields][kGroup] partial sums of the culled passes
-    int* item_nb;      // [items][kItemNb][kGroup] neighbour indices found by the culled density pass
-    int* item_nbcnt;   // [items][kGroup]
-    int* item_nbover;  // [items] nonzero: some lane's list of the item overflowed
+    float4* sub_lo;    // [n_pad / 32] bounds of every 32 particles
+    float4* sub_hi;
+    int* group_order;  // [n_pad / kGroup] i-groups by falling near-chunk count
+    int* nb;           // [kShares][nb_cap][n_pad] neighbour indices, and their number [kShares][n_pad]
+    int* nbcnt;
+    int nb_cap;
     int* ext_of_int;   // [n_pad] caller's index of the particle stored at each internal slot
     int* order;        // [n_pad] scratch: sort values / gather map
     unsigned* keys;    // [2 n_pad] sort keys (in, out)
@@ -78,8 +78,10 @@ __device__ __forceinline__ unsigned hilbert3(unsigned x0, unsigned x1, unsigned 
 }
 
 size_t spatial_sort_tmp_bytes(int64_t n_pad);
+// bounds of the chunks (and of their halves), the near chunks of every i-group, the order the groups are taken in
 cudaError_t launch_chunk_bounds(const DevArrays& a, const SpatialArrays& s, cudaStream_t st);
 cudaError_t launch_chunk_lists(const DevArrays& a, const SpatialArrays& s, float h, cudaStream_t st);
+cudaError_t launch_group_order(const DevArrays& a, const SpatialArrays& s, cudaStream_t st);
 // Sort the n real particles of `a` along the Hilbert curve and permute every per-particle array in place.
 cudaError_t reorder_particles(const DevArrays& a, const SpatialArrays& s, cudaStream_t st, int& launches);
 // The first half of it: order_out[k] = slot of the k-th particle along the curve (padding last, in place).

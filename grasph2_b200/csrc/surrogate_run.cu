@@ -30,6 +30,7 @@
 #include "../../include/grasph2_b200.h"
 
 void set_global_error(const std::string& msg);  // capi.cu
+int gsph_ctx_proposal_derivatives(gsph_ctx* c, void* stream);  // capi.cu
 
 namespace {
 constexpr int kIn = GSPH_MLP_IN, kOut = GSPH_MLP_OUT;
@@ -218,7 +219,7 @@ extern "C" {
 
 int gsph_surrogate_propose(gsph_surrogate* s, gsph_ctx* ctx, int32_t use_net, void* stream) {
     if (!s || !ctx) return sfail(s, GSPH_E_INVALID, "NULL argument");
-    const int rc = gsph_compute_derivatives(ctx, stream);
+    const int rc = use_net ? gsph_ctx_proposal_derivatives(ctx, stream) : gsph_compute_derivatives(ctx, stream);
     if (rc != GSPH_OK) return ctx_fail(s, ctx, rc, "propose: derivatives");
     return propose_from_derivatives(s, ctx, use_net, stream);
 }
@@ -233,15 +234,19 @@ int gsph_surrogate_judge(gsph_surrogate* s, gsph_ctx* ctx, int32_t use_net, doub
         if (rc != GSPH_OK) return ctx_fail(s, ctx, rc, "judge: energy");
         e_ref = d.e_kin + d.e_grav + d.e_int + d.e_shear;
     }
-    // the start state is saved with its derivatives, which the proposal and the plain integrator's first
-    // step share: the plain path is one integrate and K - 1 full steps (the same arithmetic as K steps)
-    if ((rc = gsph_compute_derivatives(ctx, stream)) != GSPH_OK) return ctx_fail(s, ctx, rc, "judge: derivatives");
+    // Without the network, the start state is saved with its derivatives, which the proposal and the plain
+    // integrator's first step share: the plain path is one integrate and K - 1 full steps (the same arithmetic as K
+    // steps). A network proposal evaluates its own, in its fixed order of summation.
+    if (!use_net && (rc = gsph_compute_derivatives(ctx, stream)) != GSPH_OK) return ctx_fail(s, ctx, rc, "judge: derivatives");
     if ((rc = gsph_snapshot(ctx, 1, 0, stream)) != GSPH_OK) return ctx_fail(s, ctx, rc, "judge: snapshot");
+    if (use_net && (rc = gsph_ctx_proposal_derivatives(ctx, stream)) != GSPH_OK)
+        return ctx_fail(s, ctx, rc, "judge: derivatives");
     if ((rc = propose_from_derivatives(s, ctx, use_net, stream)) != GSPH_OK) return rc;
     if ((rc = gsph_snapshot(ctx, 2, 0, stream)) != GSPH_OK) return ctx_fail(s, ctx, rc, "judge: snapshot");
     if ((rc = gsph_snapshot(ctx, 1, 1, stream)) != GSPH_OK) return ctx_fail(s, ctx, rc, "judge: restore");
-    if ((rc = gsph_integrate(ctx, 1, stream)) != GSPH_OK) return ctx_fail(s, ctx, rc, "judge: plain steps");
-    if ((rc = gsph_step(ctx, s->K - 1, stream)) != GSPH_OK) return ctx_fail(s, ctx, rc, "judge: plain steps");
+    if (!use_net && (rc = gsph_integrate(ctx, 1, stream)) != GSPH_OK) return ctx_fail(s, ctx, rc, "judge: plain steps");
+    if ((rc = gsph_step(ctx, use_net ? s->K : s->K - 1, stream)) != GSPH_OK)
+        return ctx_fail(s, ctx, rc, "judge: plain steps");
     double c[8];
     if ((rc = gsph_state_compare_parts(ctx, 2, 1, c, stream)) != GSPH_OK) return ctx_fail(s, ctx, rc, "judge: compare");
     out->pos_error = c[2] > 0.0 ? std::sqrt(c[1] / c[2]) : HUGE_VAL;

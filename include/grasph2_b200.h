@@ -277,11 +277,12 @@ int gsph_diagnostics_fast(gsph_ctx* ctx, double half_kick, gsph_diag* out, void*
 
 /* Autotuner (no counterpart in the reference): times candidate launch shapes on the context's current
  * state and keeps the fastest, `reps` timed launches each (median): the gravity kernel's i-blocking,
- * j-tile and j-split; the culled SPH passes' work-item count, or the all-pairs SPH tile shape. Results
+ * j-tile and j-split; the all-pairs SPH tile shape (the culled SPH passes have one shape). Results
  * change only by summation order. The next gsph_step re-captures its graph. */
 int gsph_autotune(gsph_ctx* ctx, int32_t reps, void* stream);
 typedef struct gsph_launch_shape {
     int32_t cull, grav_ipt, grav_jt, grav_nseg, grav_x2, sph_threads, sph_jt, sph_nseg, items;
+    /* items: warps that share 32 particles in the culled SPH passes (0: all pairs) */
     int32_t grav_sym_groups;  /* > 0: the symmetric gravity kernel over this many particle groups */
     int32_t reserved[6];
 } gsph_launch_shape;
