@@ -43,9 +43,8 @@ struct gsph_ctx {
     double* staging64 = nullptr;  // 9 * n doubles
     double* diag_out = nullptr;   // device, 12 doubles
     size_t part_cap = 0, gpart_cap = 0;  // floats allocated for a.part, a.gpart
-    // derivatives of network proposals (pairs_fixed.cu): launch shapes as created, buffers of the first proposal
-    Launch fixed_L;
-    FixedArrays fixed;
+    Launch fixed_L;            // gravity in the fixed order of summation (gravity_fixed.cu): its shape, as created ...
+    bool fixed_order = false;  // ... for every derivative, not only those of network proposals
     std::vector<void*> snap[4];    // gsph_snapshot slots: saved copies of the state arrays (allocated on first save)
     cudaStream_t capture_stream = nullptr;
     cudaGraph_t graph = nullptr;
@@ -234,7 +233,12 @@ const KTimer* slot_timer(gsph_ctx* c, int slot) {
     return &c->timers[slot];
 }
 
-int derivatives(gsph_ctx* c, cudaStream_t s) {
+// the gravity partials of shape L and their fold (culled path); proposal: in the fixed order of summation
+cudaError_t gravity_partials(gsph_ctx* c, const Launch& L, bool fixed, cudaStream_t s, const KTimer* t = nullptr) {
+    return fixed ? launch_fixed_gravity(c->a, c->dp, L, s, t) : launch_gravity_partials(c->a, c->dp, L, s, t);
+}
+
+int derivatives(gsph_ctx* c, cudaStream_t s, bool proposal = false) {
     const DevParams& p = c->dp;
     cudaError_t e;
     if (c->fp64) {
@@ -255,7 +259,9 @@ int derivatives(gsph_ctx* c, cudaStream_t s) {
         if (grav_kernel) {  // fork: all-pairs gravity on the side stream, joined before the finish
             e = cudaEventRecord(c->ev_fork, s);
             if (e == cudaSuccess) e = cudaStreamWaitEvent(c->side, c->ev_fork, 0);
-            if (e == cudaSuccess) e = launch_gravity_partials(c->a, p, c->L, c->side, slot_timer(c, GSPH_KSLOT_GRAVITY));
+            const bool fixed = proposal || c->fixed_order;
+            if (e == cudaSuccess)
+                e = gravity_partials(c, proposal ? c->fixed_L : c->L, fixed, c->side, slot_timer(c, GSPH_KSLOT_GRAVITY));
             if (e == cudaSuccess) e = cudaEventRecord(c->ev_join, c->side);
             if (e != cudaSuccess) return cuda_fail(c, e, "gravity pass");
             join = c->ev_join;
@@ -264,11 +270,11 @@ int derivatives(gsph_ctx* c, cudaStream_t s) {
         if (sp) {  // bounds of every chunk at the current positions, each group's near chunks, the groups' order
             e = launch_chunk_bounds(c->a, c->sp, s);
             if (e == cudaSuccess) e = launch_chunk_lists(c->a, c->sp, p.H, s);
-            if (e == cudaSuccess) e = launch_group_order(c->a, c->sp, s);
+            if (e == cudaSuccess) e = launch_group_order(c->a, c->sp, kItemsPerSM * c->sm_count, s);
             if (e != cudaSuccess) return cuda_fail(c, e, "chunk lists");
             c->launches += 3;
         }
-        if (!has(p, GSPH_INTEGRATE_DENSITY)) {
+        if (sp || !has(p, GSPH_INTEGRATE_DENSITY)) {
             e = launch_density(c->a, p, c->L, s, slot_timer(c, GSPH_KSLOT_DENSITY), sp);
             if (e != cudaSuccess) return cuda_fail(c, e, "density pass");
             c->launches += 2;
@@ -279,16 +285,15 @@ int derivatives(gsph_ctx* c, cudaStream_t s) {
         }
         const bool vgrad = has(p, GSPH_SOLIDS) || has(p, GSPH_INTEGRATE_DENSITY) || has(p, GSPH_BALSARA_SWITCH);
         const int gnseg = grav_kernel ? c->L.grav_nseg : 0;
-        const bool lists = sp && !has(p, GSPH_INTEGRATE_DENSITY);  // the density pass stored neighbour lists
         if (vgrad && has(p, GSPH_BALSARA_SWITCH)) {
-            e = launch_pairs(PASS_VGRAD, c->a, p, c->L, s, slot_timer(c, GSPH_KSLOT_VGRAD), sp, 0, nullptr, lists);
+            e = launch_pairs(PASS_VGRAD, c->a, p, c->L, s, slot_timer(c, GSPH_KSLOT_VGRAD), sp, 0, nullptr);
             if (e != cudaSuccess) return cuda_fail(c, e, "velocity-gradient pass");
-            e = launch_pairs(PASS_ACC, c->a, p, c->L, s, slot_timer(c, GSPH_KSLOT_PAIRS), sp, gnseg, join, lists);
+            e = launch_pairs(PASS_ACC, c->a, p, c->L, s, slot_timer(c, GSPH_KSLOT_PAIRS), sp, gnseg, join);
             if (e != cudaSuccess) return cuda_fail(c, e, "acceleration pass");
             c->launches += 4;
         } else {
             e = launch_pairs(vgrad ? PASS_FUSED : PASS_ACC, c->a, p, c->L, s, slot_timer(c, GSPH_KSLOT_PAIRS), sp, gnseg,
-                             join, lists);
+                             join);
             if (e != cudaSuccess) return cuda_fail(c, e, "pair pass");
             c->launches += 2;
         }
@@ -311,51 +316,6 @@ int grow(gsph_ctx* c, float** p, size_t& cap, size_t floats) {
     cudaFree(*p);
     *p = q;
     cap = floats;
-    return GSPH_OK;
-}
-
-// derivatives in the fixed order of summation (a culled context in single precision)
-int fixed_derivatives(gsph_ctx* c, cudaStream_t s) {
-    const DevParams& p = c->dp;
-    const int64_t np = c->a.n_pad;
-    cudaError_t e = cudaSuccess;
-    FixedArrays& fx = c->fixed;
-    if (!fx.item_start) {
-        // one allocation, the largest alignment first
-        const size_t items = fixed_items(np, c->sm_count);
-        const size_t parts = items * fixed_part_floats(), lists = items * fixed_list_ints();
-        int* base = static_cast<int*>(dalloc(c, (parts + lists + items * (kGroup + 1) + np / kGroup + 2) * sizeof(int), e));
-        if (e != cudaSuccess) return fail(c, GSPH_E_NOMEM, std::string("proposal buffers: ") + cudaGetErrorString(e));
-        fx.part = reinterpret_cast<float*>(base);
-        fx.nb = base + parts;
-        fx.nbcnt = fx.nb + lists;
-        fx.nbover = fx.nbcnt + items * kGroup;
-        fx.item_start = fx.nbover + items;
-    }
-    const bool grav = has(p, GSPH_SELF_GRAVITY);
-    cudaEvent_t join = nullptr;
-    if (grav) {
-        const size_t need = gravity_partial_floats(c->fixed_L, np);
-        if (need > c->gpart_cap) {
-            drop_graph(c);  // it holds the old pointer
-            const int rc = grow(c, &c->a.gpart, c->gpart_cap, need);
-            if (rc != GSPH_OK) return rc;
-        }
-        e = cudaEventRecord(c->ev_fork, s);
-        if (e == cudaSuccess) e = cudaStreamWaitEvent(c->side, c->ev_fork, 0);
-        if (e == cudaSuccess) e = launch_fixed_gravity(c->a, p, c->fixed_L, c->side);
-        if (e == cudaSuccess) e = cudaEventRecord(c->ev_join, c->side);
-        if (e != cudaSuccess) return cuda_fail(c, e, "gravity pass");
-        join = c->ev_join;
-        c->launches += 2;
-    }
-    e = launch_chunk_bounds(c->a, c->sp, s);
-    if (e == cudaSuccess) e = launch_chunk_lists(c->a, c->sp, p.H, s);
-    if (e != cudaSuccess) return cuda_fail(c, e, "chunk lists");
-    int launches = 2;
-    e = launch_fixed_sph(c->a, p, c->fixed_L, c->sp, fx, c->sm_count, grav, join, s, launches);
-    c->launches += launches;
-    if (e != cudaSuccess) return cuda_fail(c, e, "SPH passes");
     return GSPH_OK;
 }
 
@@ -410,8 +370,7 @@ bool gsph_ctx_state(gsph_ctx* c, DevArrays* a, const int** ext) {
 
 // the derivatives of a network proposal (surrogate_run.cu)
 int gsph_ctx_proposal_derivatives(gsph_ctx* c, void* stream) {
-    if (c->fp64 || !c->L.cull) return gsph_compute_derivatives(c, stream);  // the features will refuse the context
-    return fixed_derivatives(c, as_stream(stream));
+    return derivatives(c, as_stream(stream), true);
 }
 
 extern "C" {
@@ -563,15 +522,20 @@ int gsph_create(const gsph_params* p, const gsph_options* opt, int64_t n, gsph_c
         const int slots = c->sm_count * gravity_blocks_per_sm(L.grav_ipt, L.grav_threads, L.grav_jt, comp);
         L.grav_nseg = o.j_split ? std::min(o.j_split, gcap)
                                 : pick_split(n_pad / (int64_t(L.grav_threads) * L.grav_ipt), slots, gcap);
-        // the symmetric form: enough tasks (G(G+1)/2 with G up to 64) to fill the GPU twice
+        // the symmetric form, in every kernel of its own (SPH contexts without culling sum gravity in their pair pass);
+        // a caller who sets the one-sided kernel's shape keeps it below 24 blocks of 1024
         const int64_t nblocks = n_pad / 1024;
+        const bool own_kernel = (!(p->flags & GSPH_SPH) || L.cull) && !c->fp64;
+        const bool shaped = o.i_per_thread || o.j_tile || o.j_split;
         const bool sym = o.gravity_form == GSPH_GRAVITY_SYMMETRIC ||
-                         (o.gravity_form == GSPH_GRAVITY_AUTO && !o.scalar_fp32 && nblocks >= 24);
-        const bool own_kernel = !(p->flags & GSPH_SPH) || L.cull;  // gravity has a kernel of its own
-        if (sym && own_kernel && !c->fp64) sym_groups(nblocks, o.gravity_groups ? o.gravity_groups : 64, L.grav_sym_G, L.grav_sym_gs);
+                         (o.gravity_form == GSPH_GRAVITY_AUTO && !o.scalar_fp32 && (nblocks >= 24 || !shaped));
+        c->fixed_L = L;
+        if (own_kernel && sym && (o.gravity_form == GSPH_GRAVITY_SYMMETRIC || nblocks >= 24))
+            sym_groups(nblocks, o.gravity_groups ? o.gravity_groups : 64, c->fixed_L.grav_sym_G, c->fixed_L.grav_sym_gs);
+        c->fixed_order = L.cull && (p->flags & GSPH_INTEGRATE_DENSITY);
+        if (c->fixed_order) L = c->fixed_L;
+        else if (own_kernel && sym) sym_shape(n_pad, c->sm_count, o.gravity_groups, -1, L);
     }
-
-    c->fixed_L = L;
 
     cudaError_t ae = cudaSuccess;
     auto F4 = [&](void) { return static_cast<float4*>(dalloc(c, n_pad * sizeof(float4), ae)); };
@@ -582,21 +546,21 @@ int gsph_create(const gsph_params* p, const gsph_options* opt, int64_t n, gsph_c
     a.rhodot = static_cast<float*>(dalloc(c, n_pad * sizeof(float), ae));
     a.balsara = static_cast<float*>(dalloc(c, n_pad * sizeof(float), ae));
     c->part_cap = partial_floats(c->dp, L, n_pad);
-    c->gpart_cap = L.cull ? gravity_partial_floats(L, n_pad) : 4;
+    c->gpart_cap = L.cull ? std::max(gravity_partial_floats(L, n_pad), gravity_partial_floats(c->fixed_L, n_pad)) : 4;
     a.part = static_cast<float*>(dalloc(c, c->part_cap * sizeof(float), ae));
     a.gpart = static_cast<float*>(dalloc(c, c->gpart_cap * sizeof(float), ae));
     a.gfold = static_cast<double*>(dalloc(c, (L.cull ? 3 * n_pad : 4) * sizeof(double), ae));
     if (L.cull) {
         SpatialArrays& sp = c->sp;
         const int64_t nchunks = n_pad / kChunk, ngroups = n_pad / kGroup;
-        sp.group_order = static_cast<int*>(dalloc(c, ngroups * sizeof(int), ae));
+        sp.group_order = static_cast<int*>(dalloc(c, (ngroups + 1) * sizeof(int), ae));
         sp.sub_lo = static_cast<float4*>(dalloc(c, n_pad / kSub * sizeof(float4), ae));
         sp.sub_hi = static_cast<float4*>(dalloc(c, n_pad / kSub * sizeof(float4), ae));
-        // 256 neighbours per particle in equal shares; 96 in very large contexts, whose chunk lists already take
-        // n^2 / 2048 bytes (a longer list costs its warp a second search, not correctness)
-        sp.nb_cap = n_pad <= (int64_t(1) << 22) ? 64 : 24;
-        sp.nb = static_cast<int*>(dalloc(c, static_cast<size_t>(kShares) * sp.nb_cap * n_pad * sizeof(int), ae));
-        sp.nbcnt = static_cast<int*>(dalloc(c, static_cast<size_t>(kShares) * n_pad * sizeof(int), ae));
+        // 256 neighbours per particle; 96 in very large contexts, whose chunk lists already take n^2 / 2048 bytes (a
+        // longer list costs its warp a second search, not correctness)
+        sp.nb_cap = n_pad <= (int64_t(1) << 22) ? 256 : 96;
+        sp.nb = static_cast<int*>(dalloc(c, static_cast<size_t>(sp.nb_cap) * n_pad * sizeof(int), ae));
+        sp.nbcnt = static_cast<int*>(dalloc(c, static_cast<size_t>(n_pad) * sizeof(int), ae));
         a.jrec = static_cast<float4*>(dalloc(c, 4 * n_pad * sizeof(float4), ae));
         if (ae == cudaSuccess) ae = cudaMemset(a.jrec, 0, 4 * n_pad * sizeof(float4));
         sp.box_lo = static_cast<float4*>(dalloc(c, nchunks * sizeof(float4), ae));
@@ -1145,8 +1109,7 @@ int gsph_autotune(gsph_ctx* c, int32_t reps, void* stream) {
                     if (rc != GSPH_OK) break;
                     float ms = 0.0f;
                     rc = time_ms(c, s, reps, [&]() {
-                        const cudaError_t e = L.cull ? launch_gravity_partials(c->a, c->dp, t, s)
-                                                     : launch_gravity(c->a, c->dp, t, s);
+                        const cudaError_t e = L.cull ? gravity_partials(c, t, c->fixed_order, s) : launch_gravity(c->a, c->dp, t, s);
                         return e == cudaSuccess ? GSPH_OK : cuda_fail(c, e, "autotune gravity");
                     }, ms);
                     if (rc != GSPH_OK) break;
@@ -1157,26 +1120,32 @@ int gsph_autotune(gsph_ctx* c, int32_t reps, void* stream) {
                 }
                 if (rc != GSPH_OK) break;
             }
-        // the symmetric form (unless one-sided was asked for) with 32, 64 and 128 groups at most
+        // the symmetric form (unless one-sided was asked for): its block shapes with 64 and 128 groups at most (in the
+        // fixed order: blocks of 1024 in 32, 64 and 128 groups)
+        const int form = c->opt.gravity_form, asked = c->opt.gravity_groups;
         const int64_t nblocks = np / 1024;
-        const int form = c->opt.gravity_form;
-        if (rc == GSPH_OK && form != GSPH_GRAVITY_ONE_SIDED && (form == GSPH_GRAVITY_SYMMETRIC || nblocks >= 8)) {
+        if (rc == GSPH_OK && form != GSPH_GRAVITY_ONE_SIDED && (!c->fixed_order || nblocks >= 8)) {
             int last_G = -1;
-            for (int target : {32, 64, 128}) {
+            for (int cand = 0; cand < (c->fixed_order ? 3 : 2 * kSymShapes); ++cand) {
                 Launch t = best;
-                sym_groups(nblocks, c->opt.gravity_groups ? c->opt.gravity_groups : target, t.grav_sym_G, t.grav_sym_gs);
-                if (t.grav_sym_G == last_G) continue;
-                last_G = t.grav_sym_G;
+                if (c->fixed_order) {
+                    sym_groups(nblocks, asked ? asked : 32 << cand, t.grav_sym_G, t.grav_sym_gs);
+                    if (t.grav_sym_G == last_G) continue;
+                    last_G = t.grav_sym_G;
+                } else {
+                    sym_shape(np, c->sm_count, asked ? asked : (cand % 2 ? 128 : 64), cand / 2, t);
+                    if (cand % 2 && (asked || t.grav_sym_G <= 64)) continue;  // the same as the one before
+                }
                 if (L.cull) rc = grow(c, &c->a.gpart, c->gpart_cap, gravity_partial_floats(t, np));
                 else rc = grow(c, &c->a.part, c->part_cap, partial_floats(c->dp, t, np));
                 if (rc != GSPH_OK) break;
                 float ms = 0.0f;
                 rc = time_ms(c, s, reps, [&]() {
-                    const cudaError_t e = L.cull ? launch_gravity_partials(c->a, c->dp, t, s) : launch_gravity(c->a, c->dp, t, s);
+                    const cudaError_t e = L.cull ? gravity_partials(c, t, c->fixed_order, s) : launch_gravity(c->a, c->dp, t, s);
                     return e == cudaSuccess ? GSPH_OK : cuda_fail(c, e, "autotune gravity");
                 }, ms);
                 if (rc != GSPH_OK) break;
-                if (ms < best_ms || form == GSPH_GRAVITY_SYMMETRIC && best.grav_sym_G == 0) {
+                if (ms < best_ms || (form == GSPH_GRAVITY_SYMMETRIC && best.grav_sym_G == 0)) {
                     best_ms = ms;
                     best = t;
                 }
@@ -1188,6 +1157,7 @@ int gsph_autotune(gsph_ctx* c, int32_t reps, void* stream) {
             L.grav_nseg = best.grav_nseg;
             L.grav_sym_G = best.grav_sym_G;
             L.grav_sym_gs = best.grav_sym_gs;
+            L.grav_sym_shape = best.grav_sym_shape;
         }
     }
     // 2. the all-pairs SPH passes' tile shape (the culled kernels have one shape)
@@ -1247,7 +1217,7 @@ int gsph_launch_shape_get(gsph_ctx* c, gsph_launch_shape* out) {
     out->sph_threads = c->L.threads;
     out->sph_jt = c->L.jt;
     out->sph_nseg = c->L.nseg;
-    out->items = c->L.cull ? kShares : 0;
+    out->items = c->L.cull ? kItemsPerSM * c->sm_count : 0;
     return GSPH_OK;
 }
 

@@ -14,6 +14,7 @@
 // partial into a (sum, error) pair with a two-sum, and combines the j-segments in FP64.
 #include <algorithm>
 #include <cfloat>
+#include <type_traits>
 
 #include "f32x2.cuh"
 #include "pairs.cuh"
@@ -84,52 +85,150 @@ __global__ void __launch_bounds__(256) k_density(const float4* __restrict__ posm
     if (COMP) part[(seg * 2 + 1) * n_pad + i] = rho_c;
 }
 
-// Culled density sum of 32 particles per CTA, with the epilogue; every share's neighbours go to its list.
-template <bool COMP>
-__global__ void __launch_bounds__(kSub * kShares) k_density_near(const float4* __restrict__ posm, float4* __restrict__ velrho,
-                                                                 DevParams p, NearView v) {
-    __shared__ float4 sh[kShares][kSub];
-    __shared__ float red[COMP ? 2 : 1][kShares][kSub];
+// The neighbour search of 32 particles by four warps, with the density sum and its epilogue (DENS) or without (the
+// density is integrated). The group's near chunks come in batches of up to 64, cut at a stage. A: the batch's boxes are
+// tested against the 32 particles' own, 32 per warp. B: warp w takes the stages w, w + 4, ...; the positions of a near
+// box go through the warp's shared buffer, every lane gets the mask of its neighbours (0 < r^2 <= H^2) and adds
+// their terms to the stage's sum. C: with the counts of all stages known, each warp writes its stages' neighbours to
+// their places in the particle's list, and warp 0 adds the stage sums in their order.
+//
+// Bound: instruction issue (8 per test, about 2 % of the tests are neighbours). One warp alone took 154 us for 65,536
+// particles of the impact and 29 us for the 4,096 of the fluid, whose 128 warps leave the chip idle.
+constexpr int kNearWarps = 4, kBatch = 64;
+template <bool DENS, bool COMP>
+__global__ void __launch_bounds__(kSub * kNearWarps) k_near(const float4* __restrict__ posm, float4* __restrict__ velrho,
+                                                            DevParams p, NearView v) {
+    __shared__ float4 sh[kNearWarps][kSub];
+    __shared__ unsigned mk[kBatch * kHalves][kSub];   // neighbour masks of the batch's boxes
+    __shared__ float ts[DENS ? kBatch : 1][kSub];     // stage sums
+    __shared__ unsigned short cs[kBatch][kSub];       // neighbours per stage
+    __shared__ int bxs[kBatch * kHalves];
+    __shared__ unsigned nm[kBatch * kHalves / 32];    // which boxes are near
+    static_assert(kBatch * kHalves == 32 * kNearWarps, "one vote per warp and batch");
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int g = v.group();
+    const int g = v.group(), ic = v.per_item(), nc = v.count[g];
     const int64_t s0 = v.first(g), i = s0 + lane;
     if (s0 >= v.n) return;
     const float4 pi = posm[i];
-    float rho_s = 0.0f, rho_c = 0.0f;
-    int cnt = 0;
-    int* lst = v.nb + static_cast<int64_t>(warp) * v.cap * v.n_pad + i;
-    near_scan(v, posm, g, s0, __float_as_uint(p.H2), pi, sh[warp], [&](unsigned m, int jb) {
-        float t = 0.0f;
-        while (m) {
-            const int k = __ffs(m) - 1;
-            m &= m - 1;
-            const float4 q = sh[warp][k];
-            const float dx = q.x - pi.x, dy = q.y - pi.y, dz = q.z - pi.z;
-            const float r2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
-            t = fmaf(q.w, w_poly(r2 * rsqrtf(r2) * p.inv_h), t);
-            if (cnt < v.cap) lst[static_cast<int64_t>(cnt) * v.n_pad] = jb + k;
-            ++cnt;
+    const float4 l = v.lo[s0 / kSub], u = v.hi[s0 / kSub];
+    const int* chunks = v.list + static_cast<int64_t>(g) * v.nchunks;
+    const uint32_t span = __float_as_uint(p.H2);
+    // stages of [c0, c1), item ends at `ie`: f(q, first chunk, end chunk, item ends with it)
+    auto stages = [&](int c0, int c1, int ie, auto&& f) {
+        for (int q = 0, b = c0; b < c1; ++q) {
+            const int e = min(b + kStageChunks, min(ie, c1));
+            f(q, b - c0, e - c0, e == ie);
+            if (e == ie) ie += ic;
+            b = e;
         }
-        if (COMP) fold(rho_s, rho_c, t);
-        else rho_s += t;
-    });
-    v.nbcnt[static_cast<int64_t>(warp) * v.n_pad + i] = cnt;
-    red[0][warp][lane] = rho_s;
-    if (COMP) red[COMP ? 1 : 0][warp][lane] = rho_c;
-    __syncthreads();
-    if (warp != 0 || i >= v.n) return;
-    float rho;
-    if (COMP) {
-        double s = 0.0;
+        return ie;
+    };
+    int cnt = 0;                                 // neighbours so far
+    bool seen = false;                           // ... any of them of the current item
+    float rs = 0.0f, rc = 0.0f, tot = 0.0f;      // sums of the item (and its error term) and of the items before it
+    double tot2 = 0.0;
+    auto end_item = [&]() {
+        if (COMP) tot2 += static_cast<double>(rs) + static_cast<double>(rc);
+        else tot += rs;
+        rs = rc = 0.0f;
+    };
+    int ie = ic;  // end of the item that holds c0
+    for (int c0 = 0; c0 < nc;) {
+        int c1 = min(nc, c0 + kBatch);
+        if (c1 < nc) c1 -= c1 % ic % kStageChunks;  // whole stages
+        {  // A
+            const int h = threadIdx.x;
+            int bx = 0;
+            bool near = false;
+            if (h < (c1 - c0) * kHalves) {
+                bx = chunks[c0 + h / kHalves] * kHalves + h % kHalves;
+                const float4 bl = v.lo[bx], bu = v.hi[bx];
+                const float gx = fmaxf(0.0f, fmaxf(bl.x - u.x, l.x - bu.x)), gy = fmaxf(0.0f, fmaxf(bl.y - u.y, l.y - bu.y)),
+                            gz = fmaxf(0.0f, fmaxf(bl.z - u.z, l.z - bu.z));
+                near = !(gx * gx + gy * gy + gz * gz > v.hm2);
+            }
+            bxs[h] = bx;
+            const unsigned b = __ballot_sync(0xffffffffu, near);
+            if (lane == 0) nm[warp] = b;
+        }
+        __syncthreads();
+        // B
+        stages(c0, c1, ie, [&](int q, int b, int e, bool) {
+            if (q % kNearWarps != warp) return;
+            float t = 0.0f;
+            int n = 0;
+            for (int h = b * kHalves; h < e * kHalves; ++h) {
+                if (!(nm[h >> 5] >> (h & 31) & 1u)) continue;
+                const float4 q0 = posm[bxs[h] * kSub + lane];
+                __syncwarp();  // the previous box's reads are done
+                sh[warp][lane] = q0;
+                __syncwarp();
+                unsigned m4[4];  // four independent masks: no serial chain over the 32 tests
 #pragma unroll
-        for (int w = 0; w < kShares; ++w) s += static_cast<double>(red[0][w][lane]) + static_cast<double>(red[COMP ? 1 : 0][w][lane]);
-        rho = static_cast<float>(s * static_cast<double>(p.w_pref));
-    } else {
-        float s = 0.0f;
+                for (int w = 0; w < 4; ++w) {
+                    unsigned m = 0;
 #pragma unroll
-        for (int w = 0; w < kShares; ++w) s += red[0][w][lane];
-        rho = s * p.w_pref;
+                    for (int k = 0; k < 8; ++k) {
+                        const float4 r = sh[warp][8 * w + k];
+                        const float dx = r.x - pi.x, dy = r.y - pi.y, dz = r.z - pi.z;
+                        const float r2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
+                        m |= static_cast<unsigned>((__float_as_uint(r2) - 1u) < span) << k;  // 0 < r2 <= H2
+                    }
+                    m4[w] = m;
+                }
+                unsigned m = m4[0] | (m4[1] << 8) | (m4[2] << 16) | (m4[3] << 24);
+                mk[h][lane] = m;
+                n += __popc(m);
+                if (DENS) {
+                    while (m) {
+                        const float4 r = sh[warp][__ffs(m) - 1];
+                        m &= m - 1;
+                        const float dx = r.x - pi.x, dy = r.y - pi.y, dz = r.z - pi.z;
+                        const float r2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
+                        const float d = r2 * rsqrtf(r2);
+                        t = fmaf(r.w, w_poly(d * p.inv_h), t);
+                    }
+                }
+            }
+            cs[q][lane] = static_cast<unsigned short>(n);
+            if (DENS) ts[DENS ? q : 0][lane] = t;
+        });
+        __syncthreads();
+        // C
+        ie = stages(c0, c1, ie, [&](int q, int b, int e, bool item_ends) {
+            const int n = cs[q][lane];
+            if (q % kNearWarps == warp && __any_sync(0xffffffffu, n > 0)) {
+                int at = cnt;
+                bool first = !seen;
+                for (int h = b * kHalves; h < e * kHalves; ++h) {
+                    if (!(nm[h >> 5] >> (h & 31) & 1u)) continue;
+                    unsigned m = mk[h][lane];
+                    const int jb = bxs[h] * kSub;
+                    while (m) {
+                        const int j = jb + __ffs(m) - 1;
+                        m &= m - 1;
+                        if (at < v.cap) v.nb[static_cast<int64_t>(at) * v.n_pad + i] = j | (first ? kItemMark : 0);
+                        first = false;
+                        ++at;
+                    }
+                }
+            }
+            cnt += n;
+            seen = !item_ends && (seen || n > 0);
+            if (DENS && warp == 0) {
+                if (COMP) fold(rs, rc, ts[DENS ? q : 0][lane]);
+                else rs += ts[DENS ? q : 0][lane];
+                if (item_ends) end_item();
+            }
+        });
+        __syncthreads();  // before the next batch
+        c0 = c1;
     }
+    if (warp != 0) return;
+    v.nbcnt[i] = cnt;
+    if (!DENS || i >= v.n) return;
+    end_item();
+    float rho = COMP ? static_cast<float>(tot2 * static_cast<double>(p.w_pref)) : tot * p.w_pref;
     if (has(p, GSPH_DEAL_WITH_NO_PARTNERS) && rho < 0.001f) rho = p.rho0 * 0.01f;  // computeDerivatives.h:85-88
     reinterpret_cast<float*>(velrho + i)[3] = rho;
 }
@@ -276,61 +375,58 @@ __global__ void __launch_bounds__(256) k_pairs(DevArrays a, DevParams p, int jt,
                                S, C, maxv);
 }
 
-// Culled SPH pass (no gravity) of 32 particles per CTA. LISTS: an earlier pass of the step stored the neighbour lists;
-// otherwise every share first searches its boxes and stores them (for itself and a later pass). The terms then run
-// over the lists, one packed 64-byte record per neighbour, the next record and the index after it in flight; a warp
-// with an incomplete list (more than v.cap in one share) goes back to the boxes. The shares of a field are added in
-// order (compensated: in FP64; a share holds a few to tens of terms, so it carries no compensation term itself).
+// Culled SPH pass (no gravity) over the neighbour lists, one warp per 32 particles: one packed 64-byte record per
+// neighbour, the next record and the index after it in flight. A warp with an incomplete list goes back to the boxes.
 //
-// Bound: instruction issue and the L2 latency of the gathers. All neighbours of a particle in four lists instead of one
-// list per work item of a few chunks: a warp runs as long as its longest list, and the longer lists differ less
-// (18.8 of 32 lanes were active). No partial sums per item: the finish kernel reads one value per field.
-template <int PASS, bool SOLIDS, bool LISTS, bool COMP>
-__global__ void __launch_bounds__(kSub * kShares, 5) k_pairs_near(DevArrays a, DevParams p, NearView v) {
+// Bound: instruction issue and the L2 latency of the gathers. A lane goes through all its neighbours and adds an item's
+// sums when its next neighbour belongs to another one, so a warp runs as long as its longest list (a warp per
+// item of a few chunks kept 18.8 of 32 lanes active and left the items' partial sums to the finish kernel).
+template <int PASS, bool SOLIDS, bool COMP>
+__global__ void __launch_bounds__(kSub) k_pairs_near(DevArrays a, DevParams p, NearView v) {
     constexpr uint32_t MASK = field_mask<PASS, false, SOLIDS>();
-    constexpr int K = popc_c(MASK);
     constexpr bool DO_A = PASS != PASS_VGRAD;
-    __shared__ float4 sh[kShares][kSub];
-    __shared__ float red[kShares][K][kSub];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int g = v.group();
-    const int64_t s0 = v.first(g), i = s0 + lane;
+    using Sum = typename std::conditional<COMP, double, float>::type;
+    __shared__ float4 sh[kSub];
+    const int g = v.group(), ic = v.per_item();
+    const int64_t s0 = v.first(g), i = s0 + threadIdx.x;
     if (s0 >= v.n) return;
     const ISph I = load_isph<PASS, SOLIDS>(a, p, i, 0.0f);
-    int* lst = v.nb + static_cast<int64_t>(warp) * v.cap * v.n_pad + i;
-    int cnt = 0;
-    if (LISTS) {
-        cnt = v.nbcnt[static_cast<int64_t>(warp) * v.n_pad + i];
-    } else {
-        near_scan(v, a.posm, g, s0, I.span, I.pi, sh[warp], [&](unsigned m, int jb) {
-            while (m) {
-                const int k = __ffs(m) - 1;
-                m &= m - 1;
-                if (cnt < v.cap) lst[static_cast<int64_t>(cnt) * v.n_pad] = jb + k;
-                ++cnt;
-            }
-        });
-        v.nbcnt[static_cast<int64_t>(warp) * v.n_pad + i] = cnt;
-    }
-    PairAcc T;
+    const int* lst = v.nb + i;
+    const int cnt = v.nbcnt[i];
+    PairAcc T;                // the sums of the item
+    Sum S[F_COUNT];           // ... and of the items before it
 #pragma unroll
-    for (int f = 0; f < F_COUNT; ++f) T.f[f] = 0.0f;
+    for (int f = 0; f < F_COUNT; ++f) {
+        T.f[f] = 0.0f;
+        S[f] = 0;
+    }
     float maxv = 0.0f;
     const float4 zero = make_float4(0, 0, 0, 0);
+    auto end_item = [&]() {
+#pragma unroll
+        for (int f = 0; f < F_COUNT; ++f)
+            if (((MASK >> f) & 1u) && f != F_MAXV) {
+                S[f] += static_cast<Sum>(T.f[f]);
+                T.f[f] = 0.0f;
+            }
+    };
     auto term = [&](float4 q, float4 vj, float4 ja, float4 jb) {
         const float dx = q.x - I.pi.x, dy = q.y - I.pi.y, dz = q.z - I.pi.z;
-        sph_neighbour<PASS, SOLIDS>(T, maxv, I, q.w, dx, dy, dz, fmaf(dz, dz, fmaf(dy, dy, dx * dx)), vj, ja, jb, p);
+        const float r2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
+        sph_neighbour<PASS, SOLIDS>(T, maxv, I, q.w, dx, dy, dz, r2, vj, ja, jb, p);
     };
     if (!__any_sync(0xffffffffu, cnt > v.cap)) {
-        int jn = cnt > 0 ? lst[0] : 0;
-        const float4* r0 = a.jrec + 4 * static_cast<int64_t>(jn);
+        int e = cnt > 0 ? lst[0] : 0;            // the entry of neighbour k
+        int en = cnt > 1 ? lst[v.n_pad] : 0;     // ... and of k + 1
+        const float4* r0 = a.jrec + 4 * static_cast<int64_t>(e & ~kItemMark);
         float4 qn = __ldg(r0), vn = __ldg(r0 + 1);
         float4 an = DO_A ? __ldg(r0 + 2) : zero, bn = DO_A ? __ldg(r0 + 3) : zero;
-        jn = cnt > 1 ? lst[v.n_pad] : 0;  // the index of neighbour k + 1
         for (int k = 0; k < cnt; ++k) {
             const float4 q = qn, vj = vn, ja = an, jb = bn;
+            const bool first = e < 0;
+            e = en;
             if (k + 1 < cnt) {
-                const float4* r = a.jrec + 4 * static_cast<int64_t>(jn);
+                const float4* r = a.jrec + 4 * static_cast<int64_t>(e & ~kItemMark);
                 qn = __ldg(r);
                 vn = __ldg(r + 1);
                 if (DO_A) {
@@ -338,39 +434,31 @@ __global__ void __launch_bounds__(kSub * kShares, 5) k_pairs_near(DevArrays a, D
                     bn = __ldg(r + 3);
                 }
             }
-            if (k + 2 < cnt) jn = lst[static_cast<int64_t>(k + 2) * v.n_pad];
+            if (k + 2 < cnt) en = lst[static_cast<int64_t>(k + 2) * v.n_pad];
+            if (first) end_item();
             term(q, vj, ja, jb);
         }
     } else {
-        near_scan(v, a.posm, g, s0, I.span, I.pi, sh[warp], [&](unsigned m, int jb) {
+        int item = 0, next = ic, last = -1;
+        near_scan(v, a.posm, g, s0, I.span, I.pi, sh, [&](unsigned m, int jb, int c) {
+            while (c >= next) {
+                ++item;
+                next += ic;
+            }
             while (m) {
                 const float4* r = a.jrec + 4 * static_cast<int64_t>(jb + __ffs(m) - 1);
                 m &= m - 1;
+                if (item != last) end_item();
+                last = item;
                 term(r[0], r[1], DO_A ? r[2] : zero, DO_A ? r[3] : zero);
             }
         });
     }
+    end_item();
 #pragma unroll
     for (int f = 0; f < F_COUNT; ++f)
-        if ((MASK >> f) & 1u) red[warp][field_offset<MASK>(f)][lane] = f == F_MAXV ? maxv : T.f[f];
-    __syncthreads();
-    for (int o = warp; o < K; o += kShares) {  // each warp adds the shares of its fields
-        const bool mx = ((MASK >> F_MAXV) & 1u) && o == field_offset<MASK>(F_MAXV);
-        float s = red[0][o][lane];
-        if (mx) {
-#pragma unroll
-            for (int w = 1; w < kShares; ++w) s = fmaxf(s, red[w][o][lane]);
-        } else if (COMP) {
-            double d = s;
-#pragma unroll
-            for (int w = 1; w < kShares; ++w) d += static_cast<double>(red[w][o][lane]);
-            s = static_cast<float>(d);
-        } else {
-#pragma unroll
-            for (int w = 1; w < kShares; ++w) s += red[w][o][lane];
-        }
-        a.part[static_cast<int64_t>(o) * a.n_pad + i] = s;
-    }
+        if ((MASK >> f) & 1u)
+            a.part[static_cast<int64_t>(field_offset<MASK>(f)) * a.n_pad + i] = f == F_MAXV ? maxv : static_cast<float>(S[f]);
 }
 
 // Sum the slots of one field in a fixed order: FP32 in plain mode, FP64 of (sum + error) in
@@ -555,27 +643,39 @@ __global__ void __launch_bounds__(128) k_gravity_x2(const float4* __restrict__ p
 // ================================================================================================
 // symmetric all-pairs gravity (Newton's third law): every unordered pair evaluated once
 // ================================================================================================
-// Particles form blocks of kSymB = 128 threads x 8; blocks form G groups of `gs` consecutive blocks.
-// CTA t is the task (ga, gb), ga <= gb (the G(G-1)/2 pairs of distinct groups first, then the G
-// diagonal ones): for every row block a of group ga it sweeps the column blocks of group gb (those
-// after a when ga == gb) in j-tiles of kSymJT through shared memory. One 1/r^3 serves both particles
-// of a pair: the row particle's sum stays in registers (f32x2, two row particles per instruction),
-// accumulated per j-tile and then added to the running sum (plain: a sum of 256-term sums, whose
-// rounding error grows with the tile count instead of the pair count; compensated: a two-sum fold whose
-// error terms live in shared memory); the column particle's contribution is summed over the CTA's 1024 row particles -- in the thread, then
-// across the warp by rotation (each lane takes the 32 columns of a block in turn and hands each column's
-// running sum on to its neighbour), then over the four warps in shared memory -- and added to its slot
-// in the partials (plain, or two-sum when compensated). The pairs inside a block (the diagonal tile) run one-sided. Each particle has G + 1
-// slots, each written by one task (its row sums from tasks (g, gb), its column sums from tasks (ga, g),
-// g its group); the finish kernels add a particle's slots in a fixed order, so results do not depend on
-// scheduling. FMA-pipe work per pair interaction: 8 + ~0.4 operations
-// against the one-sided kernel's 12.
-constexpr int kSymT = 128, kSymI = 8, kSymB = kSymT * kSymI, kSymJT = 256;
-static_assert(kSymB % kSymJT == 0 && kSymJT % kSymT == 0 && kSymJT % 32 == 0, "symmetric gravity tiles");
-// CTAs per SM the register budget is set for. Four (128 registers, no spills with the rotating column
-// sums): Plummer N = 2^20, 128 groups, 340.5 ms plain and 340.5 ms compensated, against 338.7 / 350.6 ms
-// for a warp butterfly over batches of 8 columns at three CTAs per SM; five spill and run slower (359.6 ms)
-constexpr int kSymCtas = 4;
+// Particles form blocks of B = R T (R rows per thread, T threads); blocks form G groups of `gs` consecutive blocks.
+// CTA t is the task (ga, gb), ga <= gb (the G(G-1)/2 pairs of distinct groups first, then the G diagonal ones): for
+// every row block a of group ga it sweeps the column blocks of group gb (those after a when ga == gb) in j-tiles
+// through shared memory. One 1/r^3 serves both particles of a pair. The pairs inside a block run one-sided. Each
+// particle has G + 1 slots, each written by one task (its row sums from tasks (g, gb), its column sums from tasks
+// (ga, g), g its group); the fold adds a particle's slots in FP64 in a fixed order, so results do not depend on
+// scheduling.
+//
+// An f32x2 instruction takes one row against two columns, 32 apart: rows are duplicated once per block, columns are
+// staged as (x x' y y') (z z' m m') so that a 16-byte load brings two register pairs, and a column sum is an f32x2
+// accumulator of its own. In round r of a block of 64 columns lane l takes the columns (l + r) % 32 and (l + r) % 32 + 32,
+// adds its rows' shares and hands the sums to lane l - 1; after 32 rounds lane l holds the warp's sums of columns l and
+// l + 32. (Two rows per instruction, as gravity_fixed.cu, costs a register move per operand for the duplicated column,
+// zeroed accumulators and a horizontal add per column: 113 instructions per 512 interactions instead of 84.)
+// Row sums are accumulated per j-tile and then added to running sums in shared memory (plain: one add; compensated: a
+// two-sum fold whose error terms are there too).
+//
+// Where every row of the block has one mass and every column of the tile has one (the particle sources give equal
+// masses; it is looked up in each tile, in the barrier that publishes it), the masses leave the pair loop: 14 FP32
+// operations per unordered pair instead of 16.
+//
+// Bound: the register file. An f32x2 multiply-add of three different register pairs reads six registers and runs at
+// 0.60 of the FMA rate, multiplies and adds (four) at 0.96; six of a pair's operations are such multiply-adds, which
+// predicts 0.77. Keeping each pair that shares both factors together lets the operand cache serve the second: 0.81.
+// Measured (N = 262,144, 128 groups, one B200): row-packed 22.3 ms, column-packed 18.6 ms, equal masses 15.8 ms.
+template <int R_, int T_, int CTAS_>
+struct SymShape {
+    static constexpr int R = R_, T = T_, B = R_ * T_, CTAS = CTAS_;
+    static constexpr int JT = B < 256 ? B : 256;  // columns per tile
+    static constexpr int PF = JT / T_;            // records a thread stages
+    static constexpr int W = T_ / 32;
+    static_assert(JT % 64 == 0 && B % JT == 0 && JT % T_ == 0, "symmetric gravity tiles");
+};
 
 __host__ __device__ __forceinline__ void sym_task(int t, int G, int& ga, int& gb) {
     const int noff = G * (G - 1) / 2;
@@ -592,155 +692,194 @@ __host__ __device__ __forceinline__ void sym_task(int t, int G, int& ga, int& gb
     gb = r + 1 + rem;
 }
 
-template <int GRAV, bool COMP>
-__global__ void __launch_bounds__(kSymT, kSymCtas) k_gravity_sym(const float4* __restrict__ posm, float* __restrict__ part,
-                                                       int64_t n_pad, int G, int gs, float eps2) {
-    constexpr int P = kSymI / 2;
+// T += d s, c += d s for the three components: each pair of multiply-adds with common factors back to back
+__device__ __forceinline__ void add_both(float2& tx, float2& ty, float2& tz, float2& cx, float2& cy, float2& cz, float2 dx,
+                                         float2 dy, float2 dz, float2 s) {
+    uint64_t t0 = u64_of(tx), t1 = u64_of(ty), t2 = u64_of(tz), c0 = u64_of(cx), c1 = u64_of(cy), c2 = u64_of(cz);
+    asm("fma.rn.f32x2 %0, %6, %9, %0;\n fma.rn.f32x2 %3, %6, %9, %3;\n"
+        " fma.rn.f32x2 %1, %7, %9, %1;\n fma.rn.f32x2 %4, %7, %9, %4;\n"
+        " fma.rn.f32x2 %2, %8, %9, %2;\n fma.rn.f32x2 %5, %8, %9, %5;\n"
+        : "+l"(t0), "+l"(t1), "+l"(t2), "+l"(c0), "+l"(c1), "+l"(c2)
+        : "l"(u64_of(dx)), "l"(u64_of(dy)), "l"(u64_of(dz)), "l"(u64_of(s)));
+    tx = f2_of(t0); ty = f2_of(t1); tz = f2_of(t2);
+    cx = f2_of(c0); cy = f2_of(c1); cz = f2_of(c2);
+}
+
+template <typename S, int GRAV, bool COMP>
+__global__ void __launch_bounds__(S::T, S::CTAS) k_gravity_sym(const float4* __restrict__ posm, float* __restrict__ part,
+                                                               int64_t n_pad, int G, int gs, float eps2) {
+    constexpr int R = S::R, T = S::T, B = S::B, JT = S::JT, PF = S::PF, W = S::W;
     constexpr int K = COMP ? 6 : 3;
-    __shared__ float4 J[kSymJT];
-    __shared__ float js[kSymT / 32][kSymJT][3];
-    // the row particles' running sums (and, compensated, their rounding-error terms) stay in shared
-    // memory, touched once per j-tile; the pair loop keeps only the tile's partials in registers
-    __shared__ float2 rsh[3 * P][kSymT];
-    __shared__ float2 csh[COMP ? 3 * P : 1][kSymT];
+    __shared__ float4 XY[JT / 2], ZM[JT / 2];
+    __shared__ float js[W][3][JT];
+    __shared__ float rsh[3 * R][T];             // the row particles' running sums ...
+    __shared__ float csh[COMP ? 3 * R : 1][T];  // ... and, compensated, their rounding errors
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     int ga, gb;
     sym_task(static_cast<int>(blockIdx.x), G, ga, gb);
-    const int nb = static_cast<int>(n_pad / kSymB);
+    const int nb = static_cast<int>(n_pad / B);
     const int ra0 = ga * gs, ra1 = min(nb, ra0 + gs);
     const int cg0 = gb * gs, cg1 = min(nb, cg0 + gs);
     const bool diag = ga == gb;
-    // partials: G + 1 slots per particle, stored [slot][component][n_pad] so that a warp's 32 consecutive
-    // particles write (and the fold kernel reads) 128 contiguous bytes; a particle of group g holds its row
-    // sums from tasks (g, gb), gb = g .. G-1, in slots 0 .. G-1-g and its column sums from tasks (ga, g),
-    // ga = 0 .. g, in slots G-g .. G, each slot written by exactly one task
+    // slots [slot][component][n_pad]: a particle of group g holds its row sums from tasks (g, gb), gb = g .. G-1, in
+    // slots 0 .. G-1-g and its column sums from tasks (ga, g), ga = 0 .. g, in slots G-g .. G
     const int s_row = gb - ga, s_col = G - gb + ga;
     auto slot = [&](int64_t particle, int sl, int c) { return part + (static_cast<int64_t>(sl) * K + c) * n_pad + particle; };
     if (diag)  // the group's first block is never a column here: its column slot is zero
-        for (int e = tid; e < kSymB; e += kSymT)
-            for (int c = 0; c < K; ++c) *slot(static_cast<int64_t>(ra0) * kSymB + e, s_col, c) = 0.0f;
+        for (int e = tid; e < B; e += T)
+            for (int c = 0; c < K; ++c) *slot(static_cast<int64_t>(ra0) * B + e, s_col, c) = 0.0f;
     const float2 E2 = make_float2(eps2, eps2);
+    const float2 zero2 = make_float2(0.0f, 0.0f);
 
     for (int a = ra0; a < ra1; ++a) {
-        const int64_t base = static_cast<int64_t>(a) * kSymB + tid;
-        float2 X[P], Y[P], Z[P], MI[P];
+        const int64_t base = static_cast<int64_t>(a) * B + tid;
+        float2 X[R], Y[R], Z[R], M[R];  // negated: a difference is an addition, a column's share a product
+        const float mr = posm[static_cast<int64_t>(a) * B].w;
+        bool same = true;
 #pragma unroll
-        for (int k = 0; k < P; ++k) {
-            const float4 u = posm[base + static_cast<int64_t>(2 * k) * kSymT];
-            const float4 w = posm[base + static_cast<int64_t>(2 * k + 1) * kSymT];
-            X[k] = make_float2(u.x, w.x); Y[k] = make_float2(u.y, w.y); Z[k] = make_float2(u.z, w.z);
-            MI[k] = make_float2(-u.w, -w.w);
-            rsh[k][tid] = rsh[P + k][tid] = rsh[2 * P + k][tid] = make_float2(0.0f, 0.0f);
-            if (COMP) csh[k][tid] = csh[P + k][tid] = csh[2 * P + k][tid] = make_float2(0.0f, 0.0f);
+        for (int k = 0; k < R; ++k) {
+            const float4 u = posm[base + static_cast<int64_t>(k) * T];
+            X[k] = make_float2(-u.x, -u.x); Y[k] = make_float2(-u.y, -u.y); Z[k] = make_float2(-u.z, -u.z);
+            M[k] = make_float2(-u.w, -u.w);
+            same = same && u.w == mr;
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                rsh[c * R + k][tid] = 0.0f;
+                if (COMP) csh[COMP ? c * R + k : 0][tid] = 0.0f;
+            }
         }
+        const bool rows_equal = __syncthreads_and(same);
         // tiles: the block's own (one-sided) when diagonal, then the columns
-        const int64_t d0 = static_cast<int64_t>(a) * kSymB;
-        const int nd = diag ? kSymB / kSymJT : 0;
-        const int64_t c0 = static_cast<int64_t>(diag ? a + 1 : cg0) * kSymB, c1 = static_cast<int64_t>(cg1) * kSymB;
-        const int nc = c1 > c0 ? static_cast<int>((c1 - c0) / kSymJT) : 0;
-        const int total = nd + nc;
-        const bool first = a == ra0;
-        auto src = [&](int k) { return k < nd ? d0 + static_cast<int64_t>(k) * kSymJT : c0 + static_cast<int64_t>(k - nd) * kSymJT; };
-        constexpr int kPf = kSymJT / kSymT;  // j-records each thread stages per tile
-        float4 pf[kPf];
+        const int64_t d0 = static_cast<int64_t>(a) * B;
+        const int nd = diag ? B / JT : 0;
+        const int64_t c0 = static_cast<int64_t>(diag ? a + 1 : cg0) * B, c1 = static_cast<int64_t>(cg1) * B;
+        const int total = nd + (c1 > c0 ? static_cast<int>((c1 - c0) / JT) : 0);
+        auto src = [&](int k) { return k < nd ? d0 + static_cast<int64_t>(k) * JT : c0 + static_cast<int64_t>(k - nd) * JT; };
+        float4 pf[PF];
+        float mn = 0.0f;  // the mass of the next tile's first column
 #pragma unroll
-        for (int h = 0; h < kPf; ++h) pf[h] = make_float4(0, 0, 0, 0);
+        for (int h = 0; h < PF; ++h) pf[h] = make_float4(0, 0, 0, 0);
         if (total > 0) {
+            mn = posm[src(0)].w;
 #pragma unroll
-            for (int h = 0; h < kPf; ++h) pf[h] = posm[src(0) + h * kSymT + tid];
+            for (int h = 0; h < PF; ++h) pf[h] = posm[src(0) + h * T + tid];
         }
         for (int k = 0; k < total; ++k) {
-            __syncthreads();  // the previous tile's reads of J and js are done
+            __syncthreads();  // the previous tile's reads of XY, ZM and js are done
+            const float mc = mn;
+            bool same_c = true;
 #pragma unroll
-            for (int h = 0; h < kPf; ++h) J[tid + h * kSymT] = pf[h];
-            __syncthreads();
-            if (k + 1 < total) {
-#pragma unroll
-                for (int h = 0; h < kPf; ++h) pf[h] = posm[src(k + 1) + h * kSymT + tid];
+            for (int h = 0; h < PF; ++h) {
+                const int j = tid + h * T, half = (j >> 5) & 1, q = (j >> 6) * 32 + (j & 31);
+                float* xy = reinterpret_cast<float*>(&XY[q]);
+                float* zm = reinterpret_cast<float*>(&ZM[q]);
+                xy[half] = pf[h].x; xy[2 + half] = pf[h].y;
+                zm[half] = pf[h].z; zm[2 + half] = pf[h].w;
+                same_c = same_c && pf[h].w == mc;
             }
-            float2 TX[P], TY[P], TZ[P];
+            const bool equal = __syncthreads_and(same_c) && rows_equal;
+            if (k + 1 < total) {
+                mn = posm[src(k + 1)].w;
 #pragma unroll
-            for (int q = 0; q < P; ++q) TX[q] = TY[q] = TZ[q] = make_float2(0.0f, 0.0f);
-            if (k < nd) {  // one-sided, as k_gravity_x2
-#pragma unroll 4
-                for (int j = 0; j < kSymJT; ++j) {
-                    const float4 q = J[j];
-                    const float2 qx = make_float2(q.x, q.x), qy = make_float2(q.y, q.y), qz = make_float2(q.z, q.z),
-                                 qm = make_float2(q.w, q.w);
+                for (int h = 0; h < PF; ++h) pf[h] = posm[src(k + 1) + h * T + tid];
+            }
+            float2 TX[R], TY[R], TZ[R];
 #pragma unroll
-                    for (int m = 0; m < P; ++m) {
-                        const float2 dx = sub2(qx, X[m]), dy = sub2(qy, Y[m]), dz = sub2(qz, Z[m]);
-                        const float2 r2 = fma2(dz, dz, fma2(dy, dy, fma2(dx, dx, E2)));
-                        float2 inv = make_float2(rsqrtf(r2.x), rsqrtf(r2.y));
-                        if (GRAV == 2) inv = make_float2(fminf(inv.x, 1e12f), fminf(inv.y, 1e12f));
-                        const float2 sj = mul2(qm, mul2(mul2(inv, inv), inv));
+            for (int q = 0; q < R; ++q) TX[q] = TY[q] = TZ[q] = zero2;
+            // one column pair against row m: the separations and 1/r^3
+            auto pair = [&](int m, float4 xy, float4 zm, float2& dx, float2& dy, float2& dz) {
+                dx = add2(make_float2(xy.x, xy.y), X[m]);
+                dy = add2(make_float2(xy.z, xy.w), Y[m]);
+                dz = add2(make_float2(zm.x, zm.y), Z[m]);
+                const float2 r2 = fma2(dz, dz, fma2(dy, dy, fma2(dx, dx, E2)));
+                float2 inv = make_float2(rsqrtf(r2.x), rsqrtf(r2.y));
+                if (GRAV == 2) inv = make_float2(fminf(inv.x, 1e12f), fminf(inv.y, 1e12f));
+                return mul2(mul2(inv, inv), inv);
+            };
+            auto columns = [&](auto eq) {
+                constexpr bool EQ = decltype(eq)::value;
+                const int next = (lane + 1) & 31;
+#pragma unroll 1
+                for (int j0 = 0; j0 < JT / 2; j0 += 32) {
+                    float2 cx = zero2, cy = zero2, cz = zero2;
+#pragma unroll 2
+                    for (int r = 0; r < 32; ++r) {
+                        const int j = j0 + ((lane + r) & 31);
+                        const float4 xy = XY[j], zm = ZM[j];
+#pragma unroll
+                        for (int m = 0; m < R; ++m) {
+                            float2 dx, dy, dz;
+                            const float2 i3 = pair(m, xy, zm, dx, dy, dz);
+                            if (EQ) {
+                                add_both(TX[m], TY[m], TZ[m], cx, cy, cz, dx, dy, dz, i3);
+                            } else {
+                                const float2 sj = mul2(make_float2(zm.z, zm.w), i3), si = mul2(M[m], i3);
+                                TX[m] = fma2(dx, sj, TX[m]); TY[m] = fma2(dy, sj, TY[m]); TZ[m] = fma2(dz, sj, TZ[m]);
+                                cx = fma2(dx, si, cx); cy = fma2(dy, si, cy); cz = fma2(dz, si, cz);
+                            }
+                        }
+                        cx.x = __shfl_sync(0xffffffffu, cx.x, next); cx.y = __shfl_sync(0xffffffffu, cx.y, next);
+                        cy.x = __shfl_sync(0xffffffffu, cy.x, next); cy.y = __shfl_sync(0xffffffffu, cy.y, next);
+                        cz.x = __shfl_sync(0xffffffffu, cz.x, next); cz.y = __shfl_sync(0xffffffffu, cz.y, next);
+                    }
+                    const int j = 2 * j0 + lane;
+                    js[warp][0][j] = cx.x; js[warp][0][j + 32] = cx.y;
+                    js[warp][1][j] = cy.x; js[warp][1][j + 32] = cy.y;
+                    js[warp][2][j] = cz.x; js[warp][2][j + 32] = cz.y;
+                }
+            };
+            if (k < nd) {  // one-sided
+#pragma unroll 2
+                for (int j = 0; j < JT / 2; ++j) {
+                    const float4 xy = XY[j], zm = ZM[j];
+#pragma unroll
+                    for (int m = 0; m < R; ++m) {
+                        float2 dx, dy, dz;
+                        const float2 sj = mul2(make_float2(zm.z, zm.w), pair(m, xy, zm, dx, dy, dz));
                         TX[m] = fma2(dx, sj, TX[m]); TY[m] = fma2(dy, sj, TY[m]); TZ[m] = fma2(dz, sj, TZ[m]);
                     }
                 }
+            } else if (equal) {
+                columns(std::true_type{});
             } else {
-                // column sums by rotation: in round r of a block of 32 columns, lane l pairs its rows
-                // with column (l + r) % 32, adds its share to that column's running sum and hands the sum
-                // to lane l - 1, which takes the column in round r + 1; after 32 rounds lane l holds the
-                // warp's sum for column l (no butterfly, no selects, 3 shuffles per column)
-                const int next = (lane + 1) & 31;
-#pragma unroll 1
-                for (int j0 = 0; j0 < kSymJT; j0 += 32) {
-                    float cx = 0.0f, cy = 0.0f, cz = 0.0f;
-#pragma unroll 2
-                    for (int r = 0; r < 32; ++r) {
-                        const float4 q = J[j0 + ((lane + r) & 31)];
-                        const float2 qx = make_float2(q.x, q.x), qy = make_float2(q.y, q.y),
-                                     qz = make_float2(q.z, q.z), qm = make_float2(q.w, q.w);
-                        float2 tx = make_float2(0.0f, 0.0f), ty = tx, tz = tx;
-#pragma unroll
-                        for (int m = 0; m < P; ++m) {
-                            const float2 dx = sub2(qx, X[m]), dy = sub2(qy, Y[m]), dz = sub2(qz, Z[m]);
-                            const float2 r2 = fma2(dz, dz, fma2(dy, dy, fma2(dx, dx, E2)));
-                            float2 inv = make_float2(rsqrtf(r2.x), rsqrtf(r2.y));
-                            if (GRAV == 2) inv = make_float2(fminf(inv.x, 1e12f), fminf(inv.y, 1e12f));
-                            const float2 i3 = mul2(mul2(inv, inv), inv);
-                            const float2 sj = mul2(qm, i3), si = mul2(MI[m], i3);
-                            TX[m] = fma2(dx, sj, TX[m]); TY[m] = fma2(dy, sj, TY[m]); TZ[m] = fma2(dz, sj, TZ[m]);
-                            tx = fma2(dx, si, tx); ty = fma2(dy, si, ty); tz = fma2(dz, si, tz);
-                        }
-                        cx = __shfl_sync(0xffffffffu, cx + (tx.x + tx.y), next);
-                        cy = __shfl_sync(0xffffffffu, cy + (ty.x + ty.y), next);
-                        cz = __shfl_sync(0xffffffffu, cz + (tz.x + tz.y), next);
-                    }
-                    js[warp][j0 + lane][0] = cx;
-                    js[warp][j0 + lane][1] = cy;
-                    js[warp][j0 + lane][2] = cz;
-                }
+                columns(std::false_type{});
             }
-            // the tile's row partials into the running sums: a two-sum fold (compensated), or one add
-            // (plain: a sum of 256-term tile sums, not one running sum over the whole column group)
-#pragma unroll
-            for (int m = 0; m < P; ++m) {
-                float2 ax = rsh[m][tid], ay = rsh[P + m][tid], az = rsh[2 * P + m][tid];
+            // the tile's row partials into the running sums: a two-sum fold (compensated), or one add (plain: a sum
+            // of tile sums, not one running sum over the whole column group)
+            const float wr = k >= nd && equal ? mc : 1.0f;
+            auto row_add = [&](int o, float2 t) {
+                float x = rsh[o][tid];
                 if (COMP) {
-                    float2 cx = csh[m][tid], cy = csh[P + m][tid], cz = csh[2 * P + m][tid];
-                    fold(ax.x, cx.x, TX[m].x); fold(ax.y, cx.y, TX[m].y);
-                    fold(ay.x, cy.x, TY[m].x); fold(ay.y, cy.y, TY[m].y);
-                    fold(az.x, cz.x, TZ[m].x); fold(az.y, cz.y, TZ[m].y);
-                    csh[m][tid] = cx; csh[P + m][tid] = cy; csh[2 * P + m][tid] = cz;
+                    float e = csh[COMP ? o : 0][tid];
+                    fold(x, e, wr * (t.x + t.y));
+                    csh[COMP ? o : 0][tid] = e;
                 } else {
-                    ax = add2(ax, TX[m]); ay = add2(ay, TY[m]); az = add2(az, TZ[m]);
+                    x = fmaf(wr, t.x + t.y, x);
                 }
-                rsh[m][tid] = ax; rsh[P + m][tid] = ay; rsh[2 * P + m][tid] = az;
+                rsh[o][tid] = x;
+            };
+#pragma unroll
+            for (int m = 0; m < R; ++m) {
+                row_add(m, TX[m]);
+                row_add(R + m, TY[m]);
+                row_add(2 * R + m, TZ[m]);
             }
             if (k >= nd) {  // this tile's column sums over the CTA's row block, into the column slot
                 __syncthreads();
-                const int64_t jb = c0 + static_cast<int64_t>(k - nd) * kSymJT;
+                const float wc = equal ? -mr : 1.0f;
+                const int64_t jb = c0 + static_cast<int64_t>(k - nd) * JT;
 #pragma unroll
-                for (int h = 0; h < kSymJT / kSymT; ++h) {
-                    const int j = tid + h * kSymT;
+                for (int h = 0; h < PF; ++h) {
+                    const int j = tid + h * T;
 #pragma unroll
                     for (int c = 0; c < 3; ++c) {
-                        const float v = (js[0][j][c] + js[1][j][c]) + (js[2][j][c] + js[3][j][c]);
+                        float v = js[0][c][j] + js[1][c][j];
+                        if constexpr (W == 4) v += js[2][c][j] + js[3][c][j];
+                        v *= wc;
                         float* dst = slot(jb + j, s_col, c);
                         if (COMP) {
                             float* cdst = slot(jb + j, s_col, 3 + c);
-                            if (first) {
+                            if (a == ra0) {
                                 *dst = v;
                                 *cdst = 0.0f;
                             } else {
@@ -750,30 +889,31 @@ __global__ void __launch_bounds__(kSymT, kSymCtas) k_gravity_sym(const float4* _
                                 *cdst = cv;
                             }
                         } else {
-                            *dst = first ? v : *dst + v;
+                            *dst = a == ra0 ? v : *dst + v;
                         }
                     }
                 }
             }
         }
-        // the row sums of block a into its row slot
+        // the row sums of block a into its row slot (a thread's own shared-memory values)
 #pragma unroll
-        for (int m = 0; m < P; ++m) {
+        for (int m = 0; m < R; ++m) {
+            const int64_t pr = base + static_cast<int64_t>(m) * T;
 #pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                const int64_t pr = base + static_cast<int64_t>(2 * m + h) * kSymT;
-                *slot(pr, s_row, 0) = h ? rsh[m][tid].y : rsh[m][tid].x;
-                *slot(pr, s_row, 1) = h ? rsh[P + m][tid].y : rsh[P + m][tid].x;
-                *slot(pr, s_row, 2) = h ? rsh[2 * P + m][tid].y : rsh[2 * P + m][tid].x;
-                if (COMP) {
-                    *slot(pr, s_row, 3) = h ? csh[m][tid].y : csh[m][tid].x;
-                    *slot(pr, s_row, 4) = h ? csh[P + m][tid].y : csh[P + m][tid].x;
-                    *slot(pr, s_row, 5) = h ? csh[2 * P + m][tid].y : csh[2 * P + m][tid].x;
-                }
+            for (int c = 0; c < 3; ++c) {
+                *slot(pr, s_row, c) = rsh[c * R + m][tid];
+                if (COMP) *slot(pr, s_row, 3 + c) = csh[COMP ? c * R + m : 0][tid];
             }
         }
     }
 }
+
+// The shapes, by rows per thread, threads and CTAs per SM: larger blocks do less per column sum, smaller ones give more
+// tasks (sym_shape).
+using Sym8 = SymShape<8, 128, 3>;
+using Sym4 = SymShape<4, 128, 4>;
+using Sym2 = SymShape<2, 128, 6>;
+using Sym1 = SymShape<2, 64, 12>;
 
 template <int I, int GRAV, bool COMP>
 __global__ void __launch_bounds__(128) k_gravity(const float4* __restrict__ posm, float* __restrict__ part,
@@ -896,6 +1036,7 @@ NearView near_view(const DevArrays& a, const DevParams& p, const SpatialArrays& 
     v.order = sp.group_order;
     v.lo = sp.sub_lo;
     v.hi = sp.sub_hi;
+    v.ngroups = static_cast<int>(a.n_pad / kGroup);
     v.nchunks = a.n_pad / kChunk;
     v.n = a.n;
     v.n_pad = a.n_pad;
@@ -918,8 +1059,10 @@ cudaError_t launch_density(const DevArrays& a, const DevParams& p, const Launch&
     GSPH_TIMER_MARK(t, start);
     if (sp) {
         const NearView v = near_view(a, p, *sp);
-        if (comp) k_density_near<true><<<near_blocks(a), kSub * kShares, 0, s>>>(a.posm, a.velrho, p, v);
-        else k_density_near<false><<<near_blocks(a), kSub * kShares, 0, s>>>(a.posm, a.velrho, p, v);
+        const bool dens = !has(p, GSPH_INTEGRATE_DENSITY);
+        if (!dens) k_near<false, false><<<near_blocks(a), kSub * kNearWarps, 0, s>>>(a.posm, a.velrho, p, v);
+        else if (comp) k_near<true, true><<<near_blocks(a), kSub * kNearWarps, 0, s>>>(a.posm, a.velrho, p, v);
+        else k_near<true, false><<<near_blocks(a), kSub * kNearWarps, 0, s>>>(a.posm, a.velrho, p, v);
     } else {
         const int T = 256;
         const dim3 grid(static_cast<unsigned>(a.n_pad / T), static_cast<unsigned>(L.nseg));
@@ -945,15 +1088,14 @@ cudaError_t launch_prepare(const DevArrays& a, const DevParams& p, cudaStream_t 
 namespace {
 template <int PASS, int GRAV, bool SOLIDS, bool COMP>
 cudaError_t pairs_t(const DevArrays& a, const DevParams& p, const Launch& L, cudaStream_t s, const KTimer* t,
-                    const SpatialArrays* sp, int gnseg, cudaEvent_t join, bool lists) {
+                    const SpatialArrays* sp, int gnseg, cudaEvent_t join) {
     constexpr int NS = (PASS == PASS_VGRAD) ? 2 : 4;
     if (sp) {  // SPH terms over the near chunks; gravity partials come from elsewhere
         constexpr uint32_t MASK = field_mask<PASS, false, SOLIDS>();
         constexpr int K = popc_c(MASK);
         GSPH_TIMER_MARK(t, start);
         const NearView v = near_view(a, p, *sp);
-        if (lists) k_pairs_near<PASS, SOLIDS, true, COMP><<<near_blocks(a), kSub * kShares, 0, s>>>(a, p, v);
-        else k_pairs_near<PASS, SOLIDS, false, COMP><<<near_blocks(a), kSub * kShares, 0, s>>>(a, p, v);
+        k_pairs_near<PASS, SOLIDS, COMP><<<near_blocks(a), kSub, 0, s>>>(a, p, v);
         cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) return e;
         GSPH_TIMER_MARK(t, stop);
@@ -986,24 +1128,24 @@ cudaError_t pairs_t(const DevArrays& a, const DevParams& p, const Launch& L, cud
 
 template <int PASS, int GRAV>
 cudaError_t pairs_g(const DevArrays& a, const DevParams& p, const Launch& L, cudaStream_t s, const KTimer* t,
-                    const SpatialArrays* sp, int gnseg, cudaEvent_t join, bool lists = false) {
+                    const SpatialArrays* sp, int gnseg, cudaEvent_t join) {
     const bool solids = has(p, GSPH_SOLIDS);
     const bool comp = L.accum == GSPH_ACCUM_COMPENSATED;
     if (solids)
-        return comp ? pairs_t<PASS, GRAV, true, true>(a, p, L, s, t, sp, gnseg, join, lists)
-                    : pairs_t<PASS, GRAV, true, false>(a, p, L, s, t, sp, gnseg, join, lists);
-    return comp ? pairs_t<PASS, GRAV, false, true>(a, p, L, s, t, sp, gnseg, join, lists)
-                : pairs_t<PASS, GRAV, false, false>(a, p, L, s, t, sp, gnseg, join, lists);
+        return comp ? pairs_t<PASS, GRAV, true, true>(a, p, L, s, t, sp, gnseg, join)
+                    : pairs_t<PASS, GRAV, true, false>(a, p, L, s, t, sp, gnseg, join);
+    return comp ? pairs_t<PASS, GRAV, false, true>(a, p, L, s, t, sp, gnseg, join)
+                : pairs_t<PASS, GRAV, false, false>(a, p, L, s, t, sp, gnseg, join);
 }
 }  // namespace
 
 cudaError_t launch_pairs(int pass, const DevArrays& a, const DevParams& p, const Launch& L, cudaStream_t s,
-                         const KTimer* t, const SpatialArrays* sp, int gnseg, cudaEvent_t join, bool lists) {
+                         const KTimer* t, const SpatialArrays* sp, int gnseg, cudaEvent_t join) {
     if (sp) {  // the culled kernels carry no gravity
         switch (pass) {
-            case PASS_VGRAD: return pairs_g<PASS_VGRAD, 0>(a, p, L, s, t, sp, 0, join, lists);
-            case PASS_ACC: return pairs_g<PASS_ACC, 0>(a, p, L, s, t, sp, gnseg, join, lists);
-            default: return pairs_g<PASS_FUSED, 0>(a, p, L, s, t, sp, gnseg, join, lists);
+            case PASS_VGRAD: return pairs_g<PASS_VGRAD, 0>(a, p, L, s, t, sp, 0, join);
+            case PASS_ACC: return pairs_g<PASS_ACC, 0>(a, p, L, s, t, sp, gnseg, join);
+            default: return pairs_g<PASS_FUSED, 0>(a, p, L, s, t, sp, gnseg, join);
         }
     }
     const int grav = !has(p, GSPH_SELF_GRAVITY) ? 0 : (p.eps2 > 0.0f ? 1 : 2);
@@ -1021,6 +1163,12 @@ cudaError_t launch_pairs(int pass, const DevArrays& a, const DevParams& p, const
 }
 
 namespace {
+template <typename S, int GRAV, bool COMP>
+void sym_launch(const DevArrays& a, const DevParams& p, const Launch& L, float* out, cudaStream_t s) {
+    const int G = L.grav_sym_G;
+    k_gravity_sym<S, GRAV, COMP><<<static_cast<unsigned>(G * (G + 1) / 2), S::T, 0, s>>>(a.posm, out, a.n_pad, G,
+                                                                                        L.grav_sym_gs, p.eps2);
+}
 template <int I, int GRAV, bool COMP>
 cudaError_t gravity_t(const DevArrays& a, const DevParams& p, const Launch& L, cudaStream_t s, const KTimer* t,
                       bool finish) {
@@ -1029,9 +1177,13 @@ cudaError_t gravity_t(const DevArrays& a, const DevParams& p, const Launch& L, c
     const size_t smem = pipe_smem_bytes(1, L.grav_jt);
     GSPH_TIMER_MARK(t, start);
     if (L.grav_sym_G > 0) {
-        const int G = L.grav_sym_G;
-        k_gravity_sym<GRAV, COMP><<<static_cast<unsigned>(G * (G + 1) / 2), kSymT, 0, s>>>(
-            a.posm, finish ? a.part : a.gpart, a.n_pad, G, L.grav_sym_gs, p.eps2);
+        float* out = finish ? a.part : a.gpart;
+        switch (L.grav_sym_shape) {
+            case 0: sym_launch<Sym8, GRAV, COMP>(a, p, L, out, s); break;
+            case 1: sym_launch<Sym4, GRAV, COMP>(a, p, L, out, s); break;
+            case 2: sym_launch<Sym2, GRAV, COMP>(a, p, L, out, s); break;
+            default: sym_launch<Sym1, GRAV, COMP>(a, p, L, out, s);
+        }
     } else if constexpr (I >= 2) {
         if (L.grav_x2)
             k_gravity_x2<I, GRAV, COMP><<<grid, T, smem, s>>>(a.posm, finish ? a.part : a.gpart, a.n_pad, L.grav_jt,
@@ -1177,6 +1329,33 @@ int gravity_blocks_per_sm(int ipt, int threads, int jt, bool comp) {
     }
 #undef GSPH_OCC
     return (e == cudaSuccess && nb > 0) ? nb : 4;
+}
+
+// Model of the shapes' times: an SM takes ceil(tasks / SMs) tasks, `ctas` at a time at `rate` interactions per clock; a
+// last round of fewer takes as long as 0.6 of a full one at least (a lone CTA does not fill the FMA pipe).
+// Up to 128 groups: N = 262,144 in 15.8 ms against 16.6 ms with 64 (tasks four times as large, the last wave 68 %
+// full); 64 above 4 M particles, where a particle's slots would take 1.5 KB.
+void sym_shape(int64_t n_pad, int sms, int groups, int shape, Launch& L) {
+    const int B[kSymShapes] = {Sym8::B, Sym4::B, Sym2::B, Sym1::B};
+    const int ctas[kSymShapes] = {Sym8::CTAS, Sym4::CTAS, Sym2::CTAS, Sym1::CTAS};
+    const double rate[kSymShapes] = {14.9, 13.4, 11.0, 10.0};
+    const int target = groups ? groups : (n_pad <= (int64_t(1) << 22) ? 128 : 64);
+    double best = 1e300;
+    for (int k = 0; k < kSymShapes; ++k) {
+        if (shape >= 0 && k != shape) continue;
+        int G, gs;
+        sym_groups(n_pad / B[k], target, G, gs);
+        const int64_t per_sm = (static_cast<int64_t>(G) * (G + 1) / 2 + sms - 1) / sms;
+        const int64_t full = per_sm / ctas[k], rest = per_sm % ctas[k];
+        const double load = static_cast<double>(full * ctas[k]) + (rest ? std::max<double>(rest, 0.6 * ctas[k]) : 0.0);
+        const double pairs = static_cast<double>(gs) * B[k] * gs * B[k];
+        if (load * pairs / rate[k] < best) {
+            best = load * pairs / rate[k];
+            L.grav_sym_shape = k;
+            L.grav_sym_G = G;
+            L.grav_sym_gs = gs;
+        }
+    }
 }
 
 size_t gravity_partial_floats(const Launch& L, int64_t n_pad) {

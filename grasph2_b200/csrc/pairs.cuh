@@ -85,47 +85,56 @@ struct JTilePipe {
 };
 
 // ---- culled passes -------------------------------------------------------------------------------
-// Every 32 consecutive particles (a quarter of an i-group) belong to one CTA of kShares warps; lane l of each warp
-// holds particle l. The warps share the group's near chunks, half a chunk (32 particles, one box) at a time: half h
-// goes to warp h % kShares, since near chunks come in runs along the curve. A particle's neighbours found by a warp
-// are its share; the CTA adds the shares in order, so no partial sums leave it.
-constexpr int kShares = 4;
-constexpr int kSub = 32;                 // particles per CTA and per box
-constexpr int kSubs = kGroup / kSub;     // CTAs per i-group
+// 32 consecutive particles at a time, lane l holds particle l. One pass finds the neighbours (four warps share its
+// i-group's near chunks, half a chunk with a box of its own at a time) and stores their lists; the SPH passes walk
+// them, one warp per 32 particles. No partial sums.
+//
+// Order of summation: the near chunks of a group form items of `per_item` chunks, an item's chunks form stages of
+// kStageChunks. A particle's density is the sum over items of the sum over stages of the sum over neighbours; its SPH
+// sums are the sum over items of the sum over neighbours (compensated: stages by two-sum, items in FP64). It follows from
+// the near chunks alone, not from the launch.
+constexpr int kStageChunks = 4;
+constexpr int kSub = 32;                 // particles per warp and per box
+constexpr int kSubs = kGroup / kSub;
+constexpr int kHalves = kChunk / kSub;   // boxes per chunk
+constexpr int kItemsPerSM = 30;          // items aimed at in all
 
 struct NearView {
     const int* list;     // near chunks of each i-group, row stride nchunks
     const int* count;
-    const int* order;    // i-groups, the longest lists first
+    const int* order;    // i-groups, the longest lists first; [ngroups]: chunks per item
     const float4 *lo, *hi;  // bounds of every 32 particles
+    int ngroups;
     int64_t nchunks, n, n_pad;
     float hm2;           // (h (1 + kMargin))^2
-    int* nb;             // neighbour lists [share][cap][n_pad] ...
-    int* nbcnt;          // ... and their lengths [share][n_pad]; more than cap: the list is incomplete
+    int* nb;             // neighbour lists [cap][n_pad]; the sign bit marks the first neighbour of an item ...
+    int* nbcnt;          // ... and their lengths [n_pad]; more than cap: the list is incomplete
     int cap;
     __device__ __forceinline__ int group() const { return order[blockIdx.x / kSubs]; }
     __device__ __forceinline__ int64_t first(int g) const {
         return static_cast<int64_t>(g) * kGroup + (blockIdx.x % kSubs) * kSub;
     }
+    __device__ __forceinline__ int per_item() const { return order[ngroups]; }
 };
+constexpr int kItemMark = static_cast<int>(0x80000000u);
 
-// One warp's share of the near chunks of the 32 particles from s0 (group g): the boxes farther than h (1 + kMargin)
-// from the 32 particles' own box are skipped (32 of them per vote), the positions of the others go through the
-// warp's shared buffer `sh`, the next box's load in flight while one is tested, and body(mask, jb) gets each lane's
-// mask of the neighbours (0 < r^2 <= H^2, bit k: particle jb + k, its record in sh[k]). No block barriers.
+// The near chunks of the 32 particles from s0 (group g): boxes farther than h (1 + kMargin) from the 32 particles' own
+// box are skipped (32 of them per vote), the positions of the others go through the shared buffer `sh`, the next
+// box's load in flight while one is tested, and body(mask, jb, c) gets each lane's mask of the neighbours (0 < r^2 <= H^2,
+// bit k: particle jb + k, its record in sh[k]) and the chunk's place in the list.
 template <typename Body>
 __device__ __forceinline__ void near_scan(const NearView& v, const float4* __restrict__ posm, int g, int64_t s0,
                                           uint32_t span, float4 pi, float4* sh, Body&& body) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int lane = threadIdx.x & 31;
     const float4 l = v.lo[s0 / kSub], u = v.hi[s0 / kSub];
-    const int nh = v.count[g] * (kChunk / kSub);
+    const int nh = v.count[g] * kHalves;
     const int* chunks = v.list + static_cast<int64_t>(g) * v.nchunks;
-    for (int h0 = 0; h0 < nh; h0 += 32 * kShares) {
-        const int h = h0 + kShares * lane + warp;
+    for (int h0 = 0; h0 < nh; h0 += 32) {
+        const int h = h0 + lane;
         int bx = 0;
         bool near = false;
         if (h < nh) {
-            bx = chunks[h / (kChunk / kSub)] * (kChunk / kSub) + h % (kChunk / kSub);
+            bx = chunks[h / kHalves] * kHalves + h % kHalves;
             const float4 bl = v.lo[bx], bu = v.hi[bx];
             const float gx = fmaxf(0.0f, fmaxf(bl.x - u.x, l.x - bu.x)), gy = fmaxf(0.0f, fmaxf(bl.y - u.y, l.y - bu.y)),
                         gz = fmaxf(0.0f, fmaxf(bl.z - u.z, l.z - bu.z));
@@ -139,6 +148,7 @@ __device__ __forceinline__ void near_scan(const NearView& v, const float4* __res
             qn = posm[jn + lane];
         }
         while (todo) {
+            const int c = (h0 + __ffs(todo) - 1) / kHalves;
             todo &= todo - 1;
             const int jb = jn;
             const float4 q0 = qn;
@@ -162,7 +172,7 @@ __device__ __forceinline__ void near_scan(const NearView& v, const float4* __res
                 }
                 m4[b] = m;
             }
-            body(m4[0] | (m4[1] << 8) | (m4[2] << 16) | (m4[3] << 24), jb);
+            body(m4[0] | (m4[1] << 8) | (m4[2] << 16) | (m4[3] << 24), jb, c);
         }
     }
 }
@@ -244,8 +254,9 @@ struct Launch {
     int grav_jt;     // j-tile of the gravity kernel
     bool grav_x2;    // paired FP32 (f32x2) form of the gravity kernel
     int grav_nseg;
-    int grav_sym_G = 0;   // > 0: symmetric gravity kernel over G groups of grav_sym_gs blocks of 1024
+    int grav_sym_G = 0;   // > 0: symmetric gravity kernel over G groups of grav_sym_gs blocks
     int grav_sym_gs = 0;
+    int grav_sym_shape = 0;  // block shape of the symmetric kernel (pairs.cu)
     int accum;       // GSPH_ACCUM_*
 };
 
@@ -260,25 +271,27 @@ inline GravSum grav_sum(const Launch& L, int nseg) {
     }
     return g;
 }
-// the symmetric gravity kernel's group count for blocks of 1024 particles: groups of
-// ceil(nblocks / target) blocks
+// groups of ceil(nblocks / target) blocks
 inline void sym_groups(int64_t nblocks, int target, int& G, int& gs) {
     gs = static_cast<int>((nblocks + target - 1) / target);
     if (gs < 1) gs = 1;
     G = static_cast<int>((nblocks + gs - 1) / gs);
 }
+constexpr int kSymShapes = 4;
+// the symmetric kernel's block shape and groups for n_pad particles (at most `groups`; 0: its own choice); with
+// shape >= 0 that block shape
+void sym_shape(int64_t n_pad, int sms, int groups, int shape, Launch& L);
 
-// With `sp`, the culled density pass over the near chunks, which also stores every particle's neighbours
-// (sp->nb): the SPH passes of the same step read them instead of searching again.
+// The density pass and the j-records of the new density. With `sp`: the neighbour search over the near chunks (with
+// INTEGRATE_DENSITY the search alone), which stores the lists that the SPH passes of the step read.
 cudaError_t launch_density(const DevArrays& a, const DevParams& p, const Launch& L, cudaStream_t s,
                            const KTimer* t = nullptr, const SpatialArrays* sp = nullptr);
 cudaError_t launch_prepare(const DevArrays& a, const DevParams& p, cudaStream_t s);
-// With `sp`, the SPH terms come from the near chunks, or (`lists`) from the neighbour lists an earlier pass of the step
-// stored; the finish kernel then adds the gravity sums (a.gfold, from launch_gravity_partials), after waiting for
+// With `sp`, the SPH terms run over the neighbour lists of launch_density; the finish kernel then adds the gravity sums (a.gfold, from launch_gravity_partials), after waiting for
 // `join` when it is given (the gravity kernel may run on another stream).
 cudaError_t launch_pairs(int pass, const DevArrays& a, const DevParams& p, const Launch& L, cudaStream_t s,
                          const KTimer* t = nullptr, const SpatialArrays* sp = nullptr, int gnseg = 0,
-                         cudaEvent_t join = nullptr, bool lists = false);
+                         cudaEvent_t join = nullptr);
 cudaError_t launch_gravity_partials(const DevArrays& a, const DevParams& p, const Launch& L, cudaStream_t s,
                                     const KTimer* t = nullptr);
 cudaError_t launch_gravity(const DevArrays& a, const DevParams& p, const Launch& L, cudaStream_t s,
@@ -290,21 +303,9 @@ cudaError_t launch_gravity_raw(const float4* posm_padded, float* part, int64_t n
 cudaError_t launch_gravity_fold(const DevArrays& a, const Launch& L, int S, cudaStream_t s);
 int64_t fp32_peak_flops(int sm_count, int iters);
 
-// ---- derivatives in a fixed order of summation (pairs_fixed.cu) ---------------------------------------
-struct FixedArrays {
-    int* item_start = nullptr;  // [n_pad / kGroup + 2] first work item of each group, number of items, chunks per item
-    float* part = nullptr;      // [items][fields][kGroup] partial sums
-    int* nb = nullptr;          // [items][kItemNb][kGroup] neighbour indices the density pass found
-    int* nbcnt = nullptr;       // [items][kGroup]
-    int* nbover = nullptr;      // [items]
-};
-size_t fixed_items(int64_t n_pad, int sms);
-size_t fixed_part_floats();  // per item
-size_t fixed_list_ints();    // per item
-cudaError_t launch_fixed_gravity(const DevArrays& a, const DevParams& p, const Launch& L, cudaStream_t s);
-// near-chunk lists first; `join` as in launch_pairs
-cudaError_t launch_fixed_sph(const DevArrays& a, const DevParams& p, const Launch& L, const SpatialArrays& sp,
-                             const FixedArrays& fx, int sms, bool grav, cudaEvent_t join, cudaStream_t s, int& launches);
+// the gravity partials and their fold with the kernels of the fixed order (gravity_fixed.cu)
+cudaError_t launch_fixed_gravity(const DevArrays& a, const DevParams& p, const Launch& L, cudaStream_t s,
+                                 const KTimer* t = nullptr);
 
 size_t partial_floats(const DevParams& p, const Launch& L, int64_t n_pad);
 size_t gravity_partial_floats(const Launch& L, int64_t n_pad);

@@ -86,20 +86,37 @@ __global__ void __launch_bounds__(128) k_chunk_lists(const float4* __restrict__ 
     if (lane == 0) count[g] = n;
 }
 
-// The groups by falling near-chunk count (to a 256th of the largest), so that the CTAs of long lists start first and
-// the short ones fill the last wave. One block: counting sort. The order within a bucket is not fixed, and need not
-// be: every group's results are its own.
+// The groups by falling near-chunk count (to a 256th of the largest), so that the warps of long lists start first and
+// the short ones fill the last wave, and the chunks per item ceil(total near chunks / items). One block: counting
+// sort. The order within a bucket is not fixed, and need not be: every group's results are its own.
 constexpr int kOrderThreads = 1024, kBuckets = 256;
 __global__ void __launch_bounds__(kOrderThreads) k_group_order(const int* __restrict__ count, int* __restrict__ order,
-                                                               int ngroups) {
+                                                               int ngroups, int items) {
     __shared__ int most, bins[kBuckets], warp_sum[kBuckets / 32];
-    if (threadIdx.x == 0) most = 1;
+    __shared__ unsigned long long total;
+    if (threadIdx.x == 0) {
+        most = 1;
+        total = 0;
+    }
     if (threadIdx.x < kBuckets) bins[threadIdx.x] = 0;
     __syncthreads();
     int m = 0;
-    for (int g = threadIdx.x; g < ngroups; g += kOrderThreads) m = max(m, count[g]);
-    atomicMax(&most, m);
+    unsigned long long sum = 0;
+    for (int g = threadIdx.x; g < ngroups; g += kOrderThreads) {
+        m = max(m, count[g]);
+        sum += count[g];
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
+        sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    }
+    if ((threadIdx.x & 31) == 0) {
+        atomicMax(&most, m);
+        atomicAdd(&total, sum);
+    }
     __syncthreads();
+    if (threadIdx.x == 0) order[ngroups] = static_cast<int>(max(1ull, (total + items - 1) / items));
     const int top = most;
     auto bucket = [&](int g) {
         return kBuckets - 1 - static_cast<int>(static_cast<long long>(count[g]) * (kBuckets - 1) / top);
@@ -232,8 +249,8 @@ cudaError_t launch_chunk_lists(const DevArrays& a, const SpatialArrays& s, float
     return cudaGetLastError();
 }
 
-cudaError_t launch_group_order(const DevArrays& a, const SpatialArrays& s, cudaStream_t st) {
-    k_group_order<<<1, kOrderThreads, 0, st>>>(s.count, s.group_order, static_cast<int>(a.n_pad / kGroup));
+cudaError_t launch_group_order(const DevArrays& a, const SpatialArrays& s, int items, cudaStream_t st) {
+    k_group_order<<<1, kOrderThreads, 0, st>>>(s.count, s.group_order, static_cast<int>(a.n_pad / kGroup), items);
     return cudaGetLastError();
 }
 

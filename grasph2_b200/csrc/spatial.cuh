@@ -24,8 +24,8 @@ struct SpatialArrays {
     int* count;        // [n_pad / kGroup]
     float4* sub_lo;    // [n_pad / 32] bounds of every 32 particles
     float4* sub_hi;
-    int* group_order;  // [n_pad / kGroup] i-groups by falling near-chunk count
-    int* nb;           // [kShares][nb_cap][n_pad] neighbour indices, and their number [kShares][n_pad]
+    int* group_order;  // [n_pad / kGroup + 1] i-groups by falling near-chunk count; last: near chunks per item
+    int* nb;           // [nb_cap][n_pad] neighbour indices, and their number [n_pad]
     int* nbcnt;
     int nb_cap;
     int* ext_of_int;   // [n_pad] caller's index of the particle stored at each internal slot
@@ -78,10 +78,11 @@ __device__ __forceinline__ unsigned hilbert3(unsigned x0, unsigned x1, unsigned 
 }
 
 size_t spatial_sort_tmp_bytes(int64_t n_pad);
-// bounds of the chunks (and of their halves), the near chunks of every i-group, the order the groups are taken in
+// bounds of the chunks (and of their halves), the near chunks of every i-group, the order the groups are taken in (and
+// the chunks per item that make about `items` items)
 cudaError_t launch_chunk_bounds(const DevArrays& a, const SpatialArrays& s, cudaStream_t st);
 cudaError_t launch_chunk_lists(const DevArrays& a, const SpatialArrays& s, float h, cudaStream_t st);
-cudaError_t launch_group_order(const DevArrays& a, const SpatialArrays& s, cudaStream_t st);
+cudaError_t launch_group_order(const DevArrays& a, const SpatialArrays& s, int items, cudaStream_t st);
 // Sort the n real particles of `a` along the Hilbert curve and permute every per-particle array in place.
 cudaError_t reorder_particles(const DevArrays& a, const SpatialArrays& s, cudaStream_t st, int& launches);
 // The first half of it: order_out[k] = slot of the k-th particle along the curve (padding last, in place).

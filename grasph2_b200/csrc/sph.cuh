@@ -123,7 +123,10 @@ __device__ __forceinline__ void sph_neighbour(PairAcc& T, float& maxv, const ISp
             T.f[F_C1] = fmaf(mr, vz * gx - vx * gz, T.f[F_C1]);
             T.f[F_C2] = fmaf(mr, vx * gy - vy * gx, T.f[F_C2]);
         }
-        if (I.divv_on) T.f[F_DIVV] = fmaf(-mr, vx * gx + vy * gy + vz * gz, T.f[F_DIVV]);
+        // rounded product by product: in the first steps of a body at rest density a last place of the density is
+        // 0.6 % of its yield stress, so the rate's roundings are fixed here, not left to the compiler
+        if (I.divv_on)
+            T.f[F_DIVV] = fmaf(-mr, __fadd_rn(__fadd_rn(__fmul_rn(vx, gx), __fmul_rn(vy, gy)), __fmul_rn(vz, gz)), T.f[F_DIVV]);
     }
     if (DO_A) {
         float sxx = I.jAi.x + ja.x, syy = I.jAi.y + ja.y, szz = I.jAi.z + ja.z;
@@ -141,7 +144,9 @@ __device__ __forceinline__ void sph_neighbour(PairAcc& T, float& maxv, const ISp
         T.f[F_AY] = fmaf(mj, sxy * gx + syy * gy + syz * gz, T.f[F_AY]);
         T.f[F_AZ] = fmaf(mj, sxz * gx + syz * gy + szz * gz, T.f[F_AZ]);
         if (I.av) {  // artificialViscosity (models.h:158-185)
-            const float w = -(dx * vx + dy * vy + dz * vz) * inv_r;  // r_ij . v_ij / r
+            // r_ij . v_ij / r (the acceleration pass fixes its roundings as well)
+            const float dv = PASS == PASS_ACC ? fmaf(dz, vz, fmaf(dx, vx, dy * vy)) : dx * vx + dy * vy + dz * vz;
+            const float w = -dv * inv_r;
             if (w < 0.0f) {
                 const float vsig = p.c + p.c - p.beta * w;
                 const float rhoij = (I.vi.w + rhoj) * 0.5f;

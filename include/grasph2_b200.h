@@ -177,12 +177,13 @@ typedef struct gsph_options {
     int32_t gravity_form;    /* GSPH_GRAVITY_AUTO (default), GSPH_GRAVITY_ONE_SIDED or GSPH_GRAVITY_SYMMETRIC: the
                                 all-pairs gravity kernel evaluates every ordered pair (i gathers from all j), or
                                 every unordered pair once and applies it to both particles (Newton's third law;
-                                2/3 of the FP32 work, partials of 65 x 3 floats per particle). Auto picks the
-                                symmetric form from 24 blocks of 1024 particles up. Results agree to rounding.
+                                14 to 16 FP32 operations for both against 24, partials of up to 129 x 3 floats per
+                                particle). Auto is the symmetric form, unless scalar_fp32 or, below 24 blocks of 1024
+                                particles, a shape of the one-sided kernel is asked for. Results agree to rounding.
                                 Ensembles use the one-sided sweep fused with their density pass; SYMMETRIC
                                 gives them a queue stage of group pairs instead (slower on ensembles of
                                 1k..32k-particle simulations) */
-    int32_t gravity_groups;  /* symmetric form: particle groups G (tasks G(G+1)/2); 0 = up to 64 */
+    int32_t gravity_groups;  /* symmetric form: particle groups G at most (tasks G(G+1)/2); 0 = up to 128 */
     int32_t wait_limit_us;   /* batched ensemble: a work item that waits for another item's result (a device-side
                                 spin on a counter) gives up after this many microseconds, sets the timeout bit
                                 and its call returns GSPH_E_TIMEOUT (0 = 2 s). Waits for a bulk copy to land
@@ -282,7 +283,7 @@ int gsph_diagnostics_fast(gsph_ctx* ctx, double half_kick, gsph_diag* out, void*
 int gsph_autotune(gsph_ctx* ctx, int32_t reps, void* stream);
 typedef struct gsph_launch_shape {
     int32_t cull, grav_ipt, grav_jt, grav_nseg, grav_x2, sph_threads, sph_jt, sph_nseg, items;
-    /* items: warps that share 32 particles in the culled SPH passes (0: all pairs) */
+    /* items: runs of near chunks the culled SPH sums are ordered by, in all (0: all pairs) */
     int32_t grav_sym_groups;  /* > 0: the symmetric gravity kernel over this many particle groups */
     int32_t reserved[6];
 } gsph_launch_shape;
