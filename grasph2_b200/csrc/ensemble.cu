@@ -32,6 +32,7 @@
 #include <cub/device/device_radix_sort.cuh>
 
 #include "f32x2.cuh"
+#include "gravity_sym.cuh"
 #include "integrate.cuh"
 #include "spatial.cuh"
 #include "sph.cuh"
@@ -68,11 +69,11 @@ struct EnsView {
     int tile;            // j-particles per shared-memory stage of the DENS sweep
     int stall_sim;       // failure-path test: this simulation's SPH items wait for one DENS item more than
                          // exist, so their waits run out (-1: none)
-    // symmetric gravity (GSYM stage, first in the queue when ntasks > 0): tasks (sim, row group, column
-    // group, 0) of each simulation's group pairs, and the per-simulation partial slots they fill
+    int near;            // the DENS stage finds neighbours by boxes, gravity comes from the slots of k_ens_gravity
+    float4 *box_lo, *box_hi;  // [G][kEnsSubs] bounds of every 32 particles
+    // symmetric gravity: tasks (sim, row group, column group, 0) of each simulation's group pairs, and the
+    // per-simulation partial slots they fill
     const int4* tasks;
-    int ntasks;
-    int sym;             // gravity comes from the GSYM slots (the DENS stage then skips gravity)
     float* gslot;        // all simulations' slots; simulation k's start at slot_base[k]
     const long long* slot_base;
 };
@@ -375,137 +376,250 @@ __device__ __forceinline__ bool dens_item(const DevArrays& a, const DevParams& p
     return true;
 }
 
-// ---- GSYM: symmetric gravity over pairs of groups of one simulation --------------------------------
-// Task (sim, ga, gb), ga <= gb: every pair of a particle of group ga (the rows, four per thread in two
-// f32x2 pairs) and one of group gb (the columns, streamed by the pipe) is evaluated once and its 1/r^3
-// serves both: the rows' sums stay in registers, the columns' are summed over the task's rows (in the
-// thread, by a butterfly over the warp, then over the four warps in shared memory). The diagonal task
-// (ga == gb) runs one-sided over the group's own pairs. Every particle of a simulation with G groups has
-// G + 1 slots, [slot][component][particle of the simulation]: its row sums from tasks (g, gb) in slots
-// 0 .. G-1-g, its column sums from tasks (ga, g) in slots G-g .. G, each written by exactly one task (the
-// diagonal task zeroes slot G); the SPH stage folds them in FP64 in slot order, so results are
-// deterministic. Rows past the group's end are inert (zero mass, far away); columns past the simulation's
-// end are never read.
-constexpr int kEnsJC = 128;  // columns per shared-memory reduction round
-constexpr int kEnsJB = 8;    // columns per warp butterfly
+// ---- symmetric gravity over pairs of groups of one simulation ----------------------------------------
+// One CTA per task (sim, ga, gb), ga <= gb: every pair of a particle of group ga (the rows, four per thread) and one of
+// group gb (the columns) is evaluated once and its 1/r^3 serves both (gravity_sym.cuh: two columns per f32x2
+// instruction, tiles of equal masses without mass multiplies). A diagonal task runs one-sided over the group's own
+// pairs. Every particle of a simulation with G groups has G + 1 slots, [slot][component][particle of the simulation]: its
+// row sums from tasks (g, gb) in slots 0 .. G-1-g, its column sums from tasks (ga, g) in slots G-g .. G, each
+// written by exactly one task (the diagonal one zeroes slot G); the SPH stage folds them in FP64 in slot order. Rows and
+// columns past the simulation's end are inert: so far away that 1/r^3 is zero.
+//
+// The one-sided sweep fused with the density test spent 12 FP32 operations per ordered pair and tested a third of all
+// pairs for neighbours; this one spends 14 per unordered pair, and the density pass finds its neighbours by boxes of 32
+// particles. 512 simulations of 1,024 to 32,768 particles: 50.4 ms per step before.
+using SymE = SymShape<kEnsIpt, kEnsThreads, 4>;
+static_assert(SymE::B == kEnsGroup, "a task's rows are a group");
 
 __device__ __forceinline__ float* sim_slots(const EnsView& v, int sim) { return v.gslot + v.slot_base[sim]; }
 
 template <int GRAV, bool COMP>
-__device__ __forceinline__ bool gsym_item(const DevArrays& a, const DevParams& p, const EnsView& v, RangePipe& pipe,
-                                          int4 task, int4 sm, float (*js)[kEnsJC][3]) {
-    constexpr int P = kEnsIpt / 2;
+__global__ void __launch_bounds__(SymE::T, SymE::CTAS) k_ens_gravity(const float4* __restrict__ posm, EnsView v, float eps2) {
+    constexpr int R = SymE::R, T = SymE::T, JT = SymE::JT, PF = SymE::PF;
     constexpr int K = COMP ? 6 : 3;
+    __shared__ float4 XY[JT / 2], ZM[JT / 2];
+    __shared__ float js[SymE::W][3][JT];
+    __shared__ float rsh[3 * R][T], csh[COMP ? 3 * R : 1][T];  // running row sums, rounding errors
+    const int tid = threadIdx.x, warp = tid >> 5;
+    const int4 task = v.tasks[blockIdx.x];
+    const int4 sm = v.sims[task.x];
     const int G = sm.w, ga = task.y, gb = task.z;
     const bool diag = ga == gb;
-    const int64_t r0 = static_cast<int64_t>(sm.x) + static_cast<int64_t>(ga) * kEnsGroup;
-    const int64_t c0 = static_cast<int64_t>(sm.x) + static_cast<int64_t>(gb) * kEnsGroup;
-    const int rn = min(kEnsGroup, sm.y - ga * kEnsGroup), cn = min(kEnsGroup, sm.y - gb * kEnsGroup);
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int64_t N = sm.y;
+    const int rn = min(kEnsGroup, sm.y - ga * kEnsGroup), cn = min(kEnsGroup, sm.y - gb * kEnsGroup);
+    const float4* rp = posm + sm.x + static_cast<int64_t>(ga) * kEnsGroup;
+    const float4* cp = posm + sm.x + static_cast<int64_t>(gb) * kEnsGroup;
     float* part = sim_slots(v, task.x);
     auto slot = [&](int local, int sl, int c) { return part + (static_cast<int64_t>(sl) * K + c) * N + local; };
     const int s_row = gb - ga, s_col = G - gb + ga;
-    const float4 inert = make_float4(1e18f, 1e18f, 1e18f, 0.0f);
-    float2 X[P], Y[P], Z[P], MI[P], AX[P], AY[P], AZ[P], CX[P], CY[P], CZ[P];
+    const float mr = rp[0].w, mc = cp[0].w;
+    SymRows<SymE> rows;
+    bool same = true;
 #pragma unroll
-    for (int k = 0; k < P; ++k) {
-        const int o0 = threadIdx.x + 2 * k * kEnsThreads, o1 = o0 + kEnsThreads;
-        const float4 q0 = o0 < rn ? a.posm[r0 + o0] : inert, q1 = o1 < rn ? a.posm[r0 + o1] : inert;
-        X[k] = make_float2(q0.x, q1.x); Y[k] = make_float2(q0.y, q1.y); Z[k] = make_float2(q0.z, q1.z);
-        MI[k] = make_float2(-q0.w, -q1.w);  // the columns receive the opposite of the rows' force
-        AX[k] = AY[k] = AZ[k] = CX[k] = CY[k] = CZ[k] = make_float2(0.0f, 0.0f);
+    for (int k = 0; k < R; ++k) {
+        const int o = tid + k * T;
+        const float4 u = o < rn ? rp[o] : make_float4(-1e18f, -1e18f, -1e18f, mr);
+        rows.set(k, u);
+        same = same && u.w == mr;
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            rsh[c * R + k][tid] = 0.0f;
+            if (COMP) csh[COMP ? c * R + k : 0][tid] = 0.0f;
+        }
     }
     if (diag)  // the group never is a column of its own diagonal task: that slot is zero
-        for (int e = threadIdx.x; e < cn; e += kEnsThreads)
+        for (int e = tid; e < cn; e += T)
             for (int c = 0; c < K; ++c) *slot(gb * kEnsGroup + e, s_col, c) = 0.0f;
-    const float2 E2 = make_float2(p.eps2, p.eps2);
-    const bool ok = pipe.run(c0, c0 + cn, [&](const float4* J, int nj, int64_t jb) {
-        float2 TX[P], TY[P], TZ[P];
+    const bool rows_equal = __syncthreads_and(same);
+    const float2 E2 = make_float2(eps2, eps2);
+    auto fetch = [&](int j) { return j < cn ? cp[j] : make_float4(1e18f, 1e18f, 1e18f, mc); };
+    float4 pf[PF];
 #pragma unroll
-        for (int k = 0; k < P; ++k) TX[k] = TY[k] = TZ[k] = make_float2(0.0f, 0.0f);
-        for (int j0 = 0; j0 < nj; j0 += kEnsJC) {
-            const int jn = min(kEnsJC, nj - j0);
-#pragma unroll 1
-            for (int u0 = 0; u0 < jn; u0 += kEnsJB) {
-                float vx[kEnsJB], vy[kEnsJB], vz[kEnsJB];
+    for (int h = 0; h < PF; ++h) pf[h] = fetch(tid + h * T);
+    for (int j0 = 0; j0 < cn; j0 += JT) {
+        __syncthreads();  // the previous tile's reads are done
+        bool same_c = true;
 #pragma unroll
-                for (int u = 0; u < kEnsJB; ++u) {
-                    const float4 q = (u0 + u < jn) ? J[j0 + u0 + u] : inert;
-                    const float2 qx = make_float2(q.x, q.x), qy = make_float2(q.y, q.y), qz = make_float2(q.z, q.z),
-                                 qm = make_float2(q.w, q.w);
-                    float2 tx = make_float2(0.0f, 0.0f), ty = tx, tz = tx;
-#pragma unroll
-                    for (int k = 0; k < P; ++k) {
-                        const float2 dx = sub2(qx, X[k]), dy = sub2(qy, Y[k]), dz = sub2(qz, Z[k]);
-                        const float2 r2 = fma2(dz, dz, fma2(dy, dy, fma2(dx, dx, E2)));
-                        float2 inv = make_float2(rsqrtf(r2.x), rsqrtf(r2.y));
-                        if (GRAV == 2) inv = make_float2(fminf(inv.x, 1e12f), fminf(inv.y, 1e12f));
-                        const float2 i3 = mul2(mul2(inv, inv), inv);
-                        const float2 sj = mul2(qm, i3);
-                        TX[k] = fma2(dx, sj, TX[k]); TY[k] = fma2(dy, sj, TY[k]); TZ[k] = fma2(dz, sj, TZ[k]);
-                        if (!diag) {
-                            const float2 si = mul2(MI[k], i3);
-                            tx = fma2(dx, si, tx); ty = fma2(dy, si, ty); tz = fma2(dz, si, tz);
-                        }
-                    }
-                    vx[u] = tx.x + tx.y;
-                    vy[u] = ty.x + ty.y;
-                    vz[u] = tz.x + tz.y;
-                }
-                if (!diag) {
-                    reduce_lanes(vx, lane);
-                    reduce_lanes(vy, lane);
-                    reduce_lanes(vz, lane);
-                    if ((lane & 3) == 0) {
-                        const int u = u0 + ((lane >> 2) & (kEnsJB - 1));
-                        js[warp][u][0] = vx[0];
-                        js[warp][u][1] = vy[0];
-                        js[warp][u][2] = vz[0];
-                    }
-                }
-            }
-            if (!diag) {  // this round's column sums over the task's rows, into the column slots
-                __syncthreads();
-                const int lc0 = static_cast<int>(jb - c0) + j0;
-                for (int e = threadIdx.x; e < jn; e += kEnsThreads)
-#pragma unroll
-                    for (int c = 0; c < 3; ++c) {
-                        *slot(gb * kEnsGroup + lc0 + e, s_col, c) = (js[0][e][c] + js[1][e][c]) + (js[2][e][c] + js[3][e][c]);
-                        if (COMP) *slot(gb * kEnsGroup + lc0 + e, s_col, 3 + c) = 0.0f;
-                    }
-                __syncthreads();
-            }
+        for (int h = 0; h < PF; ++h) {
+            sym_stage(XY, ZM, tid + h * T, pf[h]);
+            same_c = same_c && pf[h].w == mc;
         }
+        const bool equal = __syncthreads_and(same_c) && rows_equal;
+        if (j0 + JT < cn) {
 #pragma unroll
-        for (int k = 0; k < P; ++k) {  // the stage's row partials into the running sums
+            for (int h = 0; h < PF; ++h) pf[h] = fetch(j0 + JT + tid + h * T);
+        }
+        rows.clear();
+        if (diag) sym_own<SymE, GRAV>(rows, XY, ZM, E2);
+        else if (equal) sym_columns<SymE, GRAV, true>(rows, XY, ZM, E2, js[warp]);
+        else sym_columns<SymE, GRAV, false>(rows, XY, ZM, E2, js[warp]);
+        const float wr = !diag && equal ? mc : 1.0f;
+        auto row_add = [&](int o, float2 t) {
+            float x = rsh[o][tid];
             if (COMP) {
-                fold(AX[k].x, CX[k].x, TX[k].x); fold(AX[k].y, CX[k].y, TX[k].y);
-                fold(AY[k].x, CY[k].x, TY[k].x); fold(AY[k].y, CY[k].y, TY[k].y);
-                fold(AZ[k].x, CZ[k].x, TZ[k].x); fold(AZ[k].y, CZ[k].y, TZ[k].y);
+                float e = csh[COMP ? o : 0][tid];
+                fold(x, e, wr * (t.x + t.y));
+                csh[COMP ? o : 0][tid] = e;
             } else {
-                AX[k] = add2(AX[k], TX[k]); AY[k] = add2(AY[k], TY[k]); AZ[k] = add2(AZ[k], TZ[k]);
+                x = fmaf(wr, t.x + t.y, x);
+            }
+            rsh[o][tid] = x;
+        };
+#pragma unroll
+        for (int m = 0; m < R; ++m) {
+            row_add(m, rows.TX[m]);
+            row_add(R + m, rows.TY[m]);
+            row_add(2 * R + m, rows.TZ[m]);
+        }
+        if (!diag) {
+            __syncthreads();
+            const float wc = equal ? -mr : 1.0f;
+#pragma unroll
+            for (int h = 0; h < PF; ++h) {
+                const int j = tid + h * T;
+                if (j0 + j >= cn) break;
+#pragma unroll
+                for (int c = 0; c < 3; ++c) {
+                    *slot(gb * kEnsGroup + j0 + j, s_col, c) = wc * ((js[0][c][j] + js[1][c][j]) + (js[2][c][j] + js[3][c][j]));
+                    if (COMP) *slot(gb * kEnsGroup + j0 + j, s_col, 3 + c) = 0.0f;
+                }
             }
         }
-    });
-    if (!ok) return false;
+    }
 #pragma unroll
-    for (int k = 0; k < P; ++k)
+    for (int m = 0; m < R; ++m) {
+        const int o = tid + m * T;
+        if (o >= rn) break;
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            const int o = threadIdx.x + (2 * k + h) * kEnsThreads;
-            if (o >= rn) continue;
-            const int l = ga * kEnsGroup + o;
-            *slot(l, s_row, 0) = h ? AX[k].y : AX[k].x;
-            *slot(l, s_row, 1) = h ? AY[k].y : AY[k].x;
-            *slot(l, s_row, 2) = h ? AZ[k].y : AZ[k].x;
-            if (COMP) {
-                *slot(l, s_row, 3) = h ? CX[k].y : CX[k].x;
-                *slot(l, s_row, 4) = h ? CY[k].y : CY[k].x;
-                *slot(l, s_row, 5) = h ? CZ[k].y : CZ[k].x;
+        for (int c = 0; c < 3; ++c) {
+            *slot(ga * kEnsGroup + o, s_row, c) = rsh[c * R + m][tid];
+            if (COMP) *slot(ga * kEnsGroup + o, s_row, 3 + c) = csh[COMP ? c * R + m : 0][tid];
+        }
+    }
+}
+
+// ---- DENS without gravity: neighbours by boxes of 32 particles -----------------------------------------
+constexpr int kEnsSub = 32, kEnsSubs = kEnsGroup / kEnsSub;  // boxes per group: box kEnsSubs * group + k
+
+// bounds of every 32 particles of each group (one CTA per group; none: lo = +inf, hi = -inf)
+__global__ void __launch_bounds__(kEnsThreads) k_ens_boxes(const float4* __restrict__ posm, EnsView v) {
+    const int4 grp = v.groups[blockIdx.x];
+    const int lane = threadIdx.x & 31;
+    for (int k = threadIdx.x >> 5; k < kEnsSubs; k += kEnsThreads / 32) {
+        const int o = k * kEnsSub + lane;
+        float mn[3] = {INFINITY, INFINITY, INFINITY}, mx[3] = {-INFINITY, -INFINITY, -INFINITY};
+        if (o < grp.z) {
+            const float4 q = posm[grp.y + o];
+            mn[0] = mx[0] = q.x; mn[1] = mx[1] = q.y; mn[2] = mx[2] = q.z;
+        }
+#pragma unroll
+        for (int w = 16; w > 0; w >>= 1)
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                mn[c] = fminf(mn[c], __shfl_xor_sync(0xffffffffu, mn[c], w));
+                mx[c] = fmaxf(mx[c], __shfl_xor_sync(0xffffffffu, mx[c], w));
+            }
+        if (lane == 0) {
+            v.box_lo[blockIdx.x * kEnsSubs + k] = make_float4(mn[0], mn[1], mn[2], 0.0f);
+            v.box_hi[blockIdx.x * kEnsSubs + k] = make_float4(mx[0], mx[1], mx[2], 0.0f);
+        }
+    }
+}
+
+// the density of 32 particles (sub k of a group) by one warp, and their neighbour lists: the simulation's boxes within
+// h (1 + 1e-3) of the 32 particles' own, in order; sums in j order, compensated per 512 particles
+template <bool COMP>
+__device__ __forceinline__ void dens_near(const DevArrays& a, const DevParams& p, const EnsView& v, int group, int4 grp, int4 sm,
+                                          int k, float4* sh) {
+    const int lane = threadIdx.x & 31;
+    const int o = k * kEnsSub + lane;
+    const bool valid = o < grp.z;
+    const int64_t i = static_cast<int64_t>(grp.y) + (valid ? o : 0);
+    const float4 pi = a.posm[i];
+    const float4 l = v.box_lo[group * kEnsSubs + k], u = v.box_hi[group * kEnsSubs + k];
+    const uint32_t span = __float_as_uint(p.H2);
+    const float hm = p.H * (1.0f + kMargin), hm2 = hm * hm;
+    const int b0 = sm.z * kEnsSubs, nb = sm.w * kEnsSubs;
+    float rho = 0.0f, rhoc = 0.0f, t = 0.0f;
+    int cnt = 0, tile = 0;
+    auto end_tile = [&]() {
+        if (COMP) {
+            fold(rho, rhoc, t);
+            t = 0.0f;
+        }
+    };
+    for (int c0 = 0; c0 < nb; c0 += 32) {
+        bool near = false;
+        if (c0 + lane < nb) {
+            const float4 bl = v.box_lo[b0 + c0 + lane], bu = v.box_hi[b0 + c0 + lane];
+            const float gx = fmaxf(0.0f, fmaxf(bl.x - u.x, l.x - bu.x)), gy = fmaxf(0.0f, fmaxf(bl.y - u.y, l.y - bu.y)),
+                        gz = fmaxf(0.0f, fmaxf(bl.z - u.z, l.z - bu.z));
+            near = !(gx * gx + gy * gy + gz * gz > hm2);
+        }
+        unsigned todo = __ballot_sync(0xffffffffu, near);
+        // the next box's positions are in flight while one is tested; particles past the end are no one's neighbours
+        auto fetch = [&](int b) {
+            const int j = (c0 + b) * kEnsSub + lane;
+            return j < sm.y ? a.posm[static_cast<int64_t>(sm.x) + j] : make_float4(INFINITY, INFINITY, INFINITY, 0.0f);
+        };
+        float4 qn = make_float4(0, 0, 0, 0);
+        if (todo) qn = fetch(__ffs(todo) - 1);
+        while (todo) {
+            const int b = __ffs(todo) - 1;
+            todo &= todo - 1;
+            const float4 q0 = qn;
+            if (todo) qn = fetch(__ffs(todo) - 1);
+            __syncwarp();  // the previous box's reads are done
+            sh[lane] = q0;
+            __syncwarp();
+            unsigned m4[4];
+#pragma unroll
+            for (int w = 0; w < 4; ++w) {
+                unsigned m = 0;
+#pragma unroll
+                for (int s = 0; s < 8; ++s) {
+                    const float4 q = sh[8 * w + s];
+                    const float dx = q.x - pi.x, dy = q.y - pi.y, dz = q.z - pi.z;
+                    const float r2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
+                    m |= static_cast<unsigned>((__float_as_uint(r2) - 1u) < span) << s;  // 0 < r2 <= H2
+                }
+                m4[w] = m;
+            }
+            unsigned m = m4[0] | (m4[1] << 8) | (m4[2] << 16) | (m4[3] << 24);
+            if (COMP && (c0 + b) / kEnsSubs != tile) {
+                end_tile();
+                tile = (c0 + b) / kEnsSubs;
+            }
+            const int jb = sm.x + (c0 + b) * kEnsSub;
+            while (m) {
+                const int s = __ffs(m) - 1;
+                m &= m - 1;
+                const float4 q = sh[s];
+                const float dx = q.x - pi.x, dy = q.y - pi.y, dz = q.z - pi.z;
+                const float r2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
+                const float w = q.w * w_poly(r2 * rsqrtf(r2) * p.inv_h);
+                if (COMP) t += w;
+                else rho += w;
+                if (valid && cnt < kEnsCap) v.nb[static_cast<int64_t>(cnt) * v.n + i] = jb + s;
+                cnt = min(cnt + 1, kEnsCap + 1);
             }
         }
-    return true;
+    }
+    end_tile();
+    if (!valid) return;
+    float4 vr = a.velrho[i];
+    if (!has(p, GSPH_INTEGRATE_DENSITY)) {  // calcDensity::do_after (:80-90)
+        float r = COMP ? static_cast<float>((static_cast<double>(rho) + static_cast<double>(rhoc)) * static_cast<double>(p.w_pref))
+                       : rho * p.w_pref;
+        if (has(p, GSPH_DEAL_WITH_NO_PARTNERS) && r < 0.001f) r = p.rho0 * 0.01f;
+        vr.w = r;
+        a.velrho[i] = vr;
+    }
+    float4 jA, jB;
+    make_jrecord(p, vr.w, a.sA[i], a.sB[i], a.balsara[i], jA, jB);
+    a.jA[i] = jA;
+    a.jB[i] = jB;
+    v.nbcnt[i] = cnt;
 }
 
 // the raw gravity sum of particle i (local index l of simulation `sim`): its G + 1 slots in FP64, in order
@@ -565,49 +679,47 @@ __device__ __forceinline__ void sph_item(const DevArrays& a, const DevParams& p,
     }
 }
 
-template <int GRAV, bool SPH, int PASS, bool SOLIDS, bool COMP, bool SYM>
+// NEAR: the density by boxes; gravity, when on, comes from the slots of k_ens_gravity. Otherwise both come from the
+// sweep of dens_item.
+template <int GRAV, bool SPH, int PASS, bool SOLIDS, bool COMP, bool NEAR>
 __global__ void __launch_bounds__(kEnsThreads) k_ensemble(DevArrays a, DevParams p, EnsView v) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ int s_item, s_flag;
     __shared__ float s_box[6 * (kEnsThreads / 32) + 12];  // reduction scratch, group box, tile box
-    __shared__ float s_js[SYM ? kEnsThreads / 32 : 1][kEnsJC][3];  // GSYM: per-warp column sums of a round
     RangePipe pipe;
-    pipe.buf = reinterpret_cast<float4*>(smem_raw);
-    pipe.tile = v.tile;
-    pipe.bar = reinterpret_cast<uint64_t*>(smem_raw + 2 * static_cast<size_t>(v.tile) * sizeof(float4));
-    pipe.src = a.posm;
-    pipe.status = a.status;
-    pipe.init();
-    const int total = v.ntasks + v.ngroups * v.nstages;
+    if (!NEAR) {
+        pipe.buf = reinterpret_cast<float4*>(smem_raw);
+        pipe.tile = v.tile;
+        pipe.bar = reinterpret_cast<uint64_t*>(smem_raw + 2 * static_cast<size_t>(v.tile) * sizeof(float4));
+        pipe.src = a.posm;
+        pipe.status = a.status;
+        pipe.init();
+    }
+    const int total = v.ngroups * v.nstages;
     for (;;) {
         if (threadIdx.x == 0) s_item = atomicAdd(v.head, 1);
         __syncthreads();
-        const int q0 = s_item;
+        const int q = s_item;
         __syncthreads();
-        if (q0 >= total) break;
-        if (q0 < v.ntasks) {  // GSYM: a pair of groups of one simulation
-            if (SYM && GRAV != 0 && SPH) {
-                const int4 task = v.tasks[q0];
-                if (!gsym_item<GRAV, COMP>(a, p, v, pipe, task, v.sims[task.x], s_js)) return;
-                signal_done(v.done + 2 * v.nsims + task.x);
-            }
-            continue;
-        }
-        const int q = q0 - v.ntasks;
+        if (q >= total) break;
         const int si = q / v.ngroups;  // (branches, not an index: keeps the parameter block out of local memory)
         const int stage = si == 0 ? v.stages[0] : (si == 1 ? v.stages[1] : v.stages[2]);
-        const int4 grp = v.groups[q % v.ngroups];
+        const int group = q % v.ngroups;
+        const int4 grp = v.groups[group];
         const int sim = grp.x;
         const int4 sm = v.sims[sim];
         if (stage == ST_DENS) {
-            const bool ok = SYM ? dens_item<0, SPH, COMP>(a, p, v, pipe, grp, sm, s_box)
-                                : dens_item<GRAV, SPH, COMP>(a, p, v, pipe, grp, sm, s_box);
-            if (!ok) return;
+            if constexpr (NEAR) {
+                float4* sh = reinterpret_cast<float4*>(smem_raw) + (threadIdx.x >> 5) * kEnsSub;
+                for (int k = threadIdx.x >> 5; k * kEnsSub < grp.z; k += kEnsThreads / 32)
+                    dens_near<COMP>(a, p, v, group, grp, sm, k, sh);
+            } else {
+                if (!dens_item<GRAV, SPH, COMP>(a, p, v, pipe, grp, sm, s_box)) return;
+            }
             signal_done(v.done + sim);
         } else if (stage == ST_SPH) {
             if (!wait_count(v.done + sim, sm.w + (sim == v.stall_sim ? 1 : 0), a.status, &s_flag)) return;
-            if (SYM && !wait_count(v.done + 2 * v.nsims + sim, sm.w * (sm.w + 1) / 2, a.status, &s_flag)) return;
-            sph_item<GRAV, PASS, SOLIDS, COMP, SYM>(a, p, v, grp, sm);
+            sph_item<GRAV, PASS, SOLIDS, COMP, NEAR && GRAV != 0>(a, p, v, grp, sm);
             signal_done(v.done + v.nsims + sim);
         } else {
             if (v.kick_dep >= 0 && !wait_count(v.done + v.kick_dep * v.nsims + sim, sm.w, a.status, &s_flag)) return;
@@ -777,11 +889,8 @@ size_t ens_smem(int tile) { return pipe_smem_bytes(1, tile); }
 template <int GRAV, bool SPH, int PASS, bool SOLIDS, bool COMP>
 cudaError_t launch_t(const DevArrays& a, const DevParams& p, const EnsView& v, int sm_count, int per_sm_cap,
                      cudaStream_t s) {
-    // the symmetric-gravity form is its own instantiation (gravity + SPH only), so the one-sided
-    // kernels keep their register budget
-    auto kern = (SPH && GRAV != 0 && v.sym) ? k_ensemble<GRAV, SPH, PASS, SOLIDS, COMP, true>
-                                            : k_ensemble<GRAV, SPH, PASS, SOLIDS, COMP, false>;
-    const size_t smem = ens_smem(v.tile);
+    auto kern = SPH && v.near ? k_ensemble<GRAV, SPH, PASS, SOLIDS, COMP, SPH> : k_ensemble<GRAV, SPH, PASS, SOLIDS, COMP, false>;
+    const size_t smem = SPH && v.near ? kEnsThreads * sizeof(float4) : ens_smem(v.tile);
     cudaError_t e = cudaSuccess;
     if (smem > 48 * 1024) e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
     if (e != cudaSuccess) return e;
@@ -790,7 +899,7 @@ cudaError_t launch_t(const DevArrays& a, const DevParams& p, const EnsView& v, i
     if (e != cudaSuccess) return e;
     per_sm = std::max(per_sm, 1);
     if (per_sm_cap > 0) per_sm = std::min(per_sm, per_sm_cap);
-    const int total = v.ntasks + v.ngroups * v.nstages;
+    const int total = v.ngroups * v.nstages;
     const int grid = std::max(1, std::min(total, sm_count * per_sm));
     kern<<<grid, kEnsThreads, smem, s>>>(a, p, v);
     return cudaGetLastError();
@@ -840,10 +949,11 @@ struct gsph_ensemble {
     std::vector<int64_t> offsets;   // host: nsims + 1
     int4* groups = nullptr;         // device tables
     int4* sims = nullptr;
-    int* counters = nullptr;        // [1 + 3 S]: queue head; finished DENS, SPH and GSYM items per simulation
-    bool sym = false;               // symmetric gravity stage (GSYM) instead of gravity in the DENS sweep
+    int* counters = nullptr;        // [1 + 2 S]: queue head; finished DENS and SPH items per simulation
+    bool near = false;              // density by boxes of 32 particles, gravity from pairs of groups
+    float4 *box_lo = nullptr, *box_hi = nullptr;
     int ntasks = 0;
-    int4* tasks = nullptr;          // GSYM tasks (sim, row group, column group, 0)
+    int4* tasks = nullptr;          // gravity tasks (sim, row group, column group, 0)
     long long* slot_base = nullptr; // [S] first float of each simulation's slots in gslot
     float* gslot = nullptr;
     int inject_stall = -1;          // failure-path test: stall this simulation's SPH items once
@@ -932,11 +1042,10 @@ EnsView view_of(const gsph_ensemble* e, const int* stages, int nstages) {
     v.kick_dt = e->dp.fixed_dt;
     v.tile = e->tile;
     v.stall_sim = -1;
-    v.sym = e->sym ? 1 : 0;
+    v.near = e->near ? 1 : 0;
+    v.box_lo = e->box_lo;
+    v.box_hi = e->box_hi;
     v.tasks = e->tasks;
-    v.ntasks = 0;
-    for (int k = 0; k < nstages; ++k)  // the GSYM tasks run with the DENS stage
-        if (stages[k] == ST_DENS && e->sym) v.ntasks = e->ntasks;
     v.gslot = e->gslot;
     v.slot_base = e->slot_base;
     return v;
@@ -948,7 +1057,18 @@ int run_stages(gsph_ensemble* e, const int* stages, int nstages, float kick_dt, 
     v.kick_dt = kick_dt;
     v.stall_sim = e->inject_stall;  // one-shot failure-path test hook
     e->inject_stall = -1;
-    ENS_CK(e, cudaMemsetAsync(e->counters, 0, (1 + 3 * static_cast<size_t>(e->nsims)) * sizeof(int), s), "counter reset");
+    ENS_CK(e, cudaMemsetAsync(e->counters, 0, (1 + 2 * static_cast<size_t>(e->nsims)) * sizeof(int), s), "counter reset");
+    if (e->near && stages[0] == ST_DENS) {
+        k_ens_boxes<<<static_cast<unsigned>(e->ngroups), kEnsThreads, 0, s>>>(e->a.posm, v);
+        if (e->ntasks) {
+            const bool comp = e->opt.accum == GSPH_ACCUM_COMPENSATED;
+            auto kern = e->dp.eps2 > 0.0f ? (comp ? k_ens_gravity<1, true> : k_ens_gravity<1, false>)
+                                          : (comp ? k_ens_gravity<2, true> : k_ens_gravity<2, false>);
+            kern<<<static_cast<unsigned>(e->ntasks), SymE::T, 0, s>>>(e->a.posm, v, e->dp.eps2);
+        }
+        ENS_CK(e, cudaGetLastError(), "boxes and gravity");
+        e->launches += 1 + (e->ntasks ? 1 : 0);
+    }
     ENS_CK(e, launch_ensemble(e->a, e->dp, v, e->opt.accum == GSPH_ACCUM_COMPENSATED, e->sm_count, e->per_sm_cap, s),
            "ensemble launch");
     e->launches += 1;
@@ -1057,16 +1177,25 @@ int gsph_ensemble_create(const gsph_params* p, const gsph_options* opt, int32_t 
                             static_cast<int>(groups.size()) - first);
     }
     e->ngroups = static_cast<int>(groups.size());
-    // symmetric gravity (GSYM) for gravity + SPH ensembles when asked for (the default is the one-sided
-    // sweep fused with the density pass, faster on ensembles of 1k..32k-particle simulations: 45.2 vs 51.6 ms
-    // per step on 512 of them, 4.63M particles): tasks (ga <= gb) of each simulation, simulations largest
-    // first and in each the off-diagonal pairs before the (half-sized) diagonal ones; G + 1 slots of K
-    // floats per particle
-    e->sym = (p->flags & GSPH_SELF_GRAVITY) && (p->flags & GSPH_SPH) && o.gravity_form == GSPH_GRAVITY_SYMMETRIC;
+    // Gravity + SPH ensembles take their gravity from pairs of groups (k_ens_gravity) unless the one-sided sweep is asked
+    // for or the slots would outgrow the 1 KB neighbour list of a particle: G + 1 slots of K floats each, so plain
+    // simulations up to about 43,000 particles on average (compensated: half of that), unless SYMMETRIC is asked for.
+    // Tasks (ga <= gb) of each simulation, simulations largest first and in each the off-diagonal pairs before the
+    // (half-sized) diagonal ones.
+    const bool sph = (p->flags & GSPH_SPH) != 0, grav = (p->flags & GSPH_SELF_GRAVITY) != 0;
+    {
+        const double K = o.accum == GSPH_ACCUM_COMPENSATED ? 6 : 3;
+        double floats = 0.0;
+        for (int s = 0; s < nsims; ++s) floats += (sims[s].w + 1.0) * K * static_cast<double>(counts[s]);
+        const bool fits = floats <= static_cast<double>(kEnsCap) * static_cast<double>(total);
+        e->near = sph && o.gravity_form != GSPH_GRAVITY_ONE_SIDED &&
+                  (!grav || o.gravity_form == GSPH_GRAVITY_SYMMETRIC || fits);
+    }
+    const bool slots = e->near && grav;
     std::vector<int4> tasks;
     std::vector<long long> slot_base(nsims, 0);
     long long slot_floats = 0;
-    if (e->sym) {
+    if (slots) {
         const int K = o.accum == GSPH_ACCUM_COMPENSATED ? 6 : 3;
         for (int s : order) {
             const int G = sims[s].w;
@@ -1096,8 +1225,12 @@ int gsph_ensemble_create(const gsph_params* p, const gsph_options* opt, int32_t 
     a.status = static_cast<int*>(ens_alloc(e, 4 * sizeof(int), ae));
     e->groups = static_cast<int4*>(ens_alloc(e, groups.size() * sizeof(int4), ae));
     e->sims = static_cast<int4*>(ens_alloc(e, sims.size() * sizeof(int4), ae));
-    e->counters = static_cast<int*>(ens_alloc(e, (1 + 3 * static_cast<size_t>(nsims)) * sizeof(int), ae));
-    if (e->sym) {
+    e->counters = static_cast<int*>(ens_alloc(e, (1 + 2 * static_cast<size_t>(nsims)) * sizeof(int), ae));
+    if (e->near) {
+        e->box_lo = static_cast<float4*>(ens_alloc(e, groups.size() * kEnsSubs * sizeof(float4), ae));
+        e->box_hi = static_cast<float4*>(ens_alloc(e, groups.size() * kEnsSubs * sizeof(float4), ae));
+    }
+    if (slots) {
         e->tasks = static_cast<int4*>(ens_alloc(e, tasks.size() * sizeof(int4), ae));
         e->slot_base = static_cast<long long*>(ens_alloc(e, slot_base.size() * sizeof(long long), ae));
         e->gslot = static_cast<float*>(ens_alloc(e, static_cast<size_t>(slot_floats) * sizeof(float), ae));
@@ -1123,9 +1256,9 @@ int gsph_ensemble_create(const gsph_params* p, const gsph_options* opt, int32_t 
     e->bbox = static_cast<float*>(ens_alloc(e, static_cast<size_t>(nsims) * 8 * sizeof(float), ae));
     if (ae == cudaSuccess) ae = cudaMemcpy(e->groups, groups.data(), groups.size() * sizeof(int4), cudaMemcpyHostToDevice);
     if (ae == cudaSuccess) ae = cudaMemcpy(e->sims, sims.data(), sims.size() * sizeof(int4), cudaMemcpyHostToDevice);
-    if (ae == cudaSuccess && e->sym)
+    if (ae == cudaSuccess && slots)
         ae = cudaMemcpy(e->tasks, tasks.data(), tasks.size() * sizeof(int4), cudaMemcpyHostToDevice);
-    if (ae == cudaSuccess && e->sym)
+    if (ae == cudaSuccess && slots)
         ae = cudaMemcpy(e->slot_base, slot_base.data(), slot_base.size() * sizeof(long long), cudaMemcpyHostToDevice);
     if (ae == cudaSuccess) {  // status[1]: the dependency-wait bound in microseconds (0: the default)
         const int lim = std::max(0, o.wait_limit_us);

@@ -17,6 +17,7 @@
 #include <type_traits>
 
 #include "f32x2.cuh"
+#include "gravity_sym.cuh"
 #include "pairs.cuh"
 #include "sph.cuh"
 
@@ -668,15 +669,6 @@ __global__ void __launch_bounds__(128) k_gravity_x2(const float4* __restrict__ p
 // 0.60 of the FMA rate, multiplies and adds (four) at 0.96; six of a pair's operations are such multiply-adds, which
 // predicts 0.77. Keeping each pair that shares both factors together lets the operand cache serve the second: 0.81.
 // Measured (N = 262,144, 128 groups, one B200): row-packed 22.3 ms, column-packed 18.6 ms, equal masses 15.8 ms.
-template <int R_, int T_, int CTAS_>
-struct SymShape {
-    static constexpr int R = R_, T = T_, B = R_ * T_, CTAS = CTAS_;
-    static constexpr int JT = B < 256 ? B : 256;  // columns per tile
-    static constexpr int PF = JT / T_;            // records a thread stages
-    static constexpr int W = T_ / 32;
-    static_assert(JT % 64 == 0 && B % JT == 0 && JT % T_ == 0, "symmetric gravity tiles");
-};
-
 __host__ __device__ __forceinline__ void sym_task(int t, int G, int& ga, int& gb) {
     const int noff = G * (G - 1) / 2;
     if (t >= noff) {
@@ -692,19 +684,6 @@ __host__ __device__ __forceinline__ void sym_task(int t, int G, int& ga, int& gb
     gb = r + 1 + rem;
 }
 
-// T += d s, c += d s for the three components: each pair of multiply-adds with common factors back to back
-__device__ __forceinline__ void add_both(float2& tx, float2& ty, float2& tz, float2& cx, float2& cy, float2& cz, float2 dx,
-                                         float2 dy, float2 dz, float2 s) {
-    uint64_t t0 = u64_of(tx), t1 = u64_of(ty), t2 = u64_of(tz), c0 = u64_of(cx), c1 = u64_of(cy), c2 = u64_of(cz);
-    asm("fma.rn.f32x2 %0, %6, %9, %0;\n fma.rn.f32x2 %3, %6, %9, %3;\n"
-        " fma.rn.f32x2 %1, %7, %9, %1;\n fma.rn.f32x2 %4, %7, %9, %4;\n"
-        " fma.rn.f32x2 %2, %8, %9, %2;\n fma.rn.f32x2 %5, %8, %9, %5;\n"
-        : "+l"(t0), "+l"(t1), "+l"(t2), "+l"(c0), "+l"(c1), "+l"(c2)
-        : "l"(u64_of(dx)), "l"(u64_of(dy)), "l"(u64_of(dz)), "l"(u64_of(s)));
-    tx = f2_of(t0); ty = f2_of(t1); tz = f2_of(t2);
-    cx = f2_of(c0); cy = f2_of(c1); cz = f2_of(c2);
-}
-
 template <typename S, int GRAV, bool COMP>
 __global__ void __launch_bounds__(S::T, S::CTAS) k_gravity_sym(const float4* __restrict__ posm, float* __restrict__ part,
                                                                int64_t n_pad, int G, int gs, float eps2) {
@@ -714,7 +693,7 @@ __global__ void __launch_bounds__(S::T, S::CTAS) k_gravity_sym(const float4* __r
     __shared__ float js[W][3][JT];
     __shared__ float rsh[3 * R][T];             // the row particles' running sums ...
     __shared__ float csh[COMP ? 3 * R : 1][T];  // ... and, compensated, their rounding errors
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int tid = threadIdx.x, warp = tid >> 5;
     int ga, gb;
     sym_task(static_cast<int>(blockIdx.x), G, ga, gb);
     const int nb = static_cast<int>(n_pad / B);
@@ -729,18 +708,16 @@ __global__ void __launch_bounds__(S::T, S::CTAS) k_gravity_sym(const float4* __r
         for (int e = tid; e < B; e += T)
             for (int c = 0; c < K; ++c) *slot(static_cast<int64_t>(ra0) * B + e, s_col, c) = 0.0f;
     const float2 E2 = make_float2(eps2, eps2);
-    const float2 zero2 = make_float2(0.0f, 0.0f);
 
     for (int a = ra0; a < ra1; ++a) {
         const int64_t base = static_cast<int64_t>(a) * B + tid;
-        float2 X[R], Y[R], Z[R], M[R];  // negated: a difference is an addition, a column's share a product
+        SymRows<S> rows;
         const float mr = posm[static_cast<int64_t>(a) * B].w;
         bool same = true;
 #pragma unroll
         for (int k = 0; k < R; ++k) {
             const float4 u = posm[base + static_cast<int64_t>(k) * T];
-            X[k] = make_float2(-u.x, -u.x); Y[k] = make_float2(-u.y, -u.y); Z[k] = make_float2(-u.z, -u.z);
-            M[k] = make_float2(-u.w, -u.w);
+            rows.set(k, u);
             same = same && u.w == mr;
 #pragma unroll
             for (int c = 0; c < 3; ++c) {
@@ -770,11 +747,7 @@ __global__ void __launch_bounds__(S::T, S::CTAS) k_gravity_sym(const float4* __r
             bool same_c = true;
 #pragma unroll
             for (int h = 0; h < PF; ++h) {
-                const int j = tid + h * T, half = (j >> 5) & 1, q = (j >> 6) * 32 + (j & 31);
-                float* xy = reinterpret_cast<float*>(&XY[q]);
-                float* zm = reinterpret_cast<float*>(&ZM[q]);
-                xy[half] = pf[h].x; xy[2 + half] = pf[h].y;
-                zm[half] = pf[h].z; zm[2 + half] = pf[h].w;
+                sym_stage(XY, ZM, tid + h * T, pf[h]);
                 same_c = same_c && pf[h].w == mc;
             }
             const bool equal = __syncthreads_and(same_c) && rows_equal;
@@ -783,67 +756,10 @@ __global__ void __launch_bounds__(S::T, S::CTAS) k_gravity_sym(const float4* __r
 #pragma unroll
                 for (int h = 0; h < PF; ++h) pf[h] = posm[src(k + 1) + h * T + tid];
             }
-            float2 TX[R], TY[R], TZ[R];
-#pragma unroll
-            for (int q = 0; q < R; ++q) TX[q] = TY[q] = TZ[q] = zero2;
-            // one column pair against row m: the separations and 1/r^3
-            auto pair = [&](int m, float4 xy, float4 zm, float2& dx, float2& dy, float2& dz) {
-                dx = add2(make_float2(xy.x, xy.y), X[m]);
-                dy = add2(make_float2(xy.z, xy.w), Y[m]);
-                dz = add2(make_float2(zm.x, zm.y), Z[m]);
-                const float2 r2 = fma2(dz, dz, fma2(dy, dy, fma2(dx, dx, E2)));
-                float2 inv = make_float2(rsqrtf(r2.x), rsqrtf(r2.y));
-                if (GRAV == 2) inv = make_float2(fminf(inv.x, 1e12f), fminf(inv.y, 1e12f));
-                return mul2(mul2(inv, inv), inv);
-            };
-            auto columns = [&](auto eq) {
-                constexpr bool EQ = decltype(eq)::value;
-                const int next = (lane + 1) & 31;
-#pragma unroll 1
-                for (int j0 = 0; j0 < JT / 2; j0 += 32) {
-                    float2 cx = zero2, cy = zero2, cz = zero2;
-#pragma unroll 2
-                    for (int r = 0; r < 32; ++r) {
-                        const int j = j0 + ((lane + r) & 31);
-                        const float4 xy = XY[j], zm = ZM[j];
-#pragma unroll
-                        for (int m = 0; m < R; ++m) {
-                            float2 dx, dy, dz;
-                            const float2 i3 = pair(m, xy, zm, dx, dy, dz);
-                            if (EQ) {
-                                add_both(TX[m], TY[m], TZ[m], cx, cy, cz, dx, dy, dz, i3);
-                            } else {
-                                const float2 sj = mul2(make_float2(zm.z, zm.w), i3), si = mul2(M[m], i3);
-                                TX[m] = fma2(dx, sj, TX[m]); TY[m] = fma2(dy, sj, TY[m]); TZ[m] = fma2(dz, sj, TZ[m]);
-                                cx = fma2(dx, si, cx); cy = fma2(dy, si, cy); cz = fma2(dz, si, cz);
-                            }
-                        }
-                        cx.x = __shfl_sync(0xffffffffu, cx.x, next); cx.y = __shfl_sync(0xffffffffu, cx.y, next);
-                        cy.x = __shfl_sync(0xffffffffu, cy.x, next); cy.y = __shfl_sync(0xffffffffu, cy.y, next);
-                        cz.x = __shfl_sync(0xffffffffu, cz.x, next); cz.y = __shfl_sync(0xffffffffu, cz.y, next);
-                    }
-                    const int j = 2 * j0 + lane;
-                    js[warp][0][j] = cx.x; js[warp][0][j + 32] = cx.y;
-                    js[warp][1][j] = cy.x; js[warp][1][j + 32] = cy.y;
-                    js[warp][2][j] = cz.x; js[warp][2][j + 32] = cz.y;
-                }
-            };
-            if (k < nd) {  // one-sided
-#pragma unroll 2
-                for (int j = 0; j < JT / 2; ++j) {
-                    const float4 xy = XY[j], zm = ZM[j];
-#pragma unroll
-                    for (int m = 0; m < R; ++m) {
-                        float2 dx, dy, dz;
-                        const float2 sj = mul2(make_float2(zm.z, zm.w), pair(m, xy, zm, dx, dy, dz));
-                        TX[m] = fma2(dx, sj, TX[m]); TY[m] = fma2(dy, sj, TY[m]); TZ[m] = fma2(dz, sj, TZ[m]);
-                    }
-                }
-            } else if (equal) {
-                columns(std::true_type{});
-            } else {
-                columns(std::false_type{});
-            }
+            rows.clear();
+            if (k < nd) sym_own<S, GRAV>(rows, XY, ZM, E2);
+            else if (equal) sym_columns<S, GRAV, true>(rows, XY, ZM, E2, js[warp]);
+            else sym_columns<S, GRAV, false>(rows, XY, ZM, E2, js[warp]);
             // the tile's row partials into the running sums: a two-sum fold (compensated), or one add (plain: a sum
             // of tile sums, not one running sum over the whole column group)
             const float wr = k >= nd && equal ? mc : 1.0f;
@@ -860,9 +776,9 @@ __global__ void __launch_bounds__(S::T, S::CTAS) k_gravity_sym(const float4* __r
             };
 #pragma unroll
             for (int m = 0; m < R; ++m) {
-                row_add(m, TX[m]);
-                row_add(R + m, TY[m]);
-                row_add(2 * R + m, TZ[m]);
+                row_add(m, rows.TX[m]);
+                row_add(R + m, rows.TY[m]);
+                row_add(2 * R + m, rows.TZ[m]);
             }
             if (k >= nd) {  // this tile's column sums over the CTA's row block, into the column slot
                 __syncthreads();
