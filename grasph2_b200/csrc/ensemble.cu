@@ -619,6 +619,8 @@ __device__ __forceinline__ void dens_near(const DevArrays& a, const DevParams& p
     make_jrecord(p, vr.w, a.sA[i], a.sB[i], a.balsara[i], jA, jB);
     a.jA[i] = jA;
     a.jB[i] = jB;
+    float4* r = a.jrec + 4 * i;
+    r[0] = pi; r[1] = vr; r[2] = jA; r[3] = jB;
     v.nbcnt[i] = cnt;
 }
 
@@ -640,7 +642,9 @@ __device__ __forceinline__ void gsym_fold(const EnsView& v, int sim, int4 sm, in
 }
 
 // ---- SPH: the neighbour lists, then the per-particle epilogue --------------------------------------
-template <int GRAV, int PASS, bool SOLIDS, bool COMP, bool SYM>
+// RECS: the DENS stage left packed 64-byte records (a.jrec): a gather touches one line instead of four, and the next
+// neighbour's record and the index after it are in flight while one is computed.
+template <int GRAV, int PASS, bool SOLIDS, bool COMP, bool RECS>
 __device__ __forceinline__ void sph_item(const DevArrays& a, const DevParams& p, const EnsView& v, int4 grp, int4 sm) {
     constexpr bool DO_A = PASS != PASS_VGRAD;
     const float4 zero = make_float4(0, 0, 0, 0);
@@ -656,20 +660,45 @@ __device__ __forceinline__ void sph_item(const DevArrays& a, const DevParams& p,
         float maxv = 0.0f;
         // the neighbour list, or every particle of the simulation when the list overflowed (same j order)
         const int cnt = v.nbcnt[i];
-        const bool over = cnt > kEnsCap;
-        const int64_t len = over ? static_cast<int64_t>(sm.y) : cnt;
-        for (int64_t m = 0; m < len; ++m) {
-            const int64_t j = over ? static_cast<int64_t>(sm.x) + m : v.nb[m * v.n + i];
-            const float4 q = __ldcg(a.posm + j);
-            const float dx = q.x - I.pi.x, dy = q.y - I.pi.y, dz = q.z - I.pi.z;
-            const float r2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
-            if (!in_open_closed(r2, 0u, span)) continue;
-            const float4 vj = __ldcg(a.velrho + j);
-            const float4 ja = DO_A ? __ldcg(a.jA + j) : zero, jb = DO_A ? __ldcg(a.jB + j) : zero;
-            sph_neighbour<PASS, SOLIDS>(T, maxv, I, q.w, dx, dy, dz, r2, vj, ja, jb, p);
+        if (RECS && cnt <= kEnsCap) {
+            const int* lst = v.nb + i;
+            const int j0 = cnt > 0 ? lst[0] : static_cast<int>(i);
+            int jn = cnt > 1 ? lst[v.n] : 0;  // the index of neighbour m + 1
+            const float4* r0 = a.jrec + 4 * static_cast<int64_t>(j0);
+            float4 qn = __ldcg(r0), vn = __ldcg(r0 + 1);
+            float4 an = DO_A ? __ldcg(r0 + 2) : zero, bn = DO_A ? __ldcg(r0 + 3) : zero;
+            for (int m = 0; m < cnt; ++m) {
+                const float4 q = qn, vj = vn, ja = an, jb = bn;
+                if (m + 1 < cnt) {
+                    const float4* r = a.jrec + 4 * static_cast<int64_t>(jn);
+                    qn = __ldcg(r);
+                    vn = __ldcg(r + 1);
+                    if (DO_A) {
+                        an = __ldcg(r + 2);
+                        bn = __ldcg(r + 3);
+                    }
+                }
+                if (m + 2 < cnt) jn = lst[static_cast<int64_t>(m + 2) * v.n];
+                const float dx = q.x - I.pi.x, dy = q.y - I.pi.y, dz = q.z - I.pi.z;
+                const float r2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
+                sph_neighbour<PASS, SOLIDS>(T, maxv, I, q.w, dx, dy, dz, r2, vj, ja, jb, p);
+            }
+        } else {
+            const bool over = cnt > kEnsCap;
+            const int64_t len = over ? static_cast<int64_t>(sm.y) : cnt;
+            for (int64_t m = 0; m < len; ++m) {
+                const int64_t j = over ? static_cast<int64_t>(sm.x) + m : v.nb[m * v.n + i];
+                const float4 q = __ldcg(a.posm + j);
+                const float dx = q.x - I.pi.x, dy = q.y - I.pi.y, dz = q.z - I.pi.z;
+                const float r2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
+                if (!in_open_closed(r2, 0u, span)) continue;
+                const float4 vj = __ldcg(a.velrho + j);
+                const float4 ja = DO_A ? __ldcg(a.jA + j) : zero, jb = DO_A ? __ldcg(a.jB + j) : zero;
+                sph_neighbour<PASS, SOLIDS>(T, maxv, I, q.w, dx, dy, dz, r2, vj, ja, jb, p);
+            }
         }
         float g[3];
-        if (SYM) {
+        if (RECS && GRAV != 0) {
             gsym_fold<COMP>(v, grp.x, sm, i, g);
         } else {
             const float4 gr = a.acc[i];
@@ -719,7 +748,7 @@ __global__ void __launch_bounds__(kEnsThreads) k_ensemble(DevArrays a, DevParams
             signal_done(v.done + sim);
         } else if (stage == ST_SPH) {
             if (!wait_count(v.done + sim, sm.w + (sim == v.stall_sim ? 1 : 0), a.status, &s_flag)) return;
-            sph_item<GRAV, PASS, SOLIDS, COMP, NEAR && GRAV != 0>(a, p, v, grp, sm);
+            sph_item<GRAV, PASS, SOLIDS, COMP, NEAR>(a, p, v, grp, sm);
             signal_done(v.done + v.nsims + sim);
         } else {
             if (v.kick_dep >= 0 && !wait_count(v.done + v.kick_dep * v.nsims + sim, sm.w, a.status, &s_flag)) return;
@@ -1229,6 +1258,7 @@ int gsph_ensemble_create(const gsph_params* p, const gsph_options* opt, int32_t 
     if (e->near) {
         e->box_lo = static_cast<float4*>(ens_alloc(e, groups.size() * kEnsSubs * sizeof(float4), ae));
         e->box_hi = static_cast<float4*>(ens_alloc(e, groups.size() * kEnsSubs * sizeof(float4), ae));
+        a.jrec = static_cast<float4*>(ens_alloc(e, 4 * n_pad * sizeof(float4), ae));
     }
     if (slots) {
         e->tasks = static_cast<int4*>(ens_alloc(e, tasks.size() * sizeof(int4), ae));
