@@ -6,6 +6,7 @@
 #include <new>
 #include <string>
 
+#include "f32x2.cuh"
 #include "umma.cuh"
 
 void set_global_error(const std::string& msg);  // capi.cu
@@ -117,13 +118,36 @@ __device__ __forceinline__ float tanh_hw(float x) {
     asm("tanh.approx.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
 }
-__device__ __forceinline__ float silu(float z) {
-    const float u = 0.5f * z;
-    return fmaf(u, tanh_hw(u), u);
+// Two columns at a time (f32x2): 2.5 instructions per value instead of 4.5 (u = (z + b) / 2 is one multiply-add with
+// half the bias, exact as scaling by 2 is), so the epilogues are bound by the tanh units.
+__device__ __forceinline__ float2 silu2(float2 v, float2 half_bias) {  // SiLU(v + bias)
+    const float2 u = fma2(make_float2(0.5f, 0.5f), v, half_bias);
+    return fma2(u, make_float2(tanh_hw(u.x), tanh_hw(u.y)), u);
 }
-__device__ __forceinline__ float dsilu(float z) {
-    const float s = fmaf(0.5f, tanh_hw(0.5f * z), 0.5f);
-    return s * fmaf(z, 1.0f - s, 1.0f);
+__device__ __forceinline__ float2 dsilu2(float2 z) {
+    const float2 h = make_float2(0.5f, 0.5f), one = make_float2(1.0f, 1.0f);
+    const float2 u = mul2(h, z);
+    const float2 s = fma2(h, make_float2(tanh_hw(u.x), tanh_hw(u.y)), h);
+    return mul2(s, fma2(z, sub2(one, s), one));
+}
+// 32 accumulator columns -> bf16 SiLU(v + bias) in row `row` of an activation buffer; HALF: `bias` holds the halves
+template <bool HALF>
+__device__ __forceinline__ void silu_store(float (&v)[32], const float* bias, unsigned char* buf, int row, int c0) {
+    const float2 half = make_float2(0.5f, 0.5f);
+#pragma unroll
+    for (int k = 0; k < 32; k += 4) {
+        const float4 b = *reinterpret_cast<const float4*>(bias + k);
+        float2 b0 = make_float2(b.x, b.y), b1 = make_float2(b.z, b.w);
+        if (!HALF) {
+            b0 = mul2(half, b0);
+            b1 = mul2(half, b1);
+        }
+        const float2 h0 = silu2(make_float2(v[k], v[k + 1]), b0);
+        const float2 h1 = silu2(make_float2(v[k + 2], v[k + 3]), b1);
+        v[k] = h0.x; v[k + 1] = h0.y; v[k + 2] = h1.x; v[k + 3] = h1.y;
+    }
+#pragma unroll
+    for (int k = 0; k < 32; k += 8) umma::st8(buf, row, c0 + k, kTileM, v + k);
 }
 
 // named CTA barrier `id` over `n` threads (a multiple of 32), and the same with an AND over a predicate
@@ -138,9 +162,9 @@ __device__ __forceinline__ bool named_and(int id, int n, bool v) {
     return r != 0;
 }
 
-// stage the packed weights (row-major bf16) into the core-matrix layout, biases as FP32
+// stage the packed weights (row-major bf16) into the core-matrix layout, biases as FP32 (the hidden layers' scaled)
 __device__ void stage_weights(unsigned char* sm, const __nv_bfloat16* __restrict__ wq, const float* __restrict__ bq,
-                              float* sbias) {
+                              float* sbias, float hidden_scale) {
     struct M { uint32_t s; int q, R, C; };
     const M mats[4] = {{sW1, qW1, kHid, kIn}, {sW2, qW2, kHid, kHid}, {sW3, qW3, kHid, kHid}, {sW4, qW4, kOutP, kHid}};
     for (int m = 0; m < 4; ++m) {
@@ -151,25 +175,7 @@ __device__ void stage_weights(unsigned char* sm, const __nv_bfloat16* __restrict
                 *reinterpret_cast<const uint4*>(wq + mats[m].q + r * C + c0);
         }
     }
-    for (int e = threadIdx.x; e < kBias; e += blockDim.x) sbias[e] = bq[e];
-}
-
-// one row of features (32 FP32) -> bf16 row t of the X buffer; zeros past the end
-__device__ __forceinline__ void load_x(unsigned char* sm, const float* __restrict__ x, int64_t p, int64_t n) {
-    float v[kIn];
-    if (p < n) {
-        const float4* src = reinterpret_cast<const float4*>(x + p * kIn);
-#pragma unroll
-        for (int k = 0; k < kIn / 4; ++k) {
-            const float4 q = src[k];
-            v[4 * k] = q.x; v[4 * k + 1] = q.y; v[4 * k + 2] = q.z; v[4 * k + 3] = q.w;
-        }
-    } else {
-#pragma unroll
-        for (int k = 0; k < kIn; ++k) v[k] = 0.0f;
-    }
-#pragma unroll
-    for (int c = 0; c < kIn; c += 8) umma::st8(sm + sX, threadIdx.x, c, kTileM, v + c);
+    for (int e = threadIdx.x; e < kBias; e += blockDim.x) sbias[e] = e < 3 * kHid ? hidden_scale * bq[e] : bq[e];
 }
 
 // thread 0: D(tD) = A * B^T, operands in shared memory (K-major: buffer rows = M/N; MN-major: buffer
@@ -202,19 +208,6 @@ __device__ __forceinline__ bool after_commit(uint64_t* bar, uint32_t& phase, int
     umma::fence_after();
     return ok;
 }
-// hidden-layer epilogue of row t: h = SiLU(D + b) into the activation buffer at `buf`
-__device__ __forceinline__ void hidden_out(uint32_t tD, const float* bias, unsigned char* buf) {
-#pragma unroll 1
-    for (int c0 = 0; c0 < kHid; c0 += 32) {
-        float v[32];
-        umma::ld32(umma::lane_addr(tD, c0), v);
-#pragma unroll
-        for (int k = 0; k < 32; ++k) v[k] = silu(v[k] + bias[c0 + k]);
-#pragma unroll
-        for (int k = 0; k < 32; k += 8) umma::st8(buf, threadIdx.x, c0 + k, kTileM, v + k);
-    }
-}
-
 // Forward over tiles of 128 rows (persistent grid): y[n][13] = MLP(x[n][32]). A CTA runs four
 // independent tile pipelines (slots) of one warpgroup each; a slot has its own buffer (inputs, then
 // activations), 128 tensor-memory columns (all 512 in use), MMA barrier and named CTA barrier, so while
@@ -230,7 +223,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1) k_mlp_forward(const float* __r
     __shared__ uint64_t bar[kSlots];
     __shared__ uint32_t tslot;
     float* sbias = reinterpret_cast<float*>(sm + sBiasF);
-    stage_weights(sm, wq, bq, sbias);
+    stage_weights(sm, wq, bq, sbias, 0.5f);
     if (threadIdx.x == 0) {
         for (int k = 0; k < kSlots; ++k) mbar_init(&bar[k], 1);
         fence_barrier_init();
@@ -274,10 +267,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1) k_mlp_forward(const float* __r
         for (int c0 = 0; c0 < kHid; c0 += 32) {
             float v[32];
             umma::ld32(umma::lane_addr(T, c0), v);
-#pragma unroll
-            for (int k = 0; k < 32; ++k) v[k] = silu(v[k] + bias[c0 + k]);
-#pragma unroll
-            for (int k = 0; k < 32; k += 8) umma::st8(sm + ho, row, c0 + k, kTileM, v + k);
+            silu_store<true>(v, bias + c0, sm + ho, row, c0);
         }
     };
     const int64_t tiles = (n + kTileM - 1) / kTileM;
@@ -323,36 +313,44 @@ __global__ void __launch_bounds__(kFwdThreads, 1) k_mlp_forward(const float* __r
 
 // ---- training: gradient of L = (1/n) sum_p sum_o w_o (y_po - t_po)^2 --------------------------------
 // Tile k goes to CTA k % grid; each CTA adds its tiles' weight and bias gradients into its own FP32
-// slice part[cta][kPartStride] (no atomics) and its loss into loss_part[cta]; a second kernel sums the
-// slices in CTA order, so the gradient is deterministic.
-__device__ __forceinline__ void rmw(float* a, float v) { *a += v; }
-// a[0..N) += v[0..N), a 16-byte aligned: N/4 vector loads and stores instead of N scalar ones (same sums)
+// slice part[cta][kPartStride] (no atomics; its first tile writes the slice) and its loss into loss_part[cta]; a second
+// kernel sums the slices in CTA order, so the gradient is deterministic.
+//
+// Four warpgroups per CTA: thread t of warpgroup c owns row t and the columns 32 c .. 32 c + 31 of every 128-column
+// accumulator. Bound: the serial chain of a tile (eight MMA groups with their waits, the epilogues between them, the L2
+// round trips of the slices); one CTA per SM, as the activations and weights fill the shared memory. One warpgroup
+// with all 128 columns took 179 us for 65,536 rows, 45 us a tile, its four schedulers a quarter busy with one warp each.
+constexpr int kTrainGroups = 4, kTrainThreads = kTrainGroups * kTileM;
+// a[0..N) = or += v[0..N), a 16-byte aligned: vector loads and stores instead of scalar ones (same sums)
 template <int N>
-__device__ __forceinline__ void rmw_row(float* a, const float* v) {
+__device__ __forceinline__ void add_row(float* a, const float* v, bool first) {
     static_assert(N % 4 == 0, "whole vectors");
     float4* q = reinterpret_cast<float4*>(a);
+    float4 r[N / 4];
+    if (!first) {
 #pragma unroll
-    for (int k = 0; k < N / 4; ++k) {
-        float4 r = q[k];
-        r.x += v[4 * k];
-        r.y += v[4 * k + 1];
-        r.z += v[4 * k + 2];
-        r.w += v[4 * k + 3];
-        q[k] = r;
+        for (int k = 0; k < N / 4; ++k) r[k] = q[k];
+    } else {
+#pragma unroll
+        for (int k = 0; k < N / 4; ++k) r[k] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     }
+#pragma unroll
+    for (int k = 0; k < N / 4; ++k)
+        q[k] = make_float4(r[k].x + v[4 * k], r[k].y + v[4 * k + 1], r[k].z + v[4 * k + 2], r[k].w + v[4 * k + 3]);
 }
+__device__ __forceinline__ void add_one(float* a, float v, bool first) { *a = first ? v : *a + v; }
 
-__global__ void __launch_bounds__(kTileM, 1) k_mlp_train(const float* __restrict__ x, const float* __restrict__ t,
-                                                        const float* __restrict__ wout, int64_t n,
-                                                        const __nv_bfloat16* __restrict__ wq,
-                                                        const float* __restrict__ bq, float* __restrict__ part,
-                                                        double* __restrict__ loss_part, int* status) {
+__global__ void __launch_bounds__(kTrainThreads, 1) k_mlp_train(const float* __restrict__ x, const float* __restrict__ t,
+                                                               const float* __restrict__ wout, int64_t n,
+                                                               const __nv_bfloat16* __restrict__ wq,
+                                                               const float* __restrict__ bq, float* __restrict__ part,
+                                                               double* __restrict__ loss_part, int* status) {
     extern __shared__ __align__(1024) unsigned char sm[];
     __shared__ uint64_t bar;
     __shared__ uint32_t tslot;
     __shared__ double red[kTileM / 32];
     float* sbias = reinterpret_cast<float*>(sm + sBiasT);
-    stage_weights(sm, wq, bq, sbias);
+    stage_weights(sm, wq, bq, sbias, 1.0f);
     for (int e = threadIdx.x; e < kTileM * 16 / 8; e += blockDim.x) {  // ones[128][16]
         const uint4 one = make_uint4(0x3F803F80u, 0x3F803F80u, 0x3F803F80u, 0x3F803F80u);  // bf16 1.0 x 8
         *reinterpret_cast<uint4*>(sm + sOnes + e * 16) = one;
@@ -372,29 +370,63 @@ __global__ void __launch_bounds__(kTileM, 1) k_mlp_train(const float* __restrict
     const float inv_n = 1.0f / static_cast<float>(n);
     uint32_t phase = 0;
     double lsum = 0.0;
-    const int t_id = threadIdx.x;
+    const int row = threadIdx.x % kTileM, grp = threadIdx.x / kTileM, c0 = 32 * grp;  // this thread's 32 columns
+    const bool lead = threadIdx.x == 0;
+    // h = SiLU(D + b) of the thread's columns into the activation buffer
+    auto hidden = [&](uint32_t tD, const float* bias, unsigned char* buf) {
+        float v[32];
+        umma::ld32(umma::lane_addr(tD, c0), v);
+        silu_store<false>(v, bias + c0, buf, row, c0);
+    };
+    // the thread's pre-activations, and dZ = dH SiLU'(z) of its columns into the layer gradient
+    auto load_z = [&](uint32_t tD, const float* bias, float (&z)[32]) {
+        umma::ld32(umma::lane_addr(tD, c0), z);
+#pragma unroll
+        for (int k = 0; k < 32; ++k) z[k] += bias[c0 + k];
+    };
+    auto layer_grad = [&](const float (&z)[32]) {
+        float v[32];
+        umma::ld32(umma::lane_addr(T3, c0), v);
+#pragma unroll
+        for (int k = 0; k < 32; k += 2) {
+            const float2 d = mul2(make_float2(v[k], v[k + 1]), dsilu2(make_float2(z[k], z[k + 1])));
+            v[k] = d.x;
+            v[k + 1] = d.y;
+        }
+#pragma unroll
+        for (int k = 0; k < 32; k += 8) umma::st8(sm + sG, row, c0 + k, kTileM, v + k);
+    };
     const int64_t tiles = (n + kTileM - 1) / kTileM;
     for (int64_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
-        const int64_t p = tile * kTileM + t_id;
-        const bool valid = p < n;
-        load_x(sm, x, p, n);
+        const int64_t p = tile * kTileM + row;
+        const bool valid = p < n, first = tile == blockIdx.x;
+        {  // eight of the row's inputs per thread; zeros past the end
+            float4 u = make_float4(0, 0, 0, 0), w = u;
+            if (valid) {
+                const float4* src = reinterpret_cast<const float4*>(x + p * kIn + 8 * grp);
+                u = src[0];
+                w = src[1];
+            }
+            const float v[8] = {u.x, u.y, u.z, u.w, w.x, w.y, w.z, w.w};
+            umma::st8(sm + sX, row, 8 * grp, kTileM, v);
+        }
         // ---- forward, keeping z1 z2 z3 in tensor memory and h1 h2 h3 in shared memory
         before_issue();
-        if (t_id == 0) { issue(T1, base + sX, kTileM, false, base + sW1, kHid, false, kHid, kIn); umma::commit(&bar); }
+        if (lead) { issue(T1, base + sX, kTileM, false, base + sW1, kHid, false, kHid, kIn); umma::commit(&bar); }
         if (!after_commit(&bar, phase, status)) break;
-        hidden_out(T1, sbias, sm + sH1);
+        hidden(T1, sbias, sm + sH1);
         before_issue();
-        if (t_id == 0) { issue(T2, base + sH1, kTileM, false, base + sW2, kHid, false, kHid, kHid); umma::commit(&bar); }
+        if (lead) { issue(T2, base + sH1, kTileM, false, base + sW2, kHid, false, kHid, kHid); umma::commit(&bar); }
         if (!after_commit(&bar, phase, status)) break;
-        hidden_out(T2, sbias + kHid, sm + sH2);
+        hidden(T2, sbias + kHid, sm + sH2);
         before_issue();
-        if (t_id == 0) { issue(T3, base + sH2, kTileM, false, base + sW3, kHid, false, kHid, kHid); umma::commit(&bar); }
+        if (lead) { issue(T3, base + sH2, kTileM, false, base + sW3, kHid, false, kHid, kHid); umma::commit(&bar); }
         if (!after_commit(&bar, phase, status)) break;
-        hidden_out(T3, sbias + 2 * kHid, sm + sH3);
+        hidden(T3, sbias + 2 * kHid, sm + sH3);
         before_issue();
-        if (t_id == 0) { issue(T4, base + sH3, kTileM, false, base + sW4, kOutP, false, kOutP, kHid); umma::commit(&bar); }
+        if (lead) { issue(T4, base + sH3, kTileM, false, base + sW4, kOutP, false, kOutP, kHid); umma::commit(&bar); }
         if (!after_commit(&bar, phase, status)) break;
-        {  // output, loss, output gradient g4 = dL/dy
+        if (grp == 0) {  // output, loss, output gradient g4 = dL/dy
             float v[16], gv[16];
             umma::ld16(umma::lane_addr(T4, 0), v);
 #pragma unroll
@@ -406,95 +438,59 @@ __global__ void __launch_bounds__(kTileM, 1) k_mlp_train(const float* __restrict
                     gv[o] = 2.0f * wout[o] * d * inv_n;
                 }
             }
-            umma::st8(sm + sG4, t_id, 0, kTileM, gv);
-            umma::st8(sm + sG4, t_id, 8, kTileM, gv + 8);
+            umma::st8(sm + sG4, row, 0, kTileM, gv);
+            umma::st8(sm + sG4, row, 8, kTileM, gv + 8);
         }
-        // z3 into registers (its columns take dH3)
-        float z[kHid];
-#pragma unroll
-        for (int c0 = 0; c0 < kHid; c0 += 32) umma::ld32(umma::lane_addr(T3, c0), z + c0);
-#pragma unroll
-        for (int c = 0; c < kHid; ++c) z[c] += sbias[2 * kHid + c];
+        float z[32];
+        load_z(T3, sbias + 2 * kHid, z);  // z3 into registers (its columns take dH3)
         // ---- layer 4: dH3 = g4 W4, dW4^T = h3^T g4, db4 = colsum(g4)
         before_issue();
-        if (t_id == 0) {
+        if (lead) {
             issue(T3, base + sG4, kTileM, false, base + sW4, kOutP, true, kHid, kOutP);
             issue(T4, base + sH3, kTileM, true, base + sG4, kTileM, true, kOutP, kTileM);
             issue_colsum(T4 + 16, base + sOnes, base + sG4, kTileM, kOutP, kTileM);
             umma::commit(&bar);
         }
         if (!after_commit(&bar, phase, status)) break;
-        {
+        layer_grad(z);  // dZ3
+        if (grp < 2) {  // warpgroup 0: dW4 (accumulator row = input feature of layer 4), 1: db4
             float v[16];
-            umma::ld16(umma::lane_addr(T4, 0), v);  // row t = input feature t of layer 4
+            umma::ld16(umma::lane_addr(T4 + 16 * grp, 0), v);
+            if (grp == 0) {
 #pragma unroll
-            for (int o = 0; o < kOut; ++o) rmw(g + oW4 + o * kHid + t_id, v[o]);
-            umma::ld16(umma::lane_addr(T4 + 16, 0), v);
-            if (t_id == 0) {
+                for (int o = 0; o < kOut; ++o) add_one(g + oW4 + o * kHid + row, v[o], first);
+            } else if (row == 0) {
 #pragma unroll
-                for (int o = 0; o < kOut; ++o) rmw(g + ob4 + o, v[o]);
+                for (int o = 0; o < kOut; ++o) add_one(g + ob4 + o, v[o], first);
             }
         }
-#pragma unroll 1
-        for (int c0 = 0; c0 < kHid; c0 += 32) {  // dZ3 = dH3 * SiLU'(z3)
-            float v[32];
-            umma::ld32(umma::lane_addr(T3, c0), v);
-#pragma unroll
-            for (int k = 0; k < 32; ++k) v[k] *= dsilu(z[c0 + k]);
-#pragma unroll
-            for (int k = 0; k < 32; k += 8) umma::st8(sm + sG, t_id, c0 + k, kTileM, v + k);
-        }
-        // z2 into registers (its columns take db3)
-#pragma unroll
-        for (int c0 = 0; c0 < kHid; c0 += 32) umma::ld32(umma::lane_addr(T2, c0), z + c0);
-#pragma unroll
-        for (int c = 0; c < kHid; ++c) z[c] += sbias[kHid + c];
+        load_z(T2, sbias + kHid, z);  // z2 (its columns take db3)
         // ---- layers 3, 2: dH = dZ W, dW = dZ^T h, db = colsum(dZ)
         bool ok = true;
 #pragma unroll 1
-        for (int layer = 3; layer >= 2 && ok; --layer) {
+        for (int layer = 3; layer >= 2; --layer) {
             const uint32_t sW = layer == 3 ? sW3 : sW2, sHin = layer == 3 ? sH2 : sH1;
             const int oW = layer == 3 ? oW3 : oW2, ob = layer == 3 ? ob3 : ob2;
             before_issue();
-            if (t_id == 0) {
+            if (lead) {
                 issue(T3, base + sG, kTileM, false, base + sW, kHid, true, kHid, kHid);
                 issue(T4, base + sG, kTileM, true, base + sHin, kTileM, true, kHid, kTileM);
                 issue_colsum(T2, base + sOnes, base + sG, kTileM, kHid, kTileM);
                 umma::commit(&bar);
             }
             if (!after_commit(&bar, phase, status)) { ok = false; break; }
-#pragma unroll 1
-            for (int c0 = 0; c0 < kHid; c0 += 32) {
-                float v[32];
-                umma::ld32(umma::lane_addr(T4, c0), v);  // row t = output unit t
-                rmw_row<32>(g + oW + t_id * kHid + c0, v);
-                umma::ld32(umma::lane_addr(T2, c0), v);
-                if (t_id == 0) rmw_row<32>(g + ob + c0, v);
-            }
-            if (layer == 2) {  // z1 from its columns
-#pragma unroll
-                for (int c0 = 0; c0 < kHid; c0 += 32) umma::ld32(umma::lane_addr(T1, c0), z + c0);
-#pragma unroll
-                for (int c = 0; c < kHid; ++c) z[c] += sbias[c];
-            }
-            umma::fence_before();
-            __syncthreads();  // every read of the dZ buffer by the MMAs is complete: overwrite it
-#pragma unroll 1
-            for (int c0 = 0; c0 < kHid; c0 += 32) {
-                float v[32];
-                umma::ld32(umma::lane_addr(T3, c0), v);
-#pragma unroll
-                for (int k = 0; k < 32; ++k) v[k] *= dsilu(z[c0 + k]);
-#pragma unroll
-                for (int k = 0; k < 32; k += 8) umma::st8(sm + sG, t_id, c0 + k, kTileM, v + k);
-            }
-            if (layer == 3) {  // z2 was loaded above; nothing to do
-            }
+            layer_grad(z);  // every MMA that reads the old dZ is complete
+            float v[32];
+            umma::ld32(umma::lane_addr(T4, c0), v);  // accumulator row = output unit
+            add_row<32>(g + oW + row * kHid + c0, v, first);
+            umma::ld32(umma::lane_addr(T2, c0), v);
+            if (row == 0) add_row<32>(g + ob + c0, v, first);
+            if (layer == 3) load_z(T1, sbias, z);
         }
         if (!ok) break;
         // ---- layer 1: dW1 = dZ1^T x, db1 = colsum(dZ1)
         before_issue();
-        if (t_id == 0) {
+        if (lead) {
             issue(T4, base + sG, kTileM, true, base + sX, kTileM, true, kIn, kTileM);
             issue_colsum(T2, base + sOnes, base + sG, kTileM, kHid, kTileM);
             umma::commit(&bar);
@@ -502,45 +498,55 @@ __global__ void __launch_bounds__(kTileM, 1) k_mlp_train(const float* __restrict
         if (!after_commit(&bar, phase, status)) break;
         {
             float v[32];
-            umma::ld32(umma::lane_addr(T4, 0), v);
-            rmw_row<kIn>(g + oW1 + t_id * kIn, v);
-#pragma unroll 1
-            for (int c0 = 0; c0 < kHid; c0 += 32) {
-                umma::ld32(umma::lane_addr(T2, c0), v);
-                if (t_id == 0) rmw_row<32>(g + ob1 + c0, v);
+            if (grp < 2) {
+                umma::ld16(umma::lane_addr(T4, 16 * grp), v);
+                add_row<16>(g + oW1 + row * kIn + 16 * grp, v, first);
             }
+            umma::ld32(umma::lane_addr(T2, c0), v);
+            if (row == 0) add_row<32>(g + ob1 + c0, v, first);
         }
         umma::fence_before();
         __syncthreads();  // the next tile overwrites X and the activation buffers
     }
     // loss of this CTA
+    if (grp == 0) {
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) lsum += __shfl_xor_sync(0xffffffffu, lsum, o);
-    if ((t_id & 31) == 0) red[t_id >> 5] = lsum;
+        for (int o = 16; o > 0; o >>= 1) lsum += __shfl_xor_sync(0xffffffffu, lsum, o);
+        if ((row & 31) == 0) red[row >> 5] = lsum;
+    }
     umma::fence_before();
     __syncthreads();
-    if (t_id == 0) {
+    if (lead) {
         double s = 0.0;
         for (int w = 0; w < kTileM / 32; ++w) s += red[w];
         loss_part[blockIdx.x] = s;
     }
-    if (t_id < 32) umma::tmem_free(tslot, 512);
+    if (threadIdx.x < 32) umma::tmem_free(tslot, 512);
 }
 
-// grad[i] = sum over CTAs c of part[c][i] (fixed order); loss = sum of loss_part / n
-__global__ void k_mlp_reduce(const float* __restrict__ part, int ncta, float* __restrict__ grad,
-                             const double* __restrict__ loss_part, double* loss, int64_t n) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < kParams) {
-        float s = 0.0f;
-        for (int c = 0; c < ncta; ++c) s += part[static_cast<int64_t>(c) * kPartStride + i];
-        grad[i] = s;
-    }
-    if (i == 0) {
+// grad[i] = sum over CTAs c of part[c][i] (fixed order); the last block: loss = sum of loss_part / n
+constexpr int kReduceThreads = 256;
+__global__ void __launch_bounds__(kReduceThreads) k_mlp_reduce(const float* __restrict__ part, int ncta, float* __restrict__ grad,
+                                                               const double* __restrict__ loss_part, double* loss, int64_t n) {
+    if (blockIdx.x == gridDim.x - 1) {
+        __shared__ double sh[kReduceThreads];
         double s = 0.0;
-        for (int c = 0; c < ncta; ++c) s += loss_part[c];
-        *loss = s / static_cast<double>(n);
+        for (int c0 = 0; c0 < ncta; c0 += kReduceThreads) {
+            __syncthreads();
+            if (c0 + static_cast<int>(threadIdx.x) < ncta) sh[threadIdx.x] = loss_part[c0 + threadIdx.x];
+            __syncthreads();
+            if (threadIdx.x == 0)
+                for (int c = 0; c < min(kReduceThreads, ncta - c0); ++c) s += sh[c];
+        }
+        if (threadIdx.x == 0) *loss = s / static_cast<double>(n);
+        return;
     }
+    const int i = blockIdx.x * kReduceThreads + threadIdx.x;
+    if (i >= kParams) return;
+    float s = 0.0f;
+#pragma unroll 16
+    for (int c = 0; c < ncta; ++c) s += part[static_cast<int64_t>(c) * kPartStride + i];
+    grad[i] = s;
 }
 
 // the squared global norm of the gradient (one block, fixed summation order) for gradient clipping
@@ -740,10 +746,9 @@ int gsph_mlp_gradient(gsph_mlp* m, const float* x, const float* target, const fl
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
     const int64_t tiles = (n + kTileM - 1) / kTileM;
     const int grid = static_cast<int>(tiles < m->grid ? tiles : m->grid);
-    MLP_CK(m, cudaMemsetAsync(m->part, 0, static_cast<size_t>(grid) * kPartStride * sizeof(float), s), "clear");
-    k_mlp_train<<<grid, kTileM, kTrainSmem, s>>>(x, target, wout, n, m->wq, m->bq, m->part, m->loss_part, m->status);
+    k_mlp_train<<<grid, kTrainThreads, kTrainSmem, s>>>(x, target, wout, n, m->wq, m->bq, m->part, m->loss_part, m->status);
     MLP_CK(m, cudaGetLastError(), "gradient launch");
-    k_mlp_reduce<<<(kParams + 255) / 256, 256, 0, s>>>(m->part, grid, m->grad, m->loss_part, m->loss, n);
+    k_mlp_reduce<<<(kParams + kReduceThreads - 1) / kReduceThreads + 1, kReduceThreads, 0, s>>>(m->part, grid, m->grad, m->loss_part, m->loss, n);
     MLP_CK(m, cudaGetLastError(), "reduce launch");
     if (grad) MLP_CK(m, cudaMemcpyAsync(grad, m->grad, kParams * sizeof(float), cudaMemcpyDeviceToHost, s), "grad copy");
     if (loss) MLP_CK(m, cudaMemcpyAsync(loss, m->loss, sizeof(double), cudaMemcpyDeviceToHost, s), "loss copy");
