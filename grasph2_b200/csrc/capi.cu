@@ -338,7 +338,8 @@ int reorder(gsph_ctx* c, cudaStream_t s) {
 
 const int* ext_map(const gsph_ctx* c) { return c->L.cull ? c->sp.ext_of_int : nullptr; }
 
-int integrate(gsph_ctx* c, int not_first_step, cudaStream_t s) {
+// after_derivatives: behind the derivatives of the same step on `s`
+int integrate(gsph_ctx* c, int not_first_step, cudaStream_t s, bool after_derivatives = false) {
     if (c->fp64) {
         int launches = 0;
         const cudaError_t e = launch64_leapfrog(c->a64, c->dp64, not_first_step, s, launches);
@@ -348,7 +349,7 @@ int integrate(gsph_ctx* c, int not_first_step, cudaStream_t s) {
     }
     const KTimer* t = slot_timer(c, GSPH_KSLOT_INTEGRATE);
     cudaError_t e = t ? timer_record(t->start, s) : cudaSuccess;
-    if (e == cudaSuccess) e = launch_leapfrog(c->a, c->dp, not_first_step, s);
+    if (e == cudaSuccess) e = launch_leapfrog(c->a, c->dp, not_first_step, s, after_derivatives && !t);
     if (e == cudaSuccess && t) e = timer_record(t->stop, s);
     if (e != cudaSuccess) return cuda_fail(c, e, "leapfrog");
     c->launches += has(c->dp, GSPH_VARIABLE_TIMESTEP) ? 3 : 1;
@@ -862,7 +863,7 @@ int gsph_step(gsph_ctx* c, int32_t nsteps, void* stream) {
             if (te != cudaSuccess) rc = cuda_fail(c, te, "timer");
         }
         if (rc == GSPH_OK) rc = derivatives(c, c->capture_stream);
-        if (rc == GSPH_OK) rc = integrate(c, 1, c->capture_stream);
+        if (rc == GSPH_OK) rc = integrate(c, 1, c->capture_stream, true);
         if (rc == GSPH_OK && st) {
             const cudaError_t te = timer_record(st->stop, c->capture_stream);
             if (te != cudaSuccess) rc = cuda_fail(c, te, "timer");

@@ -119,6 +119,30 @@ __device__ __forceinline__ void bulk_g2s(void* dst, const void* src, uint32_t by
         : "memory");
 }
 
+// ---- programmatic dependent launch -----------------------------------------------------------
+// A kernel of a step is set up while its predecessor on the stream drains, and waits here for that kernel's end before
+// it reads or writes anything. Every kernel that is launched `early` calls this first: then a kernel that has got past
+// it may rely on all the earlier ones, not only on its direct predecessor. No kernel releases its successors before its
+// end: their waiting CTAs would take room from the gravity kernel on the other stream (a step of the impact with 65,536
+// particles 1,330 -> 1,417 us that way).
+// Measured: a step of the Plummer sphere with 4,096 particles (three kernels) 18.4 -> 16.4 us.
+__device__ __forceinline__ void wait_predecessor() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+template <typename... P, typename... A>
+cudaError_t launch_kernel(bool early, void (*kernel)(P...), dim3 grid, unsigned block, cudaStream_t s, A... args) {
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(block);
+    cfg.stream = s;
+    cfg.attrs = &at;
+    cfg.numAttrs = early ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
 // ---- compensated accumulation --------------------------------------------------------------
 // Kahan-Babuska (Neumaier) fold of a tile partial `x` into the running pair (s, c): s + c is the
 // sum; c collects the rounding error of every fold exactly (two-sum).

@@ -246,7 +246,7 @@ cudaError_t launch_fixed_gravity(const DevArrays& a, const DevParams& p, const L
     else comp ? gravity_sym<2, true>(a, p, L, s) : gravity_sym<2, false>(a, p, L, s);
     e = cudaGetLastError();
     if (e == cudaSuccess && t) e = timer_record(t->stop, s);
-    return e == cudaSuccess ? launch_gravity_fold(a, L, L.grav_sym_G + 1, s) : e;
+    return e == cudaSuccess ? launch_gravity_fold(a, L, L.grav_sym_G + 1, s, !t) : e;
 }
 
 

@@ -12,7 +12,10 @@ namespace {
 
 inline unsigned blocks_for(int64_t n, int t) { return static_cast<unsigned>((n + t - 1) / t); }
 
+constexpr int kStepThreads = 128;  // per CTA of the leapfrog kernels: 4,096 particles on 32 SMs
+
 __global__ void k_leapfrog_fixed(DevArrays a, DevParams p, float kick_dt) {
+    wait_predecessor();
     const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (i >= a.n) return;
     kick_drift(a, p, i, kick_dt, p.fixed_dt);
@@ -22,6 +25,7 @@ __global__ void k_leapfrog_fixed(DevArrays a, DevParams p, float kick_dt) {
 // step and the min of the step criteria; block min, then an integer atomicMin on the positive
 // float's bit pattern
 __global__ void k_dt_criteria(DevArrays a, DevParams p) {
+    wait_predecessor();
     const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     const float dt = a.dt_state[0];
     float mindt = p.max_dt;
@@ -51,11 +55,13 @@ __global__ void k_dt_criteria(DevArrays a, DevParams p) {
 }
 
 __global__ void k_dt_first(DevArrays a, DevParams p) {
+    wait_predecessor();
     if (threadIdx.x == 0 && blockIdx.x == 0) a.dt_state[1] = p.initial_dt;  // integration.h:235-236
 }
 
 // variableTsLeapfrog_useNewTimestep (integration.h:171-217)
 __global__ void k_leapfrog_variable(DevArrays a, DevParams p) {
+    wait_predecessor();
     const float nxt = a.dt_state[1];
     const float dt = nxt < p.min_dt ? p.min_dt : nxt;
     const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
@@ -65,6 +71,7 @@ __global__ void k_leapfrog_variable(DevArrays a, DevParams p) {
 
 // commit the step chosen above as the current one (after every block has read `next`)
 __global__ void k_dt_commit(DevArrays a, DevParams p) {
+    wait_predecessor();
     if (threadIdx.x == 0 && blockIdx.x == 0) {
         const float nxt = a.dt_state[1];
         a.dt_state[0] = nxt < p.min_dt ? p.min_dt : nxt;
@@ -358,21 +365,15 @@ __global__ void k_check_finite(DevArrays a) {
 
 }  // namespace
 
-cudaError_t launch_leapfrog(const DevArrays& a, const DevParams& p, int not_first_step, cudaStream_t s) {
-    const unsigned nb = blocks_for(a.n, 256);
-    if (!has(p, GSPH_VARIABLE_TIMESTEP)) {
-        k_leapfrog_fixed<<<nb, 256, 0, s>>>(a, p, p.fixed_dt * (not_first_step ? 1.0f : 0.5f));
-        return cudaGetLastError();
-    }
-    if (not_first_step) k_dt_criteria<<<nb, 256, 0, s>>>(a, p);
-    else k_dt_first<<<1, 32, 0, s>>>(a, p);
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-    k_leapfrog_variable<<<nb, 256, 0, s>>>(a, p);
-    e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-    k_dt_commit<<<1, 32, 0, s>>>(a, p);
-    return cudaGetLastError();
+cudaError_t launch_leapfrog(const DevArrays& a, const DevParams& p, int not_first_step, cudaStream_t s, bool early) {
+    const unsigned nb = blocks_for(a.n, kStepThreads);
+    if (!has(p, GSPH_VARIABLE_TIMESTEP))
+        return launch_kernel(early, k_leapfrog_fixed, nb, kStepThreads, s, a, p, p.fixed_dt * (not_first_step ? 1.0f : 0.5f));
+    cudaError_t e = not_first_step ? launch_kernel(early, k_dt_criteria, nb, kStepThreads, s, a, p)
+                                   : launch_kernel(early, k_dt_first, 1, 32, s, a, p);
+    if (e == cudaSuccess) e = launch_kernel(true, k_leapfrog_variable, nb, kStepThreads, s, a, p);
+    if (e == cudaSuccess) e = launch_kernel(true, k_dt_commit, 1, 32, s, a, p);
+    return e;
 }
 
 int leapfrog_kernel_count(const DevParams& p) { return has(p, GSPH_VARIABLE_TIMESTEP) ? 3 : 1; }

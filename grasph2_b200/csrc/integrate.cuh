@@ -5,7 +5,8 @@
 
 namespace gsph {
 
-cudaError_t launch_leapfrog(const DevArrays& a, const DevParams& p, int not_first_step, cudaStream_t s);
+cudaError_t launch_leapfrog(const DevArrays& a, const DevParams& p, int not_first_step, cudaStream_t s,
+                            bool early = false);
 int leapfrog_kernel_count(const DevParams& p);
 size_t diag_scratch_doubles(int64_t n);
 cudaError_t launch_diagnostics(const DevArrays& a, const DevParams& p, double half_kick, double* out_dev,

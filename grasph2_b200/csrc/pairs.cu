@@ -86,26 +86,30 @@ __global__ void __launch_bounds__(256) k_density(const float4* __restrict__ posm
     if (COMP) part[(seg * 2 + 1) * n_pad + i] = rho_c;
 }
 
-// The neighbour search of 32 particles by four warps, with the density sum and its epilogue (DENS) or without (the
+// The neighbour search of 32 particles by W warps, with the density sum and its epilogue (DENS) or without (the
 // density is integrated). The group's near chunks come in batches of up to 64, cut at a stage. A: the batch's boxes are
-// tested against the 32 particles' own, 32 per warp. B: warp w takes the stages w, w + 4, ...; the positions of a near
+// tested against the 32 particles' own, 32 per warp. B: warp w takes the stages w, w + W, ...; the positions of a near
 // box go through the warp's shared buffer, every lane gets the mask of its neighbours (0 < r^2 <= H^2) and adds
 // their terms to the stage's sum. C: with the counts of all stages known, each warp writes its stages' neighbours to
 // their places in the particle's list, and warp 0 adds the stage sums in their order.
 //
 // Bound: instruction issue (8 per test, about 2 % of the tests are neighbours). One warp alone took 154 us for 65,536
-// particles of the impact and 29 us for the 4,096 of the fluid, whose 128 warps leave the chip idle.
-constexpr int kNearWarps = 4, kBatch = 64;
-template <bool DENS, bool COMP>
-__global__ void __launch_bounds__(kSub * kNearWarps) k_near(const float4* __restrict__ posm, float4* __restrict__ velrho,
+// particles of the impact and 29 us for the 4,096 of the fluid, whose 128 warps leave the chip idle. Eight warps help
+// the search alone in few groups (a rubble step with 16,384 particles 178.7 -> 174.7 us, with 4,000 73.3 -> 66.7), not the
+// search with the density sum (71.6 us for 68.5 in the fluid's step: the walk over the stages is each warp's own).
+constexpr int kBatch = 64;
+template <int W, bool DENS, bool COMP>
+__global__ void __launch_bounds__(kSub * W) k_near(const float4* __restrict__ posm, float4* __restrict__ velrho,
                                                             DevParams p, NearView v) {
-    __shared__ float4 sh[kNearWarps][kSub];
+    __shared__ float4 sh[W][kSub];
     __shared__ unsigned mk[kBatch * kHalves][kSub];   // neighbour masks of the batch's boxes
     __shared__ float ts[DENS ? kBatch : 1][kSub];     // stage sums
     __shared__ unsigned short cs[kBatch][kSub];       // neighbours per stage
     __shared__ int bxs[kBatch * kHalves];
     __shared__ unsigned nm[kBatch * kHalves / 32];    // which boxes are near
-    static_assert(kBatch * kHalves == 32 * kNearWarps, "one vote per warp and batch");
+    constexpr int kVotes = kBatch * kHalves / 32;  // one vote per batch in each of the first warps
+    static_assert(kVotes <= W, "one vote per warp and batch");
+    wait_predecessor();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int g = v.group(), ic = v.per_item(), nc = v.count[g];
     const int64_t s0 = v.first(g), i = s0 + lane;
@@ -137,7 +141,7 @@ __global__ void __launch_bounds__(kSub * kNearWarps) k_near(const float4* __rest
     for (int c0 = 0; c0 < nc;) {
         int c1 = min(nc, c0 + kBatch);
         if (c1 < nc) c1 -= c1 % ic % kStageChunks;  // whole stages
-        {  // A
+        if (warp < kVotes) {  // A
             const int h = threadIdx.x;
             int bx = 0;
             bool near = false;
@@ -155,7 +159,7 @@ __global__ void __launch_bounds__(kSub * kNearWarps) k_near(const float4* __rest
         __syncthreads();
         // B
         stages(c0, c1, ie, [&](int q, int b, int e, bool) {
-            if (q % kNearWarps != warp) return;
+            if (q % W != warp) return;
             float t = 0.0f;
             int n = 0;
             for (int h = b * kHalves; h < e * kHalves; ++h) {
@@ -198,7 +202,7 @@ __global__ void __launch_bounds__(kSub * kNearWarps) k_near(const float4* __rest
         // C
         ie = stages(c0, c1, ie, [&](int q, int b, int e, bool item_ends) {
             const int n = cs[q][lane];
-            if (q % kNearWarps == warp && __any_sync(0xffffffffu, n > 0)) {
+            if (q % W == warp && __any_sync(0xffffffffu, n > 0)) {
                 int at = cnt;
                 bool first = !seen;
                 for (int h = b * kHalves; h < e * kHalves; ++h) {
@@ -266,6 +270,7 @@ __global__ void k_density_finish(DevArrays a, DevParams p, PartView pv) {
 
 // j-records from the current density
 __global__ void k_prepare(DevArrays a, DevParams p) {
+    wait_predecessor();
     const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (i >= a.n) return;
     const float4 vr = a.velrho[i];
@@ -382,10 +387,15 @@ __global__ void __launch_bounds__(256) k_pairs(DevArrays a, DevParams p, int jt,
 // Bound: instruction issue and the L2 latency of the gathers. A lane goes through all its neighbours and adds an item's
 // sums when its next neighbour belongs to another one, so a warp runs as long as its longest list (a warp per
 // item of a few chunks kept 18.8 of 32 lanes active and left the items' partial sums to the finish kernel).
-template <int PASS, bool SOLIDS, bool COMP>
-__global__ void __launch_bounds__(kSub) k_pairs_near(DevArrays a, DevParams p, NearView v) {
-    constexpr uint32_t MASK = field_mask<PASS, false, SOLIDS>();
-    constexpr bool DO_A = PASS != PASS_VGRAD;
+// In few groups there is one warp to a scheduler at most, and the chain of one neighbour's arithmetic behind another's is
+// what it waits for. There the records of D = 4 neighbours are in flight (a rubble step with 16,384 particles 199 -> 194
+// us), and the fused pass goes to two warps, one for the velocity gradient (PART 1) and one for the acceleration (PART 2):
+// 208 -> 190 us for a step of the impact with 16,384 particles, 115 -> 98 with 4,000.
+template <int PASS, bool SOLIDS, bool COMP, int D, int PART>
+__device__ __forceinline__ void pairs_near(const DevArrays& a, const DevParams& p, const NearView& v) {
+    constexpr uint32_t ALL = field_mask<PASS, false, SOLIDS>(), FIRST = field_mask<PASS_VGRAD, false, SOLIDS>();
+    constexpr uint32_t MASK = PART == 0 ? ALL : (PART == 1 ? ALL & FIRST : ALL & ~FIRST);
+    constexpr bool DO_A = PASS != PASS_VGRAD && PART != 1;
     using Sum = typename std::conditional<COMP, double, float>::type;
     __shared__ float4 sh[kSub];
     const int g = v.group(), ic = v.per_item();
@@ -414,30 +424,38 @@ __global__ void __launch_bounds__(kSub) k_pairs_near(DevArrays a, DevParams p, N
     auto term = [&](float4 q, float4 vj, float4 ja, float4 jb) {
         const float dx = q.x - I.pi.x, dy = q.y - I.pi.y, dz = q.z - I.pi.z;
         const float r2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
-        sph_neighbour<PASS, SOLIDS>(T, maxv, I, q.w, dx, dy, dz, r2, vj, ja, jb, p);
+        sph_neighbour<PASS, SOLIDS, PART>(T, maxv, I, q.w, dx, dy, dz, r2, vj, ja, jb, p);
     };
     if (!__any_sync(0xffffffffu, cnt > v.cap)) {
-        int e = cnt > 0 ? lst[0] : 0;            // the entry of neighbour k
-        int en = cnt > 1 ? lst[v.n_pad] : 0;     // ... and of k + 1
-        const float4* r0 = a.jrec + 4 * static_cast<int64_t>(e & ~kItemMark);
-        float4 qn = __ldg(r0), vn = __ldg(r0 + 1);
-        float4 an = DO_A ? __ldg(r0 + 2) : zero, bn = DO_A ? __ldg(r0 + 3) : zero;
-        for (int k = 0; k < cnt; ++k) {
-            const float4 q = qn, vj = vn, ja = an, jb = bn;
-            const bool first = e < 0;
-            e = en;
-            if (k + 1 < cnt) {
-                const float4* r = a.jrec + 4 * static_cast<int64_t>(e & ~kItemMark);
-                qn = __ldg(r);
-                vn = __ldg(r + 1);
-                if (DO_A) {
-                    an = __ldg(r + 2);
-                    bn = __ldg(r + 3);
-                }
+        int e[D] = {}, en[D] = {};  // the entries of the next D neighbours, and of the D after them
+        float4 rec[D][4];
+        auto load = [&](int d) {
+            const float4* r = a.jrec + 4 * static_cast<int64_t>(e[d] & ~kItemMark);
+            rec[d][0] = __ldg(r);
+            rec[d][1] = __ldg(r + 1);
+            rec[d][2] = DO_A ? __ldg(r + 2) : zero;
+            rec[d][3] = DO_A ? __ldg(r + 3) : zero;
+        };
+#pragma unroll
+        for (int d = 0; d < D; ++d) {
+            e[d] = d < cnt ? lst[static_cast<int64_t>(d) * v.n_pad] : 0;
+            en[d] = D + d < cnt ? lst[static_cast<int64_t>(D + d) * v.n_pad] : 0;
+        }
+#pragma unroll
+        for (int d = 0; d < D; ++d) load(d);
+        for (int k0 = 0; k0 < cnt; k0 += D) {
+#pragma unroll
+            for (int d = 0; d < D; ++d) {
+                const int k = k0 + d;
+                if (k >= cnt) break;
+                const float4 q = rec[d][0], vj = rec[d][1], ja = rec[d][2], jb = rec[d][3];
+                const bool first = e[d] < 0;
+                e[d] = en[d];
+                if (k + D < cnt) load(d);
+                if (k + 2 * D < cnt) en[d] = lst[static_cast<int64_t>(k + 2 * D) * v.n_pad];
+                if (first) end_item();
+                term(q, vj, ja, jb);
             }
-            if (k + 2 < cnt) en = lst[static_cast<int64_t>(k + 2) * v.n_pad];
-            if (first) end_item();
-            term(q, vj, ja, jb);
         }
     } else {
         int item = 0, next = ic, last = -1;
@@ -459,7 +477,19 @@ __global__ void __launch_bounds__(kSub) k_pairs_near(DevArrays a, DevParams p, N
 #pragma unroll
     for (int f = 0; f < F_COUNT; ++f)
         if ((MASK >> f) & 1u)
-            a.part[static_cast<int64_t>(field_offset<MASK>(f)) * a.n_pad + i] = f == F_MAXV ? maxv : static_cast<float>(S[f]);
+            a.part[static_cast<int64_t>(field_offset<ALL>(f)) * a.n_pad + i] = f == F_MAXV ? maxv : static_cast<float>(S[f]);
+}
+
+template <int PASS, bool SOLIDS, bool COMP, int D>
+__global__ void __launch_bounds__(kSub) k_pairs_near(DevArrays a, DevParams p, NearView v) {
+    wait_predecessor();
+    pairs_near<PASS, SOLIDS, COMP, D, 0>(a, p, v);
+}
+template <bool SOLIDS, bool COMP>
+__global__ void __launch_bounds__(kSub) k_pairs_near_split(DevArrays a, DevParams p, NearView v) {
+    wait_predecessor();
+    if (blockIdx.y == 0) pairs_near<PASS_FUSED, SOLIDS, COMP, 1, 2>(a, p, v);
+    else pairs_near<PASS_FUSED, SOLIDS, COMP, 1, 1>(a, p, v);
 }
 
 // Sum the slots of one field in a fixed order: FP32 in plain mode, FP64 of (sum + error) in
@@ -489,57 +519,94 @@ __device__ __forceinline__ float seg_sum(const PartView& v, int64_t i, int f) {
 // ---- the FP64 fold of the gravity partials ---------------------------------------------------------
 // Both all-pairs gravity kernels leave per-particle partial sums [slot][component][n_pad]: the one-sided
 // kernel's j-segments, or the symmetric kernel's G + 1 slots (its row and column sums, each written by
-// one task). kFoldT threads fold one particle: thread q sums the slots [q R, (q + 1) R) in FP64 (with the
-// error terms of the compensated form), then the runs are added in the order q = 0, 1, 2, 3 -- a fixed
-// order, so results are deterministic. Eight particles per warp: for a slot, the eight lanes of a run
-// read 32 contiguous bytes.
-constexpr int kFoldT = 4;
-template <bool COMP>
-__device__ __forceinline__ void fold_slots(const float* __restrict__ part, int64_t n_pad, int S, int64_t i, bool valid,
-                                           double (&out)[3]) {
-    constexpr int K = COMP ? 6 : 3;
-    const int lane = threadIdx.x & 31, q = lane >> 3;
+// one task). 32 particles per CTA: warp q sums the slots [q R, (q + 1) R) in FP64 (with the error terms of
+// the compensated form), then the runs are added in the order q = 0, 1, 2, 3 -- a fixed order, so results
+// are deterministic.
+//
+// Bound: the latency of the loads in small contexts, so all 17 slots of a run of 65 are in flight at once; DRAM in large ones, where a
+// thread takes V = 4 particles in 16-byte loads. Measured (cold caches; before, with eight particles per warp and 32
+// contiguous bytes): 4,096 particles 5.8 us (11.8), 65,536 16.7 (21.2), 262,144 80 (140), 100,003 compensated 46 (61).
+constexpr int kFoldT = 4, kFoldThreads = 32 * kFoldT;
+template <int V> struct FoldVec { using type = float; };
+template <> struct FoldVec<4> { using type = float4; };
+template <int V>
+__device__ __forceinline__ float fold_get(const typename FoldVec<V>::type& x, int e) {
+    if constexpr (V == 4) return e == 0 ? x.x : (e == 1 ? x.y : (e == 2 ? x.z : x.w));
+    else return x;
+}
+// f(i, sum) for the particles of this CTA, on the threads of warp 0
+template <bool COMP, int V, typename F>
+__device__ __forceinline__ void fold_slots(const float* __restrict__ part, int64_t n, int64_t n_pad, int S, F&& f) {
+    using Vec = typename FoldVec<V>::type;
+    constexpr int K = COMP ? 6 : 3, U = (V == 4 ? 12 : 54) / K;
+    __shared__ double run[kFoldT - 1][V][3][32];
+    const int lane = threadIdx.x & 31, q = threadIdx.x >> 5;
+    const int64_t i = (static_cast<int64_t>(blockIdx.x) * 32 + lane) * V;
     const int R = (S + kFoldT - 1) / kFoldT;
     const int k0 = min(S, q * R), k1 = min(S, k0 + R);
-    double s[3] = {0.0, 0.0, 0.0};
-    if (valid) {
-#pragma unroll 4
-        for (int k = k0; k < k1; ++k) {
-            const float* p = part + static_cast<int64_t>(k) * K * n_pad + i;
+    double s[V][3];
 #pragma unroll
-            for (int c = 0; c < 3; ++c) {
-                s[c] += static_cast<double>(__ldg(p + c * n_pad));
-                if (COMP) s[c] += static_cast<double>(__ldg(p + (3 + c) * n_pad));
+    for (int e = 0; e < V; ++e) s[e][0] = s[e][1] = s[e][2] = 0.0;
+    if (i < n) {  // n_pad is a multiple of 1024: a vector of the last particles stays in its row
+        for (int k = k0; k < k1; k += U) {
+            Vec v[U][K];
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const float* p = part + static_cast<int64_t>(V == 1 ? k + u : min(k + u, k1 - 1)) * K * n_pad + i;
+#pragma unroll
+                for (int c = 0; c < K; ++c)
+                    v[u][c] = V > 1 || k + u < k1 ? __ldg(reinterpret_cast<const Vec*>(p + c * n_pad)) : Vec{};
+            }
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                if (V > 1 && k + u >= k1) break;
+#pragma unroll
+                for (int e = 0; e < V; ++e)
+#pragma unroll
+                    for (int c = 0; c < 3; ++c) {
+                        s[e][c] += static_cast<double>(fold_get<V>(v[u][c], e));
+                        if (COMP) s[e][c] += static_cast<double>(fold_get<V>(v[u][K - 3 + c], e));
+                    }
             }
         }
     }
+    if (q > 0)
 #pragma unroll
-    for (int c = 0; c < 3; ++c) {  // runs 0 + 1 + 2 + 3, in this order, on the lanes of run 0
-        double t = s[c];
-        t += __shfl_down_sync(0xffffffffu, s[c], 8);
-        t += __shfl_down_sync(0xffffffffu, s[c], 16);
-        t += __shfl_down_sync(0xffffffffu, s[c], 24);
-        out[c] = t;
+        for (int e = 0; e < V; ++e)
+#pragma unroll
+            for (int c = 0; c < 3; ++c) run[q - 1][e][c][lane] = s[e][c];
+    __syncthreads();
+    if (q > 0) return;
+#pragma unroll
+    for (int e = 0; e < V; ++e) {
+        if (i + e >= n) break;
+        double t[3];
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {  // runs 0 + 1 + 2 + 3, in this order
+            t[c] = s[e][c];
+#pragma unroll
+            for (int r = 0; r < kFoldT - 1; ++r) t[c] += run[r][e][c][lane];
+        }
+        f(i + e, t);
     }
 }
-__device__ __forceinline__ int64_t fold_particle() {
-    return (static_cast<int64_t>(blockIdx.x) * blockDim.x + (threadIdx.x & ~31u)) / kFoldT + (threadIdx.x & 7);
-}
+inline int fold_vec(int64_t n) { return n >= 32768 ? 4 : 1; }
+inline unsigned fold_blocks(int64_t n) { return static_cast<unsigned>((n + 32 * fold_vec(n) - 1) / (32 * fold_vec(n))); }
 
 // the culled path: the fold of the gravity partials into gfold[3][n_pad], on the gravity kernel's stream
-template <bool COMP>
-__global__ void __launch_bounds__(256) k_gravity_fold(const float* __restrict__ part, int64_t n, int64_t n_pad, int S,
-                                                      double* __restrict__ gfold) {
-    const int64_t i = fold_particle();
-    double t[3];
-    fold_slots<COMP>(part, n_pad, S, i, i < n, t);
-    if ((threadIdx.x & 31) < 8 && i < n)
+template <bool COMP, int V>
+__global__ void __launch_bounds__(kFoldThreads) k_gravity_fold(const float* __restrict__ part, int64_t n, int64_t n_pad, int S,
+                                                               double* __restrict__ gfold) {
+    wait_predecessor();
+    fold_slots<COMP, V>(part, n, n_pad, S, [&](int64_t i, const double (&t)[3]) {
         for (int c = 0; c < 3; ++c) gfold[c * n_pad + i] = t[c];
+    });
 }
 
 template <int PASS, bool GRAV, bool SOLIDS, bool COMP>
 __global__ void k_pairs_finish(DevArrays a, DevParams p, PartView pv, GravSum gsum) {
     constexpr uint32_t MASK = field_mask<PASS, GRAV, SOLIDS>();
+    wait_predecessor();
     const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (PASS != PASS_VGRAD && has(p, GSPH_VARIABLE_TIMESTEP) && i == 0)
         a.dt_state[1] = p.max_dt;  // nextTS reset of calcAcceleration::do_after (:306-309)
@@ -556,6 +623,14 @@ __global__ void k_pairs_finish(DevArrays a, DevParams p, PartView pv, GravSum gs
             for (int c = 0; c < 3; ++c) g[c] = static_cast<float>(a.gfold[c * a.n_pad + i]);
             grav = true;
         }
+    }
+    // the culled passes: one slot per field, all of them in flight at once (one after another, 4,000 particles took 18.4 us)
+    if (pv.nseg == 1 && !pv.err) {
+        float v[popc_c(MASK)];
+#pragma unroll
+        for (int o = 0; o < popc_c(MASK); ++o) v[o] = pv.at(0, o, i);
+        sph_finish<PASS, SOLIDS>(a, p, i, [&](int f) { return 0.0f + v[field_offset<MASK>(f)]; }, grav, g);
+        return;
     }
     sph_finish<PASS, SOLIDS>(a, p, i, [&](int f) { return seg_sum<MASK, COMP>(pv, i, f); }, grav, g);
 }
@@ -693,6 +768,7 @@ __global__ void __launch_bounds__(S::T, S::CTAS) k_gravity_sym(const float4* __r
     __shared__ float js[W][3][JT];
     __shared__ float rsh[3 * R][T];             // the row particles' running sums ...
     __shared__ float csh[COMP ? 3 * R : 1][T];  // ... and, compensated, their rounding errors
+    wait_predecessor();
     const int tid = threadIdx.x, warp = tid >> 5;
     int ga, gb;
     sym_task(static_cast<int>(blockIdx.x), G, ga, gb);
@@ -905,24 +981,24 @@ __global__ void __launch_bounds__(128) k_gravity(const float4* __restrict__ posm
     }
 }
 
-template <bool COMP>
-__global__ void __launch_bounds__(256) k_gravity_finish(DevArrays a, DevParams p, GravSum gsum) {
-    const int64_t i = fold_particle();
+template <bool COMP, int V>
+__global__ void __launch_bounds__(kFoldThreads) k_gravity_finish(DevArrays a, DevParams p, GravSum gsum) {
+    wait_predecessor();
     if (has(p, GSPH_VARIABLE_TIMESTEP) && blockIdx.x == 0 && threadIdx.x == 0) a.dt_state[1] = p.max_dt;
-    double t[3];
-    fold_slots<COMP>(a.part, a.n_pad, gsum.sym_G > 0 ? gsum.sym_G + 1 : gsum.nseg, i, i < a.n, t);
-    if ((threadIdx.x & 31) >= 8 || i >= a.n) return;
-    float acc[3];
+    fold_slots<COMP, V>(a.part, a.n, a.n_pad, gsum.sym_G > 0 ? gsum.sym_G + 1 : gsum.nseg, [&](int64_t i, const double (&t)[3]) {
+        float acc[3];
 #pragma unroll
-    for (int c = 0; c < 3; ++c)
-        acc[c] = COMP ? static_cast<float>(t[c] * static_cast<double>(p.G)) : p.G * static_cast<float>(t[c]);
-    if (a.grav) a.grav[i] = make_float4(acc[0], acc[1], acc[2], 0.0f);
-    environment(p, a.posm[i], a.velrho[i], acc[0], acc[1], acc[2]);
-    a.acc[i] = make_float4(acc[0], acc[1], acc[2], 0.0f);
-    a.xvel[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        for (int c = 0; c < 3; ++c)
+            acc[c] = COMP ? static_cast<float>(t[c] * static_cast<double>(p.G)) : p.G * static_cast<float>(t[c]);
+        if (a.grav) a.grav[i] = make_float4(acc[0], acc[1], acc[2], 0.0f);
+        environment(p, a.posm[i], a.velrho[i], acc[0], acc[1], acc[2]);
+        a.acc[i] = make_float4(acc[0], acc[1], acc[2], 0.0f);
+        a.xvel[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    });
 }
 
 inline unsigned blocks_for(int64_t n, int t) { return static_cast<unsigned>((n + t - 1) / t); }
+constexpr int kEach = 128;  // threads per CTA of the per-particle kernels: 4,096 particles on 32 SMs
 
 }  // namespace
 
@@ -964,6 +1040,15 @@ NearView near_view(const DevArrays& a, const DevParams& p, const SpatialArrays& 
     return v;
 }
 unsigned near_blocks(const DevArrays& a) { return static_cast<unsigned>(a.n_pad / kSub); }
+template <int W>
+cudaError_t near_launch(const DevArrays& a, const DevParams& p, const NearView& v, bool dens, bool comp, bool early,
+                        cudaStream_t s) {
+    auto kern = !dens ? k_near<W, false, false> : (comp ? k_near<W, true, true> : k_near<W, true, false>);
+    return launch_kernel(early, kern, near_blocks(a), kSub * W, s, a.posm, a.velrho, p, v);
+}
+// at most one warp and a half per scheduler of the 148 SMs when a warp takes 32 particles
+constexpr int kAhead = 4;  // records in flight then
+bool few_groups(const DevArrays& a) { return a.n_pad / kSub <= 900; }
 PartView seg_view(const DevArrays& a, int nseg, int KK, bool err) {
     return PartView{a.part, a.n_pad, nseg, KK, err};
 }
@@ -976,9 +1061,9 @@ cudaError_t launch_density(const DevArrays& a, const DevParams& p, const Launch&
     if (sp) {
         const NearView v = near_view(a, p, *sp);
         const bool dens = !has(p, GSPH_INTEGRATE_DENSITY);
-        if (!dens) k_near<false, false><<<near_blocks(a), kSub * kNearWarps, 0, s>>>(a.posm, a.velrho, p, v);
-        else if (comp) k_near<true, true><<<near_blocks(a), kSub * kNearWarps, 0, s>>>(a.posm, a.velrho, p, v);
-        else k_near<true, false><<<near_blocks(a), kSub * kNearWarps, 0, s>>>(a.posm, a.velrho, p, v);
+        const cudaError_t le = !dens && few_groups(a) ? near_launch<8>(a, p, v, dens, comp, !t, s)
+                                                                  : near_launch<4>(a, p, v, dens, comp, !t, s);
+        if (le != cudaSuccess) return le;
     } else {
         const int T = 256;
         const dim3 grid(static_cast<unsigned>(a.n_pad / T), static_cast<unsigned>(L.nseg));
@@ -989,16 +1074,15 @@ cudaError_t launch_density(const DevArrays& a, const DevParams& p, const Launch&
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     GSPH_TIMER_MARK(t, stop);
-    if (sp) return launch_prepare(a, p, s);  // the density is final: the j-records
+    if (sp) return launch_prepare(a, p, s, !t);  // the density is final: the j-records
     const PartView pv = seg_view(a, L.nseg, comp ? 2 : 1, comp);
     if (comp) k_density_finish<true><<<blocks_for(a.n, 256), 256, 0, s>>>(a, p, pv);
     else k_density_finish<false><<<blocks_for(a.n, 256), 256, 0, s>>>(a, p, pv);
     return cudaGetLastError();
 }
 
-cudaError_t launch_prepare(const DevArrays& a, const DevParams& p, cudaStream_t s) {
-    k_prepare<<<blocks_for(a.n, 256), 256, 0, s>>>(a, p);
-    return cudaGetLastError();
+cudaError_t launch_prepare(const DevArrays& a, const DevParams& p, cudaStream_t s, bool early) {
+    return launch_kernel(early, k_prepare, blocks_for(a.n, kEach), kEach, s, a, p);
 }
 
 namespace {
@@ -1011,17 +1095,25 @@ cudaError_t pairs_t(const DevArrays& a, const DevParams& p, const Launch& L, cud
         constexpr int K = popc_c(MASK);
         GSPH_TIMER_MARK(t, start);
         const NearView v = near_view(a, p, *sp);
-        k_pairs_near<PASS, SOLIDS, COMP><<<near_blocks(a), kSub, 0, s>>>(a, p, v);
-        cudaError_t e = cudaGetLastError();
+        void (*kern)(DevArrays, DevParams, NearView) = k_pairs_near<PASS, SOLIDS, COMP, 1>;
+        dim3 grid(near_blocks(a));
+        if (few_groups(a)) {
+            if constexpr (PASS == PASS_FUSED) {
+                kern = k_pairs_near_split<SOLIDS, COMP>;
+                grid.y = 2;
+            } else {
+                kern = k_pairs_near<PASS, SOLIDS, COMP, kAhead>;
+            }
+        }
+        cudaError_t e = launch_kernel(!t, kern, grid, kSub, s, a, p, v);
         if (e != cudaSuccess) return e;
         GSPH_TIMER_MARK(t, stop);
         if (join) {
             e = cudaStreamWaitEvent(s, join, 0);
             if (e != cudaSuccess) return e;
         }
-        k_pairs_finish<PASS, false, SOLIDS, COMP><<<blocks_for(a.n, 256), 256, 0, s>>>(
-            a, p, seg_view(a, 1, K, false), grav_sum(L, PASS == PASS_VGRAD ? 0 : gnseg));
-        return cudaGetLastError();
+        return launch_kernel(!t && !join, k_pairs_finish<PASS, false, SOLIDS, COMP>, blocks_for(a.n, kEach), kEach, s, a, p,
+                             seg_view(a, 1, K, false), grav_sum(L, PASS == PASS_VGRAD ? 0 : gnseg));
     }
     constexpr uint32_t MASK = field_mask<PASS, (GRAV != 0), SOLIDS>();
     constexpr int K = popc_c(MASK);
@@ -1115,13 +1207,9 @@ cudaError_t gravity_t(const DevArrays& a, const DevParams& p, const Launch& L, c
     if (e != cudaSuccess) return e;
     GSPH_TIMER_MARK(t, stop);
     const int S = L.grav_sym_G > 0 ? L.grav_sym_G + 1 : L.grav_nseg;
-    const unsigned fold_blocks = blocks_for(a.n * kFoldT, 256);  // kFoldT threads per particle
-    if (!finish) {  // the culled path: fold on this (the gravity) stream, the SPH finish reads a.gfold
-        k_gravity_fold<COMP><<<fold_blocks, 256, 0, s>>>(a.gpart, a.n, a.n_pad, S, a.gfold);
-        return cudaGetLastError();
-    }
-    k_gravity_finish<COMP><<<fold_blocks, 256, 0, s>>>(a, p, grav_sum(L, L.grav_nseg));
-    return cudaGetLastError();
+    if (!finish) return launch_gravity_fold(a, L, S, s, !t);  // the culled path: the SPH finish reads a.gfold
+    auto kern = fold_vec(a.n) == 4 ? k_gravity_finish<COMP, 4> : k_gravity_finish<COMP, 1>;
+    return launch_kernel(!t, kern, fold_blocks(a.n), kFoldThreads, s, a, p, grav_sum(L, L.grav_nseg));
 }
 template <int GRAV, bool COMP>
 cudaError_t gravity_i(const DevArrays& a, const DevParams& p, const Launch& L, cudaStream_t s, const KTimer* t,
@@ -1144,9 +1232,9 @@ cudaError_t gravity_any(const DevArrays& a, const DevParams& p, const Launch& L,
 cudaError_t launch_gravity(const DevArrays& a, const DevParams& p, const Launch& L, cudaStream_t s, const KTimer* t) {
     const bool comp = L.accum == GSPH_ACCUM_COMPENSATED;
     if (!has(p, GSPH_SELF_GRAVITY)) {  // neither gravity nor SPH: environment terms only
-        if (comp) k_gravity_finish<true><<<blocks_for(a.n, 256), 256, 0, s>>>(a, p, GravSum{});
-        else k_gravity_finish<false><<<blocks_for(a.n, 256), 256, 0, s>>>(a, p, GravSum{});
-        return cudaGetLastError();
+        auto kern = fold_vec(a.n) == 4 ? (comp ? k_gravity_finish<true, 4> : k_gravity_finish<false, 4>)
+                                       : (comp ? k_gravity_finish<true, 1> : k_gravity_finish<false, 1>);
+        return launch_kernel(false, kern, fold_blocks(a.n), kFoldThreads, s, a, p, GravSum{});
     }
     return gravity_any(a, p, L, s, t, true);
 }
@@ -1156,11 +1244,11 @@ cudaError_t launch_gravity_partials(const DevArrays& a, const DevParams& p, cons
     return gravity_any(a, p, L, s, t, false);
 }
 
-cudaError_t launch_gravity_fold(const DevArrays& a, const Launch& L, int S, cudaStream_t s) {
-    const unsigned nb = blocks_for(a.n * kFoldT, 256);
-    if (L.accum == GSPH_ACCUM_COMPENSATED) k_gravity_fold<true><<<nb, 256, 0, s>>>(a.gpart, a.n, a.n_pad, S, a.gfold);
-    else k_gravity_fold<false><<<nb, 256, 0, s>>>(a.gpart, a.n, a.n_pad, S, a.gfold);
-    return cudaGetLastError();
+cudaError_t launch_gravity_fold(const DevArrays& a, const Launch& L, int S, cudaStream_t s, bool early) {
+    const bool comp = L.accum == GSPH_ACCUM_COMPENSATED;
+    auto kern = fold_vec(a.n) == 4 ? (comp ? k_gravity_fold<true, 4> : k_gravity_fold<false, 4>)
+                                   : (comp ? k_gravity_fold<true, 1> : k_gravity_fold<false, 1>);
+    return launch_kernel(early, kern, fold_blocks(a.n), kFoldThreads, s, a.gpart, a.n, a.n_pad, S, a.gfold);
 }
 
 // Gravity partials of caller-provided, already padded j-records into caller-provided partials

@@ -222,7 +222,11 @@ __host__ __device__ constexpr uint32_t field_mask() {
     return m;
 }
 
-__host__ __device__ constexpr int popc_c(uint32_t x) { return x == 0 ? 0 : int(x & 1u) + popc_c(x >> 1); }
+__host__ __device__ constexpr int popc_c(uint32_t x) {  // no recursion: folds where the field is only known after unrolling
+    x -= (x >> 1) & 0x55555555u;
+    x = (x & 0x33333333u) + ((x >> 2) & 0x33333333u);
+    return static_cast<int>((((x + (x >> 4)) & 0x0f0f0f0fu) * 0x01010101u) >> 24);
+}
 
 template <uint32_t MASK>
 __host__ __device__ constexpr int field_offset(int f) {
@@ -286,7 +290,8 @@ void sym_shape(int64_t n_pad, int sms, int groups, int shape, Launch& L);
 // INTEGRATE_DENSITY the search alone), which stores the lists that the SPH passes of the step read.
 cudaError_t launch_density(const DevArrays& a, const DevParams& p, const Launch& L, cudaStream_t s,
                            const KTimer* t = nullptr, const SpatialArrays* sp = nullptr);
-cudaError_t launch_prepare(const DevArrays& a, const DevParams& p, cudaStream_t s);
+// `early`: launched early (common.cuh) behind a kernel of the same step
+cudaError_t launch_prepare(const DevArrays& a, const DevParams& p, cudaStream_t s, bool early = false);
 // With `sp`, the SPH terms run over the neighbour lists of launch_density; the finish kernel then adds the gravity sums (a.gfold, from launch_gravity_partials), after waiting for
 // `join` when it is given (the gravity kernel may run on another stream).
 cudaError_t launch_pairs(int pass, const DevArrays& a, const DevParams& p, const Launch& L, cudaStream_t s,
@@ -300,7 +305,7 @@ cudaError_t launch_fp32_peak(int sm_count, int iters, float* sink, cudaStream_t 
 cudaError_t launch_gravity_raw(const float4* posm_padded, float* part, int64_t n_pad, int ipt, int jt, int nseg,
                                float eps2, int* status, cudaStream_t s);
 // the FP64 fold of `S` slots of a.gpart into a.gfold
-cudaError_t launch_gravity_fold(const DevArrays& a, const Launch& L, int S, cudaStream_t s);
+cudaError_t launch_gravity_fold(const DevArrays& a, const Launch& L, int S, cudaStream_t s, bool early);
 int64_t fp32_peak_flops(int sm_count, int iters);
 
 // the gravity partials and their fold with the kernels of the fixed order (gravity_fixed.cu)

@@ -16,6 +16,7 @@ __global__ void __launch_bounds__(256) k_chunk_bounds(DevArrays a, SpatialArrays
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int64_t w = static_cast<int64_t>(blockIdx.x) * 8 + warp, i = w * 32 + lane;
     float mn[3] = {INFINITY, INFINITY, INFINITY}, mx[3] = {-INFINITY, -INFINITY, -INFINITY};
+    wait_predecessor();
     if (i < a.n) {
         const float4 p = a.posm[i];
         mn[0] = mx[0] = p.x; mn[1] = mx[1] = p.y; mn[2] = mx[2] = p.z;
@@ -51,6 +52,7 @@ __global__ void __launch_bounds__(128) k_chunk_lists(const float4* __restrict__ 
                                                      int* __restrict__ list, int* __restrict__ count, int64_t ngroups,
                                                      int64_t nchunks, float h2m) {
     constexpr int per_group = kGroup / kChunk;
+    wait_predecessor();
     const int lane = threadIdx.x & 31;
     const int64_t g = static_cast<int64_t>(blockIdx.x) * 4 + (threadIdx.x >> 5);
     if (g >= ngroups) return;
@@ -94,6 +96,7 @@ __global__ void __launch_bounds__(kOrderThreads) k_group_order(const int* __rest
                                                                int ngroups, int items) {
     __shared__ int most, bins[kBuckets], warp_sum[kBuckets / 32];
     __shared__ unsigned long long total;
+    wait_predecessor();
     if (threadIdx.x == 0) {
         most = 1;
         total = 0;
@@ -245,13 +248,13 @@ cudaError_t launch_chunk_bounds(const DevArrays& a, const SpatialArrays& s, cuda
 cudaError_t launch_chunk_lists(const DevArrays& a, const SpatialArrays& s, float h, cudaStream_t st) {
     const int64_t nchunks = a.n_pad / kChunk, ngroups = a.n_pad / kGroup;
     const float hm = h * (1.0f + kMargin);
-    k_chunk_lists<<<blocks_for(ngroups, 4), 128, 0, st>>>(s.box_lo, s.box_hi, s.list, s.count, ngroups, nchunks, hm * hm);
-    return cudaGetLastError();
+    return launch_kernel(true, k_chunk_lists, blocks_for(ngroups, 4), 128, st, s.box_lo, s.box_hi, s.list, s.count, ngroups,
+                         nchunks, hm * hm);
 }
 
 cudaError_t launch_group_order(const DevArrays& a, const SpatialArrays& s, int items, cudaStream_t st) {
-    k_group_order<<<1, kOrderThreads, 0, st>>>(s.count, s.group_order, static_cast<int>(a.n_pad / kGroup), items);
-    return cudaGetLastError();
+    return launch_kernel(true, k_group_order, 1, kOrderThreads, st, s.count, s.group_order,
+                         static_cast<int>(a.n_pad / kGroup), items);
 }
 
 cudaError_t launch_identity_order(const SpatialArrays& s, int64_t n_pad, cudaStream_t st) {

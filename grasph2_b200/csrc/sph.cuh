@@ -92,11 +92,12 @@ __device__ __forceinline__ ISph load_isph(const DevArrays& a, const DevParams& p
 
 // The SPH terms of one neighbour pair (0 < r <= H): velocity-gradient terms
 // (computeDerivatives.h:118-141) and acceleration terms (:237-295). d = x_j - x_i, r2 = |d|^2.
-template <int PASS, bool SOLIDS>
+// PART 1 / 2: only the first / only the second of them, in the arithmetic of both.
+template <int PASS, bool SOLIDS, int PART = 0>
 __device__ __forceinline__ void sph_neighbour(PairAcc& T, float& maxv, const ISph& I, float mj, float dx, float dy,
                                               float dz, float r2, float4 vj, float4 ja, float4 jb, const DevParams& p) {
-    constexpr bool DO_V = PASS != PASS_ACC;
-    constexpr bool DO_A = PASS != PASS_VGRAD;
+    constexpr bool DO_V = PASS != PASS_ACC && PART != 2;
+    constexpr bool DO_A = PASS != PASS_VGRAD && PART != 1;
     const float inv_r = rsqrtf(r2);
     const float r = r2 * inv_r;
     const float qq = r * p.inv_h;
