@@ -575,7 +575,7 @@ int gsph_create(const gsph_params* p, const gsph_options* opt, int64_t n, gsph_c
         sp.sort_tmp_bytes = spatial_sort_tmp_bytes(n_pad);
         sp.sort_tmp = dalloc(c, sp.sort_tmp_bytes, ae);
         sp.bbox = static_cast<int*>(dalloc(c, 8 * sizeof(int), ae));
-        sp.tmp4 = static_cast<float4*>(dalloc(c, n_pad * sizeof(float4), ae));
+        sp.tmp4 = static_cast<float4*>(dalloc(c, permute_rows(n_pad) * n_pad * sizeof(float4), ae));
         sp.tmp8 = static_cast<double*>(dalloc(c, n_pad * sizeof(double), ae));
     }
     a.dt_state = static_cast<float*>(dalloc(c, 4 * sizeof(float), ae));

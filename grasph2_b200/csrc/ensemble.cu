@@ -1281,7 +1281,7 @@ int gsph_ensemble_create(const gsph_params* p, const gsph_options* opt, int32_t 
                                     static_cast<unsigned long long*>(nullptr), static_cast<const int*>(nullptr),
                                     static_cast<int*>(nullptr), static_cast<int>(n_pad));
     e->sort_tmp = ens_alloc(e, e->sort_bytes, ae);
-    e->tmp4 = static_cast<float4*>(ens_alloc(e, n_pad * sizeof(float4), ae));
+    e->tmp4 = static_cast<float4*>(ens_alloc(e, permute_rows(n_pad) * n_pad * sizeof(float4), ae));
     e->tmp8 = static_cast<double*>(ens_alloc(e, n_pad * sizeof(double), ae));
     e->bbox = static_cast<float*>(ens_alloc(e, static_cast<size_t>(nsims) * 8 * sizeof(float), ae));
     if (ae == cudaSuccess) ae = cudaMemcpy(e->groups, groups.data(), groups.size() * sizeof(int4), cudaMemcpyHostToDevice);

@@ -1,4 +1,6 @@
 // spatial.cu -- chunk bounding boxes, per-group near-chunk lists, and the Hilbert-curve reorder.
+#include <algorithm>
+
 #include <cub/device/device_radix_sort.cuh>
 
 #include "spatial.cuh"
@@ -220,6 +222,43 @@ __global__ void k_iota(int* v, int64_t n) {
     if (i < n) v[i] = static_cast<int>(i);
 }
 
+// All the arrays of a small context at once: gathered into scratch rows (BACK: copied from there), one array or group of
+// arrays per blockIdx.y. With a gather and a copy per array, sixteen arrays of 4,096 particles took about 80 us of
+// launches; from 65,536 particles on the copies themselves count and the rows would take 200 bytes per particle.
+struct PermuteSet {
+    float4* v4[10];
+    double* v8;
+    float *f0, *f1;
+    int* ext;
+};
+template <bool BACK>
+__global__ void __launch_bounds__(256) k_permute_all(PermuteSet s, float4* __restrict__ tmp, const int* __restrict__ order,
+                                                     int64_t n) {
+    const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const int y = blockIdx.y;
+    const int64_t o = BACK ? i : order[i];
+    auto move = [&](auto* arr, auto* row) {
+        if (BACK) arr[i] = row[i];
+        else row[i] = arr[o];
+    };
+    if (y < 10) {
+        float4* arr = s.v4[0];
+#pragma unroll
+        for (int k = 1; k < 10; ++k)
+            if (y == k) arr = s.v4[k];
+        move(arr, tmp + y * n);
+    } else if (y == 10) {
+        double* row = reinterpret_cast<double*>(tmp + 10 * n);
+        for (int d = 0; d < 3; ++d) move(s.v8 + d * n, row + d * n);
+    } else {
+        float* row = reinterpret_cast<float*>(tmp + 12 * n);
+        move(s.f0, row);
+        move(s.f1, row + n);
+        move(s.ext, reinterpret_cast<int*>(row + 2 * n));
+    }
+}
+
 template <typename T>
 cudaError_t permute(T* arr, T* tmp, const int* order, int64_t n, cudaStream_t st, int& launches) {
     k_gather<T><<<blocks_for(n, 256), 256, 0, st>>>(arr, tmp, order, n);
@@ -265,7 +304,8 @@ cudaError_t launch_identity_order(const SpatialArrays& s, int64_t n_pad, cudaStr
 cudaError_t curve_order(const DevArrays& a, const SpatialArrays& s, cudaStream_t st, int& launches) {
     const int64_t np = a.n_pad;
     k_bbox_init<<<1, 32, 0, st>>>(s.bbox);
-    k_bbox<<<256, 256, 0, st>>>(a, s.bbox);
+    // four particles per thread, so that the warps' atomics stay few (256 CTAs on 4,096 particles took 10.4 us)
+    k_bbox<<<std::min(256u, blocks_for(a.n, 1024)), 256, 0, st>>>(a, s.bbox);
     k_curve_keys<<<blocks_for(np, 256), 256, 0, st>>>(a, s.bbox, s.keys, s.order);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
@@ -288,6 +328,15 @@ cudaError_t permute_particles(const DevArrays& a, const int* ord, float4* t4, do
                               cudaStream_t st, int& launches) {
     const int64_t np = a.n_pad;
     cudaError_t e = cudaSuccess;
+    if (permute_rows(np) > 1) {
+        const PermuteSet set{{a.posm, a.velrho, a.acc, a.xvel, a.sA, a.sB, a.dA, a.dB, a.jA, a.jB},
+                             a.pos64, a.rhodot, a.balsara, ext_of_int};
+        const dim3 grid(blocks_for(np, 256), 12);
+        k_permute_all<false><<<grid, 256, 0, st>>>(set, t4, ord, np);
+        k_permute_all<true><<<grid, 256, 0, st>>>(set, t4, ord, np);
+        launches += 2;
+        return cudaGetLastError();
+    }
     float4* f4s[] = {a.posm, a.velrho, a.acc, a.xvel, a.sA, a.sB, a.dA, a.dB, a.jA, a.jB};
     for (float4* arr : f4s) {
         e = permute(arr, t4, ord, np, st, launches);

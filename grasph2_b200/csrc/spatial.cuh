@@ -35,7 +35,7 @@ struct SpatialArrays {
     void* sort_tmp;    // CUB radix-sort scratch
     size_t sort_tmp_bytes;
     int* bbox;         // [6] global bounds as ordered ints
-    float4* tmp4;      // [n_pad] permutation scratch
+    float4* tmp4;      // [permute_rows(n_pad)][n_pad] permutation scratch
     double* tmp8;      // [3 n_pad]
 };
 
@@ -88,8 +88,10 @@ cudaError_t reorder_particles(const DevArrays& a, const SpatialArrays& s, cudaSt
 // The first half of it: order_out[k] = slot of the k-th particle along the curve (padding last, in place).
 cudaError_t curve_order(const DevArrays& a, const SpatialArrays& s, cudaStream_t st, int& launches);
 cudaError_t launch_identity_order(const SpatialArrays& s, int64_t n_pad, cudaStream_t st);
+// rows of float4 that the permutation takes as scratch: every array at once in small contexts, one elsewhere
+inline int permute_rows(int64_t n_pad) { return n_pad <= 65536 ? 13 : 1; }
 // Gather every per-particle array of `a` (all n_pad slots) and `ext_of_int` by `order` (new slot i takes
-// old slot order[i]); t4 / t8 are n_pad-element scratch.
+// old slot order[i]); t4 (permute_rows(n_pad) rows) and t8 are scratch.
 cudaError_t permute_particles(const DevArrays& a, const int* order, float4* t4, double* t8, int* ext_of_int,
                               cudaStream_t st, int& launches);
 
