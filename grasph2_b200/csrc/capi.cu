@@ -369,6 +369,14 @@ bool gsph_ctx_state(gsph_ctx* c, DevArrays* a, const int** ext) {
     return true;
 }
 
+// gsph_surrogate_features of the state whose derivatives gsph_ctx_proposal_derivatives has just evaluated
+int gsph_ctx_proposal_features(gsph_ctx* c, const float* mu, const float* sigma, float* feat, void* stream) {
+    if (c->fp64 || !c->L.cull || !(c->params.flags & GSPH_SPH)) return gsph_surrogate_features(c, mu, sigma, feat, stream);
+    GSPH_CK(c, launch_features(c->a, c->dp, c->sp, mu, sigma, feat, as_stream(stream), true), "features");
+    c->launches += 1;
+    return GSPH_OK;
+}
+
 // the derivatives of a network proposal (surrogate_run.cu)
 int gsph_ctx_proposal_derivatives(gsph_ctx* c, void* stream) {
     return derivatives(c, as_stream(stream), true);
@@ -984,7 +992,7 @@ int gsph_surrogate_features(gsph_ctx* c, const float* mu, const float* sigma, fl
     cudaStream_t s = as_stream(stream);
     GSPH_CK(c, launch_chunk_bounds(c->a, c->sp, s), "chunk bounds");
     GSPH_CK(c, launch_chunk_lists(c->a, c->sp, c->dp.H, s), "chunk lists");
-    GSPH_CK(c, launch_features(c->a, c->dp, c->sp, mu, sigma, feat, s), "features");
+    GSPH_CK(c, launch_features(c->a, c->dp, c->sp, mu, sigma, feat, s, false), "features");
     c->launches += 3;
     return GSPH_OK;
 }

@@ -31,6 +31,7 @@
 
 void set_global_error(const std::string& msg);  // capi.cu
 int gsph_ctx_proposal_derivatives(gsph_ctx* c, void* stream);  // capi.cu
+int gsph_ctx_proposal_features(gsph_ctx* c, const float* mu, const float* sigma, float* feat, void* stream);  // capi.cu
 
 namespace {
 constexpr int kIn = GSPH_MLP_IN, kOut = GSPH_MLP_OUT;
@@ -204,7 +205,7 @@ int propose_from_derivatives(gsph_surrogate* s, gsph_ctx* ctx, int32_t use_net, 
     gsph_size(ctx, &n);
     rc = reserve(s, n);
     if (rc != GSPH_OK) return rc;
-    rc = gsph_surrogate_features(ctx, s->stats, s->stats + kIn, s->feat, stream);
+    rc = gsph_ctx_proposal_features(ctx, s->stats, s->stats + kIn, s->feat, stream);
     if (rc != GSPH_OK) return ctx_fail(s, ctx, rc, "propose: features");
     rc = gsph_mlp_forward(s->net, s->feat, s->out, n, stream);
     if (rc != GSPH_OK) return sfail(s, rc, std::string("propose: MLP: ") + gsph_mlp_last_error(s->net));
