@@ -768,7 +768,6 @@ __global__ void __launch_bounds__(S::T, S::CTAS) k_gravity_sym(const float4* __r
     __shared__ float js[W][3][JT];
     __shared__ float rsh[3 * R][T];             // the row particles' running sums ...
     __shared__ float csh[COMP ? 3 * R : 1][T];  // ... and, compensated, their rounding errors
-    wait_predecessor();
     const int tid = threadIdx.x, warp = tid >> 5;
     int ga, gb;
     sym_task(static_cast<int>(blockIdx.x), G, ga, gb);

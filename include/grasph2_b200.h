@@ -179,10 +179,10 @@ typedef struct gsph_options {
                                 every unordered pair once and applies it to both particles (Newton's third law;
                                 14 to 16 FP32 operations for both against 24, partials of up to 129 x 3 floats per
                                 particle). Auto is the symmetric form, unless scalar_fp32 or, below 24 blocks of 1024
-                                particles, a shape of the one-sided kernel is asked for. Results agree to rounding.
-                                Ensembles use the one-sided sweep fused with their density pass; SYMMETRIC
-                                gives them a queue stage of group pairs instead (slower on ensembles of
-                                1k..32k-particle simulations) */
+                                particles, a shape of the one-sided kernel is asked for, and from 2,049 particles on
+                                (plain sums: 3,073). Results agree to rounding. Ensembles take the symmetric form
+                                too (AUTO: while its partials take at most 1 KB per particle); ONE_SIDED gives them
+                                the sweep fused with the density pass */
     int32_t gravity_groups;  /* symmetric form: particle groups G at most (tasks G(G+1)/2); 0 = up to 128 */
     int32_t wait_limit_us;   /* batched ensemble: a work item that waits for another item's result (a device-side
                                 spin on a counter) gives up after this many microseconds, sets the timeout bit
