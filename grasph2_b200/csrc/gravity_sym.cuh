@@ -53,7 +53,22 @@ __device__ __forceinline__ void sym_stage(float4* XY, float4* ZM, int j, float4 
     zm[half] = r.z; zm[2 + half] = r.w;
 }
 
-// the separations of row m from a column pair, and 1/r^3
+// How a pair's masses enter. kSymEqual: they do not (rows times the columns' mass, columns times minus the rows' are the
+// caller's). kSymMasses: they multiply 1/r^3, which one FP32 number holds for separations from 1.5e-13 to 4.3e12 only
+// (1/r^3 from 3e38 down to the smallest normal number). kSymFar: (m / r) (1 / r^2), two products more per pair, good for
+// as long as r^2 and the force are, for tiles that may reach farther (lengths in metres between stars) or, softened,
+// come nearer. A tile is far when a coordinate of its rows or columns reaches 2^40 (then, and only then, two of them can be
+// more than sqrt(3) 2^41 = 3.8e12 apart), or by its softening.
+enum SymMode { kSymEqual, kSymMasses, kSymFar };
+__device__ __forceinline__ bool sym_far(float4 q) {  // NaN counts as far
+    return !(fmaxf(fmaxf(fabsf(q.x), fabsf(q.y)), fabsf(q.z)) < 0x1p40f);
+}
+template <int GRAV>
+__device__ __forceinline__ bool sym_far_eps(float eps2) {  // 1/eps^3 above 1e38, or a larger reach
+    return GRAV == 1 && !(eps2 >= 5e-26f && eps2 <= 4e24f);
+}
+
+// the separations of row m from a column pair, and 1/r
 template <typename S, int GRAV>
 __device__ __forceinline__ float2 sym_pair(const SymRows<S>& r, int m, float4 xy, float4 zm, float2 E2, float2& dx, float2& dy,
                                            float2& dz) {
@@ -63,12 +78,12 @@ __device__ __forceinline__ float2 sym_pair(const SymRows<S>& r, int m, float4 xy
     const float2 r2 = fma2(dz, dz, fma2(dy, dy, fma2(dx, dx, E2)));
     float2 inv = make_float2(rsqrtf(r2.x), rsqrtf(r2.y));
     if (GRAV == 2) inv = make_float2(fminf(inv.x, 1e12f), fminf(inv.y, 1e12f));
-    return mul2(mul2(inv, inv), inv);
+    return inv;
 }
+__device__ __forceinline__ float2 cube2(float2 v) { return mul2(mul2(v, v), v); }
 
-// the rows against every column pair of the tile: row sums into r, the warp's column sums into js[component][column].
-// EQ: neither carries the masses (rows times the columns' mass, columns times minus the rows' are the caller's).
-template <typename S, int GRAV, bool EQ>
+// the rows against every column pair of the tile: row sums into r, the warp's column sums into js[component][column]
+template <typename S, int GRAV, SymMode MODE>
 __device__ __forceinline__ void sym_columns(SymRows<S>& rows, const float4* XY, const float4* ZM, float2 E2,
                                             float (*js)[S::JT]) {
     const int lane = threadIdx.x & 31, next = (lane + 1) & 31;
@@ -82,11 +97,13 @@ __device__ __forceinline__ void sym_columns(SymRows<S>& rows, const float4* XY, 
 #pragma unroll
             for (int m = 0; m < S::R; ++m) {
                 float2 dx, dy, dz;
-                const float2 i3 = sym_pair<S, GRAV>(rows, m, xy, zm, E2, dx, dy, dz);
-                if (EQ) {
-                    add_both(rows.TX[m], rows.TY[m], rows.TZ[m], cx, cy, cz, dx, dy, dz, i3);
+                const float2 inv = sym_pair<S, GRAV>(rows, m, xy, zm, E2, dx, dy, dz);
+                if (MODE == kSymEqual) {
+                    add_both(rows.TX[m], rows.TY[m], rows.TZ[m], cx, cy, cz, dx, dy, dz, cube2(inv));
                 } else {
-                    const float2 sj = mul2(make_float2(zm.z, zm.w), i3), si = mul2(rows.M[m], i3);
+                    const float2 mj = make_float2(zm.z, zm.w), f = MODE == kSymFar ? mul2(inv, inv) : cube2(inv);
+                    const float2 sj = mul2(MODE == kSymFar ? mul2(mj, inv) : mj, f);
+                    const float2 si = mul2(MODE == kSymFar ? mul2(rows.M[m], inv) : rows.M[m], f);
                     rows.TX[m] = fma2(dx, sj, rows.TX[m]);
                     rows.TY[m] = fma2(dy, sj, rows.TY[m]);
                     rows.TZ[m] = fma2(dz, sj, rows.TZ[m]);
@@ -105,7 +122,7 @@ __device__ __forceinline__ void sym_columns(SymRows<S>& rows, const float4* XY, 
 }
 
 // one-sided: the rows' sums over the tile's columns, masses included (a block against itself)
-template <typename S, int GRAV>
+template <typename S, int GRAV, bool FAR>
 __device__ __forceinline__ void sym_own(SymRows<S>& rows, const float4* XY, const float4* ZM, float2 E2) {
 #pragma unroll 2
     for (int j = 0; j < S::JT / 2; ++j) {
@@ -113,8 +130,8 @@ __device__ __forceinline__ void sym_own(SymRows<S>& rows, const float4* XY, cons
 #pragma unroll
         for (int m = 0; m < S::R; ++m) {
             float2 dx, dy, dz;
-            const float2 i3 = sym_pair<S, GRAV>(rows, m, xy, zm, E2, dx, dy, dz);
-            const float2 sj = mul2(make_float2(zm.z, zm.w), i3);
+            const float2 inv = sym_pair<S, GRAV>(rows, m, xy, zm, E2, dx, dy, dz), mj = make_float2(zm.z, zm.w);
+            const float2 sj = FAR ? mul2(mul2(mj, inv), mul2(inv, inv)) : mul2(mj, cube2(inv));
             rows.TX[m] = fma2(dx, sj, rows.TX[m]);
             rows.TY[m] = fma2(dy, sj, rows.TY[m]);
             rows.TZ[m] = fma2(dz, sj, rows.TZ[m]);

@@ -761,7 +761,7 @@ __host__ __device__ __forceinline__ void sym_task(int t, int G, int& ga, int& gb
 
 template <typename S, int GRAV, bool COMP>
 __global__ void __launch_bounds__(S::T, S::CTAS) k_gravity_sym(const float4* __restrict__ posm, float* __restrict__ part,
-                                                               int64_t n_pad, int G, int gs, float eps2) {
+                                                               int64_t n, int64_t n_pad, int G, int gs, float eps2) {
     constexpr int R = S::R, T = S::T, B = S::B, JT = S::JT, PF = S::PF, W = S::W;
     constexpr int K = COMP ? 6 : 3;
     __shared__ float4 XY[JT / 2], ZM[JT / 2];
@@ -788,19 +788,20 @@ __global__ void __launch_bounds__(S::T, S::CTAS) k_gravity_sym(const float4* __r
         const int64_t base = static_cast<int64_t>(a) * B + tid;
         SymRows<S> rows;
         const float mr = posm[static_cast<int64_t>(a) * B].w;
-        bool same = true;
+        bool same = true, far_r = sym_far_eps<GRAV>(eps2);
 #pragma unroll
         for (int k = 0; k < R; ++k) {
             const float4 u = posm[base + static_cast<int64_t>(k) * T];
             rows.set(k, u);
             same = same && u.w == mr;
+            far_r = far_r || (base + static_cast<int64_t>(k) * T < n && sym_far(u));  // padding lies far, without mass
 #pragma unroll
             for (int c = 0; c < 3; ++c) {
                 rsh[c * R + k][tid] = 0.0f;
                 if (COMP) csh[COMP ? c * R + k : 0][tid] = 0.0f;
             }
         }
-        const bool rows_equal = __syncthreads_and(same);
+        const bool rows_equal = __syncthreads_and(same), rows_far = __syncthreads_or(far_r);
         // tiles: the block's own (one-sided) when diagonal, then the columns
         const int64_t d0 = static_cast<int64_t>(a) * B;
         const int nd = diag ? B / JT : 0;
@@ -817,7 +818,10 @@ __global__ void __launch_bounds__(S::T, S::CTAS) k_gravity_sym(const float4* __r
             for (int h = 0; h < PF; ++h) pf[h] = posm[src(0) + h * T + tid];
         }
         for (int k = 0; k < total; ++k) {
-            __syncthreads();  // the previous tile's reads of XY, ZM and js are done
+            bool far_c = false;
+#pragma unroll
+            for (int h = 0; h < PF; ++h) far_c = far_c || (src(k) + h * T + tid < n && sym_far(pf[h]));
+            const bool far = __syncthreads_or(far_c) || rows_far;  // and the previous tile's reads of XY, ZM and js are done
             const float mc = mn;
             bool same_c = true;
 #pragma unroll
@@ -825,16 +829,17 @@ __global__ void __launch_bounds__(S::T, S::CTAS) k_gravity_sym(const float4* __r
                 sym_stage(XY, ZM, tid + h * T, pf[h]);
                 same_c = same_c && pf[h].w == mc;
             }
-            const bool equal = __syncthreads_and(same_c) && rows_equal;
+            const bool equal = __syncthreads_and(same_c) && rows_equal && !far;
             if (k + 1 < total) {
                 mn = posm[src(k + 1)].w;
 #pragma unroll
                 for (int h = 0; h < PF; ++h) pf[h] = posm[src(k + 1) + h * T + tid];
             }
             rows.clear();
-            if (k < nd) sym_own<S, GRAV>(rows, XY, ZM, E2);
-            else if (equal) sym_columns<S, GRAV, true>(rows, XY, ZM, E2, js[warp]);
-            else sym_columns<S, GRAV, false>(rows, XY, ZM, E2, js[warp]);
+            if (k < nd) far ? sym_own<S, GRAV, true>(rows, XY, ZM, E2) : sym_own<S, GRAV, false>(rows, XY, ZM, E2);
+            else if (equal) sym_columns<S, GRAV, kSymEqual>(rows, XY, ZM, E2, js[warp]);
+            else if (!far) sym_columns<S, GRAV, kSymMasses>(rows, XY, ZM, E2, js[warp]);
+            else sym_columns<S, GRAV, kSymFar>(rows, XY, ZM, E2, js[warp]);
             // the tile's row partials into the running sums: a two-sum fold (compensated), or one add (plain: a sum
             // of tile sums, not one running sum over the whole column group)
             const float wr = k >= nd && equal ? mc : 1.0f;
@@ -1173,7 +1178,7 @@ namespace {
 template <typename S, int GRAV, bool COMP>
 void sym_launch(const DevArrays& a, const DevParams& p, const Launch& L, float* out, cudaStream_t s) {
     const int G = L.grav_sym_G;
-    k_gravity_sym<S, GRAV, COMP><<<static_cast<unsigned>(G * (G + 1) / 2), S::T, 0, s>>>(a.posm, out, a.n_pad, G,
+    k_gravity_sym<S, GRAV, COMP><<<static_cast<unsigned>(G * (G + 1) / 2), S::T, 0, s>>>(a.posm, out, a.n, a.n_pad, G,
                                                                                         L.grav_sym_gs, p.eps2);
 }
 template <int I, int GRAV, bool COMP>
