@@ -122,9 +122,11 @@ __device__ __forceinline__ void bulk_g2s(void* dst, const void* src, uint32_t by
 // ---- programmatic dependent launch -----------------------------------------------------------
 // A kernel of a step is set up while its predecessor on the stream drains, and waits here for that kernel's end before
 // it reads or writes anything. Every kernel that is launched `early` calls this first: then a kernel that has got past
-// it may rely on all the earlier ones, not only on its direct predecessor. No kernel releases its successors before its
-// end: their waiting CTAs would take room from the gravity kernel on the other stream (a step of the impact with 65,536
-// particles 1,330 -> 1,417 us that way).
+// it may rely on all the earlier ones, not only on its direct predecessor. What it reads is written while it is already
+// resident, so it uses plain loads: __ldg and const __restrict__ pointers stand for memory that is read-only for the
+// kernel's whole life, and the compiler may move their loads above the wait. No kernel releases its successors before
+// its end: their waiting CTAs would take room from the gravity kernel on the other stream (a step of the impact with
+// 65,536 particles 1,330 -> 1,417 us that way).
 // Measured: a step of the Plummer sphere with 4,096 particles (three kernels) 18.4 -> 16.4 us.
 __device__ __forceinline__ void wait_predecessor() {
     asm volatile("griddepcontrol.wait;" ::: "memory");

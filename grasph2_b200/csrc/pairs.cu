@@ -99,7 +99,7 @@ __global__ void __launch_bounds__(256) k_density(const float4* __restrict__ posm
 // search with the density sum (71.6 us for 68.5 in the fluid's step: the walk over the stages is each warp's own).
 constexpr int kBatch = 64;
 template <int W, bool DENS, bool COMP>
-__global__ void __launch_bounds__(kSub * W) k_near(const float4* __restrict__ posm, float4* __restrict__ velrho,
+__global__ void __launch_bounds__(kSub * W) k_near(const float4* posm, float4* velrho,
                                                             DevParams p, NearView v) {
     __shared__ float4 sh[W][kSub];
     __shared__ unsigned mk[kBatch * kHalves][kSub];   // neighbour masks of the batch's boxes
@@ -431,10 +431,10 @@ __device__ __forceinline__ void pairs_near(const DevArrays& a, const DevParams& 
         float4 rec[D][4];
         auto load = [&](int d) {
             const float4* r = a.jrec + 4 * static_cast<int64_t>(e[d] & ~kItemMark);
-            rec[d][0] = __ldg(r);
-            rec[d][1] = __ldg(r + 1);
-            rec[d][2] = DO_A ? __ldg(r + 2) : zero;
-            rec[d][3] = DO_A ? __ldg(r + 3) : zero;
+            rec[d][0] = r[0];
+            rec[d][1] = r[1];
+            rec[d][2] = DO_A ? r[2] : zero;
+            rec[d][3] = DO_A ? r[3] : zero;
         };
 #pragma unroll
         for (int d = 0; d < D; ++d) {
@@ -536,7 +536,7 @@ __device__ __forceinline__ float fold_get(const typename FoldVec<V>::type& x, in
 }
 // f(i, sum) for the particles of this CTA, on the threads of warp 0
 template <bool COMP, int V, typename F>
-__device__ __forceinline__ void fold_slots(const float* __restrict__ part, int64_t n, int64_t n_pad, int S, F&& f) {
+__device__ __forceinline__ void fold_slots(const float* part, int64_t n, int64_t n_pad, int S, F&& f) {
     using Vec = typename FoldVec<V>::type;
     constexpr int K = COMP ? 6 : 3, U = (V == 4 ? 12 : 54) / K;
     __shared__ double run[kFoldT - 1][V][3][32];
@@ -555,7 +555,7 @@ __device__ __forceinline__ void fold_slots(const float* __restrict__ part, int64
                 const float* p = part + static_cast<int64_t>(V == 1 ? k + u : min(k + u, k1 - 1)) * K * n_pad + i;
 #pragma unroll
                 for (int c = 0; c < K; ++c)
-                    v[u][c] = V > 1 || k + u < k1 ? __ldg(reinterpret_cast<const Vec*>(p + c * n_pad)) : Vec{};
+                    v[u][c] = V > 1 || k + u < k1 ? *reinterpret_cast<const Vec*>(p + c * n_pad) : Vec{};
             }
 #pragma unroll
             for (int u = 0; u < U; ++u) {
@@ -595,8 +595,8 @@ inline unsigned fold_blocks(int64_t n) { return static_cast<unsigned>((n + 32 * 
 
 // the culled path: the fold of the gravity partials into gfold[3][n_pad], on the gravity kernel's stream
 template <bool COMP, int V>
-__global__ void __launch_bounds__(kFoldThreads) k_gravity_fold(const float* __restrict__ part, int64_t n, int64_t n_pad, int S,
-                                                               double* __restrict__ gfold) {
+__global__ void __launch_bounds__(kFoldThreads) k_gravity_fold(const float* part, int64_t n, int64_t n_pad, int S,
+                                                               double* gfold) {
     wait_predecessor();
     fold_slots<COMP, V>(part, n, n_pad, S, [&](int64_t i, const double (&t)[3]) {
         for (int c = 0; c < 3; ++c) gfold[c * n_pad + i] = t[c];

@@ -123,7 +123,7 @@ constexpr int kItemMark = static_cast<int>(0x80000000u);
 // box's load in flight while one is tested, and body(mask, jb, c) gets each lane's mask of the neighbours (0 < r^2 <= H^2,
 // bit k: particle jb + k, its record in sh[k]) and the chunk's place in the list.
 template <typename Body>
-__device__ __forceinline__ void near_scan(const NearView& v, const float4* __restrict__ posm, int g, int64_t s0,
+__device__ __forceinline__ void near_scan(const NearView& v, const float4* posm, int g, int64_t s0,
                                           uint32_t span, float4 pi, float4* sh, Body&& body) {
     const int lane = threadIdx.x & 31;
     const float4 l = v.lo[s0 / kSub], u = v.hi[s0 / kSub];

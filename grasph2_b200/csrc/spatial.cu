@@ -50,8 +50,7 @@ __device__ __forceinline__ float gap(float lo_a, float hi_a, float lo_b, float h
 }
 
 // one warp per i-group: the ordered list of chunks within h of the group's box, 128 chunks per round
-__global__ void __launch_bounds__(128) k_chunk_lists(const float4* __restrict__ lo, const float4* __restrict__ hi,
-                                                     int* __restrict__ list, int* __restrict__ count, int64_t ngroups,
+__global__ void __launch_bounds__(128) k_chunk_lists(const float4* lo, const float4* hi, int* list, int* count, int64_t ngroups,
                                                      int64_t nchunks, float h2m) {
     constexpr int per_group = kGroup / kChunk;
     wait_predecessor();
@@ -94,7 +93,7 @@ __global__ void __launch_bounds__(128) k_chunk_lists(const float4* __restrict__ 
 // the short ones fill the last wave, and the chunks per item ceil(total near chunks / items). One block: counting
 // sort. The order within a bucket is not fixed, and need not be: every group's results are its own.
 constexpr int kOrderThreads = 1024, kBuckets = 256;
-__global__ void __launch_bounds__(kOrderThreads) k_group_order(const int* __restrict__ count, int* __restrict__ order,
+__global__ void __launch_bounds__(kOrderThreads) k_group_order(const int* count, int* order,
                                                                int ngroups, int items) {
     __shared__ int most, bins[kBuckets], warp_sum[kBuckets / 32];
     __shared__ unsigned long long total;
