@@ -391,6 +391,13 @@ __global__ void __launch_bounds__(256) k_pairs(DevArrays a, DevParams p, int jt,
 // what it waits for. There the records of D = 4 neighbours are in flight (a rubble step with 16,384 particles 199 -> 194
 // us), and the fused pass goes to two warps, one for the velocity gradient (PART 1) and one for the acceleration (PART 2):
 // 208 -> 190 us for a step of the impact with 16,384 particles, 115 -> 98 with 4,000.
+// a record of the kernel before (common.cuh), loaded where it is written: left to the compiler, plain loads of the next
+// neighbours move down to their use (a rubble step with 5,000 particles 75.7 -> 81.3 us)
+__device__ __forceinline__ float4 load_here(const float4* p) {
+    float4 v;
+    asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
+    return v;
+}
 template <int PASS, bool SOLIDS, bool COMP, int D, int PART>
 __device__ __forceinline__ void pairs_near(const DevArrays& a, const DevParams& p, const NearView& v) {
     constexpr uint32_t ALL = field_mask<PASS, false, SOLIDS>(), FIRST = field_mask<PASS_VGRAD, false, SOLIDS>();
@@ -431,10 +438,10 @@ __device__ __forceinline__ void pairs_near(const DevArrays& a, const DevParams& 
         float4 rec[D][4];
         auto load = [&](int d) {
             const float4* r = a.jrec + 4 * static_cast<int64_t>(e[d] & ~kItemMark);
-            rec[d][0] = r[0];
-            rec[d][1] = r[1];
-            rec[d][2] = DO_A ? r[2] : zero;
-            rec[d][3] = DO_A ? r[3] : zero;
+            rec[d][0] = load_here(r);
+            rec[d][1] = load_here(r + 1);
+            rec[d][2] = DO_A ? load_here(r + 2) : zero;
+            rec[d][3] = DO_A ? load_here(r + 3) : zero;
         };
 #pragma unroll
         for (int d = 0; d < D; ++d) {
