@@ -383,7 +383,7 @@ __device__ __forceinline__ bool dens_item(const DevArrays& a, const DevParams& p
 // pairs. Every particle of a simulation with G groups has G + 1 slots, [slot][component][particle of the simulation]: its
 // row sums from tasks (g, gb) in slots 0 .. G-1-g, its column sums from tasks (ga, g) in slots G-g .. G, each
 // written by exactly one task (the diagonal one zeroes slot G); the SPH stage folds them in FP64 in slot order. Rows and
-// columns past the simulation's end are inert: massless, and so far away that 1/r^3 is zero where masses are left out.
+// columns past the simulation's end are inert: so far away that 1/r^3 is zero. A far task (gravity_sym.cuh) is summed apart.
 //
 // The one-sided sweep fused with the density test spent 12 FP32 operations per ordered pair and tested a third of all
 // pairs for neighbours; this one spends 14 per unordered pair, and the density pass finds its neighbours by boxes of 32
@@ -412,18 +412,29 @@ __global__ void __launch_bounds__(SymE::T, SymE::CTAS) k_ens_gravity(const float
     float* part = sim_slots(v, task.x);
     auto slot = [&](int local, int sl, int c) { return part + (static_cast<int64_t>(sl) * K + c) * N + local; };
     const int s_row = gb - ga, s_col = G - gb + ga;
+    bool far = sym_far_eps<GRAV>(eps2);
+#pragma unroll
+    for (int k = 0; k < R; ++k) {
+        if (tid + k * T < rn) far = sym_far(rp[tid + k * T]) || far;
+        if (tid + k * T < cn) far = sym_far(cp[tid + k * T]) || far;
+    }
+    if (__syncthreads_or(far)) {
+        sym_far_pass<SymE, GRAV, COMP>(rp, rn, cp, cn, eps2, XY, ZM, slot(ga * kEnsGroup, s_row, 0), N);
+        if (!diag) sym_far_pass<SymE, GRAV, COMP>(cp, cn, rp, rn, eps2, XY, ZM, slot(gb * kEnsGroup, s_col, 0), N);
+        else
+            for (int o = tid; o < cn; o += T)
+                for (int c = 0; c < K; ++c) *slot(gb * kEnsGroup + o, s_col, c) = 0.0f;
+        return;
+    }
     const float mr = rp[0].w, mc = cp[0].w;
     SymRows<SymE> rows;
-    bool same = true, far_r = sym_far_eps<GRAV>(eps2);
+    bool same = true;
 #pragma unroll
     for (int k = 0; k < R; ++k) {
         const int o = tid + k * T;
-        const float4 u = o < rn ? rp[o] : make_float4(-1e18f, -1e18f, -1e18f, 0.0f);
+        const float4 u = o < rn ? rp[o] : make_float4(-1e18f, -1e18f, -1e18f, mr);
         rows.set(k, u);
-        if (o < rn) {
-            same = same && u.w == mr;
-            far_r = far_r || sym_far(u);
-        }
+        same = same && u.w == mr;
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
             rsh[c * R + k][tid] = 0.0f;
@@ -433,33 +444,29 @@ __global__ void __launch_bounds__(SymE::T, SymE::CTAS) k_ens_gravity(const float
     if (diag)  // the group never is a column of its own diagonal task: that slot is zero
         for (int e = tid; e < cn; e += T)
             for (int c = 0; c < K; ++c) *slot(gb * kEnsGroup + e, s_col, c) = 0.0f;
-    const bool rows_equal = __syncthreads_and(same), rows_far = __syncthreads_or(far_r);
+    const bool rows_equal = __syncthreads_and(same);
     const float2 E2 = make_float2(eps2, eps2);
-    auto fetch = [&](int j) { return j < cn ? cp[j] : make_float4(1e18f, 1e18f, 1e18f, 0.0f); };
+    auto fetch = [&](int j) { return j < cn ? cp[j] : make_float4(1e18f, 1e18f, 1e18f, mc); };
     float4 pf[PF];
 #pragma unroll
     for (int h = 0; h < PF; ++h) pf[h] = fetch(tid + h * T);
     for (int j0 = 0; j0 < cn; j0 += JT) {
-        bool same_c = true, far_c = false;
+        __syncthreads();  // the previous tile's reads are done
+        bool same_c = true;
 #pragma unroll
-        for (int h = 0; h < PF; ++h)
-            if (j0 + tid + h * T < cn) {
-                same_c = same_c && pf[h].w == mc;
-                far_c = far_c || sym_far(pf[h]);
-            }
-        const bool far = __syncthreads_or(far_c) || rows_far;  // and the previous tile's reads are done
-#pragma unroll
-        for (int h = 0; h < PF; ++h) sym_stage(XY, ZM, tid + h * T, pf[h]);
-        const bool equal = __syncthreads_and(same_c) && rows_equal && !far;
+        for (int h = 0; h < PF; ++h) {
+            sym_stage(XY, ZM, tid + h * T, pf[h]);
+            same_c = same_c && pf[h].w == mc;
+        }
+        const bool equal = __syncthreads_and(same_c) && rows_equal;
         if (j0 + JT < cn) {
 #pragma unroll
             for (int h = 0; h < PF; ++h) pf[h] = fetch(j0 + JT + tid + h * T);
         }
         rows.clear();
-        if (diag) far ? sym_own<SymE, GRAV, true>(rows, XY, ZM, E2) : sym_own<SymE, GRAV, false>(rows, XY, ZM, E2);
-        else if (equal) sym_columns<SymE, GRAV, kSymEqual>(rows, XY, ZM, E2, js[warp]);
-        else if (!far) sym_columns<SymE, GRAV, kSymMasses>(rows, XY, ZM, E2, js[warp]);
-        else sym_columns<SymE, GRAV, kSymFar>(rows, XY, ZM, E2, js[warp]);
+        if (diag) sym_own<SymE, GRAV, false>(rows, XY, ZM, E2);
+        else if (equal) sym_columns<SymE, GRAV, true>(rows, XY, ZM, E2, js[warp]);
+        else sym_columns<SymE, GRAV, false>(rows, XY, ZM, E2, js[warp]);
         const float wr = !diag && equal ? mc : 1.0f;
         auto row_add = [&](int o, float2 t) {
             float x = rsh[o][tid];

@@ -3,6 +3,7 @@
 // ensemble's (ensemble.cu).
 #pragma once
 
+#include "common.cuh"
 #include "f32x2.cuh"
 
 namespace gsph {
@@ -53,21 +54,6 @@ __device__ __forceinline__ void sym_stage(float4* XY, float4* ZM, int j, float4 
     zm[half] = r.z; zm[2 + half] = r.w;
 }
 
-// How a pair's masses enter. kSymEqual: they do not (rows times the columns' mass, columns times minus the rows' are the
-// caller's). kSymMasses: they multiply 1/r^3, which one FP32 number holds for separations from 1.5e-13 to 4.3e12 only
-// (1/r^3 from 3e38 down to the smallest normal number). kSymFar: (m / r) (1 / r^2), two products more per pair, good for
-// as long as r^2 and the force are, for tiles that may reach farther (lengths in metres between stars) or, softened,
-// come nearer. A tile is far when a coordinate of its rows or columns reaches 2^40 (then, and only then, two of them can be
-// more than sqrt(3) 2^41 = 3.8e12 apart), or by its softening.
-enum SymMode { kSymEqual, kSymMasses, kSymFar };
-__device__ __forceinline__ bool sym_far(float4 q) {  // NaN counts as far
-    return !(fmaxf(fmaxf(fabsf(q.x), fabsf(q.y)), fabsf(q.z)) < 0x1p40f);
-}
-template <int GRAV>
-__device__ __forceinline__ bool sym_far_eps(float eps2) {  // 1/eps^3 above 1e38, or a larger reach
-    return GRAV == 1 && !(eps2 >= 5e-26f && eps2 <= 4e24f);
-}
-
 // the separations of row m from a column pair, and 1/r
 template <typename S, int GRAV>
 __device__ __forceinline__ float2 sym_pair(const SymRows<S>& r, int m, float4 xy, float4 zm, float2 E2, float2& dx, float2& dy,
@@ -82,8 +68,9 @@ __device__ __forceinline__ float2 sym_pair(const SymRows<S>& r, int m, float4 xy
 }
 __device__ __forceinline__ float2 cube2(float2 v) { return mul2(mul2(v, v), v); }
 
-// the rows against every column pair of the tile: row sums into r, the warp's column sums into js[component][column]
-template <typename S, int GRAV, SymMode MODE>
+// the rows against every column pair of the tile: row sums into r, the warp's column sums into js[component][column].
+// EQ: neither carries the masses (rows times the columns' mass, columns times minus the rows' are the caller's).
+template <typename S, int GRAV, bool EQ>
 __device__ __forceinline__ void sym_columns(SymRows<S>& rows, const float4* XY, const float4* ZM, float2 E2,
                                             float (*js)[S::JT]) {
     const int lane = threadIdx.x & 31, next = (lane + 1) & 31;
@@ -97,13 +84,11 @@ __device__ __forceinline__ void sym_columns(SymRows<S>& rows, const float4* XY, 
 #pragma unroll
             for (int m = 0; m < S::R; ++m) {
                 float2 dx, dy, dz;
-                const float2 inv = sym_pair<S, GRAV>(rows, m, xy, zm, E2, dx, dy, dz);
-                if (MODE == kSymEqual) {
-                    add_both(rows.TX[m], rows.TY[m], rows.TZ[m], cx, cy, cz, dx, dy, dz, cube2(inv));
+                const float2 i3 = cube2(sym_pair<S, GRAV>(rows, m, xy, zm, E2, dx, dy, dz));
+                if (EQ) {
+                    add_both(rows.TX[m], rows.TY[m], rows.TZ[m], cx, cy, cz, dx, dy, dz, i3);
                 } else {
-                    const float2 mj = make_float2(zm.z, zm.w), f = MODE == kSymFar ? mul2(inv, inv) : cube2(inv);
-                    const float2 sj = mul2(MODE == kSymFar ? mul2(mj, inv) : mj, f);
-                    const float2 si = mul2(MODE == kSymFar ? mul2(rows.M[m], inv) : rows.M[m], f);
+                    const float2 sj = mul2(make_float2(zm.z, zm.w), i3), si = mul2(rows.M[m], i3);
                     rows.TX[m] = fma2(dx, sj, rows.TX[m]);
                     rows.TY[m] = fma2(dy, sj, rows.TY[m]);
                     rows.TZ[m] = fma2(dz, sj, rows.TZ[m]);
@@ -121,7 +106,7 @@ __device__ __forceinline__ void sym_columns(SymRows<S>& rows, const float4* XY, 
     }
 }
 
-// one-sided: the rows' sums over the tile's columns, masses included (a block against itself)
+// one-sided: the rows' sums over the tile's columns, masses included (a block against itself). FAR: see below
 template <typename S, int GRAV, bool FAR>
 __device__ __forceinline__ void sym_own(SymRows<S>& rows, const float4* XY, const float4* ZM, float2 E2) {
 #pragma unroll 2
@@ -137,6 +122,73 @@ __device__ __forceinline__ void sym_own(SymRows<S>& rows, const float4* XY, cons
             rows.TZ[m] = fma2(dz, sj, rows.TZ[m]);
         }
     }
+}
+
+// ---- tasks that 1/r^3 does not suit ----------------------------------------------------------------
+// The sums above form 1/r^3 before a mass enters. One FP32 number holds it for separations from 1.5e-13 to 4.3e12 (from 3e38
+// down to the smallest normal number), not between stars in metres or atoms in metres. A task is far when a coordinate of its
+// particles reaches 2^40 (below, no two of them are more than sqrt(3) 2^41 = 3.8e12 apart), or by its softening. Its
+// sums are one-sided, (m / r) (1 / r^2) as in the one-sided kernels, and hold as long as r^2 and the force do.
+//
+// It is looked up once, before the sweep, beside the loads of the rows: a test per tile, in the barriers that are there,
+// with the far products beside the others in the loop, cost the ordinary sweep 12 % (9,000 particles, compensated, 43.2 ->
+// 48.7 us a step; now 45.2). What is left is the registers' allocation, which every such change shuffles: 9,000 plain
+// 45.1 -> 43.1 us, 45,000 plain 562.7 -> 565.7, 45,000 unequal masses 618.6 -> 629.6, 80,000 compensated 1,772 -> 1,727.
+__device__ __forceinline__ bool sym_far(float4 q) {  // NaN counts as far
+    return !(fmaxf(fmaxf(fabsf(q.x), fabsf(q.y)), fabsf(q.z)) < 0x1p40f);
+}
+template <int GRAV>
+__device__ __forceinline__ bool sym_far_eps(float eps2) {  // 1/eps^3 above 1e38, or a larger reach
+    return GRAV == 1 && !(eps2 >= 5e-26f && eps2 <= 4e24f);
+}
+// the sums of nr <= B rows over nc columns: component c of row o in out[c * stride + o], compensated the rounding errors in
+// the three components behind
+template <typename S, int GRAV, bool COMP>
+__device__ __forceinline__ void sym_far_pass(const float4* row, int nr, const float4* col, int nc, float eps2, float4* XY, float4* ZM,
+                                          float* out, int64_t stride) {
+    const float4 none = make_float4(1e18f, 1e18f, 1e18f, 0.0f);
+    SymRows<S> rows;
+    float s[3][S::R], e[3][S::R];
+#pragma unroll
+    for (int k = 0; k < S::R; ++k) {
+        const int o = threadIdx.x + k * S::T;
+        rows.set(k, o < nr ? row[o] : none);
+        for (int c = 0; c < 3; ++c) s[c][k] = e[c][k] = 0.0f;
+    }
+    for (int j0 = 0; j0 < nc; j0 += S::JT) {
+        __syncthreads();  // the previous tile's reads are done
+#pragma unroll
+        for (int h = 0; h < S::PF; ++h) {
+            const int j = threadIdx.x + h * S::T;
+            sym_stage(XY, ZM, j, j0 + j < nc ? col[j0 + j] : none);
+        }
+        __syncthreads();
+        rows.clear();
+        sym_own<S, GRAV, true>(rows, XY, ZM, make_float2(eps2, eps2));
+#pragma unroll
+        for (int k = 0; k < S::R; ++k) {
+            const float t[3] = {rows.TX[k].x + rows.TX[k].y, rows.TY[k].x + rows.TY[k].y, rows.TZ[k].x + rows.TZ[k].y};
+            for (int c = 0; c < 3; ++c) {
+                if (COMP) fold(s[c][k], e[c][k], t[c]);
+                else s[c][k] += t[c];
+            }
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < S::R; ++k) {
+        const int o = threadIdx.x + k * S::T;
+        if (o >= nr) break;
+        for (int c = 0; c < 3; ++c) {
+            out[c * stride + o] = s[c][k];
+            if (COMP) out[(3 + c) * stride + o] = e[c][k];
+        }
+    }
+}
+// the same out of line, for the shape of eight rows per thread (inlined there, N = 2^20 took 282 ms instead of 277)
+template <typename S, int GRAV, bool COMP>
+__device__ __noinline__ void sym_far_call(const float4* row, int nr, const float4* col, int nc, float eps2, float4* XY, float4* ZM,
+                                          float* out, int64_t stride) {
+    sym_far_pass<S, GRAV, COMP>(row, nr, col, nc, eps2, XY, ZM, out, stride);
 }
 
 }  // namespace gsph

@@ -786,6 +786,30 @@ __global__ void __launch_bounds__(S::T, S::CTAS) k_gravity_sym(const float4* __r
     // slots 0 .. G-1-g and its column sums from tasks (ga, g), ga = 0 .. g, in slots G-g .. G
     const int s_row = gb - ga, s_col = G - gb + ga;
     auto slot = [&](int64_t particle, int sl, int c) { return part + (static_cast<int64_t>(sl) * K + c) * n_pad + particle; };
+    bool far = sym_far_eps<GRAV>(eps2);
+    auto look = [&](int b0, int b1) {  // the padding lies far out too, but has no mass
+#pragma unroll 4
+        for (int64_t i = static_cast<int64_t>(b0) * B + tid; i < min(n, static_cast<int64_t>(b1) * B); i += T)
+            far = sym_far(posm[i]) || far;
+    };
+    look(ra0, ra1);
+    if (!diag) look(cg0, cg1);
+    if (__syncthreads_or(far)) {
+        auto pass = [&](int r0, int r1, int b0, int b1, int sl) {
+            for (int a = r0; a < r1; ++a) {
+                const float4 *row = posm + static_cast<int64_t>(a) * B, *col = posm + static_cast<int64_t>(b0) * B;
+                float* out = slot(static_cast<int64_t>(a) * B, sl, 0);
+                if constexpr (R == 8) sym_far_call<S, GRAV, COMP>(row, B, col, (b1 - b0) * B, eps2, XY, ZM, out, n_pad);
+                else sym_far_pass<S, GRAV, COMP>(row, B, col, (b1 - b0) * B, eps2, XY, ZM, out, n_pad);
+            }
+        };
+        pass(ra0, ra1, cg0, cg1, s_row);
+        if (!diag) pass(cg0, cg1, ra0, ra1, s_col);
+        else
+            for (int e = tid; e < (ra1 - ra0) * B; e += T)
+                for (int c = 0; c < K; ++c) *slot(static_cast<int64_t>(ra0) * B + e, s_col, c) = 0.0f;
+        return;
+    }
     if (diag)  // the group's first block is never a column here: its column slot is zero
         for (int e = tid; e < B; e += T)
             for (int c = 0; c < K; ++c) *slot(static_cast<int64_t>(ra0) * B + e, s_col, c) = 0.0f;
@@ -795,20 +819,19 @@ __global__ void __launch_bounds__(S::T, S::CTAS) k_gravity_sym(const float4* __r
         const int64_t base = static_cast<int64_t>(a) * B + tid;
         SymRows<S> rows;
         const float mr = posm[static_cast<int64_t>(a) * B].w;
-        bool same = true, far_r = sym_far_eps<GRAV>(eps2);
+        bool same = true;
 #pragma unroll
         for (int k = 0; k < R; ++k) {
             const float4 u = posm[base + static_cast<int64_t>(k) * T];
             rows.set(k, u);
             same = same && u.w == mr;
-            far_r = far_r || (base + static_cast<int64_t>(k) * T < n && sym_far(u));  // padding lies far, without mass
 #pragma unroll
             for (int c = 0; c < 3; ++c) {
                 rsh[c * R + k][tid] = 0.0f;
                 if (COMP) csh[COMP ? c * R + k : 0][tid] = 0.0f;
             }
         }
-        const bool rows_equal = __syncthreads_and(same), rows_far = __syncthreads_or(far_r);
+        const bool rows_equal = __syncthreads_and(same);
         // tiles: the block's own (one-sided) when diagonal, then the columns
         const int64_t d0 = static_cast<int64_t>(a) * B;
         const int nd = diag ? B / JT : 0;
@@ -825,10 +848,7 @@ __global__ void __launch_bounds__(S::T, S::CTAS) k_gravity_sym(const float4* __r
             for (int h = 0; h < PF; ++h) pf[h] = posm[src(0) + h * T + tid];
         }
         for (int k = 0; k < total; ++k) {
-            bool far_c = false;
-#pragma unroll
-            for (int h = 0; h < PF; ++h) far_c = far_c || (src(k) + h * T + tid < n && sym_far(pf[h]));
-            const bool far = __syncthreads_or(far_c) || rows_far;  // and the previous tile's reads of XY, ZM and js are done
+            __syncthreads();  // the previous tile's reads of XY, ZM and js are done
             const float mc = mn;
             bool same_c = true;
 #pragma unroll
@@ -836,17 +856,16 @@ __global__ void __launch_bounds__(S::T, S::CTAS) k_gravity_sym(const float4* __r
                 sym_stage(XY, ZM, tid + h * T, pf[h]);
                 same_c = same_c && pf[h].w == mc;
             }
-            const bool equal = __syncthreads_and(same_c) && rows_equal && !far;
+            const bool equal = __syncthreads_and(same_c) && rows_equal;
             if (k + 1 < total) {
                 mn = posm[src(k + 1)].w;
 #pragma unroll
                 for (int h = 0; h < PF; ++h) pf[h] = posm[src(k + 1) + h * T + tid];
             }
             rows.clear();
-            if (k < nd) far ? sym_own<S, GRAV, true>(rows, XY, ZM, E2) : sym_own<S, GRAV, false>(rows, XY, ZM, E2);
-            else if (equal) sym_columns<S, GRAV, kSymEqual>(rows, XY, ZM, E2, js[warp]);
-            else if (!far) sym_columns<S, GRAV, kSymMasses>(rows, XY, ZM, E2, js[warp]);
-            else sym_columns<S, GRAV, kSymFar>(rows, XY, ZM, E2, js[warp]);
+            if (k < nd) sym_own<S, GRAV, false>(rows, XY, ZM, E2);
+            else if (equal) sym_columns<S, GRAV, true>(rows, XY, ZM, E2, js[warp]);
+            else sym_columns<S, GRAV, false>(rows, XY, ZM, E2, js[warp]);
             // the tile's row partials into the running sums: a two-sum fold (compensated), or one add (plain: a sum
             // of tile sums, not one running sum over the whole column group)
             const float wr = k >= nd && equal ? mc : 1.0f;
