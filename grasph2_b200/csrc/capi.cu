@@ -382,6 +382,15 @@ int gsph_ctx_proposal_derivatives(gsph_ctx* c, void* stream) {
     return derivatives(c, as_stream(stream), true);
 }
 
+// whether a network proposal's derivatives are, to the bit, those of a step: the same gravity kernel in the same shape
+bool gsph_ctx_proposal_as_step(const gsph_ctx* c) {
+    if (!has(c->dp, GSPH_SELF_GRAVITY) || !has(c->dp, GSPH_SPH) || !c->L.cull) return true;
+    const Launch &a = c->L, &b = c->fixed_L;
+    if (a.grav_sym_G != b.grav_sym_G) return false;
+    if (a.grav_sym_G > 0) return c->fixed_order && a.grav_sym_gs == b.grav_sym_gs;
+    return a.grav_ipt == b.grav_ipt && a.grav_jt == b.grav_jt && a.grav_nseg == b.grav_nseg;
+}
+
 extern "C" {
 
 int gsph_params_reference_defaults(gsph_params* p) {

@@ -31,6 +31,7 @@
 
 void set_global_error(const std::string& msg);  // capi.cu
 int gsph_ctx_proposal_derivatives(gsph_ctx* c, void* stream);  // capi.cu
+bool gsph_ctx_proposal_as_step(const gsph_ctx* c);             // capi.cu
 int gsph_ctx_proposal_features(gsph_ctx* c, const float* mu, const float* sigma, float* feat, void* stream);  // capi.cu
 
 namespace {
@@ -235,18 +236,19 @@ int gsph_surrogate_judge(gsph_surrogate* s, gsph_ctx* ctx, int32_t use_net, doub
         if (rc != GSPH_OK) return ctx_fail(s, ctx, rc, "judge: energy");
         e_ref = d.e_kin + d.e_grav + d.e_int + d.e_shear;
     }
-    // Without the network, the start state is saved with its derivatives, which the proposal and the plain
-    // integrator's first step share: the plain path is one integrate and K - 1 full steps (the same arithmetic as K
-    // steps). A network proposal evaluates its own, in its fixed order of summation.
-    if (!use_net && (rc = gsph_compute_derivatives(ctx, stream)) != GSPH_OK) return ctx_fail(s, ctx, rc, "judge: derivatives");
-    if ((rc = gsph_snapshot(ctx, 1, 0, stream)) != GSPH_OK) return ctx_fail(s, ctx, rc, "judge: snapshot");
-    if (use_net && (rc = gsph_ctx_proposal_derivatives(ctx, stream)) != GSPH_OK)
-        return ctx_fail(s, ctx, rc, "judge: derivatives");
+    // The start state is saved with the proposal's derivatives, which the plain integrator's first step shares: the
+    // plain path is one integrate and K - 1 full steps (the same arithmetic as K steps). Where a network proposal sums
+    // its gravity in another order than the steps do (gravity_fixed.cu), the plain path is K steps of its own.
+    const bool shared = !use_net || gsph_ctx_proposal_as_step(ctx);
+    if (!shared && (rc = gsph_snapshot(ctx, 1, 0, stream)) != GSPH_OK) return ctx_fail(s, ctx, rc, "judge: snapshot");
+    rc = use_net ? gsph_ctx_proposal_derivatives(ctx, stream) : gsph_compute_derivatives(ctx, stream);
+    if (rc != GSPH_OK) return ctx_fail(s, ctx, rc, "judge: derivatives");
+    if (shared && (rc = gsph_snapshot(ctx, 1, 0, stream)) != GSPH_OK) return ctx_fail(s, ctx, rc, "judge: snapshot");
     if ((rc = propose_from_derivatives(s, ctx, use_net, stream)) != GSPH_OK) return rc;
     if ((rc = gsph_snapshot(ctx, 2, 0, stream)) != GSPH_OK) return ctx_fail(s, ctx, rc, "judge: snapshot");
     if ((rc = gsph_snapshot(ctx, 1, 1, stream)) != GSPH_OK) return ctx_fail(s, ctx, rc, "judge: restore");
-    if (!use_net && (rc = gsph_integrate(ctx, 1, stream)) != GSPH_OK) return ctx_fail(s, ctx, rc, "judge: plain steps");
-    if ((rc = gsph_step(ctx, use_net ? s->K : s->K - 1, stream)) != GSPH_OK)
+    if (shared && (rc = gsph_integrate(ctx, 1, stream)) != GSPH_OK) return ctx_fail(s, ctx, rc, "judge: plain steps");
+    if ((rc = gsph_step(ctx, shared ? s->K - 1 : s->K, stream)) != GSPH_OK)
         return ctx_fail(s, ctx, rc, "judge: plain steps");
     double c[8];
     if ((rc = gsph_state_compare_parts(ctx, 2, 1, c, stream)) != GSPH_OK) return ctx_fail(s, ctx, rc, "judge: compare");
