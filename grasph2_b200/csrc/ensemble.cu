@@ -1500,7 +1500,9 @@ int gsph_ensemble_autotune(gsph_ensemble* e, int32_t reps, int32_t* tile, int32_
     float best = 1e30f;
     int bt = e->tile, bp = e->per_sm_cap;
     int rc = GSPH_OK;
-    for (int t : {256, 512, 1024}) {
+    // the tile is the sweep's; the box search has none, and keeps the value as it is
+    const std::vector<int> tiles = e->near ? std::vector<int>{e->tile} : std::vector<int>{256, 512, 1024};
+    for (int t : tiles) {
         for (int cap : {0, 2, 3, 4}) {
             e->tile = t;
             e->per_sm_cap = cap;
