@@ -1,17 +1,21 @@
-// gravity_fixed.cu -- symmetric gravity in a fixed order of summation.
+// gravity_fixed.cu -- symmetric gravity in a kept order of summation.
 //
-// Two kinds of derivatives amplify a last-place change of the acceleration far beyond rounding, so they keep the kernel
-// (and the launch shapes that set the order of its sums) that they have always had:
+// Two kinds of derivatives amplify a last-place change of the acceleration far beyond rounding. They keep this kernel, and
+// the launch shapes that set the order of its sums as a context is made (autotuning may choose others):
 //   * network proposals (surrogate_run.cu). The network takes its inputs and keeps its activations in BF16; a change
 //     in the last place moves one of them across a rounding boundary every few thousand particles, and one such flip
-//     moves a particle's proposed stress by up to 5 % of the stress rms. It is the network's own rounding noise, but
-//     another proposal than the one a trained model was judged and shipped with;
+//     moves a particle's proposed stress by up to 5 % of the stress rms, in the proposal after the one whose acceleration
+//     changed. It is the network's own rounding noise, and the error against 64 bits is the same in either order: what is kept
+//     is that a context made today proposes what it did when the model was judged;
 //   * contexts that integrate the density (GSPH_INTEGRATE_DENSITY). The pressure, and with it the Mohr-Coulomb yield
 //     stress, comes from the distance of an FP32 density from rest: in the first steps one last place of the density is
 //     0.6 % of it.
-// Everything else takes the column-packed kernel of pairs.cu, 1.2 (equal masses: 1.4) times as fast; the results differ
-// in the last places only.
+// Everything else takes the column-packed kernel of pairs.cu, 1.2 (equal masses: 1.4) times as fast: that is the price,
+// 6.5 of the 22.4 ms of a proposal with 262,144 particles. The results differ in the last places only.
+// Both masses multiply 1/r^3 here, so separations must be within 1.5e-13 .. 4.3e12 (gravity_sym.cuh; the far tasks of that
+// kernel, in this one, cost every proposal 4.5 %).
 #include "f32x2.cuh"
+#include "gravity_sym.cuh"
 #include "pairs.cuh"
 
 namespace gsph {
@@ -28,21 +32,6 @@ constexpr int kFixT = 128, kFixI = 8, kFixB = kFixT * kFixI, kFixJT = 256;
 static_assert(kFixB % kFixJT == 0 && kFixJT % kFixT == 0 && kFixJT % 32 == 0, "symmetric gravity tiles");
 constexpr int kFixCtas = 4;
 
-__host__ __device__ __forceinline__ void fixed_sym_task(int t, int G, int& ga, int& gb) {
-    const int noff = G * (G - 1) / 2;
-    if (t >= noff) {
-        ga = gb = t - noff;
-        return;
-    }
-    int r = 0, rem = t;
-    while (rem >= G - 1 - r) {
-        rem -= G - 1 - r;
-        ++r;
-    }
-    ga = r;
-    gb = r + 1 + rem;
-}
-
 template <int GRAV, bool COMP>
 __global__ void __launch_bounds__(kFixT, kFixCtas) k_fixed_gravity_sym(const float4* __restrict__ posm, float* __restrict__ part,
                                                        int64_t n_pad, int G, int gs, float eps2) {
@@ -56,7 +45,7 @@ __global__ void __launch_bounds__(kFixT, kFixCtas) k_fixed_gravity_sym(const flo
     __shared__ float2 csh[COMP ? 3 * P : 1][kFixT];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     int ga, gb;
-    fixed_sym_task(static_cast<int>(blockIdx.x), G, ga, gb);
+    sym_task(static_cast<int>(blockIdx.x), G, ga, gb);
     const int nb = static_cast<int>(n_pad / kFixB);
     const int ra0 = ga * gs, ra1 = min(nb, ra0 + gs);
     const int cg0 = gb * gs, cg1 = min(nb, cg0 + gs);

@@ -1,6 +1,6 @@
 // gravity_sym.cuh -- the inner parts of symmetric gravity: a block of rows in registers against a tile of columns in
 // shared memory, every unordered pair once. Used by the all-pairs kernel (pairs.cu, which explains the layout) and the
-// ensemble's (ensemble.cu).
+// ensemble's (ensemble.cu); gravity_fixed.cu shares its tasks.
 #pragma once
 
 #include "common.cuh"
@@ -16,6 +16,22 @@ struct SymShape {
     static constexpr int W = T_ / 32;
     static_assert(JT % 64 == 0 && B % JT == 0 && JT % T_ == 0, "symmetric gravity tiles");
 };
+
+// the groups ga <= gb of task t: the G (G - 1) / 2 pairs of distinct groups first, then the G diagonal ones
+__host__ __device__ __forceinline__ void sym_task(int t, int G, int& ga, int& gb) {
+    const int noff = G * (G - 1) / 2;
+    if (t >= noff) {
+        ga = gb = t - noff;
+        return;
+    }
+    int r = 0, rem = t;
+    while (rem >= G - 1 - r) {
+        rem -= G - 1 - r;
+        ++r;
+    }
+    ga = r;
+    gb = r + 1 + rem;
+}
 
 // T += d s, c += d s for the three components: each pair of multiply-adds with common factors back to back
 __device__ __forceinline__ void add_both(float2& tx, float2& ty, float2& tz, float2& cx, float2& cy, float2& cz, float2 dx,

@@ -751,21 +751,6 @@ __global__ void __launch_bounds__(128) k_gravity_x2(const float4* __restrict__ p
 // 0.60 of the FMA rate, multiplies and adds (four) at 0.96; six of a pair's operations are such multiply-adds, which
 // predicts 0.77. Keeping each pair that shares both factors together lets the operand cache serve the second: 0.81.
 // Measured (N = 262,144, 128 groups, one B200): row-packed 22.3 ms, column-packed 18.6 ms, equal masses 15.8 ms.
-__host__ __device__ __forceinline__ void sym_task(int t, int G, int& ga, int& gb) {
-    const int noff = G * (G - 1) / 2;
-    if (t >= noff) {
-        ga = gb = t - noff;
-        return;
-    }
-    int r = 0, rem = t;
-    while (rem >= G - 1 - r) {
-        rem -= G - 1 - r;
-        ++r;
-    }
-    ga = r;
-    gb = r + 1 + rem;
-}
-
 template <typename S, int GRAV, bool COMP>
 __global__ void __launch_bounds__(S::T, S::CTAS) k_gravity_sym(const float4* __restrict__ posm, float* __restrict__ part,
                                                                int64_t n, int64_t n_pad, int G, int gs, float eps2) {

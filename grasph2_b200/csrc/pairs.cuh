@@ -24,11 +24,8 @@ struct JTilePipe {
     uint64_t* bar;        // shared: [2]
     const float4* src[NS];
     int jt;
-    int64_t t_begin, t_end;  // tiles t_begin .. t_end-1, or positions of `list` when it is set
-    const int* list = nullptr;
+    int64_t t_begin, t_end;  // tiles t_begin .. t_end-1
     int* status;
-
-    __device__ __forceinline__ int64_t tile_at(int64_t k) const { return list ? list[k] : k; }
 
     __device__ __forceinline__ void issue(int b, int64_t t) {
         mbar_expect_tx(&bar[b], static_cast<uint32_t>(NS * jt * sizeof(float4)));
@@ -47,8 +44,8 @@ struct JTilePipe {
         }
         __syncthreads();
         if (threadIdx.x == 0) {
-            if (t_begin < t_end) issue(0, tile_at(t_begin));
-            if (t_begin + 1 < t_end) issue(1, tile_at(t_begin + 1));
+            if (t_begin < t_end) issue(0, t_begin);
+            if (t_begin + 1 < t_end) issue(1, t_begin + 1);
         }
     }
 
@@ -66,7 +63,7 @@ struct JTilePipe {
             const float4* stage = buf + static_cast<int64_t>(b) * NS * jt;
             body(stage);
             __syncthreads();
-            if (threadIdx.x == 0 && t + 2 < t_end) issue(b, tile_at(t + 2));
+            if (threadIdx.x == 0 && t + 2 < t_end) issue(b, t + 2);
         }
     }
 
@@ -90,14 +87,15 @@ struct JTilePipe {
 // them, one warp per 32 particles. No partial sums.
 //
 // Order of summation: the near chunks of a group form items of `per_item` chunks, an item's chunks form stages of
-// kStageChunks. A particle's density is the sum over items of the sum over stages of the sum over neighbours; its SPH
-// sums are the sum over items of the sum over neighbours (compensated: stages by two-sum, items in FP64). It follows from
-// the near chunks alone, not from the launch.
+// kStageChunks. A particle's density is the sum over items of the sum over stages of the sum over neighbours (compensated:
+// stages by two-sum, items in FP64); its SPH sums are the sum over items of the sum over neighbours (compensated: items in
+// FP64, an item's neighbours in FP32 as in the plain form; in large contexts, from about 570,000 particles, an item can hold
+// all of a group's near chunks, and the two forms are then one). It follows from the near chunks alone, not from the launch.
 constexpr int kStageChunks = 4;
 constexpr int kSub = 32;                 // particles per warp and per box
 constexpr int kSubs = kGroup / kSub;
 constexpr int kHalves = kChunk / kSub;   // boxes per chunk
-constexpr int kItemsPerSM = 30;          // items aimed at in all
+constexpr int kItemsPerSM = 30;          // items aimed at in all (only the order of the SPH sums)
 
 struct NearView {
     const int* list;     // near chunks of each i-group, row stride nchunks
@@ -241,8 +239,7 @@ cudaError_t timer_record(cudaEvent_t ev, cudaStream_t s);
 
 // host launchers (pairs.cu)
 // How the finish kernels read a particle's gravity partials: segments 0 .. nseg-1 of the one-sided
-// kernel ([segment][component][particle]), or (sym_G > 0) the symmetric kernel's G + 1 slots of the
-// particle ([particle][slot][component]).
+// kernel, or (sym_G > 0) the symmetric kernel's G + 1 slots, both [slot][component][particle].
 struct GravSum {
     int nseg = 0;
     int sym_G = 0;

@@ -90,8 +90,8 @@ __global__ void __launch_bounds__(128) k_chunk_lists(const float4* lo, const flo
 }
 
 // The groups by falling near-chunk count (to a 256th of the largest), so that the warps of long lists start first and
-// the short ones fill the last wave, and the chunks per item ceil(total near chunks / items). One block: counting
-// sort. The order within a bucket is not fixed, and need not be: every group's results are its own.
+// the short ones fill the last wave, and the chunks per item ceil(total near chunks / items), which sets the order of
+// the SPH sums (pairs.cuh) and nothing else. One block: counting sort. The order within a bucket is not fixed, and need not be: every group's results are its own.
 constexpr int kOrderThreads = 1024, kBuckets = 256;
 __global__ void __launch_bounds__(kOrderThreads) k_group_order(const int* count, int* order,
                                                                int ngroups, int items) {

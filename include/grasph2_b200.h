@@ -154,7 +154,10 @@ typedef struct gsph_host_particles {
  * ------------------------------------------------------------------------------------------- */
 #define GSPH_ACCUM_PLAIN       0  /* FP32 accumulation throughout the pair sums */
 #define GSPH_ACCUM_COMPENSATED 1  /* FP32 within a j-tile, two-sum (Kahan-Babuska) fold of each
-                                     tile's partial into the running sum, FP64 combine of j-splits */
+                                     tile's partial into the running sum, FP64 combine of j-splits. The SPH
+                                     rates of culled contexts: FP32 within a run of near chunks (a few chunks
+                                     in small contexts, up to all neighbours of a particle from about 570,000
+                                     particles on), FP64 over the runs; their density folds every four chunks */
 
 typedef struct gsph_options {
     int32_t accum;           /* GSPH_ACCUM_* */
@@ -172,18 +175,24 @@ typedef struct gsph_options {
                                 (identical results; for comparison) */
     int32_t precision;       /* GSPH_PRECISION_SINGLE (default) or GSPH_PRECISION_DOUBLE: the reference's
                                 SINGLE_PRECISION / DOUBLE_PRECISION switch (settings/precisionSettings.h:16-17).
-                                Double runs every pass in FP64 with plain all-pairs tiles (no culling,
-                                accum ignored); gsph_upload_f64 / gsph_download_f64 pass values unrounded */
+                                Double runs every pass in FP64 (accum ignored), up to 4 M particles with
+                                symmetric gravity and culled SPH passes as in single precision, above them,
+                                with no_cull or with ONE_SIDED gravity by sweeps over all pairs; gsph_upload_f64 / gsph_download_f64 pass values unrounded */
     int32_t gravity_form;    /* GSPH_GRAVITY_AUTO (default), GSPH_GRAVITY_ONE_SIDED or GSPH_GRAVITY_SYMMETRIC: the
                                 all-pairs gravity kernel evaluates every ordered pair (i gathers from all j), or
                                 every unordered pair once and applies it to both particles (Newton's third law;
                                 14 to 16 FP32 operations for both against 24, partials of up to 129 x 3 floats per
                                 particle). Auto is the symmetric form, unless scalar_fp32 or, below 24 blocks of 1024
                                 particles, a shape of the one-sided kernel is asked for, and from 2,049 particles on
-                                (plain sums: 3,073). Results agree to rounding. Ensembles take the symmetric form
-                                too (AUTO: while its partials take at most 1 KB per particle); ONE_SIDED gives them
-                                the sweep fused with the density pass */
-    int32_t gravity_groups;  /* symmetric form: particle groups G at most (tasks G(G+1)/2); 0 = up to 128 */
+                                (plain sums: 3,073). Contexts that integrate the density (GSPH_INTEGRATE_DENSITY, with
+                                culling) keep one order of summation: auto is one-sided there below 24 blocks, and the
+                                symmetric form takes up to 64 groups. Results agree to rounding as far as r^2 and
+                                m / r^3 are in FP32's range (the symmetric form of contexts that integrate the density
+                                and of network proposals: 1 / r^3, separations of 1.5e-13 to 4e12). Ensembles with SPH take the symmetric form too (AUTO: while
+                                its partials take at most 1 KB per particle); ONE_SIDED gives them the sweep fused
+                                with the density pass, the only form of ensembles without SPH */
+    int32_t gravity_groups;  /* symmetric form: particle groups G at most (tasks G(G+1)/2); 0 = up to 128 (64 where the
+                                order of summation is kept) */
     int32_t wait_limit_us;   /* batched ensemble: a work item that waits for another item's result (a device-side
                                 spin on a counter) gives up after this many microseconds, sets the timeout bit
                                 and its call returns GSPH_E_TIMEOUT (0 = 2 s). Waits for a bulk copy to land
