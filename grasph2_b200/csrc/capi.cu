@@ -966,7 +966,7 @@ int diagnostics(gsph_ctx* c, double half_kick, gsph_diag* out, void* stream, boo
     if (c->fp64) GSPH_CK(c, launch64_diagnostics(c->a64, c->dp64, half_kick, c->diag64, c->diag_out, s), "diagnostics");
     else if (fast) GSPH_CK(c, launch_diagnostics_fast(c->a, c->dp, half_kick, c->diag_out, s), "diagnostics");
     else GSPH_CK(c, launch_diagnostics(c->a, c->dp, half_kick, c->diag_out, s), "diagnostics");
-    c->launches += 2;
+    c->launches += (fast && !c->fp64) || !(c->params.flags & GSPH_SELF_GRAVITY) ? 2 : 3;  // the potential's own kernel
     double h[12];
     GSPH_CK(c, cudaMemcpyAsync(h, c->diag_out, sizeof h, cudaMemcpyDeviceToHost, s), "diagnostics read");
     const int rc = check_status(c, s);

@@ -1023,7 +1023,7 @@ struct gsph_ensemble {
     cudaStream_t capture_stream = nullptr;
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t graph_exec = nullptr;
-    int64_t launches = 0;
+    int64_t launches = 0, graph_kernels = 0;
     std::string err;
 };
 
@@ -1418,7 +1418,7 @@ int gsph_ensemble_step(gsph_ensemble* e, int32_t nsteps, void* stream) {
     if (nsteps < 0) return efail(e, GSPH_E_INVALID, "nsteps < 0");
     if (nsteps == 0) return GSPH_OK;
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-    if (!e->graph_exec) {  // one launch per substep: counter reset + all three stages, captured once
+    if (!e->graph_exec) {  // one graph per substep: counter reset, boxes, gravity, all three stages; captured once
         if (!e->capture_stream)
             ENS_CK(e, cudaStreamCreateWithFlags(&e->capture_stream, cudaStreamNonBlocking), "stream");
         int st[3];
@@ -1429,6 +1429,7 @@ int gsph_ensemble_step(gsph_ensemble* e, int32_t nsteps, void* stream) {
         const int rc = run_stages(e, st, ns, e->dp.fixed_dt, e->capture_stream);
         cudaGraph_t g = nullptr;
         const cudaError_t ee = cudaStreamEndCapture(e->capture_stream, &g);
+        e->graph_kernels = e->launches - before;
         e->launches = before;
         if (rc != GSPH_OK) {
             if (g) cudaGraphDestroy(g);
@@ -1450,7 +1451,7 @@ int gsph_ensemble_step(gsph_ensemble* e, int32_t nsteps, void* stream) {
             if (rc != GSPH_OK) return rc;
         }
         ENS_CK(e, cudaGraphLaunch(e->graph_exec, s), "graph launch");
-        e->launches += 1;
+        e->launches += e->graph_kernels;
         e->steps_since_sort += 1;
     }
     return GSPH_OK;
