@@ -47,6 +47,11 @@ FLOP_DENS_NB = 10          # W(r) and the accumulation per neighbour
 FLOP_FUSED_NB = 160        # strain/rotation rates, div v, stress acceleration, AV per neighbour (solids)
 FLOP_ACC_NB = 60           # pressure acceleration + AV per neighbour (fluid, acceleration pass only)
 
+# FP32 operations (an FMA is one) that a gravity form issues per ordered pair: the symmetric kernel 14 per unordered pair
+# of equal masses, 16 of others (the fixed order always), the one-sided one 12 per ordered pair. The roofline counts
+# these, two flops each, against the FFMA rate: the flop model above credits the symmetric form with work it does not do.
+GRAV_OPS = {"equal": 7, "symmetric": 8, "one-sided": 12}
+
 FLUSH_BYTES = 256 << 20
 
 # DRAM bytes (read + write) per launch of the dominant kernel, from one ncu capture of the same kernel
@@ -56,11 +61,11 @@ FLUSH_BYTES = 256 << 20
 # traffic is its j-records (16 B per particle, read once from DRAM, then from L2) plus its partial slots
 # ((G + 1) x 12 B per particle, written once), so at fixed G it scales with N.
 MEASURED_TRAFFIC = {
-    ("plummer", "gravity", "symmetric", 128): (356643200.0, 262144),  # ncu, N = 262,144, 2 launches (mean)
-    ("impact", "gravity", "symmetric", 64): (2185728.0, 65536),  # ncu, the impact itself, 2 launches (mean)
-    # the 512-simulation ensemble itself (4,630,521 particles, DENS j-tile 512), 2 launches (mean): the
-    # neighbour lists the DENS stage writes and the SPH stage reads dominate it
-    ("ensemble", "k_ensemble", "one-sided", 512): (5093712128.0, 4630521),
+    ("plummer", "gravity", "symmetric", 128): (357415936.0, 262144),  # ncu, N = 262,144
+    ("impact", "gravity", "symmetric", 64): (1354368.0, 65536),  # ncu, the impact itself, 2 launches (mean): slots in L2
+    # 96 spheres of the same size range (965694 particles): the packed records and neighbour lists that the SPH stage reads,
+    # and the gravity slots
+    ("ensemble", "k_ens_gravity + k_ensemble", "symmetric", 512): (2000312000.0, 965694),
 }
 FLAG_DEAL_WITH_NO_PARTNERS = 1 << 3  # GSPH_DEAL_WITH_NO_PARTNERS
 
@@ -149,6 +154,19 @@ def flops_per_step(params, st, counts, culled):
     elif grav:
         out["gravity"] = FLOP_GRAV_PAIR * n2
     return out
+
+
+def gravity_issued_flops(params, masses, n, sym_groups):
+    """Flops (two per FP32 operation) that the all-pairs gravity kernel issues in one step. Contexts that integrate the
+    density keep the kernel that multiplies both masses."""
+    from grasph2_b200._abi import FLAG_BITS as F
+    if not sym_groups:
+        ops = GRAV_OPS["one-sided"]
+    elif params.flags & F["INTEGRATE_DENSITY"] or np.ptp(masses) != 0:
+        ops = GRAV_OPS["symmetric"]
+    else:
+        ops = GRAV_OPS["equal"]
+    return 2.0 * ops * n * n
 
 
 def neighbour_pairs(pos, h, device):
@@ -693,7 +711,10 @@ def run_ensemble(args, rank, world, local):
         return None
     value = whole_job_rate(args.steps, world, total_ms)
     nb = sum(neighbour_pairs(s["pos"], params.H, dev) for s in states[::8]) * 8
-    flops = FLOP_GRAV_PAIR * pairs + FLOP_DENS_PAIR * pairs + (FLOP_DENS_NB + FLOP_ACC_NB) * nb
+    form = "one-sided" if args.gravity == "one-sided" else "symmetric"  # these sizes fit the pair form's slots
+    # the sweep tests every pair for neighbours beside its gravity; the box search does not
+    per_pair = 2 * GRAV_OPS["equal"] if form == "symmetric" else 2 * GRAV_OPS["one-sided"] + FLOP_DENS_PAIR
+    flops = per_pair * pairs + (FLOP_DENS_NB + FLOP_ACC_NB) * nb
     achieved = flops / (ms_per_step * 1e-3) / 1e12
     cpu = None
     if not args.no_cpu_baseline:
@@ -715,8 +736,8 @@ def run_ensemble(args, rank, world, local):
                          "diverge at the particle level in any precision, so their energy comparison is not a "
                          "precision measure",
                  "sample": "8 simulations spanning the size range, run as an ensemble (FP32) and one by one in FP64"}
-    form = "symmetric" if args.gravity == "symmetric" else "one-sided"
-    ens_traffic = MEASURED_TRAFFIC.get(("ensemble", "k_ensemble", form, len(sizes)))
+    kernel = "k_ens_gravity + k_ensemble" if form == "symmetric" else "k_ensemble"
+    ens_traffic = MEASURED_TRAFFIC.get(("ensemble", kernel, form, len(sizes)))
     if ens_traffic is not None:
         ens_traffic = ens_traffic[0] * n_total / ens_traffic[1]
     line = {
@@ -726,7 +747,7 @@ def run_ensemble(args, rank, world, local):
         "energy_drift": drift,
         "config": {"workload": desc, "nsims": int(len(sizes)), "n_total": n_total, "form": args.accum,
                    "l2": "flushed between timed steps (256 MiB write)",
-                   "step": "every simulation: computeDerivatives + integrate, one persistent launch in a CUDA graph",
+                   "step": "every simulation: computeDerivatives + integrate, one CUDA graph",
                    "launch_shape": dict(shape, autotuned=not args.no_autotune),
                    "parallelism": ("%d ensembles of %d simulations, one per GPU" % (world, len(sizes)))
                    if world > 1 else "single GPU"},
@@ -734,7 +755,7 @@ def run_ensemble(args, rank, world, local):
         "pair_interactions_per_s": pairs * value,
         "sequential_plain_ms_per_step": seq_ms,
         "speedup_vs_sequential": (seq_ms / ms_per_step) if seq_ms else None,
-        "roofline": {"bound": "fp32", "kernel": "k_ensemble", "achieved": achieved, "peak": peak_tflops,
+        "roofline": {"bound": "fp32", "kernel": kernel, "achieved": achieved, "peak": peak_tflops,
                      "unit": "TFLOP/s", "frac": (achieved / peak_tflops) if peak_tflops else None,
                      "traffic": ens_traffic, "flops_per_launch": flops, "neighbour_pairs": nb,
                      "peak_source": "FFMA throughput measured in this run (gsph_measure_fp32_peak)"},
@@ -1015,9 +1036,10 @@ def run_context(args, rank, world, local, dist=None):
     timed = {k: prof[k][0] / prof[k][1] for k in fl if prof[k][1]}
     dominant = max(timed, key=lambda k: timed[k]) if timed else max(fl, key=lambda k: fl[k])
     ms_dom, cnt_dom = prof[dominant]
-    achieved = fl[dominant] / (ms_dom / cnt_dom * 1e-3) / 1e12 if cnt_dom else None
-    pairs_per_step = flops_pairs(params, n)
     sym_g = int(shape.get("grav_sym_groups") or 0)
+    issued = gravity_issued_flops(params, st["mass"], n, sym_g) if dominant == "gravity" else fl[dominant]
+    achieved = issued / (ms_dom / cnt_dom * 1e-3) / 1e12 if cnt_dom else None
+    pairs_per_step = flops_pairs(params, n)
     traffic = MEASURED_TRAFFIC.get((args.workload, dominant, "symmetric" if sym_g else "one-sided", sym_g))
     if traffic is not None:
         traffic = traffic[0] * n / traffic[1]  # bytes per particle of the captured case x N
@@ -1048,8 +1070,8 @@ def run_context(args, rank, world, local, dist=None):
         "kernel_ms_per_step": {k: (v[0] / v[1] if v[1] else None) for k, v in prof.items()},
         "roofline": {"bound": "fp32", "kernel": dominant, "achieved": achieved, "peak": peak_tflops,
                      "unit": "TFLOP/s", "frac": (achieved / peak_tflops) if (achieved and peak_tflops) else None,
-                     "traffic": traffic, "algorithmic_bytes": 16 * n, "flops_per_launch": fl[dominant],
-                     "neighbour_pairs": nb,
+                     "traffic": traffic, "algorithmic_bytes": 16 * n, "flops_per_launch": issued,
+                     "model_flops_per_launch": fl[dominant], "neighbour_pairs": nb,
                      "peak_source": "FFMA throughput measured in this run (gsph_measure_fp32_peak)"},
         "integrator_roofline": integrator_roofline(prof, n, params),
         "cpu_baseline": cpu,
