@@ -340,7 +340,7 @@ class Ensemble:
         return [d.as_dict() for d in arr]
 
     def autotune(self, reps=2, stream=None):
-        """Time the DENS j-tile and the persistent grid's CTAs per SM; keep the fastest."""
+        """Time the persistent grid's CTAs per SM and, for the one-sided sweep, its DENS j-tile; keep the fastest."""
         t, c = ctypes.c_int32(), ctypes.c_int32()
         self._check(self.lib.gsph_ensemble_autotune(self._h, int(reps), ctypes.byref(t), ctypes.byref(c),
                                                     _stream_handle(stream)))

@@ -287,7 +287,7 @@ int gsph_diagnostics_fast(gsph_ctx* ctx, double half_kick, gsph_diag* out, void*
 
 /* Autotuner (no counterpart in the reference): times candidate launch shapes on the context's current
  * state and keeps the fastest, `reps` timed launches each (median): the gravity kernel's i-blocking,
- * j-tile and j-split; the all-pairs SPH tile shape (the culled SPH passes have one shape). Results
+ * j-tile and j-split, the symmetric form's blocks and groups (those of network proposals too); the all-pairs SPH tile shape (the culled SPH passes have one shape). Results
  * change only by summation order. The next gsph_step re-captures its graph. */
 int gsph_autotune(gsph_ctx* ctx, int32_t reps, void* stream);
 typedef struct gsph_launch_shape {
@@ -542,9 +542,9 @@ int gsph_ensemble_integrate(gsph_ensemble* e, int32_t not_first_step, void* stre
 int gsph_ensemble_step(gsph_ensemble* e, int32_t nsteps, void* stream);
 /* FP64 diagnostics of every simulation into out[nsims] (as gsph_diagnostics); synchronises `stream` */
 int gsph_ensemble_diagnostics(gsph_ensemble* e, double half_kick, gsph_diag* out, void* stream);
-/* Autotuner: times the DENS j-tile (256, 512, 1024) and the CTAs per SM of the persistent grid on the
- * current state (derivative launches only) and keeps the fastest; tile / per_sm (nullable) receive the
- * choice (per_sm 0: as many as fit). */
+/* Autotuner: times the CTAs per SM of the persistent grid and, for the one-sided sweep, its DENS j-tile
+ * (256, 512, 1024) on the current state (derivative launches only) and keeps the fastest; tile / per_sm
+ * (nullable) receive the choice (per_sm 0: as many as fit; the symmetric form has no tile: the value it was made with). */
 int gsph_ensemble_autotune(gsph_ensemble* e, int32_t reps, int32_t* tile, int32_t* per_sm, void* stream);
 int gsph_ensemble_launch_count(const gsph_ensemble* e, int64_t* count);
 /* text of the last failure on `e` (or of the last failed gsph_ensemble_create when e is NULL) */
