@@ -10,8 +10,8 @@
 //   * contexts that integrate the density (GSPH_INTEGRATE_DENSITY). The pressure, and with it the Mohr-Coulomb yield
 //     stress, comes from the distance of an FP32 density from rest: in the first steps one last place of the density is
 //     0.6 % of it.
-// Everything else takes the column-packed kernel of pairs.cu, 1.2 (equal masses: 1.4) times as fast: that is the price,
-// 6.5 of the 22.4 ms of a proposal with 262,144 particles. The results differ in the last places only.
+// Everything else takes the column-packed kernel of pairs.cu, 1.16 (equal masses: 1.28) times as fast: that is the price,
+// 5 of the 22.4 ms of a proposal with 262,144 particles. The results differ in the last places only.
 // Both masses multiply 1/r^3 here, so separations must be within 1.5e-13 .. 4.3e12 (gravity_sym.cuh; the far tasks of that
 // kernel, in this one, cost every proposal 4.5 %).
 #include "f32x2.cuh"
