@@ -140,16 +140,12 @@ __device__ __forceinline__ void sym_own(SymRows<S>& rows, const float4* XY, cons
     }
 }
 
-// ---- tasks that 1/r^3 does not suit ----------------------------------------------------------------
+// ---- separations that 1/r^3 does not suit -----------------------------------------------------------
 // The sums above form 1/r^3 before a mass enters. One FP32 number holds it for separations from 1.5e-13 to 4.3e12 (from 3e38
-// down to the smallest normal number), not between stars in metres or atoms in metres. A task is far when a coordinate of its
-// particles reaches 2^40 (below, no two of them are more than sqrt(3) 2^41 = 3.8e12 apart), or by its softening. Its
-// sums are one-sided, (m / r) (1 / r^2) as in the one-sided kernels, and hold as long as r^2 and the force do.
-//
-// It is looked up once, before the sweep, beside the loads of the rows: a test per tile, in the barriers that are there,
-// with the far products beside the others in the loop, cost the ordinary sweep 12 % (9,000 particles, compensated, 43.2 ->
-// 48.7 us a step; now 45.2). What is left is the registers' allocation, which every such change shuffles: 9,000 plain
-// 45.1 -> 43.1 us, 45,000 plain 562.7 -> 565.7, 45,000 unequal masses 618.6 -> 629.6, 80,000 compensated 1,772 -> 1,727.
+// down to the smallest normal number), not between stars in metres or atoms in metres. Particles are far when a coordinate of
+// theirs reaches 2^40 (below, no two of them are more than sqrt(3) 2^41 = 3.8e12 apart), or by their softening. Far sums are
+// one-sided, (m / r) (1 / r^2) as in the one-sided kernels, and hold as long as r^2 and the force do: in the ensemble a
+// task's, looked up once before its sweep, in a context all of them, in the fold (pairs.cu).
 __device__ __forceinline__ bool sym_far(float4 q) {  // NaN counts as far
     return !(fmaxf(fmaxf(fabsf(q.x), fabsf(q.y)), fabsf(q.z)) < 0x1p40f);
 }
@@ -199,12 +195,6 @@ __device__ __forceinline__ void sym_far_pass(const float4* row, int nr, const fl
             if (COMP) out[(3 + c) * stride + o] = e[c][k];
         }
     }
-}
-// the same out of line, for the shape of eight rows per thread (inlined there, N = 2^20 took 282 ms instead of 277)
-template <typename S, int GRAV, bool COMP>
-__device__ __noinline__ void sym_far_call(const float4* row, int nr, const float4* col, int nc, float eps2, float4* XY, float4* ZM,
-                                          float* out, int64_t stride) {
-    sym_far_pass<S, GRAV, COMP>(row, nr, col, nc, eps2, XY, ZM, out, stride);
 }
 
 }  // namespace gsph

@@ -541,9 +541,54 @@ __device__ __forceinline__ float fold_get(const typename FoldVec<V>::type& x, in
     if constexpr (V == 4) return e == 0 ? x.x : (e == 1 ? x.y : (e == 2 ? x.z : x.w));
     else return x;
 }
+// Where 1/r^3 does not suit the separations (gravity_sym.cuh), the slots of k_gravity_sym are of no use: a group of its
+// particles reaches far, or the softening is out of range. The fold then sums over all particles itself, (m / r) (1 / r^2) as
+// the one-sided kernels do, 256 at a time in FP32. Asking costs next to nothing (the groups' flags come with the slots, the
+// vote is in its barrier), and the sweep keeps its registers: with the far sums in the sweep's kernel, looked up per tile or
+// per task, its compensated form lost 1.5 to 3.5 us at 3,000 to 12,000 particles (9,000: 38.3 -> 40.1 us; now 38.3), unequal
+// masses 2 % (45,000: 626 -> 638 us; now 625).
+struct FarView {
+    const int* groups = nullptr;  // flags of the G groups of the sweep (G = 0: slots that hold any separation)
+    int G = 0;
+    const float4* posm = nullptr;
+    float eps2 = 0.0f;
+};
+template <int V>
+__device__ __forceinline__ void far_sums(const FarView& v, int64_t n, int64_t i, int q, double (&s)[V][3]) {
+    float x[V], y[V], z[V];
+#pragma unroll
+    for (int e = 0; e < V; ++e) {
+        const float4 p = v.posm[i + e < n ? i + e : n - 1];
+        x[e] = p.x; y[e] = p.y; z[e] = p.z;
+        s[e][0] = s[e][1] = s[e][2] = 0.0;
+    }
+    const float most = v.eps2 > 0.0f ? INFINITY : 1e12f;  // eps == 0: the self pair gives 0
+    const int64_t j1 = n * (q + 1) / kFoldT;
+    for (int64_t j0 = n * q / kFoldT; j0 < j1; j0 += 256) {
+        float t[V][3];
+#pragma unroll
+        for (int e = 0; e < V; ++e) t[e][0] = t[e][1] = t[e][2] = 0.0f;
+#pragma unroll 4
+        for (int64_t j = j0; j < min(j1, j0 + 256); ++j) {
+            const float4 p = v.posm[j];
+#pragma unroll
+            for (int e = 0; e < V; ++e) {
+                const float dx = p.x - x[e], dy = p.y - y[e], dz = p.z - z[e];
+                const float inv = fminf(rsqrtf(fmaf(dz, dz, fmaf(dy, dy, fmaf(dx, dx, v.eps2)))), most);
+                const float w = p.w * inv * (inv * inv);
+                t[e][0] = fmaf(dx, w, t[e][0]);
+                t[e][1] = fmaf(dy, w, t[e][1]);
+                t[e][2] = fmaf(dz, w, t[e][2]);
+            }
+        }
+#pragma unroll
+        for (int e = 0; e < V; ++e)
+            for (int c = 0; c < 3; ++c) s[e][c] += static_cast<double>(t[e][c]);
+    }
+}
 // f(i, sum) for the particles of this CTA, on the threads of warp 0
 template <bool COMP, int V, typename F>
-__device__ __forceinline__ void fold_slots(const float* part, int64_t n, int64_t n_pad, int S, F&& f) {
+__device__ __forceinline__ void fold_slots(const float* part, int64_t n, int64_t n_pad, int S, const FarView& v, F&& f) {
     using Vec = typename FoldVec<V>::type;
     constexpr int K = COMP ? 6 : 3, U = (V == 4 ? 12 : 54) / K;
     __shared__ double run[kFoldT - 1][V][3][32];
@@ -551,18 +596,19 @@ __device__ __forceinline__ void fold_slots(const float* part, int64_t n, int64_t
     const int64_t i = (static_cast<int64_t>(blockIdx.x) * 32 + lane) * V;
     const int R = (S + kFoldT - 1) / kFoldT;
     const int k0 = min(S, q * R), k1 = min(S, k0 + R);
+    const int flag = static_cast<int>(threadIdx.x) < v.G ? v.groups[threadIdx.x] : 0;  // looked at behind the slots' loads
     double s[V][3];
 #pragma unroll
     for (int e = 0; e < V; ++e) s[e][0] = s[e][1] = s[e][2] = 0.0;
     if (i < n) {  // n_pad is a multiple of 1024: a vector of the last particles stays in its row
         for (int k = k0; k < k1; k += U) {
-            Vec v[U][K];
+            Vec w[U][K];
 #pragma unroll
             for (int u = 0; u < U; ++u) {
                 const float* p = part + static_cast<int64_t>(V == 1 ? k + u : min(k + u, k1 - 1)) * K * n_pad + i;
 #pragma unroll
                 for (int c = 0; c < K; ++c)
-                    v[u][c] = V > 1 || k + u < k1 ? *reinterpret_cast<const Vec*>(p + c * n_pad) : Vec{};
+                    w[u][c] = V > 1 || k + u < k1 ? *reinterpret_cast<const Vec*>(p + c * n_pad) : Vec{};
             }
 #pragma unroll
             for (int u = 0; u < U; ++u) {
@@ -571,18 +617,27 @@ __device__ __forceinline__ void fold_slots(const float* part, int64_t n, int64_t
                 for (int e = 0; e < V; ++e)
 #pragma unroll
                     for (int c = 0; c < 3; ++c) {
-                        s[e][c] += static_cast<double>(fold_get<V>(v[u][c], e));
-                        if (COMP) s[e][c] += static_cast<double>(fold_get<V>(v[u][K - 3 + c], e));
+                        s[e][c] += static_cast<double>(fold_get<V>(w[u][c], e));
+                        if (COMP) s[e][c] += static_cast<double>(fold_get<V>(w[u][K - 3 + c], e));
                     }
             }
         }
     }
-    if (q > 0)
+    auto hand_over = [&]() {
+        if (q > 0)
 #pragma unroll
-        for (int e = 0; e < V; ++e)
+            for (int e = 0; e < V; ++e)
 #pragma unroll
-            for (int c = 0; c < 3; ++c) run[q - 1][e][c][lane] = s[e][c];
-    __syncthreads();
+                for (int c = 0; c < 3; ++c) run[q - 1][e][c][lane] = s[e][c];
+    };
+    hand_over();
+    int far = flag;
+    for (int k = threadIdx.x + kFoldThreads; k < v.G; k += kFoldThreads) far |= v.groups[k];
+    if (__syncthreads_or(far || (v.G > 0 && v.eps2 > 0.0f && sym_far_eps<1>(v.eps2)))) {
+        far_sums<V>(v, n, i, q, s);
+        hand_over();
+        __syncthreads();
+    }
     if (q > 0) return;
 #pragma unroll
     for (int e = 0; e < V; ++e) {
@@ -603,9 +658,9 @@ inline unsigned fold_blocks(int64_t n) { return static_cast<unsigned>((n + 32 * 
 // the culled path: the fold of the gravity partials into gfold[3][n_pad], on the gravity kernel's stream
 template <bool COMP, int V>
 __global__ void __launch_bounds__(kFoldThreads) k_gravity_fold(const float* part, int64_t n, int64_t n_pad, int S,
-                                                               double* gfold) {
+                                                               double* gfold, FarView v) {
     wait_predecessor();
-    fold_slots<COMP, V>(part, n, n_pad, S, [&](int64_t i, const double (&t)[3]) {
+    fold_slots<COMP, V>(part, n, n_pad, S, v, [&](int64_t i, const double (&t)[3]) {
         for (int c = 0; c < 3; ++c) gfold[c * n_pad + i] = t[c];
     });
 }
@@ -753,7 +808,7 @@ __global__ void __launch_bounds__(128) k_gravity_x2(const float4* __restrict__ p
 // Measured (N = 262,144, 128 groups, one B200): row-packed 22.3 ms, column-packed 19.2 ms, equal masses 17.4 ms.
 template <typename S, int GRAV, bool COMP>
 __global__ void __launch_bounds__(S::T, S::CTAS) k_gravity_sym(const float4* __restrict__ posm, float* __restrict__ part,
-                                                               int64_t n, int64_t n_pad, int G, int gs, float eps2) {
+                                                               int64_t n, int64_t n_pad, int G, int gs, float eps2, int* far_groups) {
     constexpr int R = S::R, T = S::T, B = S::B, JT = S::JT, PF = S::PF, W = S::W;
     constexpr int K = COMP ? 6 : 3;
     __shared__ float4 XY[JT / 2], ZM[JT / 2];
@@ -771,33 +826,15 @@ __global__ void __launch_bounds__(S::T, S::CTAS) k_gravity_sym(const float4* __r
     // slots 0 .. G-1-g and its column sums from tasks (ga, g), ga = 0 .. g, in slots G-g .. G
     const int s_row = gb - ga, s_col = G - gb + ga;
     auto slot = [&](int64_t particle, int sl, int c) { return part + (static_cast<int64_t>(sl) * K + c) * n_pad + particle; };
-    bool far = sym_far_eps<GRAV>(eps2);
-    auto look = [&](int b0, int b1) {  // the padding lies far out too, but has no mass
-#pragma unroll 4
-        for (int64_t i = static_cast<int64_t>(b0) * B + tid; i < min(n, static_cast<int64_t>(b1) * B); i += T)
-            far = sym_far(posm[i]) || far;
-    };
-    look(ra0, ra1);
-    if (!diag) look(cg0, cg1);
-    if (__syncthreads_or(far)) {
-        auto pass = [&](int r0, int r1, int b0, int b1, int sl) {
-            for (int a = r0; a < r1; ++a) {
-                const float4 *row = posm + static_cast<int64_t>(a) * B, *col = posm + static_cast<int64_t>(b0) * B;
-                float* out = slot(static_cast<int64_t>(a) * B, sl, 0);
-                if constexpr (R == 8) sym_far_call<S, GRAV, COMP>(row, B, col, (b1 - b0) * B, eps2, XY, ZM, out, n_pad);
-                else sym_far_pass<S, GRAV, COMP>(row, B, col, (b1 - b0) * B, eps2, XY, ZM, out, n_pad);
-            }
-        };
-        pass(ra0, ra1, cg0, cg1, s_row);
-        if (!diag) pass(cg0, cg1, ra0, ra1, s_col);
-        else
-            for (int e = tid; e < (ra1 - ra0) * B; e += T)
-                for (int c = 0; c < K; ++c) *slot(static_cast<int64_t>(ra0) * B + e, s_col, c) = 0.0f;
-        return;
-    }
-    if (diag)  // the group's first block is never a column here: its column slot is zero
+    if (diag) {  // the group's first block is never a column here: its column slot is zero
         for (int e = tid; e < B; e += T)
             for (int c = 0; c < K; ++c) *slot(static_cast<int64_t>(ra0) * B + e, s_col, c) = 0.0f;
+        bool far = false;  // for the fold; the padding lies far out too, but has no mass
+        for (int64_t i = static_cast<int64_t>(ra0) * B + tid; i < min(n, static_cast<int64_t>(ra1) * B); i += T)
+            far = sym_far(posm[i]) || far;
+        const int any = __syncthreads_or(far);
+        if (tid == 0) far_groups[ga] = any;
+    }
     const float2 E2 = make_float2(eps2, eps2);
 
     for (int a = ra0; a < ra1; ++a) {
@@ -1000,7 +1037,7 @@ template <bool COMP, int V>
 __global__ void __launch_bounds__(kFoldThreads) k_gravity_finish(DevArrays a, DevParams p, GravSum gsum) {
     wait_predecessor();
     if (has(p, GSPH_VARIABLE_TIMESTEP) && blockIdx.x == 0 && threadIdx.x == 0) a.dt_state[1] = p.max_dt;
-    fold_slots<COMP, V>(a.part, a.n, a.n_pad, gsum.sym_G > 0 ? gsum.sym_G + 1 : gsum.nseg, [&](int64_t i, const double (&t)[3]) {
+    fold_slots<COMP, V>(a.part, a.n, a.n_pad, gsum.sym_G > 0 ? gsum.sym_G + 1 : gsum.nseg, FarView{a.gfar, gsum.sym_G, a.posm, p.eps2}, [&](int64_t i, const double (&t)[3]) {
         float acc[3];
 #pragma unroll
         for (int c = 0; c < 3; ++c)
@@ -1190,7 +1227,7 @@ template <typename S, int GRAV, bool COMP>
 void sym_launch(const DevArrays& a, const DevParams& p, const Launch& L, float* out, cudaStream_t s) {
     const int G = L.grav_sym_G;
     k_gravity_sym<S, GRAV, COMP><<<static_cast<unsigned>(G * (G + 1) / 2), S::T, 0, s>>>(a.posm, out, a.n, a.n_pad, G,
-                                                                                        L.grav_sym_gs, p.eps2);
+                                                                                        L.grav_sym_gs, p.eps2, a.gfar);
 }
 template <int I, int GRAV, bool COMP>
 cudaError_t gravity_t(const DevArrays& a, const DevParams& p, const Launch& L, cudaStream_t s, const KTimer* t,
@@ -1222,7 +1259,7 @@ cudaError_t gravity_t(const DevArrays& a, const DevParams& p, const Launch& L, c
     if (e != cudaSuccess) return e;
     GSPH_TIMER_MARK(t, stop);
     const int S = L.grav_sym_G > 0 ? L.grav_sym_G + 1 : L.grav_nseg;
-    if (!finish) return launch_gravity_fold(a, L, S, s, !t);  // the culled path: the SPH finish reads a.gfold
+    if (!finish) return launch_gravity_fold(a, L, S, s, !t, L.grav_sym_G, p.eps2);  // the culled path: the SPH finish reads a.gfold
     auto kern = fold_vec(a.n) == 4 ? k_gravity_finish<COMP, 4> : k_gravity_finish<COMP, 1>;
     return launch_kernel(!t, kern, fold_blocks(a.n), kFoldThreads, s, a, p, grav_sum(L, L.grav_nseg));
 }
@@ -1259,11 +1296,12 @@ cudaError_t launch_gravity_partials(const DevArrays& a, const DevParams& p, cons
     return gravity_any(a, p, L, s, t, false);
 }
 
-cudaError_t launch_gravity_fold(const DevArrays& a, const Launch& L, int S, cudaStream_t s, bool early) {
+cudaError_t launch_gravity_fold(const DevArrays& a, const Launch& L, int S, cudaStream_t s, bool early, int far_G, float eps2) {
     const bool comp = L.accum == GSPH_ACCUM_COMPENSATED;
     auto kern = fold_vec(a.n) == 4 ? (comp ? k_gravity_fold<true, 4> : k_gravity_fold<false, 4>)
                                    : (comp ? k_gravity_fold<true, 1> : k_gravity_fold<false, 1>);
-    return launch_kernel(early, kern, fold_blocks(a.n), kFoldThreads, s, a.gpart, a.n, a.n_pad, S, a.gfold);
+    return launch_kernel(early, kern, fold_blocks(a.n), kFoldThreads, s, a.gpart, a.n, a.n_pad, S, a.gfold,
+                         FarView{a.gfar, far_G, a.posm, eps2});
 }
 
 // Gravity partials of caller-provided, already padded j-records into caller-provided partials

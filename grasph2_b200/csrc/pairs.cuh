@@ -301,8 +301,9 @@ cudaError_t launch_gravity(const DevArrays& a, const DevParams& p, const Launch&
 cudaError_t launch_fp32_peak(int sm_count, int iters, float* sink, cudaStream_t s);
 cudaError_t launch_gravity_raw(const float4* posm_padded, float* part, int64_t n_pad, int ipt, int jt, int nseg,
                                float eps2, int* status, cudaStream_t s);
-// the FP64 fold of `S` slots of a.gpart into a.gfold
-cudaError_t launch_gravity_fold(const DevArrays& a, const Launch& L, int S, cudaStream_t s, bool early);
+// the FP64 fold of `S` slots of a.gpart into a.gfold; far_G: groups of k_gravity_sym whose flags it asks (0: none)
+cudaError_t launch_gravity_fold(const DevArrays& a, const Launch& L, int S, cudaStream_t s, bool early, int far_G = 0,
+                                float eps2 = 0.0f);
 int64_t fp32_peak_flops(int sm_count, int iters);
 
 // the gravity partials and their fold with the kernels of the fixed order (gravity_fixed.cu)
