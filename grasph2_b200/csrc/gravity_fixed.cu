@@ -12,8 +12,8 @@
 //     0.6 % of it.
 // Everything else takes the column-packed kernel of pairs.cu, 1.16 (equal masses: 1.28) times as fast: that is the price,
 // 5 of the 22.4 ms of a proposal with 262,144 particles. The results differ in the last places only.
-// Both masses multiply 1/r^3 here, so separations must be within 1.5e-13 .. 4.3e12 (gravity_sym.cuh; the far tasks of that
-// kernel, in this one, cost every proposal 4.5 %).
+// Both masses multiply 1/r^3 here, so separations must be within 1.5e-13 .. 4.3e12 (gravity_sym.cuh; a
+// look-up of far tiles in this kernel cost every proposal 4.5 %).
 #include "f32x2.cuh"
 #include "gravity_sym.cuh"
 #include "pairs.cuh"

@@ -805,7 +805,7 @@ __global__ void __launch_bounds__(128) k_gravity_x2(const float4* __restrict__ p
 // Bound: the register file. An f32x2 multiply-add of three different register pairs reads six registers and runs at
 // 0.60 of the FMA rate, multiplies and adds (four) at 0.96; six of a pair's operations are such multiply-adds, which
 // predicts 0.77 of the FMA rate; the pipe is 75 % busy with equal masses, 78 % with others.
-// Measured (N = 262,144, 128 groups, one B200): row-packed 22.3 ms, column-packed 19.2 ms, equal masses 17.4 ms.
+// Measured (N = 262,144, 128 groups, one B200): row-packed 22.3 ms, column-packed 19.2 ms, equal masses 17.5 ms.
 template <typename S, int GRAV, bool COMP>
 __global__ void __launch_bounds__(S::T, S::CTAS) k_gravity_sym(const float4* __restrict__ posm, float* __restrict__ part,
                                                                int64_t n, int64_t n_pad, int G, int gs, float eps2, int* far_groups) {
@@ -1389,9 +1389,8 @@ int gravity_blocks_per_sm(int ipt, int threads, int jt, bool comp) {
 }
 
 // Model of the shapes' times: an SM takes ceil(tasks / SMs) tasks, `ctas` at a time at `rate` interactions per clock (only
-// their ratios count; the largest shape now does 13.6); a
-// last round of fewer takes as long as 0.6 of a full one at least (a lone CTA does not fill the FMA pipe).
-// Up to 128 groups: N = 262,144 in 17.4 ms against 18.3 ms with 64 (tasks four times as large, the last wave 68 %
+// their ratios count; the largest shape now does 13.5); a last round of fewer takes as long as 0.6 of a full one at least (a lone CTA does not fill the FMA pipe).
+// Up to 128 groups: N = 262,144 in 17.5 ms against 18.4 ms with 64 (tasks four times as large, the last wave 68 %
 // full); 64 above 4 M particles, where a particle's slots would take 1.5 KB.
 void sym_shape(int64_t n_pad, int sms, int groups, int shape, Launch& L) {
     const int B[kSymShapes] = {Sym8::B, Sym4::B, Sym2::B, Sym1::B};
