@@ -1389,9 +1389,9 @@ int gravity_blocks_per_sm(int ipt, int threads, int jt, bool comp) {
 }
 
 // Model of the shapes' times: an SM takes ceil(tasks / SMs) tasks, `ctas` at a time at `rate` interactions per clock (only
-// their ratios count; the largest shape now does 13.5); a last round of fewer takes as long as 0.6 of a full one at least (a lone CTA does not fill the FMA pipe).
-// Up to 128 groups: N = 262,144 in 17.5 ms against 18.4 ms with 64 (tasks four times as large, the last wave 68 %
-// full); 64 above 4 M particles, where a particle's slots would take 1.5 KB.
+// their ratios count; the largest shape now does 13.5); a last round of fewer takes as long as 0.6 of a full one at least
+// (a lone CTA does not fill the FMA pipe). Up to 128 groups: N = 262,144 in 17.5 ms against 18.4 ms with 64 (tasks four
+// times as large, the last wave 68 % full); 64 above 4 M particles, where a particle's slots would take 1.5 KB.
 void sym_shape(int64_t n_pad, int sms, int groups, int shape, Launch& L) {
     const int B[kSymShapes] = {Sym8::B, Sym4::B, Sym2::B, Sym1::B};
     const int ctas[kSymShapes] = {Sym8::CTAS, Sym4::CTAS, Sym2::CTAS, Sym1::CTAS};
